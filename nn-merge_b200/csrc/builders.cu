@@ -10,9 +10,8 @@
 //
 // Random draws: each phase that the reference seeds with
 // std::mt19937(time(NULL)) gets mt19937(seed) here (the reference run with a
-// clock frozen at `seed`); the draws are generated on the host in row order
-// and copied to the device, where each row's kernel warp consumes its fixed
-// share.  std::rand() continues across phases from srand(seed).
+// clock frozen at `seed`); the draws are generated on the device in row order
+// (mt_draws), and each row's kernel warp consumes its fixed share.  std::rand() continues across phases from srand(seed).
 #include <algorithm>
 #include <vector>
 
@@ -373,12 +372,22 @@ unsigned blocks_for(size_t n, unsigned per) { return (unsigned)((n + per - 1) / 
 
 namespace {
 
-// Host-generated mt19937 stream for `rows` rows of `per_row` draws each.
-int upload_draws(Ctx& ctx, uint32_t seed_or_state_unused, std::vector<uint32_t>& host, size_t count) {
-    (void)seed_or_state_unused;
-    NNM_CUDA_TRY(ctx.ws.draws.ensure(std::max<size_t>(count, 1) * 4));
-    if (count)
-        NNM_CUDA_TRY(cudaMemcpyAsync(ctx.ws.draws.p, host.data(), count * 4, cudaMemcpyHostToDevice, ctx.stream));
+// The first `count` outputs of mt19937(seed) at the start of ws.draws: the
+// phases of a call draw from the same stream, so a later phase extends what
+// an earlier one generated.
+int mt_draws(Ctx& ctx, uint32_t seed, size_t count) {
+    Workspace& ws = ctx.ws;
+    const size_t need = mt19937_padded(std::max<size_t>(count, 1));
+    NNM_CUDA_TRY(ws.mt_ring.ensure(MT19937_RING_BYTES));
+    if (ws.mt_seed != seed || need * 4 > ws.draws.bytes) ws.mt_have = 0;
+    NNM_CUDA_TRY(ws.draws.ensure(need * 4));
+    if (need > ws.mt_have) {
+        const size_t have = ws.mt_have;
+        ws.mt_have = 0;
+        NNM_CUDA_TRY(mt19937_generate(seed, ws.draws.as<uint32_t>(), have, need, ws.mt_ring.as<uint32_t>(), ctx.stream));
+        ws.mt_seed = seed;
+        ws.mt_have = need;
+    }
     return 0;
 }
 
@@ -504,9 +513,7 @@ int kgraph_build(Ctx& ctx, GraphDev& g) {
         return run_nndescent(ctx, g, MODE_KGRAPH, 0, 0, nullptr, 0);
     }
     const uint32_t per = sds_draws(K + 1, n);
-    std::vector<uint32_t> h((size_t)n * per);
-    gen_mt19937(g.seed, h.size(), h.data());
-    int rc = upload_draws(ctx, g.seed, h, h.size());
+    int rc = mt_draws(ctx, g.seed, (size_t)n * per);
     if (rc) return rc;
     if ((rc = reset_counters(ctx))) return rc;
     InitArgs ia{g.x, g.dp, K, g.metric, g.pid, g.pdist, ctx.ws.draws.as<uint32_t>(), per, K + 1, n, 0, n,
@@ -563,9 +570,7 @@ static int cross_sample_leaves(Ctx& ctx, GraphDev& g, const std::vector<uint32_t
         per[l] = sds_draws(2 * g.cut, range);
         total += (size_t)(leaf_off[l + 1] - leaf_off[l]) * per[l];
     }
-    std::vector<uint32_t> h(total);
-    gen_mt19937(g.seed, total, h.data());
-    if ((rc = upload_draws(ctx, g.seed, h, total))) return rc;
+    if ((rc = mt_draws(ctx, g.seed, total))) return rc;
     if ((rc = reset_counters(ctx))) return rc;
     size_t off = 0;
     for (uint32_t l = 0; l < nleaf; l++) {
@@ -592,9 +597,7 @@ static int jmerge_initial_exact(Ctx& ctx, GraphDev& g, uint32_t pre) {
     g.cut = K * 3 / 6;  // jmerge.cpp:87
     const uint32_t per_old = sds_draws(2 * g.cut, n - pre), per_new = sds_draws(K + 1, n);
     size_t total = (size_t)pre * per_old + (size_t)(n - pre) * per_new;
-    std::vector<uint32_t> h(total);
-    gen_mt19937(g.seed, total, h.data());
-    if ((rc = upload_draws(ctx, g.seed, h, total))) return rc;
+    if ((rc = mt_draws(ctx, g.seed, total))) return rc;
     if ((rc = reset_counters(ctx))) return rc;
     CrossArgs ca{g.x, g.dp, K, g.metric, g.pid, g.pdist, g.cpid, g.cpdist, ctx.ws.draws.as<uint32_t>(), per_old,
                  2 * g.cut, g.cut, 0, pre, nullptr, 0, pre, n - pre, 1, ctx.ws.counters.as<IterCounters>()};
@@ -814,9 +817,7 @@ int hmerge_build(Ctx& ctx, GraphDev& g, const LayerHook& on_layer) {
         g.ncmps += (uint64_t)N0 * K;
     } else {
         const uint32_t per = sds_draws(K + 1, N0);
-        std::vector<uint32_t> h((size_t)N0 * per);
-        gen_mt19937(g.seed, h.size(), h.data());
-        if ((rc = upload_draws(ctx, g.seed, h, h.size()))) return rc;
+        if ((rc = mt_draws(ctx, g.seed, (size_t)N0 * per))) return rc;
         if ((rc = reset_counters(ctx))) return rc;
         InitArgs ia{g.x, g.dp, K, g.metric, g.pid, g.pdist, ctx.ws.draws.as<uint32_t>(), per, K + 1, N0, 0, N0,
                     0xffffffffu, ctx.ws.counters.as<IterCounters>()};
@@ -844,9 +845,7 @@ int hmerge_build(Ctx& ctx, GraphDev& g, const LayerHook& on_layer) {
         if (!g.fast) {
             const uint32_t per_old = sds_draws(2 * half, bnum), per_new = sds_draws(2 * K, sz + bnum);
             size_t tot = (size_t)sz * per_old + (size_t)bnum * per_new;
-            std::vector<uint32_t> h(tot);
-            gen_mt19937(g.seed, tot, h.data());
-            if ((rc = upload_draws(ctx, g.seed, h, tot))) return rc;
+            if ((rc = mt_draws(ctx, g.seed, tot))) return rc;
             if ((rc = reset_counters(ctx))) return rc;
             g.cut = hsize;
             CrossArgs ca{g.x, g.dp, K, g.metric, g.pid, g.pdist, g.cpid, g.cpdist, ctx.ws.draws.as<uint32_t>(), per_old,

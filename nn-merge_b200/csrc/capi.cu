@@ -168,6 +168,7 @@ int build_common(nnm_ctx* ctx, Kind kind, const float* x, bool dev, uint64_t n, 
     if (cudaSetDevice(c.device) != cudaSuccess) return fail(ctx, NNM_ERR_NO_DEVICE, "cudaSetDevice failed");
     GraphStore& store = c.store;
     GraphDev g;
+    c.ws.mt_have = 0;
     setup_graph(g, o, n, d, k);
     uint64_t sub = 0;
     EventTimer tm(c.stream);
@@ -216,6 +217,7 @@ int merge_step(nnm_merge* m, F&& step) {
     if (!m) return NNM_ERR_INVALID;
     Ctx& c = m->ctx->c;
     if (cudaSetDevice(c.device) != cudaSuccess) return fail(m->ctx, NNM_ERR_NO_DEVICE, "cudaSetDevice failed");
+    c.ws.mt_have = 0;
     int rc = step(c);
     if (!rc) {
         cudaError_t e = cudaStreamSynchronize(c.stream);
@@ -360,6 +362,7 @@ int leaves_common(nnm_ctx* ctx, bool merge, const float* x, uint64_t n, uint32_t
     Ctx& c = ctx->c;
     if (cudaSetDevice(c.device) != cudaSuccess) return fail(ctx, NNM_ERR_NO_DEVICE, "cudaSetDevice failed");
     GraphDev g;
+    c.ws.mt_have = 0;
     setup_graph(g, o, n, d, k);
     uint64_t sub = 0;
     EventTimer tm(c.stream);
@@ -553,6 +556,7 @@ int nnm_hmerge_build(nnm_ctx* ctx, const float* x, uint64_t n, uint32_t d, uint3
     if (cudaSetDevice(c.device) != cudaSuccess) return fail(ctx, NNM_ERR_NO_DEVICE, "cudaSetDevice failed");
     GraphStore& store = c.store;
     GraphDev g;
+    c.ws.mt_have = 0;
     setup_graph(g, o, n, d, k);
     nnm::DpgState dpg;
     if (layers) std::memset(layers, 0, sizeof(*layers));

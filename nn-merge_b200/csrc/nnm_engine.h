@@ -42,12 +42,17 @@ struct Workspace {
     DevBuf npairs, poff, pd, tiers, erows;
     DevBuf kth;  // every row's K-th distance, gathered per iteration
     DevBuf rtier;  // every row's join tier (k_shuffle_append), binned by k_tier_lists
-    DevBuf draws, counters, misc;
+    // outputs [0, mt_have) of mt19937(mt_seed), the generator's state, and
+    // the seed; mt_have is cleared at the start of every call
+    DevBuf draws, mt_ring;
+    uint32_t mt_seed = 0;
+    size_t mt_have = 0;
+    DevBuf counters, misc;
     DevBuf mlp_err;  // the code network's tensor-core inference: a wait that ran out
     void release_all() {
         DevBuf* all[] = {&rcnt, &rcur, &rtot, &roff, &rseg, &rscr, &rcount, &rofs, &rbuf, &cntpos, &bcnt, &bcur,
                          &boff, &bucket, &bigrev, &nflag, &scan_tmp, &npairs, &poff, &pd, &tiers, &erows, &kth, &rtier,
-                         &draws, &counters, &misc, &mlp_err};
+                         &draws, &mt_ring, &counters, &misc, &mlp_err};
         for (auto* b : all) b->release();
     }
 };
