@@ -427,16 +427,18 @@ int upload_vectors(Ctx& ctx, GraphStore& s, GraphDev& g, const float* x, bool x_
         NNM_CUDA_TRY(cudaMemcpyAsync(s.x.p, x, elems * 4, x_on_device ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice,
                                      ctx.stream));
     } else {
+        // rows padded to 16 bytes: host rows land in the proposal buckets,
+        // which are free until the first join (an allocation and its free a
+        // call, with the device idle, took 1-3 ms)
         const float* src = x;
-        DevBuf tmp;
         if (!x_on_device) {
-            NNM_CUDA_TRY(tmp.ensure((size_t)g.n_cap * g.d * 4));
-            NNM_CUDA_TRY(cudaMemcpyAsync(tmp.p, x, (size_t)g.n_cap * g.d * 4, cudaMemcpyHostToDevice, ctx.stream));
-            src = tmp.as<float>();
+            DevBuf& stage = ctx.ws.bucket;
+            NNM_CUDA_TRY(stage.ensure((size_t)g.n_cap * g.d * 4));
+            NNM_CUDA_TRY(cudaMemcpyAsync(stage.p, x, (size_t)g.n_cap * g.d * 4, cudaMemcpyHostToDevice, ctx.stream));
+            src = stage.as<float>();
         }
         k_pad_copy<<<blocks_for(elems, 256), 256, 0, ctx.stream>>>(src, s.x.as<float>(), g.n_cap, g.d, g.dp); count_launch();
-        NNM_CUDA_TRY(cudaStreamSynchronize(ctx.stream));
-        tmp.release();
+        NNM_CUDA_TRY(cudaGetLastError());
     }
     g.x = s.x.as<float>();
     if (g.init == NNM_INIT_LEARNED) {

@@ -296,6 +296,10 @@ int nnm_ctx_destroy(nnm_ctx* ctx) {
         ctx->c.init_model->release();
         delete ctx->c.init_model;
     }
+    if (ctx->c.dpg) {
+        ctx->c.dpg->release();
+        delete ctx->c.dpg;
+    }
     if (ctx->c.h_counters) cudaFreeHost(ctx->c.h_counters);
     if (ctx->c.stream) cudaStreamDestroy(ctx->c.stream);
     delete ctx;
@@ -558,7 +562,8 @@ int nnm_hmerge_build(nnm_ctx* ctx, const float* x, uint64_t n, uint32_t d, uint3
     GraphDev g;
     c.ws.mt_have = 0;
     setup_graph(g, o, n, d, k);
-    nnm::DpgState dpg;
+    if (!c.dpg) c.dpg = new nnm::DpgState();
+    nnm::DpgState& dpg = *c.dpg;
     if (layers) std::memset(layers, 0, sizeof(*layers));
     EventTimer tm(c.stream);
     rc = nnm::upload_vectors(c, store, g, x, false);
@@ -568,7 +573,6 @@ int nnm_hmerge_build(nnm_ctx* ctx, const float* x, uint64_t n, uint32_t d, uint3
         rc = nnm::hmerge_build(c, g, [&](Ctx& cc, GraphDev& gg) { return nnm::dpg_layer(cc, dpg, gg, layers); });
     if (!rc) rc = nnm::export_graph(c, g, ids, dists, flags, true);
     float ms = tm.stop();
-    dpg.release();
     if (!rc) fill_stats(stats, g, 0, ms);
     else if (layers) nnm_layers_free(layers);
     return rc;

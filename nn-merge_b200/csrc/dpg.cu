@@ -20,6 +20,7 @@
 // least, and a fixed point equals the reference's sequential result.
 #include <algorithm>
 #include <cstdlib>
+#include <memory>
 #include <vector>
 
 #include "nnm_hier.h"
@@ -312,6 +313,16 @@ __global__ void k_dpg_reverse(RevArgs a) {
     if (lane == 0) a.glen[x] = slen[w];
 }
 
+// The lists end to end (CSR), a warp per row.
+__global__ void k_dpg_pack(const uint32_t* gid, const uint32_t* glen, uint32_t N, uint32_t C, const uint64_t* off,
+                           uint32_t* adj) {
+    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const uint32_t i = blockIdx.x * WPB + w;
+    if (i >= N) return;
+    const uint32_t len = glen[i];
+    for (uint32_t l = lane; l < len; l += 32) adj[off[i] + l] = gid[(size_t)i * C + l];
+}
+
 unsigned nblk(size_t n, unsigned per) { return (unsigned)((n + per - 1) / per); }
 }  // namespace
 
@@ -389,20 +400,26 @@ int dpg_layer(Ctx& ctx, DpgState& s, GraphDev& g, nnm_layers* out) {
     s.last_rounds = rounds;
     s.rows = N;
     if (out && out->nlayers < 16) {
-        std::vector<uint32_t> len(N), ids((size_t)N * C);
-        NNM_CUDA_TRY(cudaStreamSynchronize(ctx.stream));  // the plain copies below do not order with it
-        NNM_CUDA_TRY(cudaMemcpy(len.data(), s.glen.p, (size_t)N * 4, cudaMemcpyDeviceToHost));
-        NNM_CUDA_TRY(cudaMemcpy(ids.data(), s.gid.p, (size_t)N * C * 4, cudaMemcpyDeviceToHost));
-        uint32_t L = out->nlayers;
-        uint64_t* off = static_cast<uint64_t*>(std::malloc(sizeof(uint64_t) * ((size_t)N + 1)));
-        off[0] = 0;
-        for (uint32_t i = 0; i < N; i++) off[i + 1] = off[i] + len[i];
-        uint32_t* adj = static_cast<uint32_t*>(std::malloc(sizeof(uint32_t) * std::max<uint64_t>(off[N], 1)));
-        for (uint32_t i = 0; i < N; i++)
-            for (uint32_t j = 0; j < len[i]; j++) adj[off[i] + j] = ids[(size_t)i * C + j];
+        // packed on the device, into the offers' buffer (N x C words of its
+        // 2 N x C), so that only the lists themselves are copied out
+        NNM_CUDA_TRY(exclusive_scan(s.glen.as<uint32_t>(), s.eoff.as<uint64_t>(), N, s.tmp.as<uint64_t>(), nullptr, st));
+        k_dpg_pack<<<nblk(N, WPB), WPB * 32, 0, st>>>(s.gid.as<uint32_t>(), s.glen.as<uint32_t>(), N, C,
+                                                      s.eoff.as<uint64_t>(), s.ev.as<uint32_t>()); count_launch();
+        const uint32_t L = out->nlayers;
+        std::unique_ptr<uint64_t, decltype(&std::free)> off(
+            static_cast<uint64_t*>(std::malloc(sizeof(uint64_t) * ((size_t)N + 1))), &std::free);
+        if (!off) return 4;
+        NNM_CUDA_TRY(cudaMemcpyAsync(off.get(), s.eoff.p, ((size_t)N + 1) * 8, cudaMemcpyDeviceToHost, st));
+        NNM_CUDA_TRY(cudaStreamSynchronize(st));
+        const uint64_t total = off.get()[N];
+        std::unique_ptr<uint32_t, decltype(&std::free)> adj(
+            static_cast<uint32_t*>(std::malloc(sizeof(uint32_t) * std::max<uint64_t>(total, 1))), &std::free);
+        if (!adj) return 4;
+        NNM_CUDA_TRY(cudaMemcpyAsync(adj.get(), s.ev.p, total * 4, cudaMemcpyDeviceToHost, st));
+        NNM_CUDA_TRY(cudaStreamSynchronize(st));
         out->nrows[L] = N;
-        out->off[L] = off;
-        out->adj[L] = adj;
+        out->off[L] = off.release();
+        out->adj[L] = adj.release();
         out->nlayers = L + 1;
     }
     return 0;

@@ -82,10 +82,12 @@ struct KStat {
 
 struct DevMlp;
 struct CodeViews;
+struct DpgState;
 
 struct Ctx {
     int device = 0;
     DevMlp* init_model = nullptr;  // learned-initialisation model (owned)
+    DpgState* dpg = nullptr;       // H-Merge's DPG lists, reused across calls (grow-only, owned)
     bool prof = false;
     GraphStore store;  // graph arrays, reused across calls (grow-only)
     KStat kjoin, kemit, kmerge;
