@@ -6,9 +6,9 @@
 //   1. sampling pass   k_sample_count / k_sample_fill   (kgraph.cpp:105-136)
 //      forward new/old lists from each pool, reverse entries to neighbours
 //      whose K-th distance is below the entry's distance, flags cleared.
-//   2. reverse lists   k_rev_sort_*                    (ascending source row,
+//   2. reverse lists   k_rev_sort_big, k_shuffle_exact (ascending source row,
 //      the order the reference's sequential pass pushes them in)
-//   3. shuffle         k_shuffle_append                 (kgraph.cpp:139-162)
+//   3. shuffle         k_shuffle_exact, k_shuffle_fast  (kgraph.cpp:139-162)
 //      std::random_shuffle with the std::rand() stream (rng.cu), truncation
 //      to smplNum, appended to the sample lists.
 //   4. local join      k_join<COUNT>, k_join<FILL>      (pvetex.h:111-125 ...)
@@ -41,6 +41,7 @@ namespace {
 constexpr unsigned FULL = 0xffffffffu;
 constexpr int MERGE_WARPS = 8;
 constexpr int SHUF_SMEM = 512;  // reverse-list entries a shuffling warp stages in shared memory
+constexpr uint32_t SORT_SMEM = 256;  // reverse-list entries a warp sorts and shuffles in shared memory (exact tier)
 constexpr int BIGSORT_CH = 4096;
 
 // ---------------------------------------------------------------------------
@@ -58,15 +59,48 @@ struct SampleArgs {
     const uint32_t *rnewT, *roldT, *rnewTlen, *roldTlen;  // carried reverse lists (or null)
     uint32_t smpl;
     IterCounters* ctr;
-    const float* kth;  // every row's K-th distance (k_kth_gather)
+    const float* kth;  // every row's K-th distance (k_iter_begin)
+    uint32_t* big;     // exact tier: (row | list << 31) of reverse lists with more than SORT_SMEM entries
 };
 
-// Every row's K-th distance, gathered once per iteration: the sampling and
-// the join read it for random rows, and the 4-byte array stays in L2 where
-// the pools' last entries (a sector per row) do not.
-__global__ void k_kth_gather(const float* pdist, uint32_t K, uint32_t n, float* kth) {
+// Start of an iteration, one pass over the rows: every row's K-th distance
+// into a 4-byte array (the sampling and the join read it for random rows,
+// and it stays in L2 where the pools' last entries, a sector per row, do
+// not), the lists emptied unless they are carried over, the reverse counts
+// and cursors at the carried lengths, the bucket counts and the counters at
+// zero.  One launch in place of six kernels and three memsets (about 2 us
+// apiece, 12 of an exact-tier iteration's 45 launches and copies).
+struct BeginArgs {
+    const float* pdist;
+    float* kth;
+    uint32_t n, K, carry;
+    uint32_t *newlen, *oldlen, *tn, *to;  // tn, to: carried reverse lengths (or null)
+    uint32_t *rcnt_new, *rcnt_old, *rcur_new, *rcur_old, *bcnt, *bcur;
+    IterCounters* ctr;
+};
+
+__global__ void k_iter_begin(BeginArgs a) {
+    if (blockIdx.x == 0)
+        for (uint32_t i = threadIdx.x; i < sizeof(IterCounters) / 4; i += blockDim.x)
+            reinterpret_cast<uint32_t*>(a.ctr)[i] = 0;
     const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t < n) kth[t] = pdist[(size_t)t * K + K - 1];
+    if (t >= a.n) return;
+    a.kth[t] = a.pdist[(size_t)t * a.K + a.K - 1];
+    uint32_t cn = 0, co = 0;
+    if (a.carry) {
+        cn = a.tn[t];
+        co = a.to[t];
+    } else {
+        a.newlen[t] = 0;
+        a.oldlen[t] = 0;
+        if (a.tn) {
+            a.tn[t] = 0;
+            a.to[t] = 0;
+        }
+    }
+    a.rcnt_new[t] = a.rcur_new[t] = cn;
+    a.rcnt_old[t] = a.rcur_old[t] = co;
+    a.bcnt[t] = a.bcur[t] = 0;
 }
 
 __global__ void k_sample_count(SampleArgs a) {
@@ -117,6 +151,11 @@ __global__ void k_sample_fill(SampleArgs a) {
         a.newlen[row] = base_n + nnf;
         a.oldlen[row] = base_o + (a.K - nnf);
     }
+    if (a.big && lane < 2) {  // lane l: this row's own list l, carried entries included
+        const uint64_t* off = lane ? a.roff_old : a.roff_new;
+        if (off[row + 1] - off[row] > SORT_SMEM)
+            a.big[atomicAdd(&a.ctr->nbig_rev, 1u)] = row | ((uint32_t)lane << 31);
+    }
     if (a.rnewTlen) {  // carried reverse lists go first in this row's segments
         uint32_t cn = a.rnewTlen[row], co = a.roldTlen[row];
         for (uint32_t j = lane; j < cn; j += 32) a.rseg_new[a.roff_new[row] + j] = a.rnewT[(size_t)row * a.smpl + j];
@@ -125,42 +164,19 @@ __global__ void k_sample_fill(SampleArgs a) {
 }
 
 // ---------------------------------------------------------------------------
-// 2. Reverse lists in ascending source-row order.
+// 2. Reverse lists of more than SORT_SMEM entries in ascending source-row
+// order (k_shuffle_exact sorts the shorter ones itself).
 struct RevSortArgs {
     const uint64_t* roff[2];
     uint32_t* rseg[2];
     uint32_t* rscr[2];
     const uint32_t* carry[2];  // carried prefix length per row (or null)
     uint32_t n;
-    uint32_t* big;             // (row | list << 31) of segments longer than 32
+    uint32_t* big;             // (row | list << 31) of the segments to sort
     IterCounters* ctr;
 };
 
 __device__ __forceinline__ uint32_t rkey(uint32_t v) { return v == 0xffffffffu ? 0xffffffffu : (v & LID_MASK); }
-
-__global__ void k_rev_sort_small(RevSortArgs a) {
-    uint32_t t = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    int lane = threadIdx.x & 31;
-    int l = blockIdx.y;
-    if (t >= a.n) return;
-    uint64_t lo = a.roff[l][t] + (a.carry[l] ? a.carry[l][t] : 0), hi = a.roff[l][t + 1];
-    uint32_t len = (uint32_t)(hi - lo);
-    if (len <= 1) return;
-    if (len > 32) {
-        if (lane == 0) a.big[atomicAdd(&a.ctr->nbig_rev, 1u)] = t | ((uint32_t)l << 31);
-        return;
-    }
-    uint32_t* seg = a.rseg[l] + lo;
-    uint32_t v = lane < (int)len ? seg[lane] : 0xffffffffu;
-    for (int k = 2; k <= 32; k <<= 1)
-        for (int j = k >> 1; j > 0; j >>= 1) {
-            uint32_t o = __shfl_xor_sync(FULL, v, j);
-            bool take_min = ((lane & j) == 0) == ((lane & k) == 0);
-            uint32_t kv = rkey(v), ko = rkey(o);
-            if (take_min ? (ko < kv) : (ko > kv)) v = o;
-        }
-    if (lane < (int)len) seg[lane] = v;
-}
 
 __global__ void k_rev_sort_big(RevSortArgs a) {
     __shared__ uint32_t sh[BIGSORT_CH];
@@ -241,7 +257,7 @@ struct ShufArgs {
     uint32_t *rnewT, *roldT, *rnewTlen, *roldTlen;
     uint32_t* npairs;     // pair-distance slots per row
     IterCounters* ctr;
-    uint32_t fast, seed, phase;  // fast tier: Philox sample instead of std::random_shuffle
+    uint32_t seed, phase;  // fast tier: Philox sample instead of std::random_shuffle
     uint32_t tc_max_s;    // rows with S up to this go to the tensor-core join (no stored pairs)
     int max_staged;       // highest FP32 tier whose vectors fit in shared memory (-1: none); larger lists go unstaged
     uint32_t *rscr_new, *rscr_old;  // scratch of the reverse lists' sizes (fast tier: duplicate removal)
@@ -249,14 +265,6 @@ struct ShufArgs {
     const uint32_t* phase_dev;  // non-null: the draw phase is read here (an iteration graph's replays)
     uint8_t* rtier;       // each row's join tier (0xff: no new entries, not joined); k_tier_lists bins them
 };
-
-__global__ void k_rand_count(const uint64_t* roff_new, const uint64_t* roff_old, uint32_t n, uint32_t* out) {
-    uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= n) return;
-    uint32_t ln = (uint32_t)(roff_new[t + 1] - roff_new[t]);
-    uint32_t lo = (uint32_t)(roff_old[t + 1] - roff_old[t]);
-    out[t] = (ln ? ln - 1 : 0) + (lo ? lo - 1 : 0);
-}
 
 // std::random_shuffle over seg[0..len) with draws[0..len-1), one thread.
 __device__ __forceinline__ void shuffle_seg(uint32_t* seg, uint32_t len, const int32_t* draws) {
@@ -389,29 +397,161 @@ __device__ uint32_t dedupe_ids(uint32_t* seg, uint32_t len, uint32_t* scr) {
     return out;
 }
 
-// One warp per row: lane 0 shuffles in shared memory, the warp appends.
-__global__ void k_shuffle_append(ShufArgs a) {
+// A row whose lists have grown to nl and ol entries: lengths, stored pairs
+// (new x new above the diagonal, new x old) and join tier.  Lane 0.
+__device__ __forceinline__ void shuffle_finish(const ShufArgs& a, uint32_t t, uint32_t nl, uint32_t ol) {
+    a.newlen[t] = nl;
+    a.oldlen[t] = ol;
+    const uint32_t S = nl + ol;
+    a.npairs[t] = nl && S > a.tc_max_s ? nl * (nl - 1) / 2 + nl * ol : 0u;
+    int tier = 0xff;
+    if (nl) {
+        tier = tier_of(S);
+        // next to the tensor-core join (tc_max_s != 0) longer lists take the
+        // pair kernel; without it, tiers whose staged vectors do not fit
+        if (tier < NTIER - 1 && S > a.tc_max_s && (a.tc_max_s != 0 || tier > a.max_staged)) tier = NTIER - 1;
+    }
+    a.rtier[t] = (uint8_t)tier;
+}
+
+__device__ __forceinline__ void shuffle_no_room(const ShufArgs& a, uint32_t t) {
+    atomicOr(&a.ctr->error, (unsigned)DERR_LIST_CAP);
+    a.rtier[t] = 0xff;
+}
+
+// Exact tier, one warp per row: its two reverse lists (in the order of the
+// sampling's atomics) sorted by source row after their carried prefix, then
+// std::random_shuffle, truncation and append.  A list of at most SORT_SMEM
+// entries stays in shared memory throughout: sorted by rank (each lane
+// counts the smaller entries of its own, reading the list by broadcast;
+// equal words, the same row pushed twice, keep their order), the draws'
+// remainders taken by all lanes, the swaps -- a serial chain -- run for both
+// lists at once by lanes 0 and 1.  Longer lists come sorted in place by
+// k_rev_sort_big and are shuffled there by lane 0.  Bound: issue slots of
+// the rank loops and latency of the swap chains.  Separate kernels (a
+// bitonic sort per list, a block-wide sort of lists over 32 entries, then
+// lane 0 taking remainders and swapping list after list) took 50 + 92 + 74 us
+// an iteration at 100,000 rows with k = 20.
+constexpr int SHUFX_WARPS = 8;
+__global__ void __launch_bounds__(SHUFX_WARPS * 32) k_shuffle_exact(ShufArgs a) {
+    __shared__ uint32_t s_seg[SHUFX_WARPS][2][SORT_SMEM];
+    __shared__ uint16_t s_j[SHUFX_WARPS][2][SORT_SMEM];
+    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const uint32_t t = blockIdx.x * SHUFX_WARPS + w;
+    if (t >= a.n) return;
+    uint32_t nl = a.newlen[t], ol = a.oldlen[t];
+    const uint64_t lo_n = a.roff_new[t], hi_n = a.roff_new[t + 1], lo_o = a.roff_old[t], hi_o = a.roff_old[t + 1];
+    const int32_t* draws = a.rbuf + a.rofs[t];
+    // entries carried over from the level before (they keep their order)
+    const uint32_t carry[2] = {a.rnewT ? a.rnewTlen[t] : 0u, a.roldT ? a.roldTlen[t] : 0u};
+    const uint32_t len[2] = {(uint32_t)(hi_n - lo_n), (uint32_t)(hi_o - lo_o)};
+    uint32_t* const seg[2] = {a.rseg_new + lo_n, a.rseg_old + lo_o};
+    const bool in_smem[2] = {len[0] <= SORT_SMEM, len[1] <= SORT_SMEM};
+    const int32_t* const dr[2] = {draws, draws + (len[0] ? len[0] - 1 : 0u)};
+    if (nl + min(len[0], a.smpl) > a.capn || ol + min(len[1], a.smpl) > a.capo) {
+        if (lane == 0) shuffle_no_room(a, t);
+        return;
+    }
+#pragma unroll
+    for (int l = 0; l < 2; l++) {
+        if (!in_smem[l]) continue;
+        uint32_t* sh = s_seg[w][l];
+        for (uint32_t j = lane; j < len[l]; j += 32) sh[j] = seg[l][j];
+        for (uint32_t i = 1 + lane; i < len[l]; i += 32) s_j[w][l][i] = (uint16_t)(dr[l][i - 1] % (int32_t)(i + 1));
+    }
+    __syncwarp();
+#pragma unroll
+    for (int l = 0; l < 2; l++) {
+        const uint32_t c = carry[l];
+        if (!in_smem[l] || len[l] < c + 2) continue;
+        uint32_t* sh = s_seg[w][l] + c;
+        const uint32_t m = len[l] - c;
+        uint32_t v[SORT_SMEM / 32], rank[SORT_SMEM / 32];
+        if (m <= 32) {
+            v[0] = (uint32_t)lane < m ? sh[lane] : 0u;
+            rank[0] = 0;
+            for (uint32_t i = 0; i < m; i++) {
+                const uint32_t k = sh[i] & LID_MASK, own = v[0] & LID_MASK;
+                rank[0] += k < own || (k == own && i < (uint32_t)lane);
+            }
+            __syncwarp();
+            if ((uint32_t)lane < m) sh[rank[0]] = v[0];
+        } else {
+#pragma unroll
+            for (uint32_t r = 0; r < SORT_SMEM / 32; r++) {
+                v[r] = lane + 32 * r < m ? sh[lane + 32 * r] : 0u;
+                rank[r] = 0;
+            }
+            for (uint32_t i = 0; i < m; i++) {
+                const uint32_t k = sh[i] & LID_MASK;
+#pragma unroll
+                for (uint32_t r = 0; r < SORT_SMEM / 32; r++) {
+                    if (32 * r >= m) break;
+                    const uint32_t own = v[r] & LID_MASK;
+                    rank[r] += k < own || (k == own && i < lane + 32 * r);
+                }
+            }
+            __syncwarp();
+#pragma unroll
+            for (uint32_t r = 0; r < SORT_SMEM / 32; r++)
+                if (lane + 32 * r < m) sh[rank[r]] = v[r];
+        }
+    }
+    __syncwarp();
+    if (lane < 2) {
+        const uint32_t n = lane ? len[1] : len[0];
+        if (n <= SORT_SMEM) {
+            uint32_t* sh = s_seg[w][lane];
+            const uint16_t* jj = s_j[w][lane];
+            for (uint32_t i = 1; i < n; i++) {
+                const uint32_t j = jj[i], x = sh[i], y = sh[j];
+                sh[i] = y;
+                sh[j] = x;
+            }
+        }
+    }
+    if (lane == 0) {
+        if (!in_smem[0]) shuffle_seg(seg[0], len[0], dr[0]);
+        if (!in_smem[1]) shuffle_seg(seg[1], len[1], dr[1]);
+    }
+    __syncwarp();
+#pragma unroll
+    for (int l = 0; l < 2; l++) {
+        const uint32_t keep = min(len[l], a.smpl);
+        const uint32_t* src = in_smem[l] ? s_seg[w][l] : seg[l];
+        uint32_t* L = l ? a.oldL + (size_t)t * a.capo + ol : a.newL + (size_t)t * a.capn + nl;
+        uint32_t* T = l ? a.roldT : a.rnewT;
+        for (uint32_t j = lane; j < keep; j += 32) {
+            const uint32_t v = src[j];
+            L[j] = v;
+            if (T) T[(size_t)t * a.smpl + j] = v;
+        }
+        if (l) ol += keep;
+        else nl += keep;
+        if (lane == 0 && T) (l ? a.roldTlen : a.rnewTlen)[t] = keep;
+    }
+    if (lane == 0) shuffle_finish(a, t, nl, ol);
+}
+
+// Fast tier, one warp per row: a random subset of each reverse list, appended.
+__global__ void k_shuffle_fast(ShufArgs a) {
     __shared__ uint32_t stage[8][SHUF_SMEM];
     __shared__ uint32_t hist[8][256];
     int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
     uint32_t t = blockIdx.x * 8 + w;
     if (t >= a.n) return;
-    const int32_t* draws = a.fast ? nullptr : a.rbuf + a.rofs[t];
     uint32_t nl = a.newlen[t], ol = a.oldlen[t];
     // both lists' segments read up front (independent loads in flight together)
     const uint64_t lo_n = a.roff_new[t], hi_n = a.roff_new[t + 1], lo_o = a.roff_old[t], hi_o = a.roff_old[t + 1];
-    // Fast tier, the common row: both reverse lists of at most 32 entries
+    // The common row: both reverse lists of at most 32 entries
     // and within the sample cap -- kept whole, in list order -- copied with
     // one load of each list, in flight together.
-    if (a.fast && !a.dedupe && hi_n - lo_n <= min(32u, a.smpl) && hi_o - lo_o <= min(32u, a.smpl)) {
+    if (!a.dedupe && hi_n - lo_n <= min(32u, a.smpl) && hi_o - lo_o <= min(32u, a.smpl)) {
         const uint32_t ln = (uint32_t)(hi_n - lo_n), lk = (uint32_t)(hi_o - lo_o);
         const uint32_t vn = lane < (int)ln ? a.rseg_new[lo_n + lane] : 0u;
         const uint32_t vo = lane < (int)lk ? a.rseg_old[lo_o + lane] : 0u;
         if (nl + ln > a.capn || ol + lk > a.capo) {
-            if (lane == 0) {
-                atomicOr(&a.ctr->error, (unsigned)DERR_LIST_CAP);
-                a.rtier[t] = 0xff;
-            }
+            if (lane == 0) shuffle_no_room(a, t);
             return;
         }
         if (lane < (int)ln) {
@@ -435,39 +575,21 @@ __global__ void k_shuffle_append(ShufArgs a) {
         uint32_t* seg = (l ? a.rseg_old : a.rseg_new) + lo;
         if (a.dedupe && len > 1) len = dedupe_ids(seg, len, (l ? a.rscr_old : a.rscr_new) + lo);
         uint32_t keep = min(len, a.smpl);
-        uint32_t* sh = stage[w];
-        bool staged = len <= SHUF_SMEM;
-        if (a.fast) {
-            // a uniform random subset of smplNum entries, chosen by id
-            if (len > a.smpl)
-                hash_sample(seg, len, keep, Philox{a.seed, 0x6e6e6d01u}, t, a.phase_dev ? *a.phase_dev : a.phase,
-                            (uint32_t)l, hist[w], staged ? stage[w] : nullptr);
-            __syncwarp();
-            sh = seg;
-        } else if (staged) {
-            for (uint32_t j = lane; j < len; j += 32) sh[j] = seg[j];
-            __syncwarp();
-            if (lane == 0) shuffle_seg(sh, len, draws);
-            __syncwarp();
-        } else {
-            if (lane == 0) shuffle_seg(seg, len, draws);
-            __syncwarp();
-            sh = seg;
-        }
-        draws += len ? len - 1 : 0;
+        // a uniform random subset of smplNum entries, chosen by id
+        if (len > a.smpl)
+            hash_sample(seg, len, keep, Philox{a.seed, 0x6e6e6d01u}, t, a.phase_dev ? *a.phase_dev : a.phase,
+                        (uint32_t)l, hist[w], len <= SHUF_SMEM ? stage[w] : nullptr);
+        __syncwarp();
         uint32_t* L = l ? a.oldL + (size_t)t * a.capo : a.newL + (size_t)t * a.capn;
         uint32_t base = l ? ol : nl;
         uint32_t cap = l ? a.capo : a.capn;
         uint32_t* T = l ? a.roldT : a.rnewT;
         if (base + keep > cap) {
-            if (lane == 0) {
-                atomicOr(&a.ctr->error, (unsigned)DERR_LIST_CAP);
-                a.rtier[t] = 0xff;
-            }
+            if (lane == 0) shuffle_no_room(a, t);
             return;
         }
         for (uint32_t j = lane; j < keep; j += 32) {
-            uint32_t v = sh[j];
+            uint32_t v = seg[j];
             L[base + j] = v;
             if (T) T[(size_t)t * a.smpl + j] = v;
         }
@@ -476,21 +598,7 @@ __global__ void k_shuffle_append(ShufArgs a) {
         if (lane == 0 && T) (l ? a.roldTlen : a.rnewTlen)[t] = keep;
         __syncwarp();
     }
-    if (lane == 0) {
-        a.newlen[t] = nl;
-        a.oldlen[t] = ol;
-        // stored pairs of the local join: new x new above the diagonal, new x old
-        const uint32_t S = nl + ol;
-        a.npairs[t] = nl && S > a.tc_max_s ? nl * (nl - 1) / 2 + nl * ol : 0u;
-        int tier = 0xff;
-        if (nl) {
-            tier = tier_of(S);
-            // next to the tensor-core join (tc_max_s != 0) longer lists take the
-            // pair kernel; without it, tiers whose staged vectors do not fit
-            if (tier < NTIER - 1 && S > a.tc_max_s && (a.tc_max_s != 0 || tier > a.max_staged)) tier = NTIER - 1;
-        }
-        a.rtier[t] = (uint8_t)tier;
-    }
+    if (lane == 0) shuffle_finish(a, t, nl, ol);
 }
 
 // The tier lists from the rows' tiers: a block per chunk of rows counts its
@@ -1384,28 +1492,6 @@ __global__ void k_sum_flags(const uint8_t* nflag, uint32_t n, IterCounters* ctr)
 }
 
 // ---------------------------------------------------------------------------
-// Sets `bit` of the overflow word when *total exceeds cap.
-__global__ void k_check_cap(IterCounters* ctr, const unsigned long long* total, unsigned long long cap,
-                            unsigned int bit) {
-    if (threadIdx.x == 0 && *total > cap) atomicOr(&ctr->overflow, bit);
-}
-
-__global__ void k_clear_lists(uint32_t* newlen, uint32_t* oldlen, uint32_t* tn, uint32_t* to, uint32_t n) {
-    uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= n) return;
-    newlen[t] = 0;
-    oldlen[t] = 0;
-    if (tn) {
-        tn[t] = 0;
-        to[t] = 0;
-    }
-}
-
-__global__ void k_set_u32(uint32_t* dst, const uint32_t* src, uint32_t n) {
-    uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t < n) dst[t] = src ? src[t] : 0u;
-}
-
 template <typename T> T* P(DevBuf& b) { return b.as<T>(); }
 
 }  // namespace
@@ -1494,45 +1580,50 @@ static cudaError_t prep_pairs(uint32_t caps, uint32_t dp, size_t emit_smem, int 
 // FP32 pair kernels: all tiers, or only the last one when the tensor-core
 // join takes the others.
 template <int M>
-static void launch_pairs(const JoinArgs& ja, const unsigned* ntier, uint32_t caps, uint32_t dp, int nsm,
-                         bool last_only, bool u8_last, bool u8_tc, cudaStream_t st) {
-    if (!last_only && ntier) {
-        if (ntier[0]) { k_pairs<M, 0><<<ntier[0], TIER_THREADS[0], pairs_smem(TIER_CAP[0], dp, true), st>>>(ja, TIER_CAP[0]); count_launch(); }
-        if (ntier[1]) { k_pairs<M, 1><<<ntier[1], TIER_THREADS[1], pairs_smem(TIER_CAP[1], dp, true), st>>>(ja, TIER_CAP[1]); count_launch(); }
-        if (ntier[2]) { k_pairs<M, 2><<<ntier[2], TIER_THREADS[2], pairs_smem(TIER_CAP[2], dp, true), st>>>(ja, TIER_CAP[2]); count_launch(); }
-        if (ntier[3]) { k_pairs<M, 3><<<ntier[3], TIER_THREADS[3], pairs_smem(TIER_CAP[3], dp, true), st>>>(ja, TIER_CAP[3]); count_launch(); }
+static void launch_pairs(const JoinArgs& ja, const unsigned* ntier, const unsigned* full, uint32_t caps, uint32_t dp,
+                         int nsm, bool last_only, bool u8_last, bool u8_tc, cudaStream_t st) {
+    // grids: the host's row counts, or (ntier null) full -- every block that
+    // fits on the SMs at once, looping over the rows counted on the device
+    const unsigned* g = ntier ? ntier : full;
+    if (!last_only) {
+        if (g[0]) { k_pairs<M, 0><<<g[0], TIER_THREADS[0], pairs_smem(TIER_CAP[0], dp, true), st>>>(ja, TIER_CAP[0]); count_launch(); }
+        if (g[1]) { k_pairs<M, 1><<<g[1], TIER_THREADS[1], pairs_smem(TIER_CAP[1], dp, true), st>>>(ja, TIER_CAP[1]); count_launch(); }
+        if (g[2]) { k_pairs<M, 2><<<g[2], TIER_THREADS[2], pairs_smem(TIER_CAP[2], dp, true), st>>>(ja, TIER_CAP[2]); count_launch(); }
+        if (g[3]) { k_pairs<M, 3><<<g[3], TIER_THREADS[3], pairs_smem(TIER_CAP[3], dp, true), st>>>(ja, TIER_CAP[3]); count_launch(); }
     }
-    // ntier null (the tensor-core join takes tiers 0-3): the count of the
-    // last tier is on the device only, the blocks loop over its rows; the
-    // grid is every block that fits on the SMs at once
     if (u8_tc) {  // the last tier on the tensor cores
         launch_pairs_tc(ja, caps, ntier, nsm, st);
         return;
     }
-    if (!ntier || ntier[4]) {
-        const size_t smem = u8_last ? pairs_smem_u8(caps, ja.kq) : pairs_smem(caps, dp, false);
-        int per_sm = 0;
-        if (u8_last)
-            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_pairs_u8, TIER_THREADS[4], smem);
-        else
-            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_pairs<M, 4>, TIER_THREADS[4], smem);
-        const unsigned full = (unsigned)nsm * (unsigned)std::max(per_sm, 1);
-        const unsigned g = ntier ? std::min<unsigned>(ntier[4], full) : full;
-        if (u8_last) {
-            k_pairs_u8<<<g, TIER_THREADS[4], smem, st>>>(ja, caps);
-        } else {
-            k_pairs<M, 4><<<g, TIER_THREADS[4], smem, st>>>(ja, caps);
-        }
+    if (g[4]) {
+        const unsigned blocks = std::min(g[4], full[4]);
+        if (u8_last) k_pairs_u8<<<blocks, TIER_THREADS[4], pairs_smem_u8(caps, ja.kq), st>>>(ja, caps);
+        else k_pairs<M, 4><<<blocks, TIER_THREADS[4], pairs_smem(caps, dp, false), st>>>(ja, caps);
         count_launch();
     }
 }
 
-// Grid of k_emit_rows when the row count is on the device only: every
-// block that fits on the SMs at once.
-static unsigned emit_rows_grid(uint32_t caps, int nsm) {
+template <class F>
+static unsigned resident_blocks(F fn, int threads, size_t smem, int nsm) {
     int per_sm = 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_emit_rows, EMIT_ROW_WARPS * 32, (size_t)caps * 24 + 64);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, threads, smem);
     return (unsigned)nsm * (unsigned)std::max(per_sm, 1);
+}
+
+// launch_pairs' full grids; 0 for a tier that has no rows (its vectors do
+// not fit in shared memory, or the tensor-core join takes it).
+template <int M>
+static void pair_grids(uint32_t caps, uint32_t dp, uint32_t kq, int nsm, bool last_only, bool u8_last, int max_staged,
+                       unsigned* g) {
+    auto staged = [&](int t, auto fn) {
+        return last_only || t > max_staged ? 0u : resident_blocks(fn, TIER_THREADS[t], pairs_smem(TIER_CAP[t], dp, true), nsm);
+    };
+    g[0] = staged(0, k_pairs<M, 0>);
+    g[1] = staged(1, k_pairs<M, 1>);
+    g[2] = staged(2, k_pairs<M, 2>);
+    g[3] = staged(3, k_pairs<M, 3>);
+    g[4] = u8_last ? resident_blocks(k_pairs_u8, TIER_THREADS[4], pairs_smem_u8(caps, kq), nsm)
+                   : resident_blocks(k_pairs<M, 4>, TIER_THREADS[4], pairs_smem(caps, dp, false), nsm);
 }
 
 // Sequential float mean of the per-row deltas, as the reference computes it
@@ -1560,7 +1651,6 @@ int run_nndescent(Ctx& ctx, GraphDev& g, JoinMode mode, uint32_t split, uint32_t
     NNM_CUDA_TRY(ws.roff.ensure(n1 * 2 * 8));
     NNM_CUDA_TRY(ws.rseg.ensure(rev_cap * 2 * 4));
     NNM_CUDA_TRY(ws.rscr.ensure(rev_cap * 2 * 4));
-    NNM_CUDA_TRY(ws.rcount.ensure(n1 * 4));
     NNM_CUDA_TRY(ws.rofs.ensure(n1 * 8));
     NNM_CUDA_TRY(ws.rbuf.ensure(rev_cap * 2 * 4 + 64));
     NNM_CUDA_TRY(ws.cntpos.ensure((size_t)n * caps * 2));
@@ -1582,7 +1672,6 @@ int run_nndescent(Ctx& ctx, GraphDev& g, JoinMode mode, uint32_t split, uint32_t
     uint32_t *rseg_new = P<uint32_t>(ws.rseg), *rseg_old = rseg_new + rev_cap;
     uint32_t *rscr_new = P<uint32_t>(ws.rscr), *rscr_old = rscr_new + rev_cap;
     uint64_t* scan_tmp = P<uint64_t>(ws.scan_tmp);
-    uint64_t* d_tot = P<uint64_t>(ws.scan_tmp) + scan_temp_elems(n1) + 4;  // past the scan scratch
     IterCounters* ctr = P<IterCounters>(ws.counters);
 
     const size_t emit_smem = (size_t)EMIT_WARPS * caps * 24 + 64;
@@ -1616,27 +1705,22 @@ int run_nndescent(Ctx& ctx, GraphDev& g, JoinMode mode, uint32_t split, uint32_t
     const unsigned tblocks = (unsigned)((n + 255) / 256);
     std::vector<uint8_t> h_nflag;
 
-    // Fast tier: an iteration's sampling segment -- list clears through the
-    // pair-count scan and the counter read-back -- launches the same kernels
-    // with the same arguments in every iteration but the first of a carried
-    // H-Merge level, except the draw phase of k_shuffle_append.  It is
-    // captured once per call as a CUDA graph and replayed, the phase set on
-    // the instantiated graph's node before each replay.  (The join and the
-    // merge follow host reads of tile, pair and proposal counts.)
-    struct SegGraph {
-        cudaGraph_t graph = nullptr;  // kept while exec lives: its node handle names the node to update
-        cudaGraphExec_t exec = nullptr;
-        cudaGraphNode_t shuf = nullptr;
-        cudaKernelNodeParams kp{};
-        uint64_t launches = 0;
-        bool disabled = false;
-        ~SegGraph() {
-            if (exec) cudaGraphExecDestroy(exec);
-            if (graph) cudaGraphDestroy(graph);
+    unsigned full[NTIER], emit_rows_full = 0;
+    if (g.metric == L2) pair_grids<L2>(caps, g.dp, g.kq, nsm, tc, u8_last, max_staged, full);
+    else if (g.metric == L1) pair_grids<L1>(caps, g.dp, g.kq, nsm, tc, false, max_staged, full);
+    else pair_grids<CHI2>(caps, g.dp, g.kq, nsm, tc, false, max_staged, full);
+    if (tc) emit_rows_full = resident_blocks(k_emit_rows, EMIT_ROW_WARPS * 32, (size_t)caps * 24 + 64, nsm);
+    // a buffer grown with headroom, or without where that does not fit
+    auto grow = [&](DevBuf& b, uint64_t elems, size_t each, double room) -> cudaError_t {
+        cudaError_t e = b.ensure((size_t)((double)elems * room + 1024) * each);
+        if (e == cudaErrorMemoryAllocation) {
+            cudaGetLastError();
+            e = b.ensure((size_t)elems * each);
         }
-    } seg;
-    // The whole-iteration graph of the fast tier on the tensor cores: the
-    // context's executable graph of this join mode, once it holds this
+        return e;
+    };
+
+    // The whole-iteration graph of the fast tier: the context's executable graph of this join mode, once it holds this
     // call's iteration (owned by the context).
     struct {
         cudaGraphExec_t exec = nullptr;
@@ -1646,23 +1730,6 @@ int run_nndescent(Ctx& ctx, GraphDev& g, JoinMode mode, uint32_t split, uint32_t
     // pinned host source past the host counters
     uint32_t* phase_dev = reinterpret_cast<uint32_t*>(ctr + 1);
     uint32_t* h_phase = reinterpret_cast<uint32_t*>(ctx.h_counters + 1);
-    // the node of kernel `fn` in a captured graph, and its parameters
-    auto find_kernel_node = [](cudaGraph_t graph, void* fn, cudaKernelNodeParams& out) -> cudaGraphNode_t {
-        size_t nn = 0;
-        cudaGraphGetNodes(graph, nullptr, &nn);
-        std::vector<cudaGraphNode_t> nodes(nn);
-        cudaGraphGetNodes(graph, nodes.data(), &nn);
-        for (cudaGraphNode_t nd : nodes) {
-            cudaGraphNodeType ty;
-            cudaKernelNodeParams kp{};
-            if (cudaGraphNodeGetType(nd, &ty) == cudaSuccess && ty == cudaGraphNodeTypeKernel &&
-                cudaGraphKernelNodeGetParams(nd, &kp) == cudaSuccess && kp.func == fn) {
-                out = kp;
-                return nd;
-            }
-        }
-        return nullptr;
-    };
     for (uint32_t it = 0;; it++) {
         const bool carry_now = (it == 0) && g.carry && track;
         const uint32_t phase = g.phase++;
@@ -1672,40 +1739,37 @@ int run_nndescent(Ctx& ctx, GraphDev& g, JoinMode mode, uint32_t split, uint32_t
                             g.capn, g.capo, n, g.smpl,
                             track ? g.rnewT : nullptr, track ? g.roldT : nullptr,
                             track ? g.rnewTlen : nullptr, track ? g.roldTlen : nullptr,
-                            P<uint32_t>(ws.npairs), ctr, g.fast ? 1u : 0u, g.seed, phase,
+                            P<uint32_t>(ws.npairs), ctr, g.seed, phase,
                             tc ? (g.tc_kind == 0 ? g.tile_rows : TC_MAX_S) : 0u, max_staged, rscr_new, rscr_old,
                             (g.fast && carry_now) ? 1u : 0u, nullptr, P<uint8_t>(ws.rtier)};
         };
-        // the segment; its first failing call's error is returned.  copy:
-        // read the counters back at its end (the whole-iteration graph reads
-        // them once, after the merge)
-        auto seg_a = [&](bool copy = true, const uint32_t* phase_dev = nullptr) -> cudaError_t {
+        // sampling through the pair-count scan; its first failing call's
+        // error is returned
+        auto seg_a = [&](const uint32_t* phase_dev) -> cudaError_t {
             cudaError_t e = cudaSuccess;
             auto chk = [&](cudaError_t x) {
                 if (e == cudaSuccess) e = x;
             };
-            if (!carry_now) {
-                k_clear_lists<<<tblocks, 256, 0, st>>>(g.newlen, g.oldlen,
-                                                       track ? g.rnewTlen : nullptr,
-                                                       track ? g.roldTlen : nullptr, n); count_launch();
-            }
-            chk(cudaMemsetAsync(ctr, 0, sizeof(IterCounters), st));
-            // reverse counts and cursors start at the carried lengths
-            k_set_u32<<<tblocks, 256, 0, st>>>(rcnt_new, track ? g.rnewTlen : nullptr, n); count_launch();
-            k_set_u32<<<tblocks, 256, 0, st>>>(rcnt_old, track ? g.roldTlen : nullptr, n); count_launch();
-            k_set_u32<<<tblocks, 256, 0, st>>>(rcur_new, track ? g.rnewTlen : nullptr, n); count_launch();
-            k_set_u32<<<tblocks, 256, 0, st>>>(rcur_old, track ? g.roldTlen : nullptr, n); count_launch();
+            BeginArgs ba{g.pdist, P<float>(ws.kth), n, K, carry_now ? 1u : 0u, g.newlen, g.oldlen,
+                         track ? g.rnewTlen : nullptr, track ? g.roldTlen : nullptr,
+                         rcnt_new, rcnt_old, rcur_new, rcur_old, P<uint32_t>(ws.bcnt), P<uint32_t>(ws.bcur), ctr};
+            k_iter_begin<<<tblocks, 256, 0, st>>>(ba); count_launch();
             SampleArgs sa{g.pid, g.pdist, n, K, (uint32_t)mode, split,
                           rcnt_new, rcnt_old, rcur_new, rcur_old, roff_new, roff_old, rseg_new, rseg_old,
                           g.newL, g.oldL, g.newlen, g.oldlen,
                           g.capn, g.capo,
                           carry_now ? g.rnewT : nullptr, carry_now ? g.roldT : nullptr,
                           carry_now ? g.rnewTlen : nullptr, carry_now ? g.roldTlen : nullptr,
-                          g.smpl, ctr, P<float>(ws.kth)};
-            k_kth_gather<<<tblocks, 256, 0, st>>>(g.pdist, K, n, P<float>(ws.kth)); count_launch();
+                          g.smpl, ctr, P<float>(ws.kth), g.fast ? nullptr : P<uint32_t>(ws.bigrev)};
             k_sample_count<<<warp_blocks, 256, 0, st>>>(sa); count_launch();
-            chk(exclusive_scan(rcnt_new, roff_new, n, scan_tmp, nullptr, st));
-            chk(exclusive_scan(rcnt_old, roff_old, n, scan_tmp, nullptr, st));
+            // the reverse segments and, exact tier, the std::rand() draws of
+            // every row's two shuffles
+            ScanJobs sj{};
+            sj.j[0] = ScanJob{rcnt_new, nullptr, roff_new, nullptr, nullptr, 0, 0};
+            sj.j[1] = ScanJob{rcnt_old, nullptr, roff_old, nullptr, nullptr, 0, 0};
+            sj.j[2] = ScanJob{rcnt_new, rcnt_old, P<uint64_t>(ws.rofs),
+                              reinterpret_cast<uint64_t*>(&ctr->rand_draws), nullptr, 0, 0};
+            chk(exclusive_scans(sj, g.fast ? 2 : 3, n, scan_tmp, st));
             k_sample_fill<<<warp_blocks, 256, 0, st>>>(sa); count_launch();
             RevSortArgs ra{{roff_new, roff_old}, {rseg_new, rseg_old}, {rscr_new, rscr_old},
                            {carry_now ? g.rnewTlen : nullptr, carry_now ? g.roldTlen : nullptr},
@@ -1714,25 +1778,22 @@ int run_nndescent(Ctx& ctx, GraphDev& g, JoinMode mode, uint32_t split, uint32_t
             // them; the fast tier keeps them in the (arbitrary) order the atomics
             // left: its samples and tie-break keys do not depend on list order
             if (!g.fast) {
-                k_rev_sort_small<<<dim3(warp_blocks, 2), 256, 0, st>>>(ra); count_launch();
                 k_rev_sort_big<<<nsm * 2, 512, 0, st>>>(ra); count_launch();
                 // std::rand() draws of this iteration's shuffles
-                k_rand_count<<<tblocks, 256, 0, st>>>(roff_new, roff_old, n, P<uint32_t>(ws.rcount)); count_launch();
-                chk(exclusive_scan(P<uint32_t>(ws.rcount), P<uint64_t>(ws.rofs), n, scan_tmp, d_tot, st));
-                chk(glibc_stream_generate(P<int32_t>(ws.rbuf), g.gbase, g.gpos, d_tot, rev_cap * 2, st));
-            } else {
-                chk(cudaMemsetAsync(d_tot, 0, 8, st));
+                chk(glibc_stream_generate(P<int32_t>(ws.rbuf), g.gbase, g.gpos,
+                                          reinterpret_cast<const uint64_t*>(&ctr->rand_draws), rev_cap * 2, st));
             }
             ShufArgs sh = shuf_args();
             sh.phase_dev = phase_dev;
-            k_shuffle_append<<<warp_blocks, 256, 0, st>>>(sh); count_launch();
+            if (g.fast) k_shuffle_fast<<<warp_blocks, 256, 0, st>>>(sh);
+            else k_shuffle_exact<<<warp_blocks, SHUFX_WARPS * 32, 0, st>>>(sh);
+            count_launch();
             k_tier_lists<<<(n + TIER_CHUNK - 1) / TIER_CHUNK, 256, 0, st>>>(P<uint8_t>(ws.rtier), n,
                                                                            P<uint32_t>(ws.tiers), ctr); count_launch();
-            chk(exclusive_scan(P<uint32_t>(ws.npairs), P<uint64_t>(ws.poff), n, scan_tmp,
-                               reinterpret_cast<uint64_t*>(&ctr->pairs), st));
-            chk(cudaMemsetAsync(ws.bcnt.p, 0, n1 * 4, st));
-            chk(cudaMemsetAsync(ws.bcur.p, 0, n1 * 4, st));
-            if (copy) chk(cudaMemcpyAsync(ctx.h_counters, ctr, sizeof(IterCounters), cudaMemcpyDeviceToHost, st));
+            ScanJobs pj{};
+            pj.j[0] = ScanJob{P<uint32_t>(ws.npairs), nullptr, P<uint64_t>(ws.poff),
+                              reinterpret_cast<uint64_t*>(&ctr->pairs), &ctr->overflow, ws.pd.bytes / 4, OVF_PAIRS};
+            chk(exclusive_scans(pj, 1, n, scan_tmp, st));
             chk(cudaGetLastError());
             return e;
         };
@@ -1762,12 +1823,15 @@ int run_nndescent(Ctx& ctx, GraphDev& g, JoinMode mode, uint32_t split, uint32_t
             rec(0);
             if (tc) e = launch_join_tc(0, ja, nt, nsm, st);
             if (e == cudaSuccess) {
-                if (g.metric == L2) launch_pairs<L2>(ja, nt, caps, g.dp, nsm, tc, u8_last, u8_tc, st);
-                else if (g.metric == L1) launch_pairs<L1>(ja, nt, caps, g.dp, nsm, tc, false, false, st);
-                else launch_pairs<CHI2>(ja, nt, caps, g.dp, nsm, tc, false, false, st);
+                if (g.metric == L2) launch_pairs<L2>(ja, nt, full, caps, g.dp, nsm, tc, u8_last, u8_tc, st);
+                else if (g.metric == L1) launch_pairs<L1>(ja, nt, full, caps, g.dp, nsm, tc, false, false, st);
+                else launch_pairs<CHI2>(ja, nt, full, caps, g.dp, nsm, tc, false, false, st);
                 rec(1);
-                e = exclusive_scan(P<uint32_t>(ws.bcnt), P<uint64_t>(ws.boff), n, scan_tmp,
-                                   reinterpret_cast<uint64_t*>(&ctr->proposals), st);
+                ScanJobs bj{};
+                bj.j[0] = ScanJob{P<uint32_t>(ws.bcnt), nullptr, P<uint64_t>(ws.boff),
+                                  reinterpret_cast<uint64_t*>(&ctr->proposals), &ctr->overflow,
+                                  ws.bucket.bytes / prop_bytes, OVF_PROPOSALS};
+                e = exclusive_scans(bj, 1, n, scan_tmp, st);
             }
             return e != cudaSuccess ? e : cudaGetLastError();
         };
@@ -1779,7 +1843,7 @@ int run_nndescent(Ctx& ctx, GraphDev& g, JoinMode mode, uint32_t split, uint32_t
             if (tc) e = launch_join_tc(1, ja, nt, nsm, st);
             if (e != cudaSuccess) return e;
             if (tc) {
-                const unsigned rows4 = nt ? nt[NTIER - 1] : emit_rows_grid(caps, nsm);
+                const unsigned rows4 = nt ? nt[NTIER - 1] : emit_rows_full;
                 if (rows4) {
                     k_emit_rows<<<rows4, EMIT_ROW_WARPS * 32, (size_t)caps * 24 + 64, st>>>(ja); count_launch();
                 }
@@ -1803,47 +1867,39 @@ int run_nndescent(Ctx& ctx, GraphDev& g, JoinMode mode, uint32_t split, uint32_t
             return cudaGetLastError();
         };
         auto copy_back = [&]() -> cudaError_t {
-            cudaError_t e = cudaMemcpyAsync(ctx.h_counters, ctr, sizeof(IterCounters), cudaMemcpyDeviceToHost, st);
-            if (e == cudaSuccess)
-                e = cudaMemcpyAsync(&ctx.h_counters->rand_draws, d_tot, 8, cudaMemcpyDeviceToHost, st);
+            return cudaMemcpyAsync(ctx.h_counters, ctr, sizeof(IterCounters), cudaMemcpyDeviceToHost, st);
+        };
+        // the iteration; the host reads the counters once, at its end
+        auto iteration = [&](const uint32_t* phase_dev) -> cudaError_t {
+            const JoinArgs ja = make_ja();
+            cudaError_t e = seg_a(phase_dev);
+            if (e == cudaSuccess) e = part0(ja, nullptr);
+            if (e == cudaSuccess) e = part1(ja, nullptr);
+            if (e == cudaSuccess) e = copy_back();
             return e;
         };
-        // Fast tier on the tensor cores, after the first iteration of the
-        // call has sized the pair and bucket buffers: the whole iteration --
-        // sampling, both join passes, merge, counters -- is one CUDA graph,
-        // replayed with the draw phase set on its shuffle node, and the host
-        // reads the counters once.  The buffers are sized from earlier
-        // iterations (with headroom) and checked on the device; on overflow
+        // The pair and bucket buffers are sized from earlier iterations and
+        // checked on the device (the scans that lay them out): on overflow
         // the join and merge kernels do nothing, and the host grows the
-        // buffer and reruns the skipped part directly.
-        const bool whole = g.fast && tc && !carry_now && !whole_g.disabled && !g.no_graph && it > 0;
-        bool done = false;
+        // buffer and reruns the skipped part.  Reading the pair and proposal
+        // totals before each launch that depends on them cost two further
+        // round trips an iteration (about 20 us each, a quarter of a
+        // 2,000-row build).
+        // Fast tier, after the first iteration of the call: the iteration is
+        // one CUDA graph, captured once per call and applied to the context's
+        // executable graph of this join mode (cudaGraphExecUpdate: no new
+        // instantiation while the shape of the iteration is the same); the
+        // draw phase is read from a device word, written before each replay.
+        // (The exact tier's std::rand() position is a kernel argument.)
+        const bool whole = g.fast && !carry_now && !whole_g.disabled && !g.no_graph && it > 0;
         if (whole) {
-            // The graph is captured at the call's first whole iteration and
-            // applied to the context's executable graph of this join mode
-            // (cudaGraphExecUpdate: no new instantiation while the shape of
-            // the iteration is the same); the draw phase is read from a
-            // device word, written before each replay.
             Ctx::IterGraph& ig = ctx.iter_graph[(int)mode & 3];
             if (!whole_g.exec) {
                 const uint64_t c0 = launch_counter().load();
                 cudaGraph_t graph = nullptr;
                 cudaError_t e = cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal);
                 if (e == cudaSuccess) {
-                    const JoinArgs ja = make_ja();
-                    cudaError_t e1 = seg_a(false, phase_dev);
-                    if (e1 == cudaSuccess) {
-                        k_check_cap<<<1, 32, 0, st>>>(ctr, reinterpret_cast<const unsigned long long*>(&ctr->pairs),
-                                                      (unsigned long long)(ws.pd.bytes / 4), OVF_PAIRS); count_launch();
-                        e1 = part0(ja, nullptr);
-                    }
-                    if (e1 == cudaSuccess) {
-                        k_check_cap<<<1, 32, 0, st>>>(ctr, reinterpret_cast<const unsigned long long*>(&ctr->proposals),
-                                                      (unsigned long long)(ws.bucket.bytes / prop_bytes),
-                                                      OVF_PROPOSALS); count_launch();
-                        e1 = part1(ja, nullptr);
-                    }
-                    if (e1 == cudaSuccess) e1 = copy_back();
+                    const cudaError_t e1 = iteration(phase_dev);
                     const cudaError_t e2 = cudaStreamEndCapture(st, &graph);
                     e = e1 != cudaSuccess ? e1 : e2;
                 }
@@ -1869,100 +1925,38 @@ int run_nndescent(Ctx& ctx, GraphDev& g, JoinMode mode, uint32_t split, uint32_t
             } else {
                 count_launch(ig.launches);
             }
-            if (whole_g.exec) {
-                *h_phase = phase;  // pinned; the copy is enqueued before the replay
-                NNM_CUDA_TRY(cudaMemcpyAsync(phase_dev, h_phase, 4, cudaMemcpyHostToDevice, st));
-                NNM_CUDA_TRY(cudaGraphLaunch(whole_g.exec, st));
-                NNM_CUDA_TRY(cudaStreamSynchronize(st));
-                IterCounters& h = *ctx.h_counters;
-                if (h.error) {
-                    ctx.last_error = "device capacity check failed (code " + std::to_string(h.error) + ")";
-                    return 6;
-                }
-                if (h.overflow) {
-                    // grow what was short (the graph names the old buffers:
-                    // it is captured again next iteration) and rerun what the
-                    // kernels skipped
-                    whole_g.exec = nullptr;
-                    unsigned nt[NTIER];
-                    for (int t = 0; t < NTIER; t++) nt[t] = h.ntier[t];
-                    const unsigned ovf = h.overflow;
-                    NNM_CUDA_TRY(cudaMemsetAsync(&ctr->overflow, 0, 4, st));
-                    if (ovf & OVF_PAIRS) {
-                        NNM_CUDA_TRY(ws.pd.ensure((size_t)(std::max<uint64_t>(h.pairs, 1) * 1.5 + 1024) * 4));
-                        NNM_CUDA_TRY(part0(make_ja(), nt));
-                        NNM_CUDA_TRY(cudaMemcpyAsync(ctx.h_counters, ctr, sizeof(IterCounters), cudaMemcpyDeviceToHost, st));
-                        NNM_CUDA_TRY(cudaStreamSynchronize(st));
-                    }
-                    const uint64_t nprop = ctx.h_counters->proposals;
-                    if (nprop * prop_bytes > ws.bucket.bytes)
-                        NNM_CUDA_TRY(ws.bucket.ensure((size_t)(nprop * 1.5 + 1024) * prop_bytes));
-                    NNM_CUDA_TRY(part1(make_ja(), nt));
-                    NNM_CUDA_TRY(copy_back());
-                    NNM_CUDA_TRY(cudaStreamSynchronize(st));
-                }
-                done = true;
-            }
         }
-        if (!done) {
-            const bool graphable = g.fast && !carry_now && !seg.disabled && !tc && !g.no_graph;
-            if (graphable && seg.exec) {
-                ShufArgs sh = shuf_args();
-                void* kargs[] = {&sh};
-                cudaKernelNodeParams kp = seg.kp;
-                kp.kernelParams = kargs;
-                kp.extra = nullptr;
-                cudaError_t e = cudaGraphExecKernelNodeSetParams(seg.exec, seg.shuf, &kp);
-                if (e == cudaSuccess) e = cudaGraphLaunch(seg.exec, st);
-                NNM_CUDA_TRY(e);
-                count_launch(seg.launches);
-            } else if (graphable) {
-                const uint64_t c0 = launch_counter().load();
-                cudaGraph_t& graph = seg.graph;
-                cudaError_t e = cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal);
-                if (e == cudaSuccess) {
-                    const cudaError_t e1 = seg_a();
-                    const cudaError_t e2 = cudaStreamEndCapture(st, &graph);
-                    e = e1 != cudaSuccess ? e1 : e2;
-                }
-                if (e == cudaSuccess) e = cudaGraphInstantiate(&seg.exec, graph, 0);
-                if (e == cudaSuccess) seg.shuf = find_kernel_node(graph, reinterpret_cast<void*>(k_shuffle_append), seg.kp);
-                seg.launches = launch_counter().load() - c0;
-                if (e == cudaSuccess && seg.shuf) e = cudaGraphLaunch(seg.exec, st);  // capture counted its kernels
-                if (e != cudaSuccess || !seg.shuf) {
-                    // no graph: this call launches the segment directly
-                    cudaGetLastError();
-                    if (seg.exec) cudaGraphExecDestroy(seg.exec);
-                    if (seg.graph) cudaGraphDestroy(seg.graph);
-                    seg.exec = nullptr;
-                    seg.graph = nullptr;
-                    seg.disabled = true;
-                    NNM_CUDA_TRY(seg_a());
-                }
-            } else {
-                NNM_CUDA_TRY(seg_a());
+        if (whole && whole_g.exec) {
+            *h_phase = phase;  // pinned; the copy is enqueued before the replay
+            NNM_CUDA_TRY(cudaMemcpyAsync(phase_dev, h_phase, 4, cudaMemcpyHostToDevice, st));
+            NNM_CUDA_TRY(cudaGraphLaunch(whole_g.exec, st));
+        } else {
+            NNM_CUDA_TRY(iteration(nullptr));
+        }
+        NNM_CUDA_TRY(cudaStreamSynchronize(st));
+        if (ctx.h_counters->error) {
+            ctx.last_error = "device capacity check failed (code " + std::to_string(ctx.h_counters->error) + ")";
+            return 6;
+        }
+        if (ctx.h_counters->overflow) {
+            // grow what was short (a graph names the old buffers: it is
+            // captured again next iteration) and rerun what was skipped
+            whole_g.exec = nullptr;
+            const double room = g.fast && tc ? 1.5 : 1.25;
+            unsigned nt[NTIER];
+            for (int t = 0; t < NTIER; t++) nt[t] = ctx.h_counters->ntier[t];
+            const unsigned ovf = ctx.h_counters->overflow;
+            NNM_CUDA_TRY(cudaMemsetAsync(&ctr->overflow, 0, 4, st));
+            if (ovf & OVF_PAIRS) {
+                NNM_CUDA_TRY(grow(ws.pd, ctx.h_counters->pairs, 4, room));
+                NNM_CUDA_TRY(part0(make_ja(), nt));
+                NNM_CUDA_TRY(copy_back());
+                NNM_CUDA_TRY(cudaStreamSynchronize(st));
+                if (ctx.h_counters->overflow) NNM_CUDA_TRY(cudaMemsetAsync(&ctr->overflow, 0, 4, st));
             }
-            NNM_CUDA_TRY(cudaStreamSynchronize(st));
-            if (ctx.h_counters->error) {
-                ctx.last_error = "device capacity check failed (code " + std::to_string(ctx.h_counters->error) + ")";
-                return 6;
-            }
-            unsigned ntier[NTIER];
-            for (int t = 0; t < NTIER; t++) ntier[t] = ctx.h_counters->ntier[t];
-            // headroom for the iterations the whole-iteration graph runs
-            const double room = (g.fast && tc) ? 1.5 : 1.0;
-            const size_t pd_need = (size_t)(std::max<uint64_t>(ctx.h_counters->pairs, 1) * room) * 4;
-            if (pd_need > ws.pd.bytes) NNM_CUDA_TRY(ws.pd.ensure(pd_need + 4096));
-            JoinArgs ja = make_ja();
-            NNM_CUDA_TRY(part0(ja, ntier));
-            NNM_CUDA_TRY(cudaMemcpyAsync(ctx.h_counters, ctr, sizeof(IterCounters), cudaMemcpyDeviceToHost, st));
-            NNM_CUDA_TRY(cudaStreamSynchronize(st));
             const uint64_t nprop = ctx.h_counters->proposals;
-            if (nprop * prop_bytes > ws.bucket.bytes) {
-                NNM_CUDA_TRY(ws.bucket.ensure((size_t)(nprop * (g.fast && tc ? 1.5 : 1.25) + 1024) * prop_bytes));
-                ja.bucket = ws.bucket.p;
-            }
-            NNM_CUDA_TRY(part1(ja, ntier));
+            if (nprop * prop_bytes > ws.bucket.bytes) NNM_CUDA_TRY(grow(ws.bucket, nprop, prop_bytes, room));
+            NNM_CUDA_TRY(part1(make_ja(), nt));
             NNM_CUDA_TRY(copy_back());
             NNM_CUDA_TRY(cudaStreamSynchronize(st));
         }

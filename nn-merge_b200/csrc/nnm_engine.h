@@ -37,11 +37,11 @@ struct DevBuf {
 
 // Scratch for one NN-Descent iteration, sized for the largest graph seen.
 struct Workspace {
-    DevBuf rcnt, rcur, rtot, roff, rseg, rscr, rcount, rofs, rbuf;
+    DevBuf rcnt, rcur, rtot, roff, rseg, rscr, rofs, rbuf;
     DevBuf cntpos, bcnt, bcur, boff, bucket, bigrev, nflag, scan_tmp;
     DevBuf npairs, poff, pd, tiers, erows;
     DevBuf kth;  // every row's K-th distance, gathered per iteration
-    DevBuf rtier;  // every row's join tier (k_shuffle_append), binned by k_tier_lists
+    DevBuf rtier;  // every row's join tier (k_shuffle_exact, k_shuffle_fast), binned by k_tier_lists
     // outputs [0, mt_have) of mt19937(mt_seed), the generator's state, and
     // the seed; mt_have is cleared at the start of every call
     DevBuf draws, mt_ring;
@@ -50,7 +50,7 @@ struct Workspace {
     DevBuf counters, misc;
     DevBuf mlp_err;  // the code network's tensor-core inference: a wait that ran out
     void release_all() {
-        DevBuf* all[] = {&rcnt, &rcur, &rtot, &roff, &rseg, &rscr, &rcount, &rofs, &rbuf, &cntpos, &bcnt, &bcur,
+        DevBuf* all[] = {&rcnt, &rcur, &rtot, &roff, &rseg, &rscr, &rofs, &rbuf, &cntpos, &bcnt, &bcur,
                          &boff, &bucket, &bigrev, &nflag, &scan_tmp, &npairs, &poff, &pd, &tiers, &erows, &kth, &rtier,
                          &draws, &mt_ring, &counters, &misc, &mlp_err};
         for (auto* b : all) b->release();

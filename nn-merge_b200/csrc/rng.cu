@@ -71,6 +71,9 @@ __global__ void __launch_bounds__(STREAM_WARPS * 32) k_glibc_stream(int32_t* __r
                                                                     uint64_t first_output,
                                                                     const uint64_t* __restrict__ count_ptr,
                                                                     uint64_t count_cap) {
+    __shared__ uint32_t bs[2 * DEG];
+    for (uint32_t i = threadIdx.x; i < 2 * DEG; i += blockDim.x) bs[i] = base.s[i];
+    __syncthreads();
     const int lane = threadIdx.x & 31;
     const uint64_t g = (uint64_t)blockIdx.x * STREAM_WARPS + (threadIdx.x >> 5);
     uint64_t count = count_ptr ? *count_ptr : count_cap;
@@ -79,19 +82,33 @@ __global__ void __launch_bounds__(STREAM_WARPS * 32) k_glibc_stream(int32_t* __r
     if (k0 >= count) return;
     // x^n for the s-index n of the run's first output, a hexadecimal digit at a time
     const uint64_t n = first_output + k0 + 310;
+    // (n >= 310: digit 2 or a higher one is not 0); the table reads of eight
+    // digits are in flight at once
     uint32_t c = lane == 0 ? 1u : 0u;
     bool one = true;
-    for (int j = 0; j < 16 && (n >> (4 * j)); j++) {
-        const uint32_t d = (uint32_t)(n >> (4 * j)) & 15u;
-        if (!d) continue;
-        const uint32_t pw = g_pow16[j][d - 1][lane];
-        c = one ? pw : poly_mulmod_warp(c, pw, lane);
-        one = false;
+    for (int j0 = 0; j0 < 16 && (n >> (4 * j0)); j0 += 8) {
+        uint32_t pw[8];
+#pragma unroll
+        for (int j = 0; j < 8; j++) {
+            const uint32_t d = (uint32_t)(n >> (4 * (j0 + j))) & 15u;
+            pw[j] = d ? g_pow16[j0 + j][d - 1][lane] : 0u;
+        }
+#pragma unroll 1
+        for (int j = 0; j < 8; j++) {
+            const uint32_t d = (uint32_t)(n >> (4 * (j0 + j))) & 15u;
+            uint32_t p = pw[0];
+#pragma unroll
+            for (int q = 1; q < 8; q++)
+                if (q == j) p = pw[q];
+            if (!d) continue;
+            c = one ? p : poly_mulmod_warp(c, p, lane);
+            one = false;
+        }
     }
     uint32_t w = 0;
     const int m = lane < DEG ? lane : DEG - 1;
 #pragma unroll
-    for (int j = 0; j < DEG; j++) w += __shfl_sync(FULL, c, j) * base.s[j + m];
+    for (int j = 0; j < DEG; j++) w += __shfl_sync(FULL, c, j) * bs[j + m];
     const int src = 28 + m % 3;
     const uint64_t end = k0 + DEG * RUN < count ? k0 + DEG * RUN : count;
     for (uint64_t pos = k0; pos < end; pos += DEG) {

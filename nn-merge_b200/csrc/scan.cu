@@ -1,8 +1,12 @@
 // Device-wide exclusive prefix sums (u32 counts -> u64 offsets), used to lay
 // out per-row and per-target segments (reverse lists, proposal buckets,
-// random-draw ranges).  Three passes: per-tile totals, a scan of the tile
-// totals in one block, then per-tile scans.  HBM-bound: 4 B read + 8 B
-// written per element.
+// random-draw ranges).  Two passes: per-tile totals, then per-tile scans whose
+// blocks each add up the totals before their tile; a single tile (n <= 4096)
+// needs only the second.  Up to three scans of the same length share the
+// launches.  HBM-bound at large n (4 B read + 8 B written per element),
+// launch-bound at small: a separate scan of the totals, one array at a time,
+// was 15 launches of an exact-tier iteration and 183 of the 1,110 us the GPU
+// was busy in a 2,000-row build.
 #include <cstdint>
 #include <cuda_runtime.h>
 
@@ -41,67 +45,84 @@ __device__ __forceinline__ uint64_t block_exclusive_scan(uint64_t v, uint64_t* s
     return before + x - v;
 }
 
-__global__ void k_tile_sums(const uint32_t* __restrict__ in, size_t n, uint64_t* __restrict__ sums) {
+__device__ __forceinline__ uint32_t scan_input(const ScanJob& j, size_t i) {
+    const uint32_t v = j.in[i];
+    if (!j.in2) return v;
+    const uint32_t w = j.in2[i];  // draws of two shuffles
+    return (v ? v - 1 : 0u) + (w ? w - 1 : 0u);
+}
+
+// sums: per job, one total per tile.
+__global__ void __launch_bounds__(SCAN_THREADS) k_tile_sums(ScanJobs jobs, size_t n, uint64_t* __restrict__ sums) {
     __shared__ uint64_t sh[32];
-    size_t base = (size_t)blockIdx.x * TILE + (size_t)threadIdx.x * SCAN_ITEMS;
+    const ScanJob& j = jobs.j[blockIdx.y];
+    const size_t base = (size_t)blockIdx.x * TILE;
     uint64_t s = 0;
 #pragma unroll
-    for (int i = 0; i < SCAN_ITEMS; i++)
-        if (base + i < n) s += in[base + i];
+    for (int i = 0; i < SCAN_ITEMS; i++) {
+        const size_t t = base + (size_t)i * SCAN_THREADS + threadIdx.x;
+        if (t < n) s += scan_input(j, t);
+    }
     uint64_t tot;
     block_exclusive_scan(s, sh, &tot);
-    if (threadIdx.x == 0) sums[blockIdx.x] = tot;
+    if (threadIdx.x == 0) sums[(size_t)blockIdx.y * gridDim.x + blockIdx.x] = tot;
 }
 
-__global__ void k_scan_sums(uint64_t* __restrict__ sums, size_t m, uint64_t* __restrict__ grand) {
+__global__ void __launch_bounds__(SCAN_THREADS) k_tile_scan(ScanJobs jobs, size_t n,
+                                                            const uint64_t* __restrict__ sums) {
     __shared__ uint64_t sh[32];
-    uint64_t carry = 0;
-    for (size_t b = 0; b < m; b += SCAN_THREADS) {
-        size_t i = b + threadIdx.x;
-        uint64_t v = i < m ? sums[i] : 0;
-        uint64_t tot;
-        uint64_t ex = block_exclusive_scan(v, sh, &tot);
-        if (i < m) sums[i] = carry + ex;
-        carry += tot;
+    const ScanJob& j = jobs.j[blockIdx.y];
+    uint64_t before = 0;
+    if (blockIdx.x) {  // the totals of the tiles before this one
+        const uint64_t* js = sums + (size_t)blockIdx.y * gridDim.x;
+        uint64_t p = 0;
+        for (uint32_t i = threadIdx.x; i < blockIdx.x; i += SCAN_THREADS) p += js[i];
+        block_exclusive_scan(p, sh, &before);
     }
-    if (threadIdx.x == 0 && grand) *grand = carry;
-}
-
-__global__ void k_tile_scan(const uint32_t* __restrict__ in, size_t n, const uint64_t* __restrict__ sums,
-                            uint64_t* __restrict__ out) {
-    __shared__ uint64_t sh[32];
-    size_t base = (size_t)blockIdx.x * TILE + (size_t)threadIdx.x * SCAN_ITEMS;
+    const size_t base = (size_t)blockIdx.x * TILE + (size_t)threadIdx.x * SCAN_ITEMS;
     uint32_t v[SCAN_ITEMS];
     uint64_t s = 0;
 #pragma unroll
     for (int i = 0; i < SCAN_ITEMS; i++) {
-        v[i] = base + i < n ? in[base + i] : 0;
+        v[i] = base + i < n ? scan_input(j, base + i) : 0;
         s += v[i];
     }
-    uint64_t ex = block_exclusive_scan(s, sh, nullptr) + sums[blockIdx.x];
+    uint64_t ex = block_exclusive_scan(s, sh, nullptr) + before;
 #pragma unroll
     for (int i = 0; i < SCAN_ITEMS; i++) {
-        if (base + i < n) out[base + i] = ex;
+        if (base + i < n) j.out[base + i] = ex;
         ex += v[i];
     }
-    if (base < n && base + SCAN_ITEMS >= n) out[n] = ex;  // thread owning the last element
+    if (base < n && base + SCAN_ITEMS >= n) {  // thread owning the last element
+        j.out[n] = ex;
+        if (j.total) *j.total = ex;
+        if (j.over && ex > j.cap) atomicOr(j.over, j.bit);
+    }
 }
 }  // namespace
 
-size_t scan_temp_elems(size_t n) { return (n + TILE - 1) / TILE + 1; }
+size_t scan_temp_elems(size_t n) { return ScanJobs::MAX * ((n + TILE - 1) / TILE) + 1; }
+
+cudaError_t exclusive_scans(const ScanJobs& jobs, int count, size_t n, uint64_t* temp, cudaStream_t st) {
+    if (n == 0) {
+        for (int i = 0; i < count; i++) {
+            cudaError_t e = cudaMemsetAsync(jobs.j[i].out, 0, sizeof(uint64_t), st);
+            if (e == cudaSuccess && jobs.j[i].total) e = cudaMemsetAsync(jobs.j[i].total, 0, sizeof(uint64_t), st);
+            if (e != cudaSuccess) return e;
+        }
+        return cudaSuccess;
+    }
+    const dim3 grid((unsigned)((n + TILE - 1) / TILE), (unsigned)count);
+    if (grid.x > 1) { k_tile_sums<<<grid, SCAN_THREADS, 0, st>>>(jobs, n, temp); count_launch(); }
+    k_tile_scan<<<grid, SCAN_THREADS, 0, st>>>(jobs, n, temp); count_launch();
+    return cudaGetLastError();
+}
 
 cudaError_t exclusive_scan(const uint32_t* in, uint64_t* out, size_t n, uint64_t* temp, uint64_t* d_total,
                            cudaStream_t st) {
-    if (n == 0) {
-        cudaError_t e = cudaMemsetAsync(out, 0, sizeof(uint64_t), st);
-        if (e == cudaSuccess && d_total) e = cudaMemsetAsync(d_total, 0, sizeof(uint64_t), st);
-        return e;
-    }
-    size_t tiles = (n + TILE - 1) / TILE;
-    k_tile_sums<<<(unsigned)tiles, SCAN_THREADS, 0, st>>>(in, n, temp); count_launch();
-    k_scan_sums<<<1, SCAN_THREADS, 0, st>>>(temp, tiles, d_total); count_launch();
-    k_tile_scan<<<(unsigned)tiles, SCAN_THREADS, 0, st>>>(in, n, temp, out); count_launch();
-    return cudaGetLastError();
+    ScanJobs jobs{};
+    jobs.j[0] = ScanJob{in, nullptr, out, d_total, nullptr, 0, 0};
+    return exclusive_scans(jobs, 1, n, temp, st);
 }
 
 }  // namespace nnm
