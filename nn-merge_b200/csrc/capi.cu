@@ -430,6 +430,7 @@ int nnm_merge_create(nnm_ctx* ctx, const float* x, uint64_t n, uint32_t d, uint3
     std::unique_ptr<nnm_merge> m(new nnm_merge());
     m->ctx = ctx;
     setup_graph(m->g, o, n, d, k);
+    m->g.repeats = true;  // nnm_merge_init_sgraph takes any graph
     rc = nnm::upload_vectors(c, m->store, m->g, x, false);
     if (!rc) rc = nnm::graph_alloc(c, m->store, m->g, false);
     if (!rc) {
@@ -562,6 +563,7 @@ int nnm_hmerge_build(nnm_ctx* ctx, const float* x, uint64_t n, uint32_t d, uint3
     GraphDev g;
     c.ws.mt_have = 0;
     setup_graph(g, o, n, d, k);
+    g.repeats = true;
     if (!c.dpg) c.dpg = new nnm::DpgState();
     nnm::DpgState& dpg = *c.dpg;
     if (layers) std::memset(layers, 0, sizeof(*layers));
@@ -768,21 +770,24 @@ int nnm_graph_recall(nnm_ctx* ctx, const float* x, uint64_t n, uint32_t d, const
         if (rows[i] >= n) return fail(ctx, NNM_ERR_INVALID, "recall: row out of range");
     Ctx& c = ctx->c;
     if (cudaSetDevice(c.device) != cudaSuccess) return fail(ctx, NNM_ERR_NO_DEVICE, "cudaSetDevice failed");
-    GraphStore st;
+    // the vectors in the context's graph store; the evaluated rows and the
+    // first atop ids of their lists, the only ones read, in its workspace
+    // (a call used to allocate five buffers, copy all n x k ids and free them)
     GraphDev g;
-    nnm::DevBuf ib, rb;
-    int rc = upload_plain(c, st, g, x, n, d);
-    if (!rc && (ib.ensure(n * k * 4) != cudaSuccess || rb.ensure((size_t)nrows * 4 + 4) != cudaSuccess))
-        rc = fail(ctx, NNM_ERR_OOM, "device allocation failed");
-    if (!rc && (cudaMemcpy(ib.p, ids, n * k * 4, cudaMemcpyHostToDevice) != cudaSuccess ||
-                (nrows && cudaMemcpy(rb.p, rows, (size_t)nrows * 4, cudaMemcpyHostToDevice) != cudaSuccess)))
-        rc = NNM_ERR_CUDA;
+    int rc = upload_plain(c, c.store, g, x, n, d);
+    std::vector<uint32_t> h((size_t)nrows * (atop + 1));
+    for (uint32_t i = 0; i < nrows; i++) {
+        h[i] = rows[i];
+        for (uint32_t j = 0; j < atop; j++) h[nrows + (size_t)i * atop + j] = ids[(size_t)rows[i] * k + j];
+    }
+    if (!rc && c.ws.bucket.ensure(h.size() * 4 + 4) != cudaSuccess) rc = fail(ctx, NNM_ERR_OOM, "device allocation failed");
+    uint32_t* dev = c.ws.bucket.as<uint32_t>();
+    if (!rc && !h.empty() &&
+        cudaMemcpyAsync(dev, h.data(), h.size() * 4, cudaMemcpyHostToDevice, c.stream) != cudaSuccess)
+        rc = fail(ctx, NNM_ERR_CUDA, "recall: copy failed");
     if (!rc)
-        rc = nnm::graph_recall_dev(c, g.x, (uint32_t)n, g.dp, NNM_METRIC_L2, ib.as<uint32_t>(), k, rb.as<uint32_t>(),
-                                   nrows, atop, recall);
-    st.release();
-    ib.release();
-    rb.release();
+        rc = nnm::graph_recall_dev(c, g.x, (uint32_t)n, g.dp, NNM_METRIC_L2, dev + nrows, atop, true, dev, nrows, atop,
+                                   recall);
     return rc;
 }
 
@@ -869,7 +874,7 @@ int nnm_autotune_merge_leaves(nnm_ctx* ctx, const float* x_dev, uint64_t n, uint
                 ms = std::min(ms, stt.device_ms);
             }
             double rec = 0.0;
-            int rc = nnm::graph_recall_dev(c, xe, ns, dp, (int)o.metric, ib.as<uint32_t>(), k, rb.as<uint32_t>(), ne,
+            int rc = nnm::graph_recall_dev(c, xe, ns, dp, (int)o.metric, ib.as<uint32_t>(), k, false, rb.as<uint32_t>(), ne,
                                            10, &rec);
             if (rc) return done(rc);
             const uint32_t i = res.ntrials++;

@@ -152,6 +152,7 @@ struct GraphDev {
     uint32_t *newL = nullptr, *oldL = nullptr, *newlen = nullptr, *oldlen = nullptr;  // sample lists
     uint32_t capn = 0, capo = 0;
     uint32_t *rnewT = nullptr, *roldT = nullptr, *rnewTlen = nullptr, *roldTlen = nullptr;  // H-Merge carry
+    bool repeats = false;      // exact tier: a pool may hold an id twice (H-Merge; a caller's graph)
     bool carry = false;        // lists of the last converged iteration are still present
     GlibcBase gbase;
     uint64_t gpos = 0;         // std::rand() outputs consumed since srand(seed)
