@@ -34,6 +34,7 @@
 #include "nnm_join.h"
 #include "nnm_launch.h"
 #include "nnm_scan.h"
+#include "nnm_tc.cuh"
 
 namespace nnm {
 namespace {
@@ -419,20 +420,73 @@ __device__ __forceinline__ void shuffle_no_room(const ShufArgs& a, uint32_t t) {
     a.rtier[t] = 0xff;
 }
 
+// Lane's entries of a list of m <= 32 R sorted by rank, in place in shared
+// memory: each lane counts, by broadcast reads, the entries smaller than its
+// own.  TIES: equal words (GraphDev::repeats: a row can be pushed twice) keep their order.
+template <int R, bool TIES>
+__device__ __forceinline__ void rank_sort(uint32_t* sh, uint32_t m, int lane) {
+    uint32_t v[R], rank[R];
+#pragma unroll
+    for (int r = 0; r < R; r++) {
+        v[r] = lane + 32 * r < m ? sh[lane + 32 * r] : 0u;
+        rank[r] = 0;
+    }
+#pragma unroll 4
+    for (uint32_t i = 0; i < m; i++) {
+        const uint32_t k = sh[i] & LID_MASK;
+#pragma unroll
+        for (int r = 0; r < R; r++) {
+            const uint32_t own = v[r] & LID_MASK;
+            rank[r] += TIES ? (k < own || (k == own && i < lane + 32 * r)) : k < own;
+        }
+    }
+    __syncwarp();
+#pragma unroll
+    for (int r = 0; r < R; r++)
+        if (lane + 32 * r < m) sh[rank[r]] = v[r];
+}
+
+// std::random_shuffle of a list of n <= 32 R entries, swap i exchanging
+// entries i and jj[i]: each lane traces its output positions back through
+// the swaps to the entry that ends there -- no swap waits for another's
+// memory -- and writes the first `keep` entries to L (and T).
+template <int R>
+__device__ __forceinline__ void traced_shuffle(const uint32_t* sh, const uint16_t* jj, uint32_t n, uint32_t keep,
+                                               uint32_t* L, uint32_t* T, int lane) {
+    uint32_t cur[R];
+#pragma unroll
+    for (int r = 0; r < R; r++) cur[r] = lane + 32 * r;
+#pragma unroll 4
+    for (uint32_t i = n - 1; i > 0; i--) {
+        const uint32_t j = jj[i];
+#pragma unroll
+        for (int r = 0; r < R; r++) cur[r] = cur[r] == i ? j : cur[r] == j ? i : cur[r];
+    }
+#pragma unroll
+    for (int r = 0; r < R; r++)
+        if (lane + 32 * r < keep) {
+            const uint32_t v = sh[cur[r]];
+            L[lane + 32 * r] = v;
+            if (T) T[lane + 32 * r] = v;
+        }
+}
+
 // Exact tier, one warp per row: its two reverse lists (in the order of the
 // sampling's atomics) sorted by source row after their carried prefix, then
 // std::random_shuffle, truncation and append.  A list of at most SORT_SMEM
-// entries stays in shared memory throughout: sorted by rank (each lane
-// counts the smaller entries of its own, reading the list by broadcast;
-// equal words, the same row pushed twice, keep their order), the draws'
-// remainders taken by all lanes, the swaps -- a serial chain -- run for both
-// lists at once by lanes 0 and 1.  Longer lists come sorted in place by
-// k_rev_sort_big and are shuffled there by lane 0.  Bound: issue slots of
-// the rank loops and latency of the swap chains.  Separate kernels (a
-// bitonic sort per list, a block-wide sort of lists over 32 entries, then
-// lane 0 taking remainders and swapping list after list) took 50 + 92 + 74 us
-// an iteration at 100,000 rows with k = 20.
+// entries stays in shared memory (rank_sort, traced_shuffle).  Longer lists
+// come sorted in place by k_rev_sort_big and are shuffled there by lane 0.
+// Bound: issue slots of the two loops over a list, whose instructions all
+// lanes share.  TIES: as in rank_sort.  At 100,000 rows with k = 20 separate
+// kernels (a bitonic sort per list, a block-wide sort of lists over 32
+// entries, then lane 0 taking remainders and swapping) took 50 + 92 + 74 us
+// an iteration, this kernel with the swaps a serial chain of lane 0 108 us,
+// with the traced swaps 95 us (27 and 14 us at 2,000 rows, where the longest
+// list's chain was the kernel).  The forms of 4 and 8 entries a lane out of
+// line at 48 registers (five blocks an SM instead of four) spilled: 100 and
+// 20 us.
 constexpr int SHUFX_WARPS = 8;
+template <bool TIES>
 __global__ void __launch_bounds__(SHUFX_WARPS * 32) k_shuffle_exact(ShufArgs a) {
     __shared__ uint32_t s_seg[SHUFX_WARPS][2][SORT_SMEM];
     __shared__ uint16_t s_j[SHUFX_WARPS][2][SORT_SMEM];
@@ -446,7 +500,6 @@ __global__ void __launch_bounds__(SHUFX_WARPS * 32) k_shuffle_exact(ShufArgs a) 
     const uint32_t carry[2] = {a.rnewT ? a.rnewTlen[t] : 0u, a.roldT ? a.roldTlen[t] : 0u};
     const uint32_t len[2] = {(uint32_t)(hi_n - lo_n), (uint32_t)(hi_o - lo_o)};
     uint32_t* const seg[2] = {a.rseg_new + lo_n, a.rseg_old + lo_o};
-    const bool in_smem[2] = {len[0] <= SORT_SMEM, len[1] <= SORT_SMEM};
     const int32_t* const dr[2] = {draws, draws + (len[0] ? len[0] - 1 : 0u)};
     if (nl + min(len[0], a.smpl) > a.capn || ol + min(len[1], a.smpl) > a.capo) {
         if (lane == 0) shuffle_no_room(a, t);
@@ -454,83 +507,44 @@ __global__ void __launch_bounds__(SHUFX_WARPS * 32) k_shuffle_exact(ShufArgs a) 
     }
 #pragma unroll
     for (int l = 0; l < 2; l++) {
-        if (!in_smem[l]) continue;
+        if (len[l] > SORT_SMEM) continue;
         uint32_t* sh = s_seg[w][l];
         for (uint32_t j = lane; j < len[l]; j += 32) sh[j] = seg[l][j];
         for (uint32_t i = 1 + lane; i < len[l]; i += 32) s_j[w][l][i] = (uint16_t)(dr[l][i - 1] % (int32_t)(i + 1));
     }
     __syncwarp();
-#pragma unroll
+#pragma unroll 1
     for (int l = 0; l < 2; l++) {
-        const uint32_t c = carry[l];
-        if (!in_smem[l] || len[l] < c + 2) continue;
-        uint32_t* sh = s_seg[w][l] + c;
-        const uint32_t m = len[l] - c;
-        uint32_t v[SORT_SMEM / 32], rank[SORT_SMEM / 32];
-        if (m <= 32) {
-            v[0] = (uint32_t)lane < m ? sh[lane] : 0u;
-            rank[0] = 0;
-            for (uint32_t i = 0; i < m; i++) {
-                const uint32_t k = sh[i] & LID_MASK, own = v[0] & LID_MASK;
-                rank[0] += k < own || (k == own && i < (uint32_t)lane);
-            }
-            __syncwarp();
-            if ((uint32_t)lane < m) sh[rank[0]] = v[0];
-        } else {
-#pragma unroll
-            for (uint32_t r = 0; r < SORT_SMEM / 32; r++) {
-                v[r] = lane + 32 * r < m ? sh[lane + 32 * r] : 0u;
-                rank[r] = 0;
-            }
-            for (uint32_t i = 0; i < m; i++) {
-                const uint32_t k = sh[i] & LID_MASK;
-#pragma unroll
-                for (uint32_t r = 0; r < SORT_SMEM / 32; r++) {
-                    if (32 * r >= m) break;
-                    const uint32_t own = v[r] & LID_MASK;
-                    rank[r] += k < own || (k == own && i < lane + 32 * r);
-                }
-            }
-            __syncwarp();
-#pragma unroll
-            for (uint32_t r = 0; r < SORT_SMEM / 32; r++)
-                if (lane + 32 * r < m) sh[rank[r]] = v[r];
-        }
-    }
-    __syncwarp();
-    if (lane < 2) {
-        const uint32_t n = lane ? len[1] : len[0];
-        if (n <= SORT_SMEM) {
-            uint32_t* sh = s_seg[w][lane];
-            const uint16_t* jj = s_j[w][lane];
-            for (uint32_t i = 1; i < n; i++) {
-                const uint32_t j = jj[i], x = sh[i], y = sh[j];
-                sh[i] = y;
-                sh[j] = x;
-            }
-        }
-    }
-    if (lane == 0) {
-        if (!in_smem[0]) shuffle_seg(seg[0], len[0], dr[0]);
-        if (!in_smem[1]) shuffle_seg(seg[1], len[1], dr[1]);
-    }
-    __syncwarp();
-#pragma unroll
-    for (int l = 0; l < 2; l++) {
-        const uint32_t keep = min(len[l], a.smpl);
-        const uint32_t* src = in_smem[l] ? s_seg[w][l] : seg[l];
+        const uint32_t n = l ? len[1] : len[0], c = l ? carry[1] : carry[0], keep = min(n, a.smpl);
         uint32_t* L = l ? a.oldL + (size_t)t * a.capo + ol : a.newL + (size_t)t * a.capn + nl;
         uint32_t* T = l ? a.roldT : a.rnewT;
-        for (uint32_t j = lane; j < keep; j += 32) {
-            const uint32_t v = src[j];
-            L[j] = v;
-            if (T) T[(size_t)t * a.smpl + j] = v;
+        if (T) T += (size_t)t * a.smpl;
+        if (n > SORT_SMEM) {
+            uint32_t* g = l ? seg[1] : seg[0];
+            if (lane == 0) shuffle_seg(g, n, l ? dr[1] : dr[0]);
+            __syncwarp();
+            for (uint32_t j = lane; j < keep; j += 32) {
+                const uint32_t v = g[j];
+                L[j] = v;
+                if (T) T[j] = v;
+            }
+        } else if (n) {
+            uint32_t* sh = s_seg[w][l];
+            const uint16_t* jj = s_j[w][l];
+            const uint32_t m = n - c;
+            if (m > 128) rank_sort<SORT_SMEM / 32, TIES>(sh + c, m, lane);
+            else if (m > 64) rank_sort<4, TIES>(sh + c, m, lane);
+            else if (m > 32) rank_sort<2, TIES>(sh + c, m, lane);
+            else if (m > 1) rank_sort<1, TIES>(sh + c, m, lane);
+            __syncwarp();
+            if (n > 128) traced_shuffle<SORT_SMEM / 32>(sh, jj, n, keep, L, T, lane);
+            else if (n > 64) traced_shuffle<4>(sh, jj, n, keep, L, T, lane);
+            else if (n > 32) traced_shuffle<2>(sh, jj, n, keep, L, T, lane);
+            else traced_shuffle<1>(sh, jj, n, keep, L, T, lane);
         }
-        if (l) ol += keep;
-        else nl += keep;
         if (lane == 0 && T) (l ? a.roldTlen : a.rnewTlen)[t] = keep;
     }
-    if (lane == 0) shuffle_finish(a, t, nl, ol);
+    if (lane == 0) shuffle_finish(a, t, nl + min(len[0], a.smpl), ol + min(len[1], a.smpl));
 }
 
 // Fast tier, one warp per row: a random subset of each reverse list, appended.
@@ -631,7 +645,7 @@ __global__ void __launch_bounds__(256) k_tier_lists(const uint8_t* rtier, uint32
 
 // ---------------------------------------------------------------------------
 // 4. Local join, in two kernels.
-//   k_pairs: every pair of a row's lists once -- new x new above the
+//   k_pairs_*: every pair of a row's lists once -- new x new above the
 //     diagonal and new x old -- with the exact sequential distance, stored
 //     in the row's slice of the pair buffer; per list position, the number
 //     of proposals that pass the K-th-distance filter (for bucket sizes).
@@ -644,13 +658,180 @@ __global__ void __launch_bounds__(256) k_tier_lists(const uint8_t* rtier, uint32
 __device__ __forceinline__ uint32_t vrow(uint32_t q, uint32_t vstride) { return q * vstride + (q >> 2); }
 __host__ __device__ __forceinline__ uint32_t vec_stride(uint32_t units) { return ((units + 7) & ~7u) + 1; }
 
-// Where pairs_row reads a row's vectors: FP32 from global memory (L2), FP32
-// staged in shared memory, or the u8 operand copy of the tensor-core join
-// staged in shared memory.  The u8 form is used only when every component
-// is an integer in [0, 255]: d(a, b) = |a|^2 + |b|^2 - 2 a.b is then an
-// exact integer below 2^24, the value of the reference's sequential float
-// sum of the same terms, so all three give the same distances.
-constexpr int VEC_GLOBAL = 0, VEC_F32 = 1, VEC_U8 = 2;
+// Where pairs_row reads a row's vectors: FP32 from global memory (L2), or the
+// u8 operand copy of the tensor-core join staged in shared memory.  The u8
+// form is used only when every component is an integer in [0, 255]:
+// d(a, b) = |a|^2 + |b|^2 - 2 a.b is then an exact integer below 2^24, the
+// value of the reference's sequential float sum of the same terms, so both
+// give the same distances.
+constexpr int VEC_GLOBAL = 0, VEC_U8 = 2;
+
+// Tiers 0-3: the row's FP32 vectors staged in shared memory, PS_WARPS[t]
+// warps a row (four rows side by side in a block of tier 0), a TA x TB tile
+// of pairs a thread.  The tile is the largest that keeps the threads busy,
+// chosen per row: after the first iterations a row has few new entries (3
+// new of 24 is 66 pairs), and 4 x 4 tiles alone ran with 4.4 of 32 lanes on.
+// 4 x 4 and 2 x 2 for the metrics of three operations a term (the larger
+// tile reads half the shared memory a pair), 1 x 1 below; chi-square, a
+// division a term and bound by issue, takes 2 x 2 (tiers 1-3) and 1 x 1.
+// Measured over a build, against 4 x 4 tiles at 64 threads a row: 30,011 x
+// 100 rows, k = 16, L2: tiers 0-2 3.70 -> 1.83 ms; 10,007 x 65, k = 10,
+// chi-square: tiers 0-3 7.9 -> 3.3 ms.  Copying the vectors with cp.async
+// instead of through registers measured the same.
+constexpr int PS_WARPS[4] = {1, 2, 2, 4};
+constexpr int PS_MAX_THREADS[4] = {128, 64, 64, 128};
+
+// Slots of a staged row, 16-byte units: the member arrays (four words a list
+// slot) and the vectors.
+__host__ __device__ __forceinline__ uint32_t staged_units(uint32_t R, uint32_t dq) {
+    return R + R * vec_stride(dq) + R / 4 + 1;
+}
+
+__host__ __device__ __forceinline__ uint32_t tile_count(uint32_t nn, uint32_t S, uint32_t t) {  // t x t tiles
+    const uint32_t ntA = (nn + t - 1) / t, ntB = (S + t - 1) / t;
+    return ntA * ntB - ntA * (ntA - 1) / 2;
+}
+
+// A row's members in shared memory.
+struct PairRow {
+    const uint32_t *ids, *grp;
+    const float* kth;
+    uint32_t* cnt;
+    const float4* vec;
+};
+
+// This thread's T x T tiles of the row, threads apart: distances, stored and
+// counted against the filters.  Returns the distance evaluations.
+template <int M, uint32_t T>
+__device__ __forceinline__ uint32_t pair_tiles(const JoinArgs& a, const PairRow& r, float* pd, uint32_t nn, uint32_t no,
+                                               uint32_t tid, uint32_t threads) {
+    const uint32_t S = nn + no, dq = a.dp >> 2, vstride = vec_stride(dq);
+    const uint32_t ntA = (nn + T - 1) / T, ntB = (S + T - 1) / T;
+    uint32_t ta = 0, rem = tid, cmps = 0;
+    for (;;) {
+        while (ta < ntA && rem >= ntB - ta) {
+            rem -= ntB - ta;
+            ta++;
+        }
+        if (ta >= ntA) break;
+        const uint32_t a0 = ta * T, b0 = (ta + rem) * T;
+        rem += threads;
+        const float4* pa[T];
+        const float4* pb[T];
+#pragma unroll
+        for (uint32_t i = 0; i < T; i++) {
+            pa[i] = r.vec + vrow(min(a0 + i, nn - 1), vstride);
+            pb[i] = r.vec + vrow(min(b0 + i, S - 1), vstride);
+        }
+        float acc[T][T];
+#pragma unroll
+        for (uint32_t i = 0; i < T; i++)
+#pragma unroll
+            for (uint32_t j = 0; j < T; j++) acc[i][j] = 0.f;
+#pragma unroll(T == 1 ? 4 : 1)
+        for (uint32_t c = 0; c < dq; c++) {
+            float4 A[T], B[T];
+#pragma unroll
+            for (uint32_t i = 0; i < T; i++) {
+                A[i] = pa[i][c];
+                B[i] = pb[i][c];
+            }
+#pragma unroll
+            for (uint32_t i = 0; i < T; i++)
+#pragma unroll
+                for (uint32_t j = 0; j < T; j++) {
+                    acc[i][j] = dist_step<M>(acc[i][j], A[i].x, B[j].x);
+                    acc[i][j] = dist_step<M>(acc[i][j], A[i].y, B[j].y);
+                    acc[i][j] = dist_step<M>(acc[i][j], A[i].z, B[j].z);
+                    acc[i][j] = dist_step<M>(acc[i][j], A[i].w, B[j].w);
+                }
+        }
+#pragma unroll
+        for (uint32_t i = 0; i < T; i++) {
+            const uint32_t av = a0 + i;
+            if (av >= nn) continue;
+#pragma unroll
+            for (uint32_t j = 0; j < T; j++) {
+                const uint32_t bv = b0 + j;
+                if (bv >= S || bv <= av) continue;
+                const float dd = acc[i][j];
+                pd[pair_slot(av, bv, nn, no)] = dd;
+                uint32_t outer, inner;
+                if (!pair_order(a.mode, a.verse, av, bv, nn, r.ids[av], r.ids[bv], r.grp[av], r.grp[bv], outer, inner))
+                    continue;
+                cmps++;
+                if (dd < r.kth[outer]) atomicAdd(&r.cnt[outer], 1u);
+                if (dd < r.kth[inner]) atomicAdd(&r.cnt[inner], 1u);
+            }
+        }
+    }
+    return cmps;
+}
+
+template <int M, int TIER>
+__global__ void __launch_bounds__(PS_MAX_THREADS[TIER]) k_pairs_staged(JoinArgs a) {
+    extern __shared__ __align__(16) unsigned char smem[];
+    if (a.ctr->overflow) return;
+    constexpr uint32_t R = TIER_CAP[TIER], T = PS_WARPS[TIER] * 32;
+    const uint32_t grp = T == PS_MAX_THREADS[TIER] ? 0 : threadIdx.x / T, tid = threadIdx.x % T;
+    const uint32_t rpb = T == PS_MAX_THREADS[TIER] ? 1 : blockDim.x / T;
+    const uint32_t dq = a.dp >> 2, vstride = vec_stride(dq);
+    float4* base = reinterpret_cast<float4*>(smem) + (size_t)grp * staged_units(R, dq);
+    uint32_t* s_ids = reinterpret_cast<uint32_t*>(base);
+    float* s_kth = reinterpret_cast<float*>(s_ids + R);
+    uint32_t* s_cnt = reinterpret_cast<uint32_t*>(s_kth + R);
+    uint32_t* s_grp = s_cnt + R;
+    float4* s_vec = reinterpret_cast<float4*>(s_grp + R);
+    const float4* x4 = reinterpret_cast<const float4*>(a.x);
+    const uint32_t vec_base = smem_u32(s_vec);
+    const PairRow pr{s_ids, s_grp, s_kth, s_cnt, s_vec};
+    auto row_sync = [&]() {  // a block of several rows has a warp for each
+        if (T == 32) __syncwarp();
+        else __syncthreads();
+    };
+    const uint32_t cnt = a.ctr->ntier[TIER];
+    const uint32_t* rows = a.tier_rows + (size_t)TIER * a.n;
+    uint32_t cmps = 0, sum_s = 0;
+    for (uint32_t ri = blockIdx.x * rpb + grp; ri < cnt; ri += gridDim.x * rpb) {
+        const uint32_t row = rows[ri];
+        const uint32_t nn = a.newlen[row], no = a.oldlen[row], S = nn + no;
+        for (uint32_t q = tid; q < S; q += T) {
+            const uint32_t e = q < nn ? a.newL[(size_t)row * a.capn + q] : a.oldL[(size_t)row * a.capo + q - nn];
+            const uint32_t id = e & LID_MASK;
+            s_ids[q] = e;
+            s_kth[q] = a.kthv[id];
+            s_cnt[q] = 0;
+            s_grp[q] = a.mode == MODE_SMERGE ? leaf_of(id, a.leaf_off, a.nleaf) : (e >> 31);
+        }
+        row_sync();
+        for (uint32_t i = tid; i < S * dq; i += T) {
+            const uint32_t q = i / dq, c = i - q * dq;
+            cp_async16(vec_base + (vrow(q, vstride) + c) * 16, x4 + (size_t)(s_ids[q] & LID_MASK) * dq + c);
+        }
+        asm volatile("cp.async.wait_all;" ::: "memory");
+        row_sync();
+        if (tid == 0) sum_s += S;
+        float* pd = a.pd + a.poff[row];
+        if (M != CHI2 && tile_count(nn, S, 4) * 4 >= T * 3) cmps += pair_tiles<M, M == CHI2 ? 1 : 4>(a, pr, pd, nn, no, tid, T);
+        else if ((M != CHI2 || TIER > 0) && tile_count(nn, S, 2) * 4 >= T * 3) cmps += pair_tiles<M, 2>(a, pr, pd, nn, no, tid, T);
+        else cmps += pair_tiles<M, 1>(a, pr, pd, nn, no, tid, T);
+        row_sync();
+        for (uint32_t q = tid; q < S; q += T) {
+            const uint32_t c = s_cnt[q];
+            a.cntpos[(size_t)row * a.caps + q] = (uint16_t)c;
+            if (c) atomicAdd(&a.bcnt[s_ids[q] & LID_MASK], c);
+        }
+        row_sync();
+    }
+    for (int o = 16; o > 0; o >>= 1) {
+        cmps += __shfl_xor_sync(FULL, cmps, o);
+        sum_s += __shfl_xor_sync(FULL, sum_s, o);
+    }
+    if ((threadIdx.x & 31) == 0) {
+        if (cmps) atomicAdd(&a.ctr->ncmps, (unsigned long long)cmps);
+        if (sum_s) atomicAdd(&a.ctr->sum_s, (unsigned long long)sum_s);
+    }
+}
 
 template <int M, int VEC>
 __device__ void pairs_row(const JoinArgs& a, uint32_t row, unsigned char* smem, uint32_t R) {
@@ -674,7 +855,7 @@ __device__ void pairs_row(const JoinArgs& a, uint32_t row, unsigned char* smem, 
         if (VEC == VEC_U8) s_nrm[q] = a.nrm[id];
     }
     __syncthreads();
-    if (VEC != VEC_GLOBAL) {
+    if (VEC == VEC_U8) {
         for (uint32_t i = threadIdx.x; i < S * dq; i += blockDim.x) {
             uint32_t q = i / dq, c = i - q * dq;
             s_vec[vrow(q, vstride) + c] = x4[(size_t)(s_ids[q] & LID_MASK) * dq + c];
@@ -698,8 +879,8 @@ __device__ void pairs_row(const JoinArgs& a, uint32_t row, unsigned char* smem, 
 #pragma unroll
         for (int i = 0; i < 4; i++) {
             uint32_t ai = min(ta * 4 + i, nn - 1), bj = min(tb * 4 + i, S - 1);
-            pa[i] = VEC != VEC_GLOBAL ? s_vec + vrow(ai, vstride) : x4 + (size_t)(s_ids[ai] & LID_MASK) * dq;
-            pb[i] = VEC != VEC_GLOBAL ? s_vec + vrow(bj, vstride) : x4 + (size_t)(s_ids[bj] & LID_MASK) * dq;
+            pa[i] = VEC == VEC_U8 ? s_vec + vrow(ai, vstride) : x4 + (size_t)(s_ids[ai] & LID_MASK) * dq;
+            pb[i] = VEC == VEC_U8 ? s_vec + vrow(bj, vstride) : x4 + (size_t)(s_ids[bj] & LID_MASK) * dq;
         }
         float acc[4][4];
         if (VEC == VEC_U8) {
@@ -785,19 +966,20 @@ __device__ void pairs_row(const JoinArgs& a, uint32_t row, unsigned char* smem, 
     __syncthreads();
 }
 
-template <int M, int TIER>
-__global__ void __launch_bounds__(TIER_THREADS[TIER]) k_pairs(JoinArgs a, uint32_t R) {
+// Rows of the last tier, and of tiers whose staged vectors do not fit in
+// shared memory: the vectors read from L2.
+template <int M>
+__global__ void __launch_bounds__(LAST_THREADS) k_pairs_last(JoinArgs a, uint32_t R) {
     extern __shared__ __align__(16) unsigned char smem[];
     if (a.ctr->overflow) return;
-    const uint32_t cnt = a.ctr->ntier[TIER];
-    const uint32_t* rows = a.tier_rows + (size_t)TIER * a.n;
-    for (uint32_t b = blockIdx.x; b < cnt; b += gridDim.x)
-        pairs_row<M, (TIER < NTIER - 1 ? VEC_F32 : VEC_GLOBAL)>(a, rows[b], smem, R);
+    const uint32_t cnt = a.ctr->ntier[NTIER - 1];
+    const uint32_t* rows = a.tier_rows + (size_t)(NTIER - 1) * a.n;
+    for (uint32_t b = blockIdx.x; b < cnt; b += gridDim.x) pairs_row<M, VEC_GLOBAL>(a, rows[b], smem, R);
 }
 
 // Rows of the last tier (S > 128) next to the u8 tensor-core join: the u8
 // vectors staged in shared memory, integer dot products (dp4a).
-__global__ void __launch_bounds__(TIER_THREADS[NTIER - 1]) k_pairs_u8(JoinArgs a, uint32_t R) {
+__global__ void __launch_bounds__(LAST_THREADS) k_pairs_u8(JoinArgs a, uint32_t R) {
     extern __shared__ __align__(16) unsigned char smem[];
     if (a.ctr->overflow) return;
     const uint32_t cnt = a.ctr->ntier[NTIER - 1];
@@ -805,9 +987,9 @@ __global__ void __launch_bounds__(TIER_THREADS[NTIER - 1]) k_pairs_u8(JoinArgs a
     for (uint32_t b = blockIdx.x; b < cnt; b += gridDim.x) pairs_row<L2, VEC_U8>(a, rows[b], smem, R);
 }
 
-// One warp per row: proposals from the stored pair distances.  With the
-// tensor-core join active, only the rows of the last tier have stored pairs.
-constexpr int EMIT_WARPS = 4;
+// Proposals from the stored pair distances: a warp per row of tiers 0-3
+// (FP32 join), a block per row of the last tier.
+constexpr int EMIT_WARPS = 8;
 
 // Members of one row (bucket bases, ids, K-th distances, cursors, groups)
 // in shared memory, 24 bytes a list slot.
@@ -846,58 +1028,71 @@ __device__ __forceinline__ bool emit_load_row(const JoinArgs& a, uint32_t row, u
     return any_c;
 }
 
-// Proposals of the pairs (av, bv) of a row with av = av0, av0 + av_step, ...
-// (a warp's share), lanes over bv; FAST: the fast tier's 8-byte form.
+// Proposals of the row's pairs p = p0, p0 + step, ... in the order of their
+// stored distances (pair_slot), so that every lane of a warp has a pair and
+// the reads are coalesced; FAST: the fast tier's 8-byte form.
 template <bool FAST>
 __device__ __forceinline__ void emit_pairs(const JoinArgs& a, uint32_t row, uint32_t nn, uint32_t no,
-                                           EmitRow m, uint32_t av0, uint32_t av_step) {
-    const int lane = threadIdx.x & 31;
-    const uint32_t S = nn + no;
+                                           EmitRow m, uint32_t p0, uint32_t step) {
+    const uint32_t S = nn + no, tri = nn * (nn - 1) / 2, np = tri + nn * no;
     const unsigned long long* s_base = m.base;
     const uint32_t* s_ids = m.ids;
     const float* s_kth = m.kth;
     uint32_t* s_cur = m.cur;
     const uint32_t* s_grp = m.grp;
     const float* pd = a.pd + a.poff[row];
-    for (uint32_t av = av0; av < nn; av += av_step) {
-        for (uint32_t bv = av + 1 + lane; bv < S; bv += 32) {
-            uint32_t outer, inner;
-            if (!pair_order(a.mode, a.verse, av, bv, nn, s_ids[av], s_ids[bv], s_grp[av], s_grp[bv], outer, inner))
-                continue;
-            const float dd = pd[pair_slot(av, bv, nn, no)];
-            const uint32_t pidx = outer * S + inner;
-            if (dd < s_kth[outer]) {
-                unsigned long long slot = s_base[outer] + atomicAdd(&s_cur[outer], 1u);
-                put_prop<FAST>(a.bucket, slot, dd, s_ids[inner], row, pidx, 0);
+    uint32_t ta = 0, rem = p0;  // new x new: pair `rem` after row ta's first
+    for (uint32_t p = p0; p < np; p += step) {
+        uint32_t av, bv;
+        if (p < tri) {
+            while (rem >= nn - 1 - ta) {
+                rem -= nn - 1 - ta;
+                ta++;
             }
-            if (dd < s_kth[inner]) {
-                unsigned long long slot = s_base[inner] + atomicAdd(&s_cur[inner], 1u);
-                put_prop<FAST>(a.bucket, slot, dd, s_ids[outer], row, pidx, 1);
-            }
+            av = ta;
+            bv = ta + 1 + rem;
+            rem += step;
+        } else {
+            av = (p - tri) / no;
+            bv = nn + (p - tri) - av * no;
+        }
+        const float dd = pd[p];
+        uint32_t outer, inner;
+        if (!pair_order(a.mode, a.verse, av, bv, nn, s_ids[av], s_ids[bv], s_grp[av], s_grp[bv], outer, inner))
+            continue;
+        const uint32_t pidx = outer * S + inner;
+        if (dd < s_kth[outer]) {
+            const unsigned long long slot = s_base[outer] + atomicAdd(&s_cur[outer], 1u);
+            put_prop<FAST>(a.bucket, slot, dd, s_ids[inner], row, pidx, 0);
+        }
+        if (dd < s_kth[inner]) {
+            const unsigned long long slot = s_base[inner] + atomicAdd(&s_cur[inner], 1u);
+            put_prop<FAST>(a.bucket, slot, dd, s_ids[outer], row, pidx, 1);
         }
     }
 }
 
-// FP32 join: a warp per row.
+// FP32 join, rows of tiers 0-3: a warp per row (24 bytes of shared memory a
+// list slot of tier 3; sized for the longest possible list, 22 KB for four
+// warps, it held 40 warps an SM, and each warp's lanes ran over the entries of
+// one outer member at a time, a dozen of them at most in tier 0).
 __global__ void __launch_bounds__(EMIT_WARPS * 32) k_emit(JoinArgs a) {
-    extern __shared__ __align__(16) unsigned char smem[];
+    __shared__ __align__(16) unsigned char smem[EMIT_WARPS][TIER_CAP[3] * 24];
     if (a.ctr->overflow) return;
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const uint32_t row = blockIdx.x * EMIT_WARPS + w;
     if (row >= a.n) return;
     const uint32_t nn = a.newlen[row], no = a.oldlen[row];
-    if (nn == 0) return;
-    const EmitRow m = emit_row_smem(smem + (size_t)w * a.caps * 24, a.caps);
+    if (nn == 0 || a.rtier[row] == NTIER - 1) return;
+    const EmitRow m = emit_row_smem(smem[w], TIER_CAP[3]);
     if (!__any_sync(FULL, emit_load_row(a, row, nn, nn + no, m, lane, 32))) return;
     __syncwarp();
-    if (a.fast_key) emit_pairs<true>(a, row, nn, no, m, 0, 1);
-    else emit_pairs<false>(a, row, nn, no, m, 0, 1);
+    if (a.fast_key) emit_pairs<true>(a, row, nn, no, m, lane, 32);
+    else emit_pairs<false>(a, row, nn, no, m, lane, 32);
 }
 
-// Rows of the last tier next to the tensor-core join (lists of more than
-// 128 entries, up to caps^2 / 2 pairs each, a few thousand rows): a block
-// per row, its warps taking the outer entries in turn, so that no row is a
-// single warp's long chain of loads.
+// Rows of the last tier (up to caps^2 / 2 pairs each, a few thousand rows): a
+// block per row, so that no row is a single warp's long chain of loads.
 constexpr int EMIT_ROW_WARPS = 8;
 
 __global__ void __launch_bounds__(EMIT_ROW_WARPS * 32) k_emit_rows(JoinArgs a) {
@@ -911,8 +1106,8 @@ __global__ void __launch_bounds__(EMIT_ROW_WARPS * 32) k_emit_rows(JoinArgs a) {
         const EmitRow m = emit_row_smem(smem, a.caps);
         const bool any = __syncthreads_or(emit_load_row(a, row, nn, nn + no, m, threadIdx.x, blockDim.x));
         if (any) {
-            if (a.fast_key) emit_pairs<true>(a, row, nn, no, m, threadIdx.x >> 5, EMIT_ROW_WARPS);
-            else emit_pairs<false>(a, row, nn, no, m, threadIdx.x >> 5, EMIT_ROW_WARPS);
+            if (a.fast_key) emit_pairs<true>(a, row, nn, no, m, threadIdx.x, blockDim.x);
+            else emit_pairs<false>(a, row, nn, no, m, threadIdx.x, blockDim.x);
         }
         __syncthreads();  // the row's members in shared memory are read before the next row's load
     }
@@ -1534,12 +1729,8 @@ int graph_alloc(Ctx& ctx, GraphStore& s, GraphDev& g, bool with_carry) {
     return 0;
 }
 
-// Shared memory of a k_pairs block: member arrays (16 B per list slot) and,
-// for the staged tiers, the swizzled vectors.
-static size_t pairs_smem(uint32_t R, uint32_t dp, bool staged) {
-    const uint32_t vstride = vec_stride(dp / 4);
-    return (size_t)R * 16 + (staged ? ((size_t)R * vstride + R / 4 + 1) * 16 : 0) + 64;
-}
+// Shared memory of a k_pairs_last block: the member arrays, 16 B a list slot.
+static size_t pairs_smem(uint32_t R) { return (size_t)R * 16 + 64; }
 
 // k_pairs_u8: the member arrays, the norms, then kq bytes a row.
 static size_t pairs_smem_u8(uint32_t R, uint32_t kq) {
@@ -1547,58 +1738,74 @@ static size_t pairs_smem_u8(uint32_t R, uint32_t kq) {
     return (size_t)R * 16 + (size_t)((R + 3) & ~3u) * 4 + ((size_t)R * vstride + R / 4 + 1) * 16 + 64;
 }
 
+// Launch shape of k_pairs_staged at tier t: as many rows side by side as the
+// block's threads and shared memory (`optin` bytes) hold.
+struct StagedShape {
+    uint32_t rows, threads;
+    size_t smem;
+};
+static StagedShape staged_shape(int t, uint32_t dp, size_t optin) {
+    const size_t row = (size_t)staged_units(TIER_CAP[t], dp / 4) * 16;
+    const uint32_t rows = (uint32_t)std::min<size_t>(PS_MAX_THREADS[t] / (PS_WARPS[t] * 32), optin / row);
+    return {rows, rows * PS_WARPS[t] * 32, rows * row};
+}
+
 // Highest list-size tier whose staged vectors fit in a CTA's shared memory
 // at this dimension (3: all; lower at large d, -1 for none -- those rows
 // take the unstaged kernel of the last tier, with the same sums).
-static int max_staged_tier(uint32_t dp, int device) {
-    int optin = 0;
-    cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, device);
+static int max_staged_tier(uint32_t dp, size_t optin) {
     int t = 0;
-    while (t < NTIER - 1 && pairs_smem(TIER_CAP[t], dp, true) <= (size_t)optin) t++;
+    while (t < NTIER - 1 && staged_shape(t, dp, optin).rows > 0) t++;
     return t - 1;
 }
 
 template <int M>
-static cudaError_t prep_pairs(uint32_t caps, uint32_t dp, size_t emit_smem, int max_staged) {
+static const void* staged_fn(int t) {
+    const void* f[4] = {(const void*)k_pairs_staged<M, 0>, (const void*)k_pairs_staged<M, 1>,
+                        (const void*)k_pairs_staged<M, 2>, (const void*)k_pairs_staged<M, 3>};
+    return f[t];
+}
+
+template <int M>
+static cudaError_t prep_pairs(uint32_t caps, uint32_t dp, size_t optin, int max_staged) {
     cudaError_t e;
-    if (max_staged >= 0 && (e = cudaFuncSetAttribute(k_pairs<M, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                     (int)pairs_smem(TIER_CAP[0], dp, true))) != cudaSuccess) return e;
-    if (max_staged >= 1 && (e = cudaFuncSetAttribute(k_pairs<M, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                     (int)pairs_smem(TIER_CAP[1], dp, true))) != cudaSuccess) return e;
-    if (max_staged >= 2 && (e = cudaFuncSetAttribute(k_pairs<M, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                     (int)pairs_smem(TIER_CAP[2], dp, true))) != cudaSuccess) return e;
-    if (max_staged >= 3 && (e = cudaFuncSetAttribute(k_pairs<M, 3>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                     (int)pairs_smem(TIER_CAP[3], dp, true))) != cudaSuccess) return e;
-    if ((e = cudaFuncSetAttribute(k_pairs<M, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (int)pairs_smem(caps, dp, false))) != cudaSuccess) return e;
-    if ((e = cudaFuncSetAttribute(k_emit_rows, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(caps * 24 + 64))) !=
-        cudaSuccess)
+    for (int t = 0; t <= max_staged; t++)
+        if ((e = cudaFuncSetAttribute(staged_fn<M>(t), cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                      (int)staged_shape(t, dp, optin).smem)) != cudaSuccess)
+            return e;
+    if ((e = cudaFuncSetAttribute(k_pairs_last<M>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  (int)pairs_smem(caps))) != cudaSuccess)
         return e;
-    return cudaFuncSetAttribute(k_emit, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)emit_smem);
+    return cudaFuncSetAttribute(k_emit_rows, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(caps * 24 + 64));
 }
 
 // FP32 pair kernels: all tiers, or only the last one when the tensor-core
 // join takes the others.
 template <int M>
 static void launch_pairs(const JoinArgs& ja, const unsigned* ntier, const unsigned* full, uint32_t caps, uint32_t dp,
-                         int nsm, bool last_only, bool u8_last, bool u8_tc, cudaStream_t st) {
+                         size_t optin, int nsm, bool last_only, bool u8_last, bool u8_tc, cudaStream_t st) {
     // grids: the host's row counts, or (ntier null) full -- every block that
     // fits on the SMs at once, looping over the rows counted on the device
-    const unsigned* g = ntier ? ntier : full;
+    auto staged = [&](int t, auto fn) {
+        if (!full[t] || (ntier && !ntier[t])) return;
+        const StagedShape s = staged_shape(t, dp, optin);
+        const unsigned blocks = ntier ? std::min(full[t], (ntier[t] + s.rows - 1) / s.rows) : full[t];
+        fn<<<blocks, s.threads, s.smem, st>>>(ja); count_launch();
+    };
     if (!last_only) {
-        if (g[0]) { k_pairs<M, 0><<<g[0], TIER_THREADS[0], pairs_smem(TIER_CAP[0], dp, true), st>>>(ja, TIER_CAP[0]); count_launch(); }
-        if (g[1]) { k_pairs<M, 1><<<g[1], TIER_THREADS[1], pairs_smem(TIER_CAP[1], dp, true), st>>>(ja, TIER_CAP[1]); count_launch(); }
-        if (g[2]) { k_pairs<M, 2><<<g[2], TIER_THREADS[2], pairs_smem(TIER_CAP[2], dp, true), st>>>(ja, TIER_CAP[2]); count_launch(); }
-        if (g[3]) { k_pairs<M, 3><<<g[3], TIER_THREADS[3], pairs_smem(TIER_CAP[3], dp, true), st>>>(ja, TIER_CAP[3]); count_launch(); }
+        staged(0, k_pairs_staged<M, 0>);
+        staged(1, k_pairs_staged<M, 1>);
+        staged(2, k_pairs_staged<M, 2>);
+        staged(3, k_pairs_staged<M, 3>);
     }
     if (u8_tc) {  // the last tier on the tensor cores
         launch_pairs_tc(ja, caps, ntier, nsm, st);
         return;
     }
-    if (g[4]) {
-        const unsigned blocks = std::min(g[4], full[4]);
-        if (u8_last) k_pairs_u8<<<blocks, TIER_THREADS[4], pairs_smem_u8(caps, ja.kq), st>>>(ja, caps);
-        else k_pairs<M, 4><<<blocks, TIER_THREADS[4], pairs_smem(caps, dp, false), st>>>(ja, caps);
+    const unsigned blocks = ntier ? std::min(ntier[4], full[4]) : full[4];
+    if (blocks) {
+        if (u8_last) k_pairs_u8<<<blocks, LAST_THREADS, pairs_smem_u8(caps, ja.kq), st>>>(ja, caps);
+        else k_pairs_last<M><<<blocks, LAST_THREADS, pairs_smem(caps), st>>>(ja, caps);
         count_launch();
     }
 }
@@ -1613,17 +1820,16 @@ static unsigned resident_blocks(F fn, int threads, size_t smem, int nsm) {
 // launch_pairs' full grids; 0 for a tier that has no rows (its vectors do
 // not fit in shared memory, or the tensor-core join takes it).
 template <int M>
-static void pair_grids(uint32_t caps, uint32_t dp, uint32_t kq, int nsm, bool last_only, bool u8_last, int max_staged,
-                       unsigned* g) {
-    auto staged = [&](int t, auto fn) {
-        return last_only || t > max_staged ? 0u : resident_blocks(fn, TIER_THREADS[t], pairs_smem(TIER_CAP[t], dp, true), nsm);
-    };
-    g[0] = staged(0, k_pairs<M, 0>);
-    g[1] = staged(1, k_pairs<M, 1>);
-    g[2] = staged(2, k_pairs<M, 2>);
-    g[3] = staged(3, k_pairs<M, 3>);
-    g[4] = u8_last ? resident_blocks(k_pairs_u8, TIER_THREADS[4], pairs_smem_u8(caps, kq), nsm)
-                   : resident_blocks(k_pairs<M, 4>, TIER_THREADS[4], pairs_smem(caps, dp, false), nsm);
+static void pair_grids(uint32_t caps, uint32_t dp, uint32_t kq, size_t optin, int nsm, bool last_only, bool u8_last,
+                       int max_staged, unsigned* g) {
+    for (int t = 0; t < 4; t++) {
+        g[t] = 0;
+        if (last_only || t > max_staged) continue;
+        const StagedShape s = staged_shape(t, dp, optin);
+        g[t] = resident_blocks(staged_fn<M>(t), (int)s.threads, s.smem, nsm);
+    }
+    g[4] = u8_last ? resident_blocks(k_pairs_u8, LAST_THREADS, pairs_smem_u8(caps, kq), nsm)
+                   : resident_blocks(k_pairs_last<M>, LAST_THREADS, pairs_smem(caps), nsm);
 }
 
 // Sequential float mean of the per-row deltas, as the reference computes it
@@ -1674,11 +1880,13 @@ int run_nndescent(Ctx& ctx, GraphDev& g, JoinMode mode, uint32_t split, uint32_t
     uint64_t* scan_tmp = P<uint64_t>(ws.scan_tmp);
     IterCounters* ctr = P<IterCounters>(ws.counters);
 
-    const size_t emit_smem = (size_t)EMIT_WARPS * caps * 24 + 64;
-    const int max_staged = max_staged_tier(g.dp, ctx.device);
-    cudaError_t ae = g.metric == L2 ? prep_pairs<L2>(caps, g.dp, emit_smem, max_staged)
-                     : g.metric == L1 ? prep_pairs<L1>(caps, g.dp, emit_smem, max_staged)
-                                      : prep_pairs<CHI2>(caps, g.dp, emit_smem, max_staged);
+    int optin_i = 0;
+    NNM_CUDA_TRY(cudaDeviceGetAttribute(&optin_i, cudaDevAttrMaxSharedMemoryPerBlockOptin, ctx.device));
+    const size_t optin = (size_t)optin_i;
+    const int max_staged = max_staged_tier(g.dp, optin);
+    cudaError_t ae = g.metric == L2 ? prep_pairs<L2>(caps, g.dp, optin, max_staged)
+                     : g.metric == L1 ? prep_pairs<L1>(caps, g.dp, optin, max_staged)
+                                      : prep_pairs<CHI2>(caps, g.dp, optin, max_staged);
     NNM_CUDA_TRY(ae);
     NNM_CUDA_TRY(ws.npairs.ensure(n1 * 4));
     NNM_CUDA_TRY(ws.poff.ensure(n1 * 8));
@@ -1691,13 +1899,11 @@ int run_nndescent(Ctx& ctx, GraphDev& g, JoinMode mode, uint32_t split, uint32_t
     if (tc) {
         NNM_CUDA_TRY(tc_set_attributes(g.kq, g.tc_kind));
         NNM_CUDA_TRY(ws.erows.ensure((size_t)n * 4 * 4 + 16));
-        int optin = 0;
-        NNM_CUDA_TRY(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, ctx.device));
         const size_t u8_smem = pairs_smem_u8(caps, g.kq);
-        u8_last = g.tc_kind == 0 && g.metric == L2 && u8_smem <= (size_t)optin;
+        u8_last = g.tc_kind == 0 && g.metric == L2 && u8_smem <= optin;
         if (u8_last)
             NNM_CUDA_TRY(cudaFuncSetAttribute(k_pairs_u8, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)u8_smem));
-        u8_tc = u8_last && pairs_tc_smem(caps, g.kq) <= (size_t)optin;
+        u8_tc = u8_last && pairs_tc_smem(caps, g.kq) <= optin;
         if (u8_tc) NNM_CUDA_TRY(pairs_tc_set_attributes(caps, g.kq));
     }
 
@@ -1706,10 +1912,10 @@ int run_nndescent(Ctx& ctx, GraphDev& g, JoinMode mode, uint32_t split, uint32_t
     std::vector<uint8_t> h_nflag;
 
     unsigned full[NTIER], emit_rows_full = 0;
-    if (g.metric == L2) pair_grids<L2>(caps, g.dp, g.kq, nsm, tc, u8_last, max_staged, full);
-    else if (g.metric == L1) pair_grids<L1>(caps, g.dp, g.kq, nsm, tc, false, max_staged, full);
-    else pair_grids<CHI2>(caps, g.dp, g.kq, nsm, tc, false, max_staged, full);
-    if (tc) emit_rows_full = resident_blocks(k_emit_rows, EMIT_ROW_WARPS * 32, (size_t)caps * 24 + 64, nsm);
+    if (g.metric == L2) pair_grids<L2>(caps, g.dp, g.kq, optin, nsm, tc, u8_last, max_staged, full);
+    else if (g.metric == L1) pair_grids<L1>(caps, g.dp, g.kq, optin, nsm, tc, false, max_staged, full);
+    else pair_grids<CHI2>(caps, g.dp, g.kq, optin, nsm, tc, false, max_staged, full);
+    emit_rows_full = resident_blocks(k_emit_rows, EMIT_ROW_WARPS * 32, (size_t)caps * 24 + 64, nsm);
     // a buffer grown with headroom, or without where that does not fit
     auto grow = [&](DevBuf& b, uint64_t elems, size_t each, double room) -> cudaError_t {
         cudaError_t e = b.ensure((size_t)((double)elems * room + 1024) * each);
@@ -1786,7 +1992,8 @@ int run_nndescent(Ctx& ctx, GraphDev& g, JoinMode mode, uint32_t split, uint32_t
             ShufArgs sh = shuf_args();
             sh.phase_dev = phase_dev;
             if (g.fast) k_shuffle_fast<<<warp_blocks, 256, 0, st>>>(sh);
-            else k_shuffle_exact<<<warp_blocks, SHUFX_WARPS * 32, 0, st>>>(sh);
+            else if (g.repeats) k_shuffle_exact<true><<<warp_blocks, SHUFX_WARPS * 32, 0, st>>>(sh);
+            else k_shuffle_exact<false><<<warp_blocks, SHUFX_WARPS * 32, 0, st>>>(sh);
             count_launch();
             k_tier_lists<<<(n + TIER_CHUNK - 1) / TIER_CHUNK, 256, 0, st>>>(P<uint8_t>(ws.rtier), n,
                                                                            P<uint32_t>(ws.tiers), ctr); count_launch();
@@ -1812,7 +2019,7 @@ int run_nndescent(Ctx& ctx, GraphDev& g, JoinMode mode, uint32_t split, uint32_t
                             P<float>(ws.pd), P<uint16_t>(ws.cntpos), P<uint32_t>(ws.bcnt), P<uint32_t>(ws.bcur),
                             P<uint64_t>(ws.boff), ws.bucket.p, ctr,
                             g.xq, g.nrm, g.kq, tc ? 1u : 0u, &ctr->error, tc ? P<uint32_t>(ws.erows) : nullptr,
-                            g.fast ? 1u : 0u, g.tc_kind, g.err_c, g.scl, g.audit ? 1u : 0u, P<float>(ws.kth)};
+                            g.fast ? 1u : 0u, g.tc_kind, g.err_c, g.scl, g.audit ? 1u : 0u, P<float>(ws.kth), P<uint8_t>(ws.rtier)};
         };
         // local join, pass 1: per-target proposal counts (and, on the FP32
         // path, the stored pair distances), then the bucket offsets.  nt:
@@ -1823,9 +2030,9 @@ int run_nndescent(Ctx& ctx, GraphDev& g, JoinMode mode, uint32_t split, uint32_t
             rec(0);
             if (tc) e = launch_join_tc(0, ja, nt, nsm, st);
             if (e == cudaSuccess) {
-                if (g.metric == L2) launch_pairs<L2>(ja, nt, full, caps, g.dp, nsm, tc, u8_last, u8_tc, st);
-                else if (g.metric == L1) launch_pairs<L1>(ja, nt, full, caps, g.dp, nsm, tc, false, false, st);
-                else launch_pairs<CHI2>(ja, nt, full, caps, g.dp, nsm, tc, false, false, st);
+                if (g.metric == L2) launch_pairs<L2>(ja, nt, full, caps, g.dp, optin, nsm, tc, u8_last, u8_tc, st);
+                else if (g.metric == L1) launch_pairs<L1>(ja, nt, full, caps, g.dp, optin, nsm, tc, false, false, st);
+                else launch_pairs<CHI2>(ja, nt, full, caps, g.dp, optin, nsm, tc, false, false, st);
                 rec(1);
                 ScanJobs bj{};
                 bj.j[0] = ScanJob{P<uint32_t>(ws.bcnt), nullptr, P<uint64_t>(ws.boff),
@@ -1842,13 +2049,12 @@ int run_nndescent(Ctx& ctx, GraphDev& g, JoinMode mode, uint32_t split, uint32_t
             rec(2);
             if (tc) e = launch_join_tc(1, ja, nt, nsm, st);
             if (e != cudaSuccess) return e;
-            if (tc) {
-                const unsigned rows4 = nt ? nt[NTIER - 1] : emit_rows_full;
-                if (rows4) {
-                    k_emit_rows<<<rows4, EMIT_ROW_WARPS * 32, (size_t)caps * 24 + 64, st>>>(ja); count_launch();
-                }
-            } else if (n > 0) {
-                k_emit<<<(n + EMIT_WARPS - 1) / EMIT_WARPS, EMIT_WARPS * 32, emit_smem, st>>>(ja); count_launch();
+            if (!tc) {
+                k_emit<<<(n + EMIT_WARPS - 1) / EMIT_WARPS, EMIT_WARPS * 32, 0, st>>>(ja); count_launch();
+            }
+            const unsigned rows4 = nt ? std::min(nt[NTIER - 1], emit_rows_full) : emit_rows_full;
+            if (rows4) {
+                k_emit_rows<<<rows4, EMIT_ROW_WARPS * 32, (size_t)caps * 24 + 64, st>>>(ja); count_launch();
             }
             MergeArgs ma{g.pid, g.pdist, n, K, P<uint32_t>(ws.bcnt), P<uint64_t>(ws.boff),
                          ja.bucket, P<uint8_t>(ws.nflag), ctr, g.x, g.dp, g.nrm, g.err_c, ctx.prof ? 1u : 0u};

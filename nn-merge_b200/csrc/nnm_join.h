@@ -13,7 +13,7 @@ namespace nnm {
 // join packs 8, 4, 2 or 1 rows of the first four tiers into one 128-slot tile.
 constexpr int NTIER = 5;
 constexpr uint32_t TIER_CAP[4] = {16, 32, 64, 128};
-constexpr int TIER_THREADS[NTIER] = {64, 64, 64, 128, 128};
+constexpr int LAST_THREADS = 512;  // threads per row of the last tier's pair kernels
 constexpr uint32_t TC_MAX_S = 128;  // rows the tensor-core join takes
 
 __host__ __device__ __forceinline__ int tier_of(uint32_t S) {
@@ -51,6 +51,7 @@ struct JoinArgs {
     const float* scl;     // FP8: per-row inverse scales
     uint32_t audit;       // reduced precision: check every pair's d~ against its exact distance
     const float* kthv;    // every row's K-th distance at the iteration's start (compact copy of pdist's)
+    const uint8_t* rtier; // every row's tier (0xff: not joined)
 };
 
 // Tie-break key of the exact tier's proposal "target gets the other entry"
