@@ -8,6 +8,7 @@
 namespace nnm {
 
 constexpr uint32_t SEARCH_MAX_BEAM = 1024;
+constexpr size_t INDEX_IO_BYTES = 256 * 1024;  // IndexDev::h_io
 
 // Device state of LyNNDescent::graph, which the reference never clears
 // between layers (lynndescent.cpp:644): each layer starts from the previous
@@ -48,6 +49,10 @@ struct IndexDev {
     DevEntry* net = nullptr;                   // entry network, owned
     uint32_t nprobe = 0, entry_layer = 0, n_classes = 0;
     uint32_t width = 4;  // fast kernel: most unexpanded entries expanded together
+    // small batches from host memory: queries, beams, counters and results
+    // pass through this pinned block, so that a call waits for the device once
+    unsigned char* h_io = nullptr;
+    cudaEvent_t ev[3] = {};
     void release();
 };
 
@@ -75,8 +80,10 @@ int index_run_fast(Ctx& ctx, IndexDev& ix, const SearchReq& r);
 // Seeds of nndFlatSrch for every beam width up to beam_max (cached).
 int index_flat_seeds(Ctx& ctx, IndexDev& ix, uint32_t beam_max);
 // Waits for the stream, reads the distance and expansion counts of the last
-// run and turns its self-check flags into an error.
+// run and turns its self-check flags into an error.  index_check: the same on
+// the counters' 24 bytes once they are in host memory.
 int index_counters(Ctx& ctx, IndexDev& ix, uint64_t* ncmps, uint64_t* nexp);
+int index_check(Ctx& ctx, const unsigned long long* c, uint64_t* ncmps, uint64_t* nexp);
 
 int search_host(Ctx& ctx, const float* x, uint64_t n, uint32_t d, const nnm_layers* layers, const float* q,
                 uint64_t nq, uint32_t topk, uint32_t seed, int metric, uint32_t* out_ids, float* out_dists,

@@ -454,7 +454,8 @@ int index_run_exact(Ctx& ctx, IndexDev& ix, const SearchReq& r) {
     NNM_CUDA_TRY(cudaFuncSetAttribute(k_search, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     int per_sm = 1;
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_search, SWARPS * 32, smem);
-    const uint32_t blocks = (uint32_t)std::min(std::max(1, per_sm), 4) * (uint32_t)nsm;
+    const uint32_t blocks = std::min((uint32_t)std::min(std::max(1, per_sm), 4) * (uint32_t)nsm,
+                                     (r.nq + SWARPS - 1) / SWARPS);
     const uint32_t words = (uint32_t)((ix.n + 31) / 32);
     const size_t slots = (size_t)blocks * SWARPS;
     if (ix.visited.bytes < slots * words * 4) {
@@ -549,6 +550,10 @@ int index_counters(Ctx& ctx, IndexDev& ix, uint64_t* ncmps, uint64_t* nexp) {
     unsigned long long c[3] = {0, 0, 0};
     NNM_CUDA_TRY(cudaMemcpyAsync(c, ix.ctr.p, 24, cudaMemcpyDeviceToHost, ctx.stream));
     NNM_CUDA_TRY(cudaStreamSynchronize(ctx.stream));
+    return index_check(ctx, c, ncmps, nexp);
+}
+
+int index_check(Ctx& ctx, const unsigned long long* c, uint64_t* ncmps, uint64_t* nexp) {
     if (ncmps) *ncmps = c[1];
     if (nexp) *nexp = c[2];
     const unsigned serr = (unsigned)(c[0] >> 32);  // bytes 4..7
@@ -565,6 +570,12 @@ void IndexDev::release() {
     DevBuf* all[] = {&x,     &off,   &adj,  &visited, &vlist,  &cand,     &ctr,      &qpad,
                      &beams, &probes, &hid, &scores,  &out,    &flat_off, &flat_pool};
     for (auto* b : all) b->release();
+    if (h_io) cudaFreeHost(h_io);
+    h_io = nullptr;
+    for (auto& e : ev) {
+        if (e) cudaEventDestroy(e);
+        e = nullptr;
+    }
 }
 
 int search_host(Ctx& ctx, const float* x, uint64_t n, uint32_t d, const nnm_layers* layers, const float* q,

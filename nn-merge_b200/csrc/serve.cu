@@ -76,6 +76,7 @@ struct ServeArgs {
     unsigned* overflow;
     unsigned long long* ncmps;
     unsigned long long* nexp;
+    uint32_t spec_blocks;  // k_serve_team: prefetch the next list's rows with at most this many blocks
 };
 
 template <int M>
@@ -514,10 +515,533 @@ __global__ void __launch_bounds__(FW * 32, 5) k_serve(ServeArgs a) {
     }
 }
 
+// A few queries: a block per query (k_serve_team).  The steps, the beam and
+// the counts are k_serve's; what a step waits for is shared or taken off the
+// chain, since one warp alone spends a step of 20 fresh rows in three
+// dependent batches of row reads and two round trips to L2 for the offsets,
+// the list and the visited bits:
+//   - warp 0 leads; a batch of up to 32 rows is measured by the four warps at
+//     once, eight rows each (two block barriers a batch);
+//   - the visited bitmap lies in shared memory (cleared per query);
+//   - the helpers prefetch what later steps read: the fresh rows' offsets and
+//     lists, and (no more blocks than SMs) the rows of the list that is
+//     expanded next if no nearer entry turns up;
+//   - accepted rows are placed by rank (one shuffle pair per accepted row)
+//     instead of a 15-stage sort.
+// Sums have the same tree as warp_dists', so the results are the same bits.
+// Bound: the latency of the leader's chain, 4,900 cycles a step of which the
+// row reads are 1,900 (2,600 without the prefetched rows).  Beam 64,
+// 100,000 x 128 rows, device time against k_serve's: 1 query 250 -> 155 us,
+// 148 queries 415 -> 239, 592 queries 489 -> 288; faster as long as every
+// query has a resident block (740 here: 472 -> 296), which is the rule that
+// picks it.  The beam in registers (up to 192 entries) against shared memory:
+// 177 -> 155 us.
+constexpr int TEAM = 4;
+
+__device__ __forceinline__ void prefetch_l1(const void* p) { asm volatile("prefetch.global.L1 [%0];" ::"l"(p)); }
+
+// Distances to rows [first, first + 8) of the cnt <= 32 ids that the lanes
+// hold, into out[0, 8) (shared memory).  NB rows at a time are summed by a
+// transposing butterfly (NB - 1 + 5 - log2 NB shuffles).
+template <int M, int QV>
+__device__ __forceinline__ void team_rows(const float4 (&qr)[QV], const float4* __restrict__ x4, uint32_t dp4,
+                                          uint32_t fid, uint32_t first, uint32_t cnt, uint32_t lane, float* out) {
+    constexpr uint32_t NB = QV == 1 ? 8 : (QV == 2 ? 4 : 2);  // rows in flight per lane
+#pragma unroll
+    for (uint32_t b0 = 0; b0 < 8; b0 += NB) {
+        if (first + b0 >= cnt) break;
+        float4 r[NB][QV];
+#pragma unroll
+        for (uint32_t b = 0; b < NB; b++) {
+            const uint32_t id = __shfl_sync(FULL, fid, (first + b0 + b) & 31);
+#pragma unroll
+            for (int t = 0; t < QV; t++) {
+                const uint32_t c4 = lane + 32u * t;
+                r[b][t] = make_float4(0.f, 0.f, 0.f, 0.f);
+                if (first + b0 + b < cnt && c4 < dp4) r[b][t] = __ldg(x4 + (size_t)id * dp4 + c4);
+            }
+        }
+        float v[NB];
+#pragma unroll
+        for (uint32_t b = 0; b < NB; b++) {
+            v[b] = 0.f;
+#pragma unroll
+            for (int t = 0; t < QV; t++) v[b] = part4<M>(qr[t], r[b][t], v[b]);
+        }
+        uint32_t s = 16;
+#pragma unroll
+        for (uint32_t n = NB / 2; n >= 1; n >>= 1, s >>= 1) {
+            const bool up = (lane & s) != 0;
+#pragma unroll
+            for (uint32_t i = 0; i < n; i++) {
+                const float send = up ? v[i] : v[i + n], keep = up ? v[i + n] : v[i];
+                v[i] = keep + __shfl_xor_sync(FULL, send, s);
+            }
+        }
+#pragma unroll
+        for (; s >= 1; s >>= 1) v[0] += __shfl_xor_sync(FULL, v[0], s);
+        constexpr uint32_t PER = 32 / NB;  // lanes b PER .. hold row b
+        if ((lane & (PER - 1)) == 0) out[b0 + lane / PER] = v[0];
+    }
+}
+
+__host__ __device__ constexpr size_t team_words(uint32_t words) { return ((size_t)words + 3) & ~(size_t)3; }
+__host__ __device__ constexpr size_t team_smem(uint32_t words, uint32_t cap) {
+    return (team_words(words) + (size_t)cap * 4 + 4 * 32 + GROUP * 32 + 8) * 4;
+}
+
+// A batch handed to the helpers; cnt 0: the query is done.
+struct TeamCmd {
+    uint32_t cnt, next;  // ids of the batch; entry likely expanded next (or ~0)
+};
+
+// ER > 0: the beam (at most 32 ER entries) in the leader's registers, entry i
+// in slot i / 32 of lane i % 32; 0: in shared memory, placed by binary search.
+template <int M, int QV, int ER>
+__global__ void __launch_bounds__(TEAM * 32) k_serve_team(ServeArgs a) {
+    extern __shared__ __align__(16) unsigned char smem[];
+    const uint32_t tid = threadIdx.x, w = tid >> 5, lane = tid & 31;
+    uint32_t* vis = reinterpret_cast<uint32_t*>(smem);
+    float* bd = reinterpret_cast<float*>(vis + team_words(a.words));
+    uint32_t* bi = reinterpret_cast<uint32_t*>(bd + a.cap);
+    float* td = reinterpret_cast<float*>(bi + a.cap);
+    uint32_t* ti = reinterpret_cast<uint32_t*>(td + a.cap);
+    float* nd = reinterpret_cast<float*>(ti + a.cap);
+    uint32_t* ni = reinterpret_cast<uint32_t*>(nd + 32);
+    float* raw = reinterpret_cast<float*>(ni + 32);              // the batch's distances
+    uint32_t* ids = reinterpret_cast<uint32_t*>(raw + 32);       // the batch's ids
+    uint32_t* fr = ids + 32;                                     // fresh ids of a group
+    TeamCmd* cmd = reinterpret_cast<TeamCmd*>(fr + GROUP * 32);  // two, in turn
+    const float4* x4 = reinterpret_cast<const float4*>(a.x);
+    const uint32_t nlast = a.nrows[a.L - 1];
+    const uint64_t* off_last = a.off_all + a.off_base[a.L - 1];
+    const bool spec = gridDim.x <= a.spec_blocks;
+    unsigned long long cmps = 0, nexp = 0;
+    for (uint32_t qi = blockIdx.x; qi < a.nq; qi += gridDim.x) {
+        for (uint32_t i = tid; i < team_words(a.words) / 4; i += TEAM * 32)
+            reinterpret_cast<uint4*>(vis)[i] = make_uint4(0u, 0u, 0u, 0u);
+        float4 qr[QV];
+#pragma unroll
+        for (int t = 0; t < QV; t++) {
+            const uint32_t c4 = lane + 32u * t;
+            qr[t] = c4 < a.dp4 ? __ldg(reinterpret_cast<const float4*>(a.q) + (size_t)qi * a.dp4 + c4)
+                               : make_float4(0.f, 0.f, 0.f, 0.f);
+        }
+        __syncthreads();  // the bitmap is clear
+        uint32_t turn = 0;
+        if (w > 0) {  // helpers
+            for (;; turn ^= 1) {
+                __syncthreads();  // a batch is posted
+                const TeamCmd c = cmd[turn];
+                if (c.cnt == 0) break;
+                const uint32_t fid = lane < c.cnt ? ids[lane] : 0u;
+                team_rows<M, QV>(qr, x4, a.dp4, fid, 8 * w, c.cnt, lane, raw + 8 * w);
+                __syncthreads();  // the batch is measured
+                if (w == TEAM - 1) {
+                    if (lane < c.cnt && fid < nlast) {
+                        const uint64_t b = off_last[fid], e = off_last[fid + 1];
+                        for (uint64_t t = b; t < e; t += 32) prefetch_l1(a.adj_all + t);
+                        if (e > b) prefetch_l1(a.adj_all + e - 1);
+                    }
+                } else if (spec) {
+                    // the rows of the list that the next step reads, of one of
+                    // two entries: the first open one, or the nearest of this batch
+                    uint32_t cand = c.next;
+                    if (w == 1) {
+                        const uint32_t u = lane < c.cnt ? __float_as_uint(raw[lane]) : 0u;
+                        const uint32_t key = lane < c.cnt ? (u >> 31 ? ~u : u | 0x80000000u) : 0xffffffffu;
+                        const unsigned at = __ballot_sync(FULL, key == __reduce_min_sync(FULL, key));
+                        cand = __shfl_sync(FULL, fid, __ffs(at) - 1);
+                    }
+                    if (cand < nlast) {
+                        const uint64_t b = off_last[cand], e = off_last[cand + 1];
+                        if (b + lane < e) {
+                            const uint32_t id = a.adj_all[b + lane];
+                            if (!(vis[id >> 5] >> (id & 31) & 1u)) {  // a hint: the leader may be setting bits
+                                const float4* r = x4 + (size_t)id * a.dp4;
+                                for (uint32_t t = 0; t < a.dp4; t += 8) prefetch_l1(r + t);
+                            }
+                        }
+                    }
+                }
+            }
+            __syncthreads();  // the results are out
+            continue;
+        }
+        // leader
+        uint32_t ef = a.beams ? a.beams[qi] : a.beam;
+        if (ef < a.out_k || ef > a.cap) {
+            if (lane == 0) atomicOr(a.overflow, FERR_BEAM_RANGE);
+            ef = min(max(ef, a.out_k), a.cap);
+        }
+        const uint32_t width = max(1u, min(a.width, ef / 64));
+        // distances of the cnt <= 32 ids in the lanes
+        auto dists = [&](uint32_t fid, uint32_t cnt, uint32_t next) -> float {
+            if (lane < cnt) ids[lane] = fid;
+            if (lane == 0) cmd[turn] = TeamCmd{cnt, next};
+            turn ^= 1;
+            __syncthreads();
+            team_rows<M, QV>(qr, x4, a.dp4, fid, 0, cnt, lane, raw);
+            __syncthreads();
+            return raw[lane];
+        };
+        uint32_t cur = 0, g0;
+        float cur_d = 0.f;
+        if (a.flat) {
+            g0 = a.L - 1;
+        } else if (a.probes) {
+            g0 = a.g0;
+            uint32_t pid = 0;
+            if (lane < a.nprobe) {
+                pid = a.probes[(size_t)qi * a.nprobe + lane];
+                if (pid >= a.nrows[g0]) {
+                    atomicOr(a.overflow, FERR_BAD_ID);
+                    pid = 0;
+                }
+            }
+            uint32_t l;
+            warp_argmin(dists(pid, a.nprobe, ~0u), a.nprobe, lane, cur_d, l);
+            cur = __shfl_sync(FULL, pid, l & 31);
+            cmps += a.nprobe;
+        } else {
+            g0 = 0;
+            cur = a.entry;
+            cur_d = __shfl_sync(FULL, dists(cur, 1, ~0u), 0);
+            cmps++;
+        }
+        // greedy descent, as k_serve
+        for (uint32_t g = g0; g + 1 < a.L; g++) {
+            const uint64_t* off = a.off_all + a.off_base[g];
+            uint32_t moves = 0;
+            for (;;) {
+                if (cur >= a.nrows[g] || ++moves > a.nrows[g]) {
+                    if (lane == 0) atomicOr(a.overflow, cur >= a.nrows[g] ? FERR_BAD_ID : FERR_LOOP);
+                    cur = 0;
+                    break;
+                }
+                const uint64_t b = off[cur], e = off[cur + 1];
+                float best = cur_d;
+                uint32_t bid = cur;
+                for (uint64_t c0 = b; c0 < e; c0 += 32) {
+                    const uint32_t cnt = (uint32_t)(e - c0 < 32 ? e - c0 : 32);
+                    const uint32_t nn = lane < cnt ? a.adj_all[c0 + lane] : 0u;
+                    if (lane < cnt) prefetch_l1(off + nn);
+                    const float dd = dists(nn, cnt, ~0u);
+                    cmps += cnt;
+                    float md;
+                    uint32_t ml;
+                    warp_argmin(dd, cnt, lane, md, ml);
+                    const uint32_t mid = __shfl_sync(FULL, nn, ml & 31);
+                    if (md < best) {
+                        best = md;
+                        bid = mid;
+                    }
+                }
+                if (bid == cur) break;
+                cur = bid;
+                cur_d = best;
+            }
+        }
+        uint32_t m = 0, p = 0;
+        constexpr int ES = ER ? ER : 1;
+        float rd[ES];
+        uint32_t ri[ES];
+#pragma unroll
+        for (int r = 0; r < ES; r++) {
+            rd[r] = INFINITY;
+            ri[r] = 0xffffffffu;
+        }
+        // the first unexpanded entry from s0 on (its position; m: none)
+        auto first_open = [&](uint32_t s0) -> uint32_t {
+            if (ER) {
+                uint32_t at = m;
+#pragma unroll
+                for (int r = ES - 1; r >= 0; r--) {
+                    const uint32_t i = 32u * r + lane;
+                    const unsigned bal = __ballot_sync(FULL, i >= s0 && i < m && !(ri[r] & EXP_BIT));
+                    if (bal) at = 32u * r + __ffs(bal) - 1;
+                }
+                return at;
+            }
+            for (; s0 < m; s0 += 32) {
+                const unsigned bal = __ballot_sync(FULL, s0 + lane < m && !(bi[s0 + lane] & EXP_BIT));
+                if (bal) return s0 + __ffs(bal) - 1;
+            }
+            return m;
+        };
+        // id word of entry `at` < m
+        auto id_at = [&](uint32_t at) -> uint32_t {
+            if (!ER) return bi[at];
+            uint32_t v = ri[0];
+#pragma unroll
+            for (int r = 1; r < ES; r++)
+                if ((at >> 5) == (uint32_t)r) v = ri[r];
+            return __shfl_sync(FULL, v, at & 31);
+        };
+        auto dist_at = [&](uint32_t at) -> float {
+            if (!ER) return bd[at];
+            float v = rd[0];
+#pragma unroll
+            for (int r = 1; r < ES; r++)
+                if ((at >> 5) == (uint32_t)r) v = rd[r];
+            return __shfl_sync(FULL, v, at & 31);
+        };
+        auto mark = [&](uint32_t at) {
+            if (ER) {
+#pragma unroll
+                for (int r = 0; r < ES; r++)
+                    if (at == 32u * r + lane) ri[r] |= EXP_BIT;
+            } else {
+                __syncwarp();
+                if (lane == 0) bi[at] |= EXP_BIT;
+                __syncwarp();
+            }
+        };
+        // k_serve's offer; next: see TeamCmd
+        auto offer = [&](uint32_t fid, uint32_t nf, uint32_t next) {
+            cmps += nf;
+            float wd = INFINITY;
+            uint32_t wi = 0xffffffffu;
+            if (m >= ef) {
+                wd = dist_at(m - 1);
+                wi = id_at(m - 1) & IDM;
+            }
+            const float dd = dists(fid, nf, next);
+            const bool acc = lane < nf && (m < ef || key_less(dd, fid, wd, wi));
+            const unsigned am = __ballot_sync(FULL, acc);
+            const uint32_t nk = __popc(am);
+            if (nk == 0) return;
+            const uint32_t m2 = min(ef, m + nk);
+            uint32_t rank = 0;
+            if (ER) {
+                // every accepted row against the beam and the other rows: its
+                // place, and how far each entry moves up
+                uint32_t place = 0, move[ES];
+#pragma unroll
+                for (int r = 0; r < ES; r++) move[r] = 0;
+#pragma unroll 2
+                for (unsigned q = am; q; q &= q - 1) {
+                    const int j = __ffs(q) - 1;
+                    const float od = __shfl_sync(FULL, dd, j);
+                    const uint32_t oi = __shfl_sync(FULL, fid, j);
+                    rank += key_less(od, oi, dd, fid) || (od == dd && oi == fid && j < (int)lane);
+                    uint32_t before = 0;
+#pragma unroll
+                    for (int r = 0; r < ES; r++) {
+                        const bool less = key_less(rd[r], ri[r] & IDM, od, oi);
+                        before += __popc(__ballot_sync(FULL, less));
+                        move[r] += !less;
+                    }
+                    if ((int)lane == j) place = before;
+                }
+#pragma unroll
+                for (int r = 0; r < ES; r++) {
+                    const uint32_t i = 32u * r + lane, to = i + move[r];
+                    if (i < m && to < m2) {
+                        bd[to] = rd[r];
+                        bi[to] = ri[r];
+                    }
+                }
+                if (acc && place + rank < m2) {
+                    bd[place + rank] = dd;
+                    bi[place + rank] = fid;
+                }
+                __syncwarp();
+#pragma unroll
+                for (int r = 0; r < ES; r++) {
+                    const uint32_t i = 32u * r + lane;
+                    if (i < m2) {
+                        rd[r] = bd[i];
+                        ri[r] = bi[i];
+                    }
+                }
+                __syncwarp();
+                m = m2;
+                return;
+            }
+            for (unsigned r = am; r; r &= r - 1) {
+                const int j = __ffs(r) - 1;
+                const float od = __shfl_sync(FULL, dd, j);
+                const uint32_t oi = __shfl_sync(FULL, fid, j);
+                rank += key_less(od, oi, dd, fid) || (od == dd && oi == fid && j < (int)lane);
+            }
+            uint32_t npos = 0xffffffffu;
+            if (acc) {
+                uint32_t lo = 0, hi = m;
+                while (lo < hi) {
+                    const uint32_t md = (lo + hi) >> 1;
+                    const float v = bd[md];
+                    if (v < dd || (v == dd && (bi[md] & IDM) < fid)) lo = md + 1;
+                    else hi = md;
+                }
+                npos = rank + lo;
+                nd[rank] = dd;
+                ni[rank] = fid;
+            }
+            const uint32_t lo0 = __reduce_min_sync(FULL, npos);
+            for (uint32_t i = lo0 + lane; i < m; i += 32) {
+                td[i - lo0] = bd[i];
+                ti[i - lo0] = bi[i];
+            }
+            __syncwarp();
+            for (uint32_t i = lo0 + lane; i < m; i += 32) {
+                const float d0 = td[i - lo0];
+                const uint32_t i0 = ti[i - lo0];
+                uint32_t lo = 0, hi = nk;
+                while (lo < hi) {
+                    const uint32_t md = (lo + hi) >> 1;
+                    if (key_less(nd[md], ni[md], d0, i0 & IDM)) lo = md + 1;
+                    else hi = md;
+                }
+                if (i + lo < m2) {
+                    bd[i + lo] = d0;
+                    bi[i + lo] = i0;
+                }
+            }
+            if (acc && npos < m2) {
+                bd[npos] = dd;
+                bi[npos] = fid;
+            }
+            __syncwarp();
+            m = m2;
+            if (lo0 < p) p = lo0;
+        };
+        if (a.flat) {
+            const uint32_t* sd = a.flat_pool + a.flat_off[ef];
+            for (uint32_t c0 = 0; c0 < ef; c0 += 32) {
+                const uint32_t cnt = min(32u, ef - c0);
+                uint32_t id = 0;
+                if (lane < cnt) {
+                    id = sd[c0 + lane];
+                    atomicOr(&vis[id >> 5], 1u << (id & 31));
+                }
+                offer(id, cnt, ~0u);
+            }
+        } else if (cur < nlast) {
+            if (lane == 0) {
+                rd[0] = bd[0] = cur_d;
+                ri[0] = bi[0] = cur;
+                atomicOr(&vis[cur >> 5], 1u << (cur & 31));
+            }
+            m = 1;
+        } else if (lane == 0) {
+            atomicOr(a.overflow, FERR_BAD_ID);
+        }
+        uint32_t expansions = 0;
+        for (;;) {
+            __syncwarp();  // the last merge is visible
+            // lane e: the e-th of the first `width` unexpanded entries
+            uint32_t ne = 0, mine = 0, at = first_open(p);
+            while (at < m) {
+                const uint32_t id = id_at(at) & IDM;
+                if (lane == ne) mine = id;
+                mark(at);
+                if (!ER) p = at + 1;
+                if (++ne >= width) break;
+                at = first_open(at + 1);
+            }
+            if (ne == 0) break;
+            expansions += ne;
+            if (expansions > nlast) {
+                if (lane == 0) atomicOr(a.overflow, FERR_LOOP);
+                break;
+            }
+            nexp += ne;
+            uint64_t lb = 0, le = 0;
+            if (lane < ne) {
+                lb = off_last[mine];
+                le = off_last[mine + 1];
+            }
+            const uint32_t open = first_open(p), next = open < m ? id_at(open) & IDM : ~0u;  // while those load
+            const uint32_t len = (uint32_t)(le - lb);
+            uint32_t pre = len;
+            uint64_t base_l = lb;
+            if (ne > 1) {
+#pragma unroll
+                for (int o = 1; o < 4; o <<= 1) {
+                    const uint32_t v = __shfl_up_sync(FULL, pre, o);
+                    if (lane >= (uint32_t)o) pre += v;
+                }
+                base_l = lb - (pre - len);  // list e: adjacency index base_e + t
+            }
+            const uint32_t total = __shfl_sync(FULL, pre, ne - 1);
+            for (uint32_t t0 = 0; t0 < total; t0 += 32 * GROUP) {
+                uint32_t nn[GROUP];
+#pragma unroll
+                for (uint32_t c = 0; c < GROUP; c++) {
+                    if (t0 + 32 * c >= total) break;
+                    const uint32_t t = t0 + 32 * c + lane;
+                    uint64_t bs = __shfl_sync(FULL, base_l, 0);
+                    for (uint32_t e = 1; e < ne; e++) {  // entry t belongs to list e when end_{e-1} <= t
+                        const uint32_t end = __shfl_sync(FULL, pre, e - 1);
+                        const uint64_t be = __shfl_sync(FULL, base_l, e);
+                        if (t >= end) bs = be;
+                    }
+                    nn[c] = t < total ? a.adj_all[bs + t] : 0u;
+                }
+                uint32_t nf = 0;
+#pragma unroll
+                for (uint32_t c = 0; c < GROUP; c++) {
+                    if (t0 + 32 * c >= total) break;
+                    bool fresh = false;
+                    if (t0 + 32 * c + lane < total) {
+                        const uint32_t bit = 1u << (nn[c] & 31);
+                        fresh = !(atomicOr(&vis[nn[c] >> 5], bit) & bit);
+                    }
+                    const unsigned fb = __ballot_sync(FULL, fresh);
+                    if (fresh) {
+                        fr[nf + __popc(fb & ((1u << lane) - 1u))] = nn[c];
+                        prefetch_l1(off_last + nn[c]);
+                    }
+                    nf += __popc(fb);
+                }
+                __syncwarp();
+                for (uint32_t f0 = 0; f0 < nf; f0 += 32) {
+                    const uint32_t cnt = min(32u, nf - f0);
+                    const uint32_t fid = lane < cnt ? fr[f0 + lane] : 0u;
+                    offer(fid, cnt, next);
+                }
+                __syncwarp();
+            }
+        }
+        if (lane == 0) cmd[turn] = TeamCmd{0, 0};
+        __syncthreads();  // the helpers stop
+        if (ER) {  // the marks are in the registers only; ids and distances are staged
+#pragma unroll
+            for (int r = 0; r < ES; r++) {
+                const uint32_t i = 32u * r + lane;
+                if (i < m) {
+                    bd[i] = rd[r];
+                    bi[i] = ri[r];
+                }
+            }
+            __syncwarp();
+        }
+        for (uint32_t t = lane; t < a.out_k; t += 32) {
+            const size_t o = (size_t)qi * a.out_k + t;
+            a.out_ids[o] = t < m ? (bi[t] & IDM) : 0xffffffffu;
+            if (a.out_d) a.out_d[o] = t < m ? bd[t] : 0.f;
+        }
+        __syncthreads();
+    }
+    if (tid == 0) {
+        atomicAdd(a.ncmps, cmps);
+        atomicAdd(a.nexp, nexp);
+    }
+}
+
 using ServeFn = void (*)(ServeArgs);
 template <int M>
 ServeFn pick_qv(uint32_t qv) {
     return qv == 1 ? k_serve<M, 1> : (qv == 2 ? k_serve<M, 2> : k_serve<M, 4>);
+}
+template <int M, int QV>
+ServeFn pick_team_beam(uint32_t beam) {
+    return beam <= 64 ? k_serve_team<M, QV, 2> : (beam <= 192 ? k_serve_team<M, QV, 6> : k_serve_team<M, QV, 0>);
+}
+template <int M>
+ServeFn pick_team(uint32_t qv, uint32_t beam) {
+    return qv == 1 ? pick_team_beam<M, 1>(beam) : (qv == 2 ? pick_team_beam<M, 2>(beam) : pick_team_beam<M, 4>(beam));
 }
 }  // namespace
 
@@ -529,20 +1053,38 @@ int index_run_fast(Ctx& ctx, IndexDev& ix, const SearchReq& r) {
     }
     const uint32_t dp4 = ix.dp / 4;
     const uint32_t qv = dp4 <= 32 ? 1 : (dp4 <= 64 ? 2 : 4);
-    const ServeFn fn = ix.metric == L2 ? pick_qv<L2>(qv) : (ix.metric == L1 ? pick_qv<L1>(qv) : pick_qv<CHI2>(qv));
-    const size_t smem = (size_t)FW * ((size_t)r.beam_max * 16 + WARP_EXTRA);
-    NNM_CUDA_TRY(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    int nsm = 148, per_sm = 1;
-    cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, ctx.device);
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, FW * 32, smem);
-    const uint32_t blocks = (uint32_t)std::min(std::max(1, per_sm), 8) * (uint32_t)nsm;
+    int nsm = 148, per_sm = 1, optin = 0;
+    NNM_CUDA_TRY(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, ctx.device));
+    NNM_CUDA_TRY(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, ctx.device));
     const uint32_t words = (ix.n + 31) / 32;
-    const size_t slots = (size_t)blocks * FW;
-    if (ix.visited.bytes < slots * words * 4) {
-        NNM_CUDA_TRY(ix.visited.ensure(slots * words * 4));
-        NNM_CUDA_TRY(cudaMemsetAsync(ix.visited.p, 0, slots * words * 4, st));
+    // a block per query while the blocks resident at once hold them all, and
+    // the visited bitmap fits in shared memory
+    const ServeFn team = ix.metric == L2 ? pick_team<L2>(qv, r.beam_max)
+                         : (ix.metric == L1 ? pick_team<L1>(qv, r.beam_max) : pick_team<CHI2>(qv, r.beam_max));
+    const size_t tsmem = team_smem(words, r.beam_max);
+    bool use_team = tsmem <= (size_t)optin;
+    if (use_team) {
+        NNM_CUDA_TRY(cudaFuncSetAttribute(team, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tsmem));
+        int pt = 0;
+        NNM_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&pt, team, TEAM * 32, tsmem));
+        use_team = r.nq <= (uint32_t)std::max(pt, 0) * (uint32_t)nsm;
     }
-    NNM_CUDA_TRY(ix.vlist.ensure(slots * FVCAP * 4));
+    const ServeFn fn = use_team ? team
+                       : ix.metric == L2 ? pick_qv<L2>(qv)
+                                         : (ix.metric == L1 ? pick_qv<L1>(qv) : pick_qv<CHI2>(qv));
+    const size_t smem = use_team ? tsmem : (size_t)FW * ((size_t)r.beam_max * 16 + WARP_EXTRA);
+    uint32_t blocks = r.nq;
+    if (!use_team) {
+        NNM_CUDA_TRY(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, FW * 32, smem);
+        blocks = std::min((uint32_t)std::min(std::max(1, per_sm), 8) * (uint32_t)nsm, (r.nq + FW - 1) / FW);
+        const size_t slots = (size_t)blocks * FW;
+        if (ix.visited.bytes < slots * words * 4) {
+            NNM_CUDA_TRY(ix.visited.ensure(slots * words * 4));
+            NNM_CUDA_TRY(cudaMemsetAsync(ix.visited.p, 0, slots * words * 4, st));
+        }
+        NNM_CUDA_TRY(ix.vlist.ensure(slots * FVCAP * 4));
+    }
     ServeArgs a{};
     a.x = ix.x.as<float>();
     a.dp4 = dp4;
@@ -577,7 +1119,8 @@ int index_run_fast(Ctx& ctx, IndexDev& ix, const SearchReq& r) {
     a.overflow = reinterpret_cast<unsigned*>(c + 4);
     a.ncmps = reinterpret_cast<unsigned long long*>(c + 8);
     a.nexp = reinterpret_cast<unsigned long long*>(c + 16);
-    fn<<<blocks, FW * 32, smem, st>>>(a); count_launch();
+    a.spec_blocks = (uint32_t)nsm;
+    fn<<<blocks, (use_team ? TEAM : FW) * 32, smem, st>>>(a); count_launch();
     NNM_CUDA_TRY(cudaGetLastError());
     return 0;
 }
