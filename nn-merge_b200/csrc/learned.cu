@@ -443,6 +443,9 @@ __global__ void k_refresh(const float* __restrict__ w1, const float* __restrict_
     }
 }
 
+// Both weight matrices: below d = 32 the second one is the larger.
+uint32_t refresh_blocks(uint32_t d) { return (std::max<uint32_t>(MLP_H * d, MLP_O * MLP_H) + 255) / 256; }
+
 __global__ void k_sample_triplets(uint32_t* idx, uint32_t B, uint32_t n, const uint32_t* graph, uint32_t K,
                                   uint32_t seed, const uint32_t* step) {
     const uint32_t b = blockIdx.x * blockDim.x + threadIdx.x;
@@ -563,7 +566,7 @@ int mlp_upload(Ctx& ctx, DevMlp& m, const nnm_mlp& h) {
     NNM_CUDA_TRY(m.b2.ensure(MLP_O * 4));
     NNM_CUDA_TRY(cudaMemcpyAsync(tmp.p, f.data(), L.total * 4, cudaMemcpyHostToDevice, ctx.stream));
     const float* t = tmp.as<float>();
-    k_refresh<<<(MLP_H * d + 255) / 256, 256, 0, ctx.stream>>>(t + L.w1, t + L.w2, d, m.w1t.as<__nv_bfloat16>(),
+    k_refresh<<<refresh_blocks(d), 256, 0, ctx.stream>>>(t + L.w1, t + L.w2, d, m.w1t.as<__nv_bfloat16>(),
                                                              m.w2t.as<__nv_bfloat16>()); count_launch();
     NNM_CUDA_TRY(cudaMemcpyAsync(m.b1.p, t + L.b1, MLP_H * 4, cudaMemcpyDeviceToDevice, ctx.stream));
     NNM_CUDA_TRY(cudaMemcpyAsync(m.b2.p, t + L.b2, MLP_O * 4, cudaMemcpyDeviceToDevice, ctx.stream));
@@ -624,7 +627,7 @@ int mlp_grad(Ctx& ctx, const nnm_mlp& model, const float* x_dev, uint32_t n, uin
     std::vector<float> f = flatten(model, L);
     NNM_CUDA_TRY(cudaMemcpyAsync(p.flat.p, f.data(), L.total * 4, cudaMemcpyHostToDevice, ctx.stream));
     const float* fl = p.flat.as<float>();
-    k_refresh<<<(MLP_H * d + 255) / 256, 256, 0, ctx.stream>>>(fl + L.w1, fl + L.w2, d, p.w1t.as<__nv_bfloat16>(),
+    k_refresh<<<refresh_blocks(d), 256, 0, ctx.stream>>>(fl + L.w1, fl + L.w2, d, p.w1t.as<__nv_bfloat16>(),
                                                              p.w2t.as<__nv_bfloat16>()); count_launch();
     enqueue_pass(pass_view(p, L, model), x_dev, dp, B, margin, p, L, nullptr, ctx.stream);
     count_launch(6);
@@ -655,7 +658,7 @@ int mlp_train(Ctx& ctx, const float* x_dev, uint32_t n, uint32_t dp, const uint3
     NNM_CUDA_TRY(cudaMemsetAsync(p.vel.p, 0, L.total * 4, st));
     NNM_CUDA_TRY(cudaMemsetAsync(p.step.p, 0, 4, st));
     float* fl = p.flat.as<float>();
-    k_refresh<<<(MLP_H * d + 255) / 256, 256, 0, st>>>(fl + L.w1, fl + L.w2, d, p.w1t.as<__nv_bfloat16>(),
+    k_refresh<<<refresh_blocks(d), 256, 0, st>>>(fl + L.w1, fl + L.w2, d, p.w1t.as<__nv_bfloat16>(),
                                                      p.w2t.as<__nv_bfloat16>()); count_launch();
     NNM_CUDA_TRY(cudaStreamSynchronize(st));
     const MlpView mv = pass_view(p, L, model);
@@ -668,7 +671,7 @@ int mlp_train(Ctx& ctx, const float* x_dev, uint32_t n, uint32_t dp, const uint3
     enqueue_pass(mv, x_dev, dp, B, o.margin, p, L, step, st);
     k_adam<<<(unsigned)((L.total + 255) / 256), 256, 0, st>>>(fl, p.mom.as<float>(), p.vel.as<float>(),
                                                               p.grad.as<float>(), (uint32_t)L.total, o.lr, step);
-    k_refresh<<<(MLP_H * d + 255) / 256, 256, 0, st>>>(fl + L.w1, fl + L.w2, d, p.w1t.as<__nv_bfloat16>(),
+    k_refresh<<<refresh_blocks(d), 256, 0, st>>>(fl + L.w1, fl + L.w2, d, p.w1t.as<__nv_bfloat16>(),
                                                      p.w2t.as<__nv_bfloat16>());
     k_step_inc<<<1, 1, 0, st>>>(step);
     cudaError_t ce = cudaStreamEndCapture(st, &graph);
