@@ -698,11 +698,9 @@ int nnm_mlp_grad(nnm_ctx* ctx, const nnm_mlp* model, const float* x, uint64_t n,
         if (triplets[i] >= n) return fail(ctx, NNM_ERR_INVALID, "triplet index out of range");
     Ctx& c = ctx->c;
     if (cudaSetDevice(c.device) != cudaSuccess) return fail(ctx, NNM_ERR_NO_DEVICE, "cudaSetDevice failed");
-    GraphStore st;
     GraphDev g;
-    int rc = upload_plain(c, st, g, x, n, d);
+    int rc = upload_plain(c, c.store, g, x, n, d);
     if (!rc) rc = nnm::mlp_grad(c, *model, g.x, (uint32_t)n, g.dp, triplets, ntrip, margin, loss, *grad);
-    st.release();
     return rc;
 }
 

@@ -32,7 +32,7 @@ namespace {
 using bf16 = __nv_bfloat16;
 constexpr uint32_t EH = ENTRY_H;
 constexpr uint32_t ERB = 32;          // rows per block
-constexpr uint64_t STEP_KERNELS = 11; // kernels of one captured training step
+constexpr uint64_t STEP_KERNELS = 12; // kernels of one captured training step
 
 struct EView {
     const bf16* w1t;  // d x 256
@@ -622,7 +622,7 @@ void enqueue_pass(const EView& v, const float* x, uint32_t dp, uint32_t B, EPass
     k_ent_gw2<<<(v.C + GC - 1) / GC, 256, 0, st>>>(p.s.as<float>(), p.h.as<float>(), B, v.C, g + L.w2, g + L.b2);
     launch_grad_w1(p.dh.as<float>(), x, dp, p.idx.as<uint32_t>(), B, v.d, v.scale, v.shift, g + L.w1, g + L.b1, st);
 }
-constexpr uint64_t PASS_KERNELS = 7;
+constexpr uint64_t PASS_KERNELS = 8;
 
 }  // namespace
 

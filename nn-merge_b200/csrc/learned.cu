@@ -28,7 +28,7 @@ namespace {
 
 constexpr uint32_t RB = 32;  // rows per forward block
 constexpr int FWD_THREADS = 256;
-constexpr uint64_t STEP_KERNELS = 10;  // kernels of one captured training step
+constexpr uint64_t STEP_KERNELS = 12;  // kernels of one captured training step
 
 __device__ __forceinline__ float bf(__nv_bfloat16 v) { return __bfloat162float(v); }
 
@@ -357,61 +357,156 @@ __global__ void k_triplet(const float* __restrict__ t, uint32_t B, float margin,
     }
 }
 
-__global__ void k_loss_final(const float* partial, uint32_t nblk, uint32_t B, float* loss, const uint32_t* step) {
+// One block; the sum itself runs in partial's order on one thread.
+__global__ void __launch_bounds__(256) k_loss_final(const float* partial, uint32_t nblk, uint32_t B, float* loss,
+                                                    const uint32_t* step) {
+    __shared__ float part[1024];
     float s = 0.f;
-    for (uint32_t i = 0; i < nblk; i++) s += partial[i];
-    loss[step ? *step : 0] = s / (float)B;
+    for (uint32_t i0 = 0; i0 < nblk; i0 += 1024) {
+        const uint32_t n = min(1024u, nblk - i0);
+        __syncthreads();
+        for (uint32_t i = threadIdx.x; i < n; i += blockDim.x) part[i] = partial[i0 + i];
+        __syncthreads();
+        if (threadIdx.x == 0)
+            for (uint32_t i = 0; i < n; i++) s += part[i];
+    }
+    if (threadIdx.x == 0) loss[step ? *step : 0] = s / (float)B;
 }
 
-// dL/d(pre-activation of h): (h > 0) * sum_o dz_o W2[o][j].
-__global__ void k_bwd_h(const float* __restrict__ dz, const float* __restrict__ h, MlpView m, uint32_t R,
-                        float* __restrict__ dh) {
-    const size_t t = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= (size_t)R * MLP_H) return;
-    const uint32_t r = (uint32_t)(t / MLP_H), j = (uint32_t)(t - (size_t)r * MLP_H);
+// dL/d(pre-activation of h): (h > 0) * sum_o dz_o W2[o][j], o ascending.
+// Thread j keeps its 32 weights in registers over BH_ROWS rows, whose dz come
+// from shared memory by broadcast (a thread per value, 64 bytes of weights
+// each, took 98 us for 6,144 rows; this 14).
+constexpr uint32_t BH_ROWS = 16;
+__global__ void __launch_bounds__(MLP_H) k_bwd_h(const float* __restrict__ dz, const float* __restrict__ h, MlpView m,
+                                                 uint32_t R, float* __restrict__ dh) {
+    __shared__ __align__(16) float ds[BH_ROWS][MLP_O];
+    const uint32_t j = threadIdx.x, r0 = blockIdx.x * BH_ROWS, nr = min(BH_ROWS, R - r0);
+    for (uint32_t i = j; i < nr * MLP_O; i += MLP_H) ds[i / MLP_O][i % MLP_O] = dz[(size_t)r0 * MLP_O + i];
+    float w[MLP_O];
+#pragma unroll
+    for (uint32_t o = 0; o < MLP_O; o++) w[o] = bf(m.w2t[j * MLP_O + o]);
+    __syncthreads();
+#pragma unroll 2
+    for (uint32_t r = 0; r < nr; r++) {
+        float acc = 0.f;
+#pragma unroll
+        for (uint32_t o = 0; o < MLP_O; o += 4) {
+            const float4 z = *reinterpret_cast<const float4*>(&ds[r][o]);
+            acc = fmaf(z.x, w[o], acc);
+            acc = fmaf(z.y, w[o + 1], acc);
+            acc = fmaf(z.z, w[o + 2], acc);
+            acc = fmaf(z.w, w[o + 3], acc);
+        }
+        const size_t t = (size_t)(r0 + r) * MLP_H + j;
+        dh[t] = h[t] > 0.f ? acc : 0.f;
+    }
+}
+
+// Weight gradients: g[a][b] = sum_r p[r][a] q[r][b] for a < na, b < nb, the
+// rows added in ascending order by one FMA chain per value, so that the
+// result does not depend on the launch.  q's row r is the vector
+// x[idx[r]] * scale + shift (GATHER) or row r of q itself; ldq floats a row,
+// a multiple of 4.  A block takes 16 x 16 values and streams 128 rows at a
+// time through shared memory, transposed so that one read brings four rows; the
+// next rows, and the indices of those after, load into registers meanwhile.  Bound: the chain, R x 4 cycles
+// (13 us for 6,144 rows): 533 -> 65 us for 256 x 128 values, 228 -> 61
+// for 32 x 256, against a thread per value reading its operands itself.
+constexpr uint32_t GO_T = 16, GO_R = 128, GO_LD = GO_R + 4;
+template <bool GATHER>
+__global__ void __launch_bounds__(GO_T * GO_T) k_grad_outer(const float* __restrict__ p, uint32_t na,
+                                                            const float* __restrict__ q, uint32_t nb, uint32_t ldq,
+                                                            const uint32_t* __restrict__ idx, float scale, float shift,
+                                                            uint32_t R, float* __restrict__ g) {
+    __shared__ __align__(16) float ps[2][GO_T][GO_LD], qs[2][GO_T][GO_LD];
+    const uint32_t tid = threadIdx.x, ta = tid / GO_T, tb = tid % GO_T, lr = tid >> 2, c = (tid & 3) * 4;
+    const uint32_t a0 = blockIdx.y * GO_T, b0 = blockIdx.x * GO_T;
+    constexpr uint32_t NF = GO_R / 64;  // rows of a chunk per thread, 64 apart
+    float4 np[NF], nq[NF];  // four columns of this thread's rows of the chunk to come
+    uint32_t ni[NF];        // GATHER: and the rows of x of the chunk after it
+    auto fetch_idx = [&](uint32_t r0) {
+#pragma unroll
+        for (uint32_t f = 0; f < NF; f++) {
+            const uint32_t r = r0 + lr + 64 * f;
+            ni[f] = GATHER ? (r < R ? idx[r] : 0u) : r;
+        }
+    };
+    auto fetch = [&](uint32_t r0) {
+#pragma unroll
+        for (uint32_t f = 0; f < NF; f++) {
+            np[f] = nq[f] = make_float4(0.f, 0.f, 0.f, 0.f);
+            const uint32_t r = r0 + lr + 64 * f;
+            if (r < R) {
+                np[f] = *reinterpret_cast<const float4*>(p + (size_t)r * na + a0 + c);
+                if (b0 + c < ldq) nq[f] = *reinterpret_cast<const float4*>(q + (size_t)ni[f] * ldq + b0 + c);
+            }
+        }
+    };
+    auto put = [&](uint32_t b) {
+#pragma unroll
+        for (uint32_t f = 0; f < NF; f++) {
+            const uint32_t r = lr + 64 * f;
+            const float pv[4] = {np[f].x, np[f].y, np[f].z, np[f].w}, qv[4] = {nq[f].x, nq[f].y, nq[f].z, nq[f].w};
+#pragma unroll
+            for (uint32_t i = 0; i < 4; i++) {
+                ps[b][c + i][r] = pv[i];
+                qs[b][c + i][r] = GATHER ? fmaf(qv[i], scale, shift) : qv[i];  // past R: times p = 0
+            }
+        }
+    };
     float acc = 0.f;
-#pragma unroll 8
-    for (uint32_t o = 0; o < MLP_O; o++) acc = fmaf(dz[(size_t)r * MLP_O + o], bf(m.w2t[j * MLP_O + o]), acc);
-    dh[t] = h[t] > 0.f ? acc : 0.f;
+    fetch_idx(0);
+    fetch(0);
+    fetch_idx(GO_R);
+    put(0);
+    uint32_t b = 0;
+    for (uint32_t r0 = 0; r0 < R; r0 += GO_R, b ^= 1) {
+        __syncthreads();
+        if (r0 + GO_R < R) {
+            fetch(r0 + GO_R);
+            fetch_idx(r0 + 2 * GO_R);
+        }
+#pragma unroll 16
+        for (uint32_t r = 0; r < GO_R; r += 4) {
+            const float4 u = *reinterpret_cast<const float4*>(&ps[b][ta][r]);
+            const float4 v = *reinterpret_cast<const float4*>(&qs[b][tb][r]);
+            acc = fmaf(u.x, v.x, acc);
+            acc = fmaf(u.y, v.y, acc);
+            acc = fmaf(u.z, v.z, acc);
+            acc = fmaf(u.w, v.w, acc);
+        }
+        if (r0 + GO_R < R) put(b ^ 1);
+    }
+    if (b0 + tb < nb) g[(size_t)(a0 + ta) * nb + b0 + tb] = acc;
 }
 
-// Block o: dW2[o][j] = sum_r dz[r][o] h[r][j] (thread j), db2[o].
-__global__ void k_grad_w2(const float* __restrict__ dz, const float* __restrict__ h, uint32_t R,
-                          float* __restrict__ gw2, float* __restrict__ gb2) {
-    __shared__ float red[MLP_H];
-    const uint32_t o = blockIdx.x, j = threadIdx.x;
-    float acc = 0.f, sb = 0.f;
-    for (uint32_t r = 0; r < R; r++) acc = fmaf(dz[(size_t)r * MLP_O + o], h[(size_t)r * MLP_H + j], acc);
-    for (uint32_t r = j; r < R; r += MLP_H) sb += dz[(size_t)r * MLP_O + o];
-    gw2[(size_t)o * MLP_H + j] = acc;
-    red[j] = sb;
+// Bias gradients: g[a] = sum_r p[r][a] as 256 sums over r = k, k + 256, ...,
+// added in a tree over k.  A block takes 32 columns, a warp's lanes one each.
+constexpr uint32_t GB_THREADS = 1024, GB_K = 256;
+__global__ void __launch_bounds__(GB_THREADS) k_grad_bias(const float* __restrict__ p, uint32_t na, uint32_t R,
+                                                          float* __restrict__ g) {
+    __shared__ float red[GB_K][33];
+    const uint32_t lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const float* col = p + blockIdx.x * 32 + lane;
+    constexpr uint32_t NK = GB_K / (GB_THREADS / 32);
+    float s[NK];
+#pragma unroll
+    for (uint32_t i = 0; i < NK; i++) s[i] = 0.f;
+#pragma unroll 4
+    for (uint32_t r0 = 0; r0 < R; r0 += GB_K)
+#pragma unroll
+        for (uint32_t i = 0; i < NK; i++) {
+            const uint32_t r = r0 + w * NK + i;
+            if (r < R) s[i] += col[(size_t)r * na];
+        }
+#pragma unroll
+    for (uint32_t i = 0; i < NK; i++) red[w * NK + i][lane] = s[i];
     __syncthreads();
-    for (uint32_t s = MLP_H / 2; s > 0; s >>= 1) {
-        if (j < s) red[j] += red[j + s];
+    for (uint32_t n = GB_K / 2; n > 0; n >>= 1) {
+        for (uint32_t k = w; k < n; k += GB_THREADS / 32) red[k][lane] += red[k + n][lane];
         __syncthreads();
     }
-    if (j == 0) gb2[o] = red[0];
-}
-
-// Block j: dW1[j][k] = sum_r dh[r][j] u[r][k] (thread k), db1[j].
-__global__ void k_grad_w1(const float* __restrict__ dh, const float* __restrict__ x, uint32_t dp,
-                          const uint32_t* __restrict__ idx, uint32_t R, MlpView m, float* __restrict__ gw1,
-                          float* __restrict__ gb1) {
-    __shared__ float red[256];
-    const uint32_t j = blockIdx.x, k = threadIdx.x;
-    float acc = 0.f, sb = 0.f;
-    if (k < m.d)
-        for (uint32_t r = 0; r < R; r++)
-            acc = fmaf(dh[(size_t)r * MLP_H + j], fmaf(x[(size_t)idx[r] * dp + k], m.scale, m.shift), acc);
-    for (uint32_t r = k; r < R; r += blockDim.x) sb += dh[(size_t)r * MLP_H + j];
-    if (k < m.d) gw1[(size_t)j * m.d + k] = acc;
-    red[k] = sb;
-    __syncthreads();
-    for (uint32_t s = blockDim.x / 2; s > 0; s >>= 1) {
-        if (k < s) red[k] += red[k + s];
-        __syncthreads();
-    }
-    if (k == 0) gb1[j] = red[0];
+    if (w == 0) g[blockIdx.x * 32 + lane] = red[0][lane];
 }
 
 // Adam (Kingma & Ba, 2015) on the flat parameter vector, step t = *step + 1.
@@ -473,12 +568,20 @@ cudaError_t set_fwd_attrs(uint32_t d) {
     return cudaFuncSetAttribute(k_mlp_fwd<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fwd_smem(d));
 }
 
-// Scratch of one training/gradient pass over B triplets.
+// Scratch of one training/gradient pass over B triplets, laid out in the
+// context's training workspace (a call allocated and freed 13 buffers, 2-3 ms
+// with the frees' waits).  A workspace above KEEP bytes is given back at the end.
 struct Pass {
-    DevBuf idx, h, t, dz, dh, partial, flat, grad, mom, vel, w1t, w2t, loss, step;
+    struct Span {
+        void* p = nullptr;
+        template <class T> T* as() const { return static_cast<T*>(p); }
+    };
+    static constexpr size_t KEEP = (size_t)256 << 20;
+    DevBuf& arena;
+    Span idx, h, t, dz, dh, partial, flat, grad, mom, vel, w1t, w2t, loss, step;
+    explicit Pass(Ctx& ctx) : arena(ctx.ws.train) {}
     ~Pass() {
-        for (DevBuf* b : {&idx, &h, &t, &dz, &dh, &partial, &flat, &grad, &mom, &vel, &w1t, &w2t, &loss, &step})
-            b->release();
+        if (arena.bytes > KEEP) arena.release();
     }
 };
 
@@ -491,27 +594,36 @@ void enqueue_pass(const MlpView& mv, const float* x, uint32_t dp, uint32_t B, fl
                                                                            nullptr, nullptr);
     const uint32_t nblk = (B + 7) / 8;
     k_triplet<<<nblk, 256, 0, st>>>(p.t.as<float>(), B, margin, p.dz.as<float>(), p.partial.as<float>());
-    k_loss_final<<<1, 1, 0, st>>>(p.partial.as<float>(), nblk, B, p.loss.as<float>(), step);
-    k_bwd_h<<<(unsigned)(((size_t)R * MLP_H + 255) / 256), 256, 0, st>>>(p.dz.as<float>(), p.h.as<float>(), mv, R,
-                                                                        p.dh.as<float>());
+    k_loss_final<<<1, 256, 0, st>>>(p.partial.as<float>(), nblk, B, p.loss.as<float>(), step);
+    k_bwd_h<<<(R + BH_ROWS - 1) / BH_ROWS, MLP_H, 0, st>>>(p.dz.as<float>(), p.h.as<float>(), mv, R,
+                                                           p.dh.as<float>());
     float* g = p.grad.as<float>();
-    k_grad_w2<<<MLP_O, MLP_H, 0, st>>>(p.dz.as<float>(), p.h.as<float>(), R, g + L.w2, g + L.b2);
-    k_grad_w1<<<MLP_H, 256, 0, st>>>(p.dh.as<float>(), x, dp, p.idx.as<uint32_t>(), R, mv, g + L.w1, g + L.b1);
+    k_grad_outer<false><<<dim3(MLP_H / GO_T, MLP_O / GO_T), GO_T * GO_T, 0, st>>>(
+        p.dz.as<float>(), MLP_O, p.h.as<float>(), MLP_H, MLP_H, nullptr, 0.f, 0.f, R, g + L.w2);
+    k_grad_bias<<<MLP_O / 32, GB_THREADS, 0, st>>>(p.dz.as<float>(), MLP_O, R, g + L.b2);
+    launch_grad_w1(p.dh.as<float>(), x, dp, p.idx.as<uint32_t>(), R, mv.d, mv.scale, mv.shift, g + L.w1, g + L.b1, st);
 }
 
-int alloc_pass(Ctx& ctx, Pass& p, uint32_t B, const Layout& L, uint32_t d) {
+// Lays out p over ctx's training workspace; loss_floats: entries of the loss
+// trace; train: with Adam's moments.
+int alloc_pass(Ctx& ctx, Pass& p, uint32_t B, const Layout& L, uint32_t d, size_t loss_floats, bool train) {
     const size_t R = 3 * (size_t)B;
-    NNM_CUDA_TRY(p.idx.ensure(R * 4));
-    NNM_CUDA_TRY(p.h.ensure(R * MLP_H * 4));
-    NNM_CUDA_TRY(p.t.ensure(R * MLP_O * 4));
-    NNM_CUDA_TRY(p.dz.ensure(R * MLP_O * 4));
-    NNM_CUDA_TRY(p.dh.ensure(R * MLP_H * 4));
-    NNM_CUDA_TRY(p.partial.ensure(((B + 7) / 8) * 4 + 64));
-    NNM_CUDA_TRY(p.flat.ensure(L.total * 4));
-    NNM_CUDA_TRY(p.grad.ensure(L.total * 4));
-    NNM_CUDA_TRY(p.w1t.ensure((size_t)d * MLP_H * 2));
-    NNM_CUDA_TRY(p.w2t.ensure((size_t)MLP_H * MLP_O * 2));
-    NNM_CUDA_TRY(p.step.ensure(64));
+    const struct {
+        Pass::Span* s;
+        size_t bytes;
+    } parts[] = {{&p.idx, R * 4}, {&p.h, R * MLP_H * 4}, {&p.t, R * MLP_O * 4}, {&p.dz, R * MLP_O * 4},
+                 {&p.dh, R * MLP_H * 4}, {&p.partial, ((B + 7) / 8) * 4 + 64}, {&p.flat, L.total * 4},
+                 {&p.grad, L.total * 4}, {&p.w1t, (size_t)d * MLP_H * 2}, {&p.w2t, (size_t)MLP_H * MLP_O * 2},
+                 {&p.step, 64}, {&p.loss, loss_floats * 4 + 64}, {&p.mom, train ? L.total * 4 : 0},
+                 {&p.vel, train ? L.total * 4 : 0}};
+    size_t total = 0;
+    for (const auto& q : parts) total += (q.bytes + 255) & ~(size_t)255;
+    NNM_CUDA_TRY(p.arena.ensure(total));
+    unsigned char* at = p.arena.as<unsigned char>();
+    for (const auto& q : parts) {
+        q.s->p = at;
+        at += (q.bytes + 255) & ~(size_t)255;
+    }
     return 0;
 }
 
@@ -542,11 +654,9 @@ MlpView pass_view(const Pass& p, const Layout& L, const nnm_mlp& m) {
 
 void launch_grad_w1(const float* dh, const float* x, uint32_t dp, const uint32_t* idx, uint32_t R, uint32_t d,
                     float scale, float shift, float* gw1, float* gb1, cudaStream_t st) {
-    MlpView m{};
-    m.d = d;
-    m.scale = scale;
-    m.shift = shift;
-    k_grad_w1<<<MLP_H, 256, 0, st>>>(dh, x, dp, idx, R, m, gw1, gb1);
+    k_grad_outer<true><<<dim3((d + GO_T - 1) / GO_T, MLP_H / GO_T), GO_T * GO_T, 0, st>>>(dh, MLP_H, x, d, dp, idx,
+                                                                                          scale, shift, R, gw1);
+    k_grad_bias<<<MLP_H / 32, GB_THREADS, 0, st>>>(dh, MLP_H, R, gb1);
 }
 
 void launch_adam(float* p, float* mo, float* ve, const float* g, uint32_t cnt, float lr, const uint32_t* step,
@@ -614,10 +724,9 @@ int mlp_grad(Ctx& ctx, const nnm_mlp& model, const float* x_dev, uint32_t n, uin
     (void)n;
     const uint32_t d = model.d_in, B = ntrip;
     const Layout L(d);
-    Pass p;
-    int rc = alloc_pass(ctx, p, B, L, d);
+    Pass p(ctx);
+    int rc = alloc_pass(ctx, p, B, L, d, 1, false);
     if (rc) return rc;
-    NNM_CUDA_TRY(p.loss.ensure(64));
     NNM_CUDA_TRY(set_fwd_attrs(d));
     // triplets (anchor, positive, negative) -> idx = anchors | positives | negatives
     std::vector<uint32_t> h(3 * (size_t)B);
@@ -630,7 +739,7 @@ int mlp_grad(Ctx& ctx, const nnm_mlp& model, const float* x_dev, uint32_t n, uin
     k_refresh<<<refresh_blocks(d), 256, 0, ctx.stream>>>(fl + L.w1, fl + L.w2, d, p.w1t.as<__nv_bfloat16>(),
                                                              p.w2t.as<__nv_bfloat16>()); count_launch();
     enqueue_pass(pass_view(p, L, model), x_dev, dp, B, margin, p, L, nullptr, ctx.stream);
-    count_launch(6);
+    count_launch(8);
     NNM_CUDA_TRY(cudaGetLastError());
     std::vector<float> g(L.total);
     NNM_CUDA_TRY(cudaMemcpyAsync(g.data(), p.grad.p, L.total * 4, cudaMemcpyDeviceToHost, ctx.stream));
@@ -644,12 +753,9 @@ int mlp_train(Ctx& ctx, const float* x_dev, uint32_t n, uint32_t dp, const uint3
               const nnm_train_opts& o, nnm_mlp& model, float* loss_trace) {
     const uint32_t d = model.d_in, B = o.batch;
     const Layout L(d);
-    Pass p;
-    int rc = alloc_pass(ctx, p, B, L, d);
+    Pass p(ctx);
+    int rc = alloc_pass(ctx, p, B, L, d, o.steps, true);
     if (rc) return rc;
-    NNM_CUDA_TRY(p.mom.ensure(L.total * 4));
-    NNM_CUDA_TRY(p.vel.ensure(L.total * 4));
-    NNM_CUDA_TRY(p.loss.ensure((size_t)o.steps * 4 + 64));
     NNM_CUDA_TRY(set_fwd_attrs(d));
     std::vector<float> f = flatten(model, L);
     cudaStream_t st = ctx.stream;

@@ -48,11 +48,12 @@ struct Workspace {
     uint32_t mt_seed = 0;
     size_t mt_have = 0;
     DevBuf counters, misc;
+    DevBuf train;    // one training or gradient pass of the code network
     DevBuf mlp_err;  // the code network's tensor-core inference: a wait that ran out
     void release_all() {
         DevBuf* all[] = {&rcnt, &rcur, &rtot, &roff, &rseg, &rscr, &rofs, &rbuf, &cntpos, &bcnt, &bcur,
                          &boff, &bucket, &bigrev, &nflag, &scan_tmp, &npairs, &poff, &pd, &tiers, &erows, &kth, &rtier,
-                         &draws, &mt_ring, &counters, &misc, &mlp_err};
+                         &draws, &mt_ring, &counters, &misc, &train, &mlp_err};
         for (auto* b : all) b->release();
     }
 };
