@@ -12,20 +12,33 @@
 //   - best-first beam search on the last layer with the reference's two
 //     std::priority_queue<pair<float,unsigned>> heaps (results: max-heap on
 //     distance, size <= topk, in shared memory; candidates: max-heap on
-//     minus the distance, in a per-warp HBM slot).  Lane 0 replays
-//     libstdc++'s push_heap/pop_heap steps exactly, so the order among equal
-//     distances -- which the heaps decide -- is the reference's too.  The
+//     minus the distance, its first CAND_SMEM entries in shared memory and the
+//     rest in a per-warp HBM slot).  The heaps hold what libstdc++'s
+//     push_heap/pop_heap steps leave, so the order among equal distances --
+//     which the heaps decide -- is the reference's too.  Up to COOP entries
+//     the warp takes a step at once: a push compares every ancestor in its own
+//     lane, a pop picks every node's larger child by ballot and moves the path
+//     from the root together; larger heaps replay the steps on lane 0.  The
 //     neighbours of an expanded node are checked against a per-warp visited
 //     bitmap and their distances computed in parallel first, then offered in
 //     list order.
 // Distances are the reference's sequential float sums (one lane per
-// distance), equal to vmath.cpp:56-88 bit for bit.
+// distance), equal to vmath.cpp:56-88 bit for bit.  The rows come through
+// shared memory, a coalesced copy each: a lane reading its own row from global
+// memory 16 bytes at a time touched 20 lines per load instruction, and the
+// candidate heap in HBM put an L2 round trip under every level of a pop.
+// Bound: latency of a query's chain (lane 0's heap steps, then list, visited
+// bits and rows), all queries of a batch at once.  2,000 queries, beam 60,
+// 100,000 x 128 rows: 1,366 -> 1,215 us, the length of the longest query's
+// chain (120 expansions, 2M cycles: offers 1,700 each, 2,300 before; rows
+// 5,000 and a pop 1,350 an expansion, 2,100 before).
 #include <algorithm>
 #include <string>
 #include <vector>
 
 #include "nnm_hier.h"
 #include "nnm_launch.h"
+#include "nnm_tc.cuh"
 
 namespace nnm {
 namespace {
@@ -41,8 +54,16 @@ struct HP {
     uint32_t id;
 };
 
+// The candidate heap: entries below CAND_SMEM in shared memory.
+constexpr uint32_t CAND_SMEM = 256;
+struct CandHeap {
+    HP *s, *g;
+    __device__ __forceinline__ HP& operator[](int i) const { return i < (int)CAND_SMEM ? s[i] : g[i]; }
+};
+
 // libstdc++ push_heap / pop_heap on a max-heap by .f (one thread).
-__device__ __forceinline__ void heap_push(HP* h, uint32_t& n, HP v) {
+template <class H>
+__device__ __forceinline__ void heap_push(H h, uint32_t& n, HP v) {
     int hole = (int)n++;
     int parent = (hole - 1) / 2;
     while (hole > 0 && h[parent].f < v.f) {
@@ -52,7 +73,8 @@ __device__ __forceinline__ void heap_push(HP* h, uint32_t& n, HP v) {
     }
     h[hole] = v;
 }
-__device__ __forceinline__ void heap_pop(HP* h, uint32_t& n) {
+template <class H>
+__device__ __forceinline__ void heap_pop(H h, uint32_t& n) {
     if (n == 0) return;
     if (n > 1) {
         const int len = (int)n - 1;
@@ -79,6 +101,115 @@ __device__ __forceinline__ void heap_pop(HP* h, uint32_t& n) {
         h[hole] = v;
     }
     n--;
+}
+
+constexpr uint32_t COOP = 256;  // entries of the heaps that the warp handles together
+
+// heap_push of v on the n entries of h (shared memory), by the whole warp.
+__device__ __forceinline__ void coop_push(HP* h, uint32_t n, HP v, int lane) {
+    const uint32_t at = n + 1;  // 1-based: the parent of i is i / 2
+    const uint32_t up = lane < 31 ? at >> (lane + 1) : 0u;
+    HP a{0.f, 0u};
+    if (up) a = h[up - 1];
+    const uint32_t k = __ffs(__ballot_sync(FULL, !(up && a.f < v.f))) - 1;  // ancestors that move down
+    if ((uint32_t)lane < k) h[(at >> lane) - 1] = a;
+    if (lane == 0) h[(at >> k) - 1] = v;
+    __syncwarp();
+}
+
+// heap_pop of the n <= COOP entries of h (shared memory), by the whole warp:
+// the hole follows the larger children to a leaf, then the last entry v climbs
+// from there -- so with the path p_0 = 0, p_1, .., p_k, the entries up to the
+// last one that is not smaller than v move up by one and v follows them.
+__device__ __forceinline__ void coop_pop(HP* h, uint32_t n, int lane) {
+    if (n < 2) return;
+    const uint32_t len = n - 1, inner = (len - 1) / 2;  // nodes with two children
+    const HP v = h[len];
+    uint32_t left[COOP / 64];
+#pragma unroll
+    for (uint32_t q = 0; q < COOP / 64; q++) {
+        left[q] = 0;
+        if (32 * q >= inner) break;
+        const uint32_t i = 32 * q + lane;
+        left[q] = __ballot_sync(FULL, i < inner && h[2 * i + 2].f < h[2 * i + 1].f);
+    }
+    uint32_t pos = 0, k = 0, mine = 0;  // lane i: p_i
+    while (pos < inner) {
+        uint32_t w = left[0];
+#pragma unroll
+        for (uint32_t q = 1; q < COOP / 64; q++)
+            if (pos >> 5 == q) w = left[q];
+        pos = 2 * pos + 2 - (w >> (pos & 31) & 1u);
+        k++;
+        if ((uint32_t)lane == k) mine = pos;
+    }
+    if ((len & 1) == 0 && pos == (len - 2) / 2) {
+        pos = 2 * pos + 1;
+        k++;
+        if ((uint32_t)lane == k) mine = pos;
+    }
+    const bool on = lane > 0 && (uint32_t)lane <= k;
+    HP o{0.f, 0u};
+    if (on) o = h[mine];
+    const unsigned keep = __ballot_sync(FULL, on && !(o.f < v.f));
+    const int last = keep ? 31 - __clz(keep) : 0;
+    const uint32_t prev = __shfl_up_sync(FULL, mine, 1);
+    if (on && lane <= last) h[prev] = o;
+    if (lane == last) h[mine] = v;
+    __syncwarp();
+}
+
+// Pushes and pops of either size.
+__device__ __forceinline__ void warp_push(const CandHeap& h, uint32_t& n, HP v, int lane) {
+    if (n < COOP) {
+        coop_push(h.s, n, v, lane);
+        n++;
+    } else {
+        uint32_t m = n;
+        if (lane == 0) heap_push(h, m, v);
+        n++;
+        __syncwarp();
+    }
+}
+__device__ __forceinline__ void warp_pop(const CandHeap& h, uint32_t& n, int lane) {
+    if (n <= COOP) {
+        coop_pop(h.s, n, lane);
+    } else {
+        uint32_t m = n;
+        if (lane == 0) heap_pop(h, m);
+        __syncwarp();
+    }
+    if (n) n--;
+}
+__device__ __forceinline__ void warp_push(HP* h, uint32_t& n, HP v, int lane) {
+    coop_push(h, n, v, lane);  // any size in shared memory: at most 11 ancestors
+    n++;
+}
+__device__ __forceinline__ void warp_pop(HP* h, uint32_t& n, int lane) {
+    if (n <= COOP) {
+        coop_pop(h, n, lane);
+    } else {
+        uint32_t m = n;
+        if (lane == 0) heap_pop(h, m);
+        __syncwarp();
+    }
+    if (n) n--;
+}
+
+// The reference's sequential sum over staged rows, four reads of each side
+// in flight.
+template <int M>
+__device__ __forceinline__ float dist_staged(const float* a, const float* b, uint32_t dp) {
+    float acc = 0.f;
+#pragma unroll 4
+    for (uint32_t t = 0; t < dp; t += 4) {
+        const float4 va = *reinterpret_cast<const float4*>(a + t), vb = *reinterpret_cast<const float4*>(b + t);
+        acc = dist_step<M>(acc, va.x, vb.x);
+        acc = dist_step<M>(acc, va.y, vb.y);
+        acc = dist_step<M>(acc, va.z, vb.z);
+        acc = dist_step<M>(acc, va.w, vb.w);
+    }
+    return acc;
 }
 
 struct SearchArgs {
@@ -110,6 +241,7 @@ struct SearchArgs {
     unsigned long long* nexp;
     unsigned* overflow;     // bit 0: candidate heap full; bits 1..: self-check failures
     uint32_t nrows[16];     // rows of each layer
+    uint32_t rb;            // rows staged in shared memory at a time (0: read from global memory)
 };
 
 enum : unsigned {
@@ -120,19 +252,60 @@ enum : unsigned {
     SERR_BEAM_RANGE = 32u, // a per-query beam width outside [out_k, beam_cap]
 };
 
-__global__ void k_search(SearchArgs a) {
+// Shared memory of one warp: the query, the staged rows (an odd number of
+// 16-byte units apart, so that lanes reading their own rows at the same offset
+// fall in different banks), the results heap, the offered distances and ids, the
+// candidate heap's head.
+__host__ __device__ constexpr uint32_t row_units(uint32_t dp) { return (dp / 4) | 1u; }
+__host__ __device__ constexpr size_t search_warp_bytes(uint32_t dp, uint32_t beam_cap, uint32_t rb) {
+    return ((size_t)dp * 4 + (size_t)rb * row_units(dp) * 16 + (size_t)(beam_cap + 1) * 8 + 32 * 8 + CAND_SMEM * 8 + 15) &
+           ~(size_t)15;
+}
+
+// Exact distances from qv to the rows nn of the lanes with `want` (0 in the
+// others), rb rows at a time through `rows`.
+__device__ __forceinline__ float rows_exact(const SearchArgs& a, const float* qv, float4* rows, uint32_t nn, bool want,
+                                            int lane) {
+    if (!a.rb) return want ? dist_seq_rt(a.metric, qv, a.x + (size_t)nn * a.dp, a.dp) : 0.f;
+    const uint32_t dq = a.dp >> 2, units = row_units(a.dp), base = smem_u32(rows);
+    unsigned todo = __ballot_sync(FULL, want);
+    float dd = 0.f;
+    while (todo) {
+        unsigned left = todo;
+        uint32_t mine = 0xffffffffu;
+        for (uint32_t k = 0; k < a.rb && left; k++, left &= left - 1) {
+            const int j = __ffs(left) - 1;
+            if (lane == j) mine = k;
+            const uint32_t id = __shfl_sync(FULL, nn, j);
+            for (uint32_t c = lane; c < dq; c += 32)
+                cp_async16(base + (k * units + c) * 16, reinterpret_cast<const float4*>(a.x) + (size_t)id * dq + c);
+        }
+        asm volatile("cp.async.wait_all;" ::: "memory");
+        __syncwarp();
+        if (mine != 0xffffffffu) {
+            const float* r = reinterpret_cast<const float*>(rows + mine * units);
+            dd = a.metric == L2 ? dist_staged<L2>(qv, r, a.dp)
+                                : (a.metric == L1 ? dist_staged<L1>(qv, r, a.dp) : dist_staged<CHI2>(qv, r, a.dp));
+        }
+        __syncwarp();
+        todo = left;
+    }
+    return dd;
+}
+
+__global__ void __launch_bounds__(SWARPS * 32) k_search(SearchArgs a) {
     extern __shared__ __align__(16) unsigned char smem[];
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const uint32_t slot = blockIdx.x * SWARPS + w;
-    const size_t wbytes = (size_t)a.dp * 4 + (size_t)(a.beam_cap + 1) * 8 + 32 * 8;
-    unsigned char* base = smem + (size_t)w * ((wbytes + 15) & ~(size_t)15);
+    unsigned char* base = smem + (size_t)w * search_warp_bytes(a.dp, a.beam_cap, a.rb);
     float* qv = reinterpret_cast<float*>(base);
-    HP* top = reinterpret_cast<HP*>(base + (size_t)a.dp * 4);
+    float4* rows = reinterpret_cast<float4*>(base + (size_t)a.dp * 4);
+    HP* top = reinterpret_cast<HP*>(rows + (size_t)a.rb * row_units(a.dp));
     float* stage_d = reinterpret_cast<float*>(top + a.beam_cap + 1);
     uint32_t* stage_i = reinterpret_cast<uint32_t*>(stage_d + 32);
     uint32_t* vis = a.visited + (size_t)slot * a.words;
     uint32_t* vl = a.vlist + (size_t)slot * VCAP;
-    HP* cand = a.cand + (size_t)slot * CCAP;
+    const CandHeap cand{reinterpret_cast<HP*>(stage_i + 32), a.cand + (size_t)slot * CCAP};
     unsigned long long cmps = 0, nexp = 0;
     for (;;) {
         unsigned qi = 0;
@@ -190,12 +363,8 @@ __global__ void k_search(SearchArgs a) {
                 }
                 const uint64_t b = off[cur], e = off[cur + 1];  // the list of the node at loop entry
                 for (uint64_t c0 = b; c0 < e; c0 += 32) {
-                    uint32_t nn = 0;
-                    float dd = 0.f;
-                    if (c0 + lane < e) {
-                        nn = a.adj_all[c0 + lane];
-                        dd = dist_seq_rt(a.metric, qv, a.x + (size_t)nn * a.dp, a.dp);
-                    }
+                    const uint32_t nn = c0 + lane < e ? a.adj_all[c0 + lane] : 0u;
+                    const float dd = rows_exact(a, qv, rows, nn, c0 + lane < e, lane);
                     const uint32_t cnt = (uint32_t)(e - c0 < 32 ? e - c0 : 32);
                     cmps += cnt;
                     for (uint32_t j = 0; j < cnt; j++) {
@@ -222,23 +391,23 @@ __global__ void k_search(SearchArgs a) {
             nvis = 0;
             for (uint32_t c0 = 0; c0 < topk; c0 += 32) {
                 const uint32_t cnt = min(32u, topk - c0);
+                const uint32_t id = lane < cnt ? sd[c0 + lane] : 0u;
+                const float dd = rows_exact(a, qv, rows, id, lane < cnt, lane);
                 if (lane < cnt) {
-                    const uint32_t id = sd[c0 + lane];
                     stage_i[lane] = id;
-                    stage_d[lane] = dist_seq_rt(a.metric, qv, a.x + (size_t)id * a.dp, a.dp);
+                    stage_d[lane] = dd;
                     atomicOr(&vis[id >> 5], 1u << (id & 31));
                     if (nvis + lane < VCAP) vl[nvis + lane] = id;
                 }
                 __syncwarp();
-                if (lane == 0)
-                    for (uint32_t r = 0; r < cnt; r++) {
-                        if (ncand >= CCAP) {
-                            atomicOr(a.overflow, SERR_HEAP);
-                            break;
-                        }
-                        heap_push(cand, ncand, HP{-stage_d[r], stage_i[r]});
-                        heap_push(top, ntop, HP{stage_d[r], stage_i[r]});
+                for (uint32_t r = 0; r < cnt; r++) {
+                    if (ncand >= CCAP) {
+                        if (lane == 0) atomicOr(a.overflow, SERR_HEAP);
+                        break;
                     }
+                    warp_push(cand, ncand, HP{-stage_d[r], stage_i[r]}, lane);
+                    warp_push(top, ntop, HP{stage_d[r], stage_i[r]}, lane);
+                }
                 __syncwarp();
                 nvis += cnt;
                 cmps += cnt;
@@ -246,37 +415,34 @@ __global__ void k_search(SearchArgs a) {
             if (nvis > VCAP) vis_overflow = true;
         } else {
             start_ok = cur < a.nrows[a.L - 1];  // false only after a failed greedy check
-            if (lane == 0 && start_ok) {
-                heap_push(cand, ncand, HP{-cur_d, cur});
-                heap_push(top, ntop, HP{cur_d, cur});
-                atomicOr(&vis[cur >> 5], 1u << (cur & 31));
-                vl[0] = cur;
+            if (start_ok) {
+                warp_push(cand, ncand, HP{-cur_d, cur}, lane);
+                warp_push(top, ntop, HP{cur_d, cur}, lane);
+                if (lane == 0) {
+                    atomicOr(&vis[cur >> 5], 1u << (cur & 31));
+                    vl[0] = cur;
+                }
             }
         }
-        ncand = __shfl_sync(FULL, ncand, 0);
-        ntop = __shfl_sync(FULL, ntop, 0);
         __syncwarp();
         if (!start_ok) nvis = 0;
-        float lwbnd = 0.f;
-        if (lane == 0 && start_ok) lwbnd = top[0].f;
-        lwbnd = __shfl_sync(FULL, lwbnd, 0);
+        float lwbnd = start_ok ? top[0].f : 0.f;
         const uint32_t nlast = a.nrows[a.L - 1];
         uint32_t expansions = 0;
         while (ncand > 0) {
-            // Lane 0 alone reads the heaps and broadcasts through registers:
-            // a value every lane loaded itself could be re-read after lane
-            // 0's next update, and lanes that disagree would diverge.
-            HP c{0.f, 0u};
-            if (lane == 0) c = cand[0];
+            // Every heap update ends with a warp barrier; a value read from a
+            // heap is broadcast, so that lanes cannot disagree on it whatever
+            // the compiler does with the read.
+            HP c = cand.s[0];
             c.f = __shfl_sync(FULL, c.f, 0);
             c.id = __shfl_sync(FULL, c.id, 0);
+            __syncwarp();
             if (-c.f > lwbnd) break;
             if (c.id >= nlast || ++expansions > nlast + 1) {
                 if (lane == 0) atomicOr(a.overflow, c.id >= nlast ? SERR_BAD_ID : SERR_BEAM_CAP);
                 break;
             }
-            if (lane == 0) heap_pop(cand, ncand);
-            ncand = __shfl_sync(FULL, ncand, 0);
+            warp_pop(cand, ncand, lane);
             nexp++;
             const uint64_t b = off[c.id], e = off[c.id + 1];
             for (uint64_t c0 = b; c0 < e; c0 += 32) {
@@ -292,10 +458,11 @@ __global__ void k_search(SearchArgs a) {
                     }
                 }
                 const unsigned fb = __ballot_sync(FULL, fresh);
+                const float dd = rows_exact(a, qv, rows, nn, fresh, lane);
                 if (fresh) {
                     const uint32_t r = __popc(fb & ((1u << lane) - 1u));
                     if (nvis + r < VCAP) vl[nvis + r] = nn;
-                    stage_d[r] = dist_seq_rt(a.metric, qv, a.x + (size_t)nn * a.dp, a.dp);
+                    stage_d[r] = dd;
                     stage_i[r] = nn;
                 }
                 const uint32_t nf = __popc(fb);
@@ -303,43 +470,41 @@ __global__ void k_search(SearchArgs a) {
                 if (nvis > VCAP) vis_overflow = true;
                 cmps += nf;
                 __syncwarp();
-                if (lane == 0) {  // offers in list order (lysearch.cpp:284-295)
-                    for (uint32_t r = 0; r < nf; r++) {
-                        const float dj = stage_d[r];
-                        if (top[0].f > dj || ntop < topk) {
-                            if (ncand >= CCAP) {
-                                atomicOr(a.overflow, SERR_HEAP);
-                                continue;
-                            }
-                            heap_push(cand, ncand, HP{-dj, stage_i[r]});
-                            heap_push(top, ntop, HP{dj, stage_i[r]});
-                            if (ntop > topk) heap_pop(top, ntop);
+                for (uint32_t r = 0; r < nf; r++) {  // offers in list order (lysearch.cpp:284-295)
+                    const float dj = __shfl_sync(FULL, stage_d[r], 0);
+                    const uint32_t ij = __shfl_sync(FULL, stage_i[r], 0);
+                    const float worst = __shfl_sync(FULL, top[0].f, 0);
+                    __syncwarp();
+                    if (worst > dj || ntop < topk) {
+                        if (ncand >= CCAP) {
+                            if (lane == 0) atomicOr(a.overflow, SERR_HEAP);
+                            continue;
                         }
+                        warp_push(cand, ncand, HP{-dj, ij}, lane);
+                        warp_push(top, ntop, HP{dj, ij}, lane);
+                        if (ntop > topk) warp_pop(top, ntop, lane);
                     }
                 }
                 __syncwarp();
-                ncand = __shfl_sync(FULL, ncand, 0);
-                ntop = __shfl_sync(FULL, ntop, 0);
-                float lw = 0.f;
-                if (lane == 0) lw = top[0].f;
-                lwbnd = __shfl_sync(FULL, lw, 0);
+                lwbnd = __shfl_sync(FULL, top[0].f, 0);
             }
         }
         // results ascending, popped from the max-heap into place (lysearch.cpp:302-312);
         // the first out_k are kept
-        if (lane == 0) {
-            const size_t o = (size_t)qi * a.out_k;
-            for (uint32_t t = ntop; t < a.out_k; t++) {
-                a.out_ids[o + t] = 0xffffffffu;
-                if (a.out_d) a.out_d[o + t] = 0.f;
+        const size_t o = (size_t)qi * a.out_k;
+        for (uint32_t t = ntop + lane; t < a.out_k; t += 32) {
+            a.out_ids[o + t] = 0xffffffffu;
+            if (a.out_d) a.out_d[o + t] = 0.f;
+        }
+        __syncwarp();
+        while (ntop > 0) {
+            const uint32_t loc = ntop - 1;
+            if (loc < a.out_k && lane == 0) {
+                a.out_ids[o + loc] = top[0].id;
+                if (a.out_d) a.out_d[o + loc] = top[0].f;
             }
-            for (int loc = (int)ntop - 1; loc >= 0; loc--) {
-                if ((uint32_t)loc < a.out_k) {
-                    a.out_ids[o + loc] = top[0].id;
-                    if (a.out_d) a.out_d[o + loc] = top[0].f;
-                }
-                heap_pop(top, ntop);
-            }
+            __syncwarp();
+            warp_pop(top, ntop, lane);
         }
         // clear the visited bits of this query
         if (!vis_overflow) {
@@ -445,9 +610,14 @@ int index_run_exact(Ctx& ctx, IndexDev& ix, const SearchReq& r) {
     const uint32_t dp = ix.dp;
     int nsm = 148;
     cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, ctx.device);
-    const size_t wbytes = (size_t)dp * 4 + (size_t)(r.beam_max + 1) * 8 + 32 * 8;
-    const size_t smem = (size_t)SWARPS * ((wbytes + 15) & ~(size_t)15) + 64;
-    if (smem > 200 * 1024) {
+    // rows staged at a time: 16 while four blocks fit on an SM, fewer for long
+    // rows and wide beams, none where two rows no longer fit beside the heaps
+    auto bytes_of = [&](uint32_t rb) { return (size_t)SWARPS * search_warp_bytes(dp, r.beam_max, rb) + 64; };
+    uint32_t rb = 16;
+    while (rb > 2 && bytes_of(rb) > 56 * 1024) rb /= 2;
+    if (bytes_of(rb) > 112 * 1024) rb = 0;
+    const size_t smem = bytes_of(rb);
+    if (smem > 200 * 1024 + (size_t)SWARPS * CAND_SMEM * 8) {
         ctx.last_error = "beam too wide for shared memory at this dimension";
         return 1;
     }
@@ -491,6 +661,7 @@ int index_run_exact(Ctx& ctx, IndexDev& ix, const SearchReq& r) {
     a.flat_pool = r.flat_pool;
     a.out_ids = r.out_ids;
     a.out_d = r.out_d;
+    a.rb = rb;
     a.visited = ix.visited.as<uint32_t>();
     a.words = words;
     a.vlist = ix.vlist.as<uint32_t>();
