@@ -424,8 +424,8 @@ int upload_vectors(Ctx& ctx, GraphStore& s, GraphDev& g, const float* x, bool x_
     const size_t elems = (size_t)g.n_cap * g.dp;
     NNM_CUDA_TRY(s.x.ensure(elems * 4));
     if (g.dp == g.d) {
-        NNM_CUDA_TRY(cudaMemcpyAsync(s.x.p, x, elems * 4, x_on_device ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice,
-                                     ctx.stream));
+        if (x_on_device) NNM_CUDA_TRY(cudaMemcpyAsync(s.x.p, x, elems * 4, cudaMemcpyDeviceToDevice, ctx.stream));
+        else NNM_CUDA_TRY(host_to_dev(ctx, s.x.p, x, elems * 4));
     } else {
         // rows padded to 16 bytes: host rows land in the proposal buckets,
         // which are free until the first join (an allocation and its free a
@@ -434,7 +434,7 @@ int upload_vectors(Ctx& ctx, GraphStore& s, GraphDev& g, const float* x, bool x_
         if (!x_on_device) {
             DevBuf& stage = ctx.ws.bucket;
             NNM_CUDA_TRY(stage.ensure((size_t)g.n_cap * g.d * 4));
-            NNM_CUDA_TRY(cudaMemcpyAsync(stage.p, x, (size_t)g.n_cap * g.d * 4, cudaMemcpyHostToDevice, ctx.stream));
+            NNM_CUDA_TRY(host_to_dev(ctx, stage.p, x, (size_t)g.n_cap * g.d * 4));
             src = stage.as<float>();
         }
         k_pad_copy<<<blocks_for(elems, 256), 256, 0, ctx.stream>>>(src, s.x.as<float>(), g.n_cap, g.d, g.dp); count_launch();
@@ -467,10 +467,8 @@ int export_graph(Ctx& ctx, const GraphDev& g, uint32_t* ids, float* dists, uint8
     float* dd = reinterpret_cast<float*>(di + cnt);
     uint8_t* df = reinterpret_cast<uint8_t*>(dd + cnt);
     k_export<<<blocks_for(cnt, 256), 256, 0, ctx.stream>>>(g.pid, g.pdist, cnt, di, dd, df); count_launch();
-    if (ids) NNM_CUDA_TRY(cudaMemcpyAsync(ids, di, cnt * 4, cudaMemcpyDeviceToHost, ctx.stream));
-    if (dists) NNM_CUDA_TRY(cudaMemcpyAsync(dists, dd, cnt * 4, cudaMemcpyDeviceToHost, ctx.stream));
-    if (flags) NNM_CUDA_TRY(cudaMemcpyAsync(flags, df, cnt, cudaMemcpyDeviceToHost, ctx.stream));
-    NNM_CUDA_TRY(cudaStreamSynchronize(ctx.stream));
+    const HostPiece out[] = {{ids, di, cnt * 4}, {dists, dd, cnt * 4}, {flags, df, cnt}};
+    NNM_CUDA_TRY(dev_to_host(ctx, out, 3));
     return 0;
 }
 

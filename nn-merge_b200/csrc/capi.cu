@@ -300,6 +300,7 @@ int nnm_ctx_destroy(nnm_ctx* ctx) {
         ctx->c.dpg->release();
         delete ctx->c.dpg;
     }
+    ctx->c.stage.release();
     if (ctx->c.h_counters) cudaFreeHost(ctx->c.h_counters);
     if (ctx->c.stream) cudaStreamDestroy(ctx->c.stream);
     delete ctx;
@@ -1007,7 +1008,7 @@ int index_search_impl(nnm_index* h, const float* q, uint64_t nq, const uint32_t*
     } else if (!dev || dp != d) {
         if ((rc = cu(ix.qpad.ensure((size_t)nq * dp * 4)))) return rc;
         const cudaMemcpyKind kind = dev ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice;
-        if (dp == d) rc = cu(cudaMemcpyAsync(ix.qpad.p, q, (size_t)nq * d * 4, kind, st));
+        if (dp == d) rc = cu(nnm::host_to_dev(c, ix.qpad.p, q, (size_t)nq * d * 4));  // not dev: dp != d there
         else {
             rc = cu(cudaMemset2DAsync(ix.qpad.p, dp * 4, 0, dp * 4, nq, st));
             if (!rc) rc = cu(cudaMemcpy2DAsync(ix.qpad.p, dp * 4, q, d * 4, d * 4, nq, kind, st));
@@ -1076,9 +1077,8 @@ int index_search_impl(nnm_index* h, const float* q, uint64_t nq, const uint32_t*
         rc = nnm::index_counters(c, ix, &ncmps, &nexp);
     }
     if (!rc && !dev && !small) {
-        rc = cu(cudaMemcpyAsync(out_ids, oi, (size_t)nq * out_k * 4, cudaMemcpyDeviceToHost, st));
-        if (!rc && out_d) rc = cu(cudaMemcpyAsync(out_d, od, (size_t)nq * out_k * 4, cudaMemcpyDeviceToHost, st));
-        if (!rc) rc = cu(cudaStreamSynchronize(st));
+        const nnm::HostPiece out[] = {{out_ids, oi, (size_t)nq * out_k * 4}, {out_d, od, (size_t)nq * out_k * 4}};
+        rc = cu(nnm::dev_to_host(c, out, 2));
     }
     if (!rc && stats) {
         float a = 0.f, b = 0.f;

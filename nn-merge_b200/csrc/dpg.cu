@@ -409,14 +409,14 @@ int dpg_layer(Ctx& ctx, DpgState& s, GraphDev& g, nnm_layers* out) {
         std::unique_ptr<uint64_t, decltype(&std::free)> off(
             static_cast<uint64_t*>(std::malloc(sizeof(uint64_t) * ((size_t)N + 1))), &std::free);
         if (!off) return 4;
-        NNM_CUDA_TRY(cudaMemcpyAsync(off.get(), s.eoff.p, ((size_t)N + 1) * 8, cudaMemcpyDeviceToHost, st));
-        NNM_CUDA_TRY(cudaStreamSynchronize(st));
+        const HostPiece po{off.get(), s.eoff.p, ((size_t)N + 1) * 8};
+        NNM_CUDA_TRY(dev_to_host(ctx, &po, 1));
         const uint64_t total = off.get()[N];
         std::unique_ptr<uint32_t, decltype(&std::free)> adj(
             static_cast<uint32_t*>(std::malloc(sizeof(uint32_t) * std::max<uint64_t>(total, 1))), &std::free);
         if (!adj) return 4;
-        NNM_CUDA_TRY(cudaMemcpyAsync(adj.get(), s.ev.p, total * 4, cudaMemcpyDeviceToHost, st));
-        NNM_CUDA_TRY(cudaStreamSynchronize(st));
+        const HostPiece pa{adj.get(), s.ev.p, total * 4};
+        NNM_CUDA_TRY(dev_to_host(ctx, &pa, 1));
         out->nrows[L] = N;
         out->off[L] = off.release();
         out->adj[L] = adj.release();

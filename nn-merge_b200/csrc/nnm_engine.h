@@ -9,6 +9,7 @@
 
 #include <cuda_runtime.h>
 
+#include "nnm_hostcopy.h"
 #include "nnm_nnd.h"
 #include "nnm_rng.h"
 
@@ -115,6 +116,7 @@ struct Ctx {
         uint64_t launches = 0;
     } iter_graph[4];
     cudaStream_t stream = nullptr;
+    HostStage stage;  // pinned slots of host copies
     Workspace ws;
     IterCounters* h_counters = nullptr;  // pinned
     std::string last_error;

@@ -584,7 +584,7 @@ int index_upload(Ctx& ctx, IndexDev& ix, const float* x, uint64_t n, uint32_t d,
     NNM_CUDA_TRY(ix.adj.ensure(std::max<uint64_t>(adj_total, 1) * 4));
     NNM_CUDA_TRY(ix.ctr.ensure(64));
     if (dp == d) {
-        NNM_CUDA_TRY(cudaMemcpyAsync(ix.x.p, x, (size_t)n * d * 4, cudaMemcpyHostToDevice, st));
+        NNM_CUDA_TRY(host_to_dev(ctx, ix.x.p, x, (size_t)n * d * 4));
     } else {
         NNM_CUDA_TRY(cudaMemset2DAsync(ix.x.p, dp * 4, 0, dp * 4, n, st));
         NNM_CUDA_TRY(cudaMemcpy2DAsync(ix.x.p, dp * 4, x, d * 4, d * 4, n, cudaMemcpyHostToDevice, st));
@@ -599,9 +599,10 @@ int index_upload(Ctx& ctx, IndexDev& ix, const float* x, uint64_t n, uint32_t d,
         NNM_CUDA_TRY(cudaMemcpy(ix.off.as<uint64_t>() + ix.off_base[g], off.data(), off.size() * 8,
                                 cudaMemcpyHostToDevice));
         uint64_t cnt = layers->off[g][layers->nrows[g]];
-        if (cnt) NNM_CUDA_TRY(cudaMemcpy(ix.adj.as<uint32_t>() + adj_total, layers->adj[g], cnt * 4, cudaMemcpyHostToDevice));
+        if (cnt) NNM_CUDA_TRY(host_to_dev(ctx, ix.adj.as<uint32_t>() + adj_total, layers->adj[g], cnt * 4));
         adj_total += cnt;
     }
+    NNM_CUDA_TRY(cudaStreamSynchronize(st));  // the caller's arrays are free again
     return 0;
 }
 
