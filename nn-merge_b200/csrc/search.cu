@@ -739,7 +739,7 @@ int index_check(Ctx& ctx, const unsigned long long* c, uint64_t* ncmps, uint64_t
 }
 
 void IndexDev::release() {
-    DevBuf* all[] = {&x,     &off,   &adj,  &visited, &vlist,  &cand,     &ctr,      &qpad,
+    DevBuf* all[] = {&x,     &off,   &adj,  &visited, &vlist,  &cand,         &ctr,      &qpad,
                      &beams, &probes, &hid, &scores,  &out,    &flat_off, &flat_pool};
     for (auto* b : all) b->release();
     if (h_io) cudaFreeHost(h_io);

@@ -42,8 +42,11 @@ constexpr uint32_t FVCAP = 65536;        // visited ids recorded per warp slot
 constexpr uint32_t EXP_BIT = 1u << 31;   // beam entry already expanded
 constexpr uint32_t IDM = 0x7fffffffu;
 constexpr uint32_t FAST_MAX_DP = 512;    // 4 float4 per lane
+constexpr uint32_t DENSE_WARPS = 28;                    // k_serve's dense form: warps per SM ..
+constexpr uint32_t DENSE_QUERIES = 2 * DENSE_WARPS;     // .. for more queries per SM than these
+constexpr size_t DENSE_BITMAPS = (size_t)128 << 20;     // .. and at most this much of visited bitmaps
 constexpr uint32_t GROUP = 4;            // 32-id chunks of a step whose loads and atomics overlap
-constexpr uint32_t WARP_EXTRA = 256 + GROUP * 32 * 4;  // nd, ni and fr after the two beam arrays
+constexpr uint32_t WARP_EXTRA = 256 + GROUP * 32 * 4;  // nd, ni and fr after the beam's two arrays
 
 // self-check codes, shared with the exact kernel's report
 enum : unsigned { FERR_LOOP = 4u, FERR_BAD_ID = 8u, FERR_BEAM_RANGE = 32u };
@@ -168,6 +171,52 @@ __device__ __forceinline__ float warp_dists(const float4 (&qr)[QV], const float4
     return v[0];
 }
 
+// The same distances, NB rows at a time from load to sum: 40 registers fewer,
+// so that seven CTAs fit on an SM, for a longer chain per batch (see k_serve).
+template <int M, int QV>
+__device__ __forceinline__ float warp_dists_short(const float4 (&qr)[QV], const float4* __restrict__ x4, uint32_t dp4,
+                                                  uint32_t fid, uint32_t nf, uint32_t lane) {
+    constexpr uint32_t NB = QV == 1 ? 8 : (QV == 2 ? 4 : 2);  // rows in flight per lane
+    constexpr uint32_t PER = 32 / NB;                         // lanes b PER .. end with row b's sum
+    float out = 0.f;
+#pragma unroll 1
+    for (uint32_t j0 = 0; j0 < nf; j0 += NB) {
+        float4 r[NB][QV];
+#pragma unroll
+        for (uint32_t b = 0; b < NB; b++) {
+            const uint32_t id = __shfl_sync(FULL, fid, (j0 + b) & 31);
+#pragma unroll
+            for (int t = 0; t < QV; t++) {
+                const uint32_t c4 = lane + 32u * t;
+                r[b][t] = make_float4(0.f, 0.f, 0.f, 0.f);
+                if (j0 + b < nf && c4 < dp4) r[b][t] = __ldg(x4 + (size_t)id * dp4 + c4);
+            }
+        }
+        float v[NB];
+#pragma unroll
+        for (uint32_t b = 0; b < NB; b++) {
+            v[b] = 0.f;
+#pragma unroll
+            for (int t = 0; t < QV; t++) v[b] = part4<M>(qr[t], r[b][t], v[b]);
+        }
+        uint32_t s = 16;
+#pragma unroll
+        for (uint32_t n = NB / 2; n >= 1; n >>= 1, s >>= 1) {
+            const bool up = (lane & s) != 0;
+#pragma unroll
+            for (uint32_t i = 0; i < n; i++) {
+                const float send = up ? v[i] : v[i + n], keep = up ? v[i + n] : v[i];
+                v[i] = keep + __shfl_xor_sync(FULL, send, s);
+            }
+        }
+#pragma unroll
+        for (; s >= 1; s >>= 1) v[0] += __shfl_xor_sync(FULL, v[0], s);
+        const float mine = __shfl_sync(FULL, v[0], ((lane - j0) & (NB - 1)) * PER);
+        if (lane >= j0 && lane < j0 + NB && lane < nf) out = mine;
+    }
+    return out;
+}
+
 __device__ __forceinline__ bool key_less(float da, uint32_t ia, float db, uint32_t ib) {
     return da < db || (da == db && ia < ib);
 }
@@ -211,27 +260,39 @@ __device__ __forceinline__ void warp_sort(float& d, uint32_t& id, uint32_t lane,
     }
 }
 
-// Five CTAs per SM (registers capped at 96, a few spilled): the kernel is
-// bound by memory latency, and 20 warps per SM hide it better than 16 --
-// 6 % faster on the 1M hierarchy than the uncapped 126 registers; six CTAs
-// spill more and lose again.
-template <int M, int QV>
-__global__ void __launch_bounds__(FW * 32, 5) k_serve(ServeArgs a) {
+__device__ __forceinline__ void prefetch_l1(const void* p) { asm volatile("prefetch.global.L1 [%0];" ::"l"(p)); }
+__device__ __forceinline__ void prefetch_l2(const void* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
+
+// Bound: memory latency of a step's chain (offsets, list ids, visited set,
+// rows) at the warps that are resident.  Two forms, the same steps and sums:
+// DENSE, for batches of several queries per resident warp: seven CTAs per SM
+// (72 registers: the rows of a list summed eight at a time, prefetched into L2
+// when their ids are known); otherwise five CTAs (96 registers, 32 rows summed
+// together), whose single query is shorter.  The line: 20,000 queries, 100,000
+// rows, five CTAs against seven: beams 16 872 -> 761 us, 64 2,690 -> 2,442,
+// 32..512 6,492 -> 5,206, d = 160 8,448 -> 5,962; 3,000 queries (one each) 1,726
+// -> 2,062.  At 1M rows the 28 warps' bitmaps (518 MB, allocated and cleared
+// by an index's first batch) gain 3 to 7 %, not worth it: so at most
+// DENSE_BITMAPS of them.  A hash table per query instead of a bitmap there took
+// 1.5 times as long.
+template <int M, int QV, bool DENSE>
+__global__ void __launch_bounds__(FW * 32, DENSE ? 7 : 5) k_serve(ServeArgs a) {
     extern __shared__ __align__(16) unsigned char smem[];
     const uint32_t w = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const uint32_t slot = blockIdx.x * FW + w;
-    unsigned char* base = smem + (size_t)w * ((size_t)a.cap * 16 + WARP_EXTRA);
+    unsigned char* base = smem + (size_t)w * ((size_t)a.cap * 8 + WARP_EXTRA);
     float* bd = reinterpret_cast<float*>(base);
     uint32_t* bi = reinterpret_cast<uint32_t*>(bd + a.cap);
-    float* td = reinterpret_cast<float*>(bi + a.cap);
-    uint32_t* ti = reinterpret_cast<uint32_t*>(td + a.cap);
-    float* nd = reinterpret_cast<float*>(ti + a.cap);
+    float* nd = reinterpret_cast<float*>(bi + a.cap);
     uint32_t* ni = reinterpret_cast<uint32_t*>(nd + 32);
     uint32_t* fr = ni + 32;  // fresh ids of one group of a step
     uint32_t* vis = a.visited + (size_t)slot * a.words;
     uint32_t* vl = a.vlist + (size_t)slot * FVCAP;
     const float4* x4 = reinterpret_cast<const float4*>(a.x);
     const uint32_t nlast = a.nrows[a.L - 1];
+    auto dists = [](const float4(&qr)[QV], const float4* x, uint32_t dp4, uint32_t fid, uint32_t nf, uint32_t lane) {
+        return DENSE ? warp_dists_short<M, QV>(qr, x, dp4, fid, nf, lane) : warp_dists<M, QV>(qr, x, dp4, fid, nf, lane);
+    };
     unsigned long long cmps = 0, nexp = 0;
     for (;;) {
         uint32_t qi = 0;
@@ -267,7 +328,7 @@ __global__ void __launch_bounds__(FW * 32, 5) k_serve(ServeArgs a) {
                     pid = 0;
                 }
             }
-            const float pd = warp_dists<M, QV>(qr, x4, a.dp4, pid, a.nprobe, lane);
+            const float pd = dists(qr, x4, a.dp4, pid, a.nprobe, lane);
             uint32_t l;
             warp_argmin(pd, a.nprobe, lane, cur_d, l);
             cur = __shfl_sync(FULL, pid, l & 31);
@@ -275,7 +336,7 @@ __global__ void __launch_bounds__(FW * 32, 5) k_serve(ServeArgs a) {
         } else {
             g0 = 0;
             cur = a.entry;
-            cur_d = __shfl_sync(FULL, warp_dists<M, QV>(qr, x4, a.dp4, cur, 1, lane), 0);
+            cur_d = __shfl_sync(FULL, dists(qr, x4, a.dp4, cur, 1, lane), 0);
             cmps++;
         }
         // greedy descent (lysearch.cpp:397-420); upper-layer ids were checked
@@ -295,7 +356,7 @@ __global__ void __launch_bounds__(FW * 32, 5) k_serve(ServeArgs a) {
                 for (uint64_t c0 = b; c0 < e; c0 += 32) {
                     const uint32_t cnt = (uint32_t)(e - c0 < 32 ? e - c0 : 32);
                     const uint32_t nn = lane < cnt ? a.adj_all[c0 + lane] : 0u;
-                    const float dd = warp_dists<M, QV>(qr, x4, a.dp4, nn, cnt, lane);
+                    const float dd = dists(qr, x4, a.dp4, nn, cnt, lane);
                     cmps += cnt;
                     float md;
                     uint32_t ml;
@@ -317,11 +378,10 @@ __global__ void __launch_bounds__(FW * 32, 5) k_serve(ServeArgs a) {
         // Offers the fresh rows whose ids lanes [0, nf) hold: distances, the
         // ones below the worst entry of a full beam sorted by a bitonic
         // network over those lanes and merged in place -- entries before the
-        // first new one keep their slots; the suffix [lo0, m) is staged, then
-        // every entry of the merged range [lo0, m2) is written once.
+        // first new one keep their slots.
         auto offer = [&](uint32_t fid, uint32_t nf) {
             cmps += nf;
-            const float dd = warp_dists<M, QV>(qr, x4, a.dp4, fid, nf, lane);
+            const float dd = dists(qr, x4, a.dp4, fid, nf, lane);
             bool acc = lane < nf;
             if (m >= ef) acc = acc && key_less(dd, fid, bd[m - 1], bi[m - 1] & IDM);
             const uint32_t nk = __popc(__ballot_sync(FULL, acc));
@@ -346,24 +406,32 @@ __global__ void __launch_bounds__(FW * 32, 5) k_serve(ServeArgs a) {
                 npos = lane + lo;
             }
             const uint32_t lo0 = __shfl_sync(FULL, npos, 0);
-            for (uint32_t i = lo0 + lane; i < m; i += 32) {
-                td[i - lo0] = bd[i];
-                ti[i - lo0] = bi[i];
-            }
             __syncwarp();
-            for (uint32_t i = lo0 + lane; i < m; i += 32) {
-                const float d0 = td[i - lo0];
-                const uint32_t i0 = ti[i - lo0];
-                uint32_t lo = 0, hi = nk;
-                while (lo < hi) {
-                    const uint32_t md = (lo + hi) >> 1;
-                    if (key_less(nd[md], ni[md], d0, i0 & IDM)) lo = md + 1;
-                    else hi = md;
+            // entries from lo0 on move up by the number of new entries before
+            // them, 32 at a time from the last: a chunk's places lie at or after
+            // its own, so the chunks still to come are intact
+            for (uint32_t s0 = m > lo0 ? lo0 + ((m - lo0 - 1) & ~31u) : 0u, more = m > lo0; more; s0 -= 32) {
+                const uint32_t i = s0 + lane;
+                float d0 = 0.f;
+                uint32_t i0 = 0;
+                if (i < m) {
+                    d0 = bd[i];
+                    i0 = bi[i];
                 }
-                if (i + lo < m2) {
-                    bd[i + lo] = d0;
-                    bi[i + lo] = i0;
+                __syncwarp();
+                if (i < m) {
+                    uint32_t lo = 0, hi = nk;
+                    while (lo < hi) {
+                        const uint32_t md = (lo + hi) >> 1;
+                        if (key_less(nd[md], ni[md], d0, i0 & IDM)) lo = md + 1;
+                        else hi = md;
+                    }
+                    if (i + lo < m2) {
+                        bd[i + lo] = d0;
+                        bi[i + lo] = i0;
+                    }
                 }
+                more = s0 > lo0;
             }
             if (lane < nk && npos < m2) {
                 bd[npos] = kd;
@@ -477,6 +545,8 @@ __global__ void __launch_bounds__(FW * 32, 5) k_serve(ServeArgs a) {
                     const unsigned fb = __ballot_sync(FULL, fresh[c]);
                     if (fresh[c]) {
                         const uint32_t r = nf + __popc(fb & ((1u << lane) - 1u));
+                        if (DENSE)
+                            for (uint32_t t = 0; t < a.dp4; t += 8) prefetch_l2(x4 + (size_t)nn[c] * a.dp4 + t);
                         fr[r] = nn[c];
                         if (nvis + r < FVCAP) vl[nvis + r] = nn[c];
                     }
@@ -537,8 +607,6 @@ __global__ void __launch_bounds__(FW * 32, 5) k_serve(ServeArgs a) {
 // picks it.  The beam in registers (up to 192 entries) against shared memory:
 // 177 -> 155 us.
 constexpr int TEAM = 4;
-
-__device__ __forceinline__ void prefetch_l1(const void* p) { asm volatile("prefetch.global.L1 [%0];" ::"l"(p)); }
 
 // Distances to rows [first, first + 8) of the cnt <= 32 ids that the lanes
 // hold, into out[0, 8) (shared memory).  NB rows at a time are summed by a
@@ -1031,9 +1099,13 @@ __global__ void __launch_bounds__(TEAM * 32) k_serve_team(ServeArgs a) {
 }
 
 using ServeFn = void (*)(ServeArgs);
-template <int M>
+template <int M, bool DENSE>
 ServeFn pick_qv(uint32_t qv) {
-    return qv == 1 ? k_serve<M, 1> : (qv == 2 ? k_serve<M, 2> : k_serve<M, 4>);
+    return qv == 1 ? k_serve<M, 1, DENSE> : (qv == 2 ? k_serve<M, 2, DENSE> : k_serve<M, 4, DENSE>);
+}
+template <bool DENSE>
+ServeFn pick_warp(int metric, uint32_t qv) {
+    return metric == L2 ? pick_qv<L2, DENSE>(qv) : (metric == L1 ? pick_qv<L1, DENSE>(qv) : pick_qv<CHI2, DENSE>(qv));
 }
 template <int M, int QV>
 ServeFn pick_team_beam(uint32_t beam) {
@@ -1069,10 +1141,11 @@ int index_run_fast(Ctx& ctx, IndexDev& ix, const SearchReq& r) {
         NNM_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&pt, team, TEAM * 32, tsmem));
         use_team = r.nq <= (uint32_t)std::max(pt, 0) * (uint32_t)nsm;
     }
-    const ServeFn fn = use_team ? team
-                       : ix.metric == L2 ? pick_qv<L2>(qv)
-                                         : (ix.metric == L1 ? pick_qv<L1>(qv) : pick_qv<CHI2>(qv));
-    const size_t smem = use_team ? tsmem : (size_t)FW * ((size_t)r.beam_max * 16 + WARP_EXTRA);
+    // several queries per resident warp: the form with more warps
+    const bool dense = !use_team && r.nq > DENSE_QUERIES * (uint32_t)nsm &&
+                       (size_t)words * 4 * DENSE_WARPS * nsm <= DENSE_BITMAPS;
+    const ServeFn fn = use_team ? team : dense ? pick_warp<true>(ix.metric, qv) : pick_warp<false>(ix.metric, qv);
+    const size_t smem = use_team ? tsmem : (size_t)FW * ((size_t)r.beam_max * 8 + WARP_EXTRA);
     uint32_t blocks = r.nq;
     if (!use_team) {
         NNM_CUDA_TRY(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
