@@ -1215,7 +1215,12 @@ __device__ __forceinline__ void merge_round(uint32_t pd, unsigned long long pk, 
         if (s < tot) {
             keep = true;
             MEnt me = sm[s];
-            for (int q = (int)s - 1; q >= 0 && sm[q].d == me.d; q--)
+            // a proposal equal to an earlier entry; entries of the start pool
+            // (keys below 2^63) stay even where the pool repeats an id, as
+            // the reference leaves them (an H-Merge level of fewer rows than
+            // its cross samples draws the same ids twice, and without the
+            // repeats fewer than K entries were left)
+            for (int q = (int)s - 1; (me.k >> 63) && q >= 0 && sm[q].d == me.d; q--)
                 if ((sm[q].e & ID_MASK) == (me.e & ID_MASK)) {
                     keep = false;
                     break;
