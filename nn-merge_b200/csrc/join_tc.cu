@@ -25,11 +25,11 @@
 // that pass the K-th-distance filter (the bucket sizes); pass 1 recomputes
 // the distances and writes the proposals.  Nothing per pair is stored.
 //
-// Synchronisation: persistent CTAs of 256 threads, at most four per SM (the
-// TMEM columns and the shared memory request both allow four), each holding
-// 128 TMEM columns for its lifetime.  Producer warps load tile k+1 into one
-// buffer while the consumer warps run tile k from the other (full/empty
-// mbarriers per buffer); consumer thread 0 issues the MMAs and commits them
+// Synchronisation: persistent CTAs of 256 to 512 threads, at most four per SM
+// (the TMEM columns and the shared memory request both allow four), each
+// holding 128 TMEM columns for its lifetime.  Producer warps load tile k+1
+// into one buffer while the consumer warps run tile k from the other
+// (full/empty mbarriers per buffer); consumer thread 0 issues the MMAs and commits them
 // to an mbarrier.  Every mbarrier wait is bounded in time; when a bound runs
 // out the group stops (decided by a barrier-OR over its threads), the CTA
 // records DERR_TC_WAIT, waits (bounded) once more for its MMA, frees its
@@ -52,12 +52,23 @@
 namespace nnm {
 namespace {
 
-// Consumer threads per CTA: the emit pass runs two warps per TMEM lane
-// quarter (warps 0-7), the count pass one (warps 0-3); the producers are
-// the next four warps, one thread per tile slot.
+// Consumer threads per CTA: two warps per TMEM lane quarter (warps 0-7) in
+// the emit pass, one (warps 0-3) in the count pass; then the producers, one
+// thread per tile slot, a group for both buffers (u8) or for each
+// (reduced-precision kinds).  BF16 and FP8 operand rows leave room for two
+// CTAs on an SM, and their joins waited for the producers, whose reads from
+// tile to tile form one chain (eight consumer warps in the count pass
+// changed nothing): a group per buffer took 6 % off a 1M x 96 BF16 build,
+// 209.1 -> 196.9 ms.  Four u8 CTAs a SM overlap each other.
 constexpr int TC_PROD = 128;
 __host__ __device__ constexpr int tc_cons(int pass) { return pass == 1 ? 256 : 128; }
-__host__ __device__ constexpr int tc_threads(int pass) { return tc_cons(pass) + TC_PROD; }
+__host__ __device__ constexpr int tc_prods(uint32_t kind) { return kind != 0 ? 2 : 1; }  // producer groups
+__host__ __device__ constexpr int tc_threads(int pass, uint32_t kind) {
+    return tc_cons(pass) + tc_prods(kind) * TC_PROD;
+}
+// Columns the epilogue works through together: their reads and tests have no
+// branch between them (1M x 128 u8 build 95.2 -> 92.1 ms; 8: 93.5, 2: 92.0).
+constexpr uint32_t TC_GROUP = 4;
 constexpr uint32_t TC_SLOTS = 128;             // M = N = 128: one TMEM lane and one column per slot
 constexpr uint32_t TC_COLS = 128;              // TMEM columns held by a CTA
 constexpr uint32_t TC_SMEM_FLOOR = 50 * 1024;  // keeps residency at <= 4 CTAs per SM (4 x 128 columns)
@@ -120,7 +131,7 @@ __host__ __device__ constexpr size_t tc_smem_bytes(uint32_t kq) { return 2 * tc_
 
 struct SlotBuf {
     unsigned char* vec;
-    uint4* info;    // per slot: list entry, K-th distance (bits), norm, group -- one 16-byte read
+    uint4* info;    // per slot: list entry, K-th distance (slot_kth), norm, pair word (pair_word) -- one 16-byte read
     uint32_t* cnt;  // pass 0: counts; pass 1: bucket cursors
     uint32_t* lim;  // pass 1: the slot's reserved bucket range (its pass-0 count)
     float* scl;     // KIND_FP8: the row's inverse scale 2^-e
@@ -139,8 +150,8 @@ __device__ __forceinline__ SlotBuf slot_buf(unsigned char* smem, uint32_t kq, ui
     return s;
 }
 
-// Barriers of one thread group (producers: 1, consumers: 2).
-constexpr uint32_t BAR_PROD = 1, BAR_CONS = 2;
+// Barriers of one thread group.
+constexpr uint32_t BAR_PROD = 1, BAR_CONS = 3;  // BAR_PROD + g: producer group g
 
 __device__ __forceinline__ void group_sync(uint32_t id, uint32_t nthreads) {
     asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(nthreads) : "memory");
@@ -162,10 +173,34 @@ __device__ __forceinline__ bool group_any(uint32_t id, bool p, uint32_t nthreads
     return r != 0;
 }
 
+// The reference's pair filter (pair_order) as one word per slot: a pair of
+// slots with words u and v is evaluated when ((u ^ v) & pair_mask) != 0 and
+// u | v | pair_set has its top bit.  k-NN graph and whole merges: the ids (a
+// pair is skipped when they are equal); S-Merge: the leaves (equal ids have
+// equal leaves); J-Merge's first pass: the entry, id and group bit, and one
+// of the two must be of group 1.
+__device__ __forceinline__ bool pair_by_entry(const JoinArgs& a) {
+    return a.mode != MODE_KGRAPH && a.mode != MODE_SMERGE && !a.verse;
+}
+__device__ __forceinline__ uint32_t pair_word(const JoinArgs& a, uint32_t e) {
+    if (a.mode == MODE_SMERGE) return leaf_of(e & LID_MASK, a.leaf_off, a.nleaf);
+    return pair_by_entry(a) ? e : e & LID_MASK;
+}
+
+// A slot's K-th distance as the epilogue compares it: float bits, or for the
+// integer distances of KIND_U8 the smallest integer not below it (d < kth
+// for an integer d exactly when d < that; beyond the integers it saturates
+// above every distance).
+template <int KIND>
+__device__ __forceinline__ uint32_t slot_kth(float kth) {
+    return KIND == KIND_U8 ? (uint32_t)__float2int_ru(kth) : __float_as_uint(kth);
+}
+
 // Persistent CTAs in two groups over two tile buffers:
-//   producers (the last four warps): for tile k, wait until buffer k%2 is released,
-//     write its header and slot metadata, gather the slot vectors with
-//     cp.async, then arrive on full[k%2];
+//   producers (the last four warps, for tile k in buffer k%2; or eight, each
+//     four with a buffer and tiles of their own): wait until the buffer is
+//     released, write its header and slot metadata, gather the slot vectors
+//     with cp.async, then arrive on its full barrier;
 //   consumers (warps 0-3; in the emit pass warps 0-7, warps w and w + 4
 //     reading TMEM lanes 32 (w % 4) .. + 31 and sharing their columns in
 //     8-column blocks): wait for full[k%2], run the MMA chain (thread 0) and
@@ -191,10 +226,10 @@ __device__ __forceinline__ bool group_any(uint32_t id, bool p, uint32_t nthreads
 // AUDIT (pass 0 of the reduced-precision kinds): every pair's d~ is also
 // checked against its exact distance.
 template <int PASS, int KIND, bool FAST, bool AUDIT = false>
-__global__ void __launch_bounds__(tc_threads(PASS), PASS == 0 ? 4 : KIND == KIND_U8 ? 3 : 2) k_join_tc(JoinArgs a) {
+__global__ void __launch_bounds__(tc_threads(PASS, KIND), KIND != KIND_U8 ? 2 : PASS == 0 ? 4 : 3) k_join_tc(JoinArgs a) {
     extern __shared__ __align__(1024) unsigned char smem[];
     __shared__ TcShared sh;
-    constexpr uint32_t CONS = tc_cons(PASS), HALVES = CONS / 128;
+    constexpr uint32_t CONS = tc_cons(PASS), HALVES = CONS / 128, PG = tc_prods(KIND);
     if (a.ctr->overflow) return;  // a buffer sized ahead was too small: the host reruns
     const uint32_t tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const uint32_t kq = a.kq, nchunk = kq >> 4;
@@ -240,7 +275,8 @@ __global__ void __launch_bounds__(tc_threads(PASS), PASS == 0 ? 4 : KIND == KIND
         // of dependent reads; it is fetched into registers for tile k+1
         // while the vector copies of tile k are in flight, and stored into
         // the buffer once that buffer is released.
-        const uint32_t ptid = tid - CONS;
+        const uint32_t ptid = (tid - CONS) & (TC_PROD - 1), pg = PG == 2 ? (tid - CONS) / TC_PROD : 0u;
+        const uint32_t bar_prod = BAR_PROD + pg;
         unsigned long long sum_s = 0;
         struct SlotMeta {
             uint32_t t, lgB, nrows, row, nn, S, e, nrm, grp, lim;
@@ -275,7 +311,7 @@ __global__ void __launch_bounds__(tc_threads(PASS), PASS == 0 ? 4 : KIND == KIND
                     m.kth = a.kthv[id];
                     m.nrm = a.nrm[id];
                     m.scl = KIND == KIND_FP8 ? a.scl[id] : 1.f;
-                    m.grp = a.mode == MODE_SMERGE ? leaf_of(id, a.leaf_off, a.nleaf) : (e >> 31);
+                    m.grp = pair_word(a, e);
                     if (PASS == 1) {
                         const uint32_t c = a.cntpos[(size_t)row * a.caps + q];
                         m.lim = c;
@@ -289,13 +325,14 @@ __global__ void __launch_bounds__(tc_threads(PASS), PASS == 0 ? 4 : KIND == KIND
         // that finish early take more).  After the last tile the producers
         // hand the consumers a buffer marked done.
         SlotMeta cur{};
-        uint32_t tile = blockIdx.x;
+        const uint32_t lgc = nchunk > 4 ? 3u : nchunk > 2 ? 2u : 1u, cl = ptid & ((1u << lgc) - 1u);
+        uint32_t tile = blockIdx.x + pg * gridDim.x;
         if (tile < total) fetch(tile, cur);
         for (uint32_t k = 0;; k++) {
-            const uint32_t b = k & 1, use = k >> 1;
+            const uint32_t b = PG == 2 ? pg : k & 1, use = PG == 2 ? k : k >> 1;
             if (use > 0) {
                 const bool ok = mbar_wait_bounded(smem_u32(&sh.empty[b]), (use - 1) & 1);
-                if (group_any(BAR_PROD, !ok, TC_PROD)) {
+                if (group_any(bar_prod, !ok, TC_PROD)) {
                     failed = true;
                     break;
                 }
@@ -308,7 +345,7 @@ __global__ void __launch_bounds__(tc_threads(PASS), PASS == 0 ? 4 : KIND == KIND
             }
             if (ptid == 0) {
                 H.done = 0;
-                H.next = gridDim.x + atomicAdd(&a.ctr->tc_next[PASS], 1u);
+                H.next = PG * gridDim.x + atomicAdd(&a.ctr->tc_next[PASS], 1u);
             }
             const SlotBuf S = slot_buf(smem, kq, b);
             const uint32_t B = 1u << cur.lgB, r = ptid >> cur.lgB, q = ptid & (B - 1);
@@ -324,7 +361,7 @@ __global__ void __launch_bounds__(tc_threads(PASS), PASS == 0 ? 4 : KIND == KIND
                 H.S[r] = cur.S;
                 sum_s += cur.S;
             }
-            S.info[ptid] = cur.e != NO_SLOT ? make_uint4(cur.e, __float_as_uint(cur.kth), cur.nrm, cur.grp)
+            S.info[ptid] = cur.e != NO_SLOT ? make_uint4(cur.e, slot_kth<KIND>(cur.kth), cur.nrm, cur.grp)
                                             : make_uint4(NO_SLOT, 0u, 0u, 0u);
             if (cur.e != NO_SLOT) {
                 if (KIND == KIND_FP8) S.scl[ptid] = cur.scl;
@@ -334,17 +371,28 @@ __global__ void __launch_bounds__(tc_threads(PASS), PASS == 0 ? 4 : KIND == KIND
                     S.base[ptid] = cur.base;
                 }
             }
-            group_sync(BAR_PROD, TC_PROD);
+            group_sync(bar_prod, TC_PROD);
             // gather: 16-byte chunk c of slot s -> column c / 8, row s, chunk
             // (c % 8) ^ (s % 8) (the 128-byte swizzle); a row's chunks by
-            // consecutive threads
-            const uint32_t vbase = smem_u32(S.vec);
-            for (uint32_t i = ptid; i < TC_SLOTS * nchunk; i += 128) {
-                const uint32_t sl = i / nchunk, c = i - sl * nchunk;
-                const uint32_t e = S.info[sl].x;
-                if (e != NO_SLOT)
-                    cp_async16(vbase + (c >> 3) * TC_COL_BYTES + sl * 128 + (((c & 7) ^ (sl & 7)) << 4),
-                               a.xq + (size_t)(e & LID_MASK) * kq + c * 16);
+            // consecutive lanes, as many as a 128-byte column of it has
+            // (rounded up to a power of two), four rows a lane at a time
+            const uint32_t vbase = smem_u32(S.vec), step = TC_PROD >> lgc;
+            for (uint32_t s0 = ptid >> lgc; s0 < TC_SLOTS; s0 += 4 * step) {
+                uint32_t e[4];
+#pragma unroll
+                for (uint32_t u = 0; u < 4; u++) {
+                    const uint32_t sl = s0 + u * step;
+                    e[u] = sl < TC_SLOTS ? S.info[sl].x : NO_SLOT;
+                }
+                for (uint32_t c = cl, col = 0; c < nchunk; c += 8, col += TC_COL_BYTES) {
+#pragma unroll
+                    for (uint32_t u = 0; u < 4; u++) {
+                        const uint32_t sl = s0 + u * step;
+                        if (e[u] != NO_SLOT)
+                            cp_async16(vbase + col + sl * 128 + ((cl ^ (sl & 7)) << 4),
+                                       a.xq + (size_t)(e[u] & LID_MASK) * kq + c * 16);
+                    }
+                }
             }
             // the next tile's metadata while these copies land
             const uint32_t nxt = H.next;
@@ -364,15 +412,21 @@ __global__ void __launch_bounds__(tc_threads(PASS), PASS == 0 ? 4 : KIND == KIND
     } else {
         // ---------------- consumers ----------------
         uint32_t cmps = 0;
+        uint32_t ended = 0;  // buffers whose producers have no more tiles
         for (uint32_t k = 0;; k++) {
             const uint32_t b = k & 1, use = k >> 1;
+            if (PG == 2 && ((ended >> b) & 1u)) continue;
             const bool okf = mbar_wait_bounded(smem_u32(&sh.full[b]), use & 1);
             if (group_any(BAR_CONS, !okf, CONS)) {
                 failed = true;
                 break;
             }
             const TileHdr& H = sh.hdr[b];
-            if (H.done) break;
+            if (H.done) {
+                ended |= 1u << b;
+                if (PG == 1 || ended == 3u) break;
+                continue;
+            }
             const SlotBuf S = slot_buf(smem, kq, b);
             const uint32_t t = H.t, lgB = H.lgB, nrows = H.nrows, B = 1u << lgB;
             if (tid == 0) {
@@ -444,8 +498,10 @@ __global__ void __launch_bounds__(tc_threads(PASS), PASS == 0 ? 4 : KIND == KIND
             const uint32_t r_b = slot >> lgB, q_b = slot & (B - 1);
             const uint32_t nn_b = valid_b ? H.nn[r_b] : 0u, S_b = valid_b ? H.S[r_b] : 0u;
             const uint32_t row_b = valid_b ? H.row[r_b] : 0u;
-            const float kth_b = __uint_as_float(info_b.y);
+            const float kth_b = __uint_as_float(info_b.y);  // KIND_U8: an integer's bits
             const uint32_t nrm_b = info_b.z, grp_b = info_b.w;
+            const uint32_t pair_mask = pair_by_entry(a) ? LID_MASK : 0xffffffffu;
+            const uint32_t pair_set = grp_b | (pair_by_entry(a) ? 0u : 0x80000000u);
             const float scl_b = KIND == KIND_FP8 ? S.scl[slot] : 1.f;
             const uint32_t lim_b = PASS == 1 ? S.lim[slot] : 0u;
             // this slot's bucket range start, read once (the proposal stores
@@ -453,14 +509,17 @@ __global__ void __launch_bounds__(tc_threads(PASS), PASS == 0 ? 4 : KIND == KIND
             const unsigned long long base_b = PASS == 1 ? S.base[slot] : 0ull;
             bool over = false;  // pass 1, reduced precision: a write beyond a reserved range
             const uint32_t blk = slot & ~(B - 1);
+            // this slot pairs with the columns blk .. blk + ncol - 1: earlier
+            // slots of its row, in the new list
+            const int ncol = valid_b ? (int)min(q_b, nn_b) : 0;
             uint32_t cb = 0;
-            // Rows of at most 32 slots lie inside one lane quarter, so every
-            // proposal to slot s of such a tile comes from the two warps
-            // holding s: each keeps its counter in a register of lane s % 32
-            // (read by shuffle) instead of shared memory (an atomic round trip
-            // per pair).  In the emit pass half 0 fills the slot's reserved
-            // range from its start, half 1 from its end.
-            const bool wl_tile = lgB <= 5;
+            // Emit pass: rows of at most 32 slots lie inside one lane quarter,
+            // so every proposal to slot s of such a tile comes from the two
+            // warps holding s: each keeps its counter in a register of lane
+            // s % 32 (read by shuffle) instead of shared memory, half 0
+            // filling the slot's reserved range from its start, half 1 from
+            // its end.
+            const bool wl_tile = PASS == 1 && lgB <= 5;
             uint32_t cnt_r = 0;
             const uint32_t c_first = B >= 32 ? ((quarter * 32) & ~(B - 1)) : quarter * 32;
             // the loop specialised for the tile's counter kind, so that the
@@ -470,11 +529,11 @@ __global__ void __launch_bounds__(tc_threads(PASS), PASS == 0 ? 4 : KIND == KIND
                 constexpr bool wl = decltype(wl_kind)::value;
                 uint32_t blocks = 0;  // 8-column blocks of this lane quarter so far
                 for (uint32_t c0 = c_first; c0 <= quarter * 32; c0 += 32) {
-                    // columns a of a pair are new-list entries: a < blk + nn_b; the
-                    // bound is made warp-uniform (lanes of different rows take the max)
-                    const int lim = valid_b ? (int)(blk + nn_b) - (int)c0 : 0;
+                    // the last column any lane of the warp pairs with
+                    const int lim = ncol ? (int)blk + ncol - (int)c0 : 0;
                     const uint32_t jend = (uint32_t)__reduce_max_sync(0xffffffffu, lim < 0 ? 0 : (lim > 32 ? 32 : lim));
                     if (jend == 0) continue;
+                    uint32_t cnt_w = 0;  // pass 0: proposals of this warp to slot c0 + lane
                     // 8 columns per TMEM load: no spills at 64 registers, a short unrolled body
                     for (uint32_t h = 0; h < jend; h += 8) {
                         // blocks 0, 3, 4, 7, ... to half 0 and 1, 2, 5, 6, ... to
@@ -483,94 +542,119 @@ __global__ void __launch_bounds__(tc_threads(PASS), PASS == 0 ? 4 : KIND == KIND
                         if (HALVES == 2 && ((bi + (bi >> 1)) & 1u) != half) continue;
                         uint32_t v[8];
                         tmem_ld8(tmem + ((quarter * 32) << 16) + c0 + h, v);
+                        // bit j: this slot pairs with column c0 + h + j
+                        const int lo = (int)blk - (int)(c0 + h), hi = lo + ncol;
+                        const uint32_t pm = hi > 0 && lo < 8 ? ((1u << min(hi, 8)) - 1u) & ~((1u << max(lo, 0)) - 1u) : 0u;
+                        // TC_GROUP columns at a time without a branch between
+                        // them, so that their reads and tests overlap
 #pragma unroll
-                        for (uint32_t j8 = 0; j8 < 8; j8++) {
-                            const uint32_t jj = h + j8;
-                            if (jj >= jend) break;
-                            const uint32_t av = c0 + jj;
-                            const uint32_t q_a = av & (B - 1);
-                            const bool pv = valid_b && (av & ~(B - 1)) == blk && q_a < q_b && q_a < nn_b;
-                            const uint4 info_a = S.info[av];
-                            const uint32_t e_a = info_a.x;
-                            float dd, lb;
-                            if (KIND == KIND_U8) {
-                                dd = (float)((int)(info_a.z + nrm_b) - 2 * (int)v[j8]);
-                                lb = dd;
-                            } else {
-                                // d~ and its lower bound (distances are >= 0)
-                                const float ns = __uint_as_float(info_a.z) + __uint_as_float(nrm_b);
-                                float gd = __uint_as_float(v[j8]);
-                                if (KIND == KIND_FP8) gd *= S.scl[av] * scl_b;
-                                dd = fmaxf(ns - 2.f * gd, 0.f);
-                                lb = dd - a.err_c * ns;
-                                if (PASS == 0 && AUDIT && pv) {  // the bound against the exact distance
-                                    const float ex = audit_l2(a.x, a.dp, e_a & LID_MASK, e_b & LID_MASK);
-                                    if (!(ex >= lb && ex <= dd + a.err_c * ns)) atomicOr(a.tc_err, (unsigned)DERR_BOUND);
-                                    if (ns > 0.f) atomicMax(&a.ctr->audit_max, __float_as_uint(fabsf(ex - dd) / ns));
+                        for (uint32_t g = 0; g < 8; g += TC_GROUP) {
+                            if (g && h + g >= jend) break;
+                            const uint32_t av0 = c0 + h + g;
+                            uint32_t e_a[TC_GROUP], m[TC_GROUP];
+                            float dd[TC_GROUP];
+                            bool pa[TC_GROUP], pb[TC_GROUP];
+#pragma unroll
+                            for (uint32_t j = 0; j < TC_GROUP; j++) {
+                                const uint4 info_a = S.info[av0 + j];
+                                e_a[j] = info_a.x;
+                                const bool pv = (pm >> (g + j)) & 1u;
+                                const bool ok = pv && ((info_a.w ^ grp_b) & pair_mask) != 0 &&
+                                                (int)(info_a.w | pair_set) < 0;
+                                if (KIND == KIND_U8) {
+                                    const int di = (int)(info_a.z + nrm_b) - 2 * (int)v[g + j];
+                                    pa[j] = ok && di < (int)info_a.y;
+                                    pb[j] = ok && di < __float_as_int(kth_b);
+                                    dd[j] = __int_as_float(di);
+                                } else {
+                                    // d~ and its lower bound (distances are >= 0)
+                                    const float ns = __uint_as_float(info_a.z) + __uint_as_float(nrm_b);
+                                    float gd = __uint_as_float(v[g + j]);
+                                    if (KIND == KIND_FP8) gd *= S.scl[av0 + j] * scl_b;
+                                    dd[j] = fmaxf(ns - 2.f * gd, 0.f);
+                                    const float lb = dd[j] - a.err_c * ns;
+                                    if (PASS == 0 && AUDIT && pv) {  // the bound against the exact distance
+                                        const float ex = audit_l2(a.x, a.dp, e_a[j] & LID_MASK, e_b & LID_MASK);
+                                        if (!(ex >= lb && ex <= dd[j] + a.err_c * ns))
+                                            atomicOr(a.tc_err, (unsigned)DERR_BOUND);
+                                        if (ns > 0.f)
+                                            atomicMax(&a.ctr->audit_max, __float_as_uint(fabsf(ex - dd[j]) / ns));
+                                    }
+                                    pa[j] = ok && lb < __uint_as_float(info_a.y);
+                                    pb[j] = ok && lb < kth_b;
+                                }
+                                m[j] = __ballot_sync(0xffffffffu, pa[j]);
+                                if (PASS == 0) {
+                                    cmps += ok;
+                                    cb += pb[j];
+                                    if (lane == h + g + j) cnt_w += __popc(m[j]);
                                 }
                             }
-                            const uint32_t axb = APPROX ? APPROX_BIT : 0u;
-                            uint32_t outer = 0, inner = 0;
-                            const bool ok = pv && pair_order(a.mode, a.verse, q_a, q_b, nn_b, e_a, e_b, info_a.w,
-                                                             grp_b, outer, inner);
-                            const float kth_a = __uint_as_float(info_a.y);
-                            if (PASS == 0) {
-                                cmps += ok;
-                                cb += (ok && lb < kth_b);
-                                const unsigned m = __ballot_sync(0xffffffffu, ok && lb < kth_a);
-                                if (wl) {
-                                    if (lane == (av & 31)) cnt_r += __popc(m);
-                                } else if (m && lane == 0) {
-                                    atomicAdd(&S.cnt[av], (uint32_t)__popc(m));
+                            if constexpr (PASS == 1) {
+                                const uint32_t axb = APPROX ? APPROX_BIT : 0u;
+                                // the proposal of entry e at distance dd[j] to position `at` of a
+                                // bucket; side 0: into the pair's outer element's pool
+                                auto put = [&](uint32_t j, unsigned long long at, uint32_t e, bool to_a) {
+                                    const uint32_t q_a = (av0 + j) & (B - 1);
+                                    const bool swap = !FAST && a.mode == MODE_KGRAPH && q_b < nn_b &&
+                                                      (e_b & LID_MASK) < (e_a[j] & LID_MASK);  // pair_order
+                                    const uint32_t pidx = swap ? q_b * S_b + q_a : q_a * S_b + q_b;
+                                    put_prop<FAST>(a.bucket, at, KIND == KIND_U8 ? (float)__float_as_int(dd[j]) : dd[j],
+                                                   e | axb, row_b, pidx, to_a != swap ? 0u : 1u);
+                                };
+                                uint32_t base4 = 0, pos = 0;
+                                if (!wl) {
+                                    // the group's positions in two reservations: lane j < TC_GROUP for
+                                    // the proposals to column j's slot, every lane for those to its own
+                                    uint32_t mine = m[0];
+    #pragma unroll
+                                    for (uint32_t j = 1; j < TC_GROUP; j++) mine = lane == j ? m[j] : mine;
+                                    if (lane < TC_GROUP && mine) base4 = atomicAdd(&S.cnt[av0 + lane], (uint32_t)__popc(mine));
+                                    uint32_t npb = 0;
+    #pragma unroll
+                                    for (uint32_t j = 0; j < TC_GROUP; j++) npb += pb[j];
+                                    if (npb) pos = atomicAdd(&S.cnt[slot], npb);
                                 }
-                            } else {
-                                const uint32_t pidx = outer * S_b + inner;
-                                const bool pa = ok && lb < kth_a;
-                                const unsigned m = __ballot_sync(0xffffffffu, pa);
-                                if (m) {
-                                    uint32_t base;
-                                    if (wl) {
-                                        // the owner of slot av is lane av % 32; its own
-                                        // pair with av is not a pair (q_a == q_b), so it
-                                        // takes no b-side proposal in this step
-                                        base = __shfl_sync(0xffffffffu, cnt_r, av & 31);
-                                        if (lane == (av & 31)) cnt_r += __popc(m);
-                                        if (half) base = S.lim[av] - base - __popc(m);  // from the range's end
-                                    } else {
-                                        const uint32_t leader = __ffs(m) - 1;
-                                        base = 0;
-                                        if (lane == leader) base = atomicAdd(&S.cnt[av], (uint32_t)__popc(m));
-                                        base = __shfl_sync(0xffffffffu, base, leader);
+    #pragma unroll
+                                for (uint32_t j = 0; j < TC_GROUP; j++) {
+                                    if (m[j]) {
+                                        const uint32_t av = av0 + j;
+                                        uint32_t base;
+                                        if (wl) {
+                                            // the owner of slot av is lane av % 32; its own
+                                            // pair with av is not a pair (q_a == q_b), so it
+                                            // takes no b-side proposal in this step
+                                            base = __shfl_sync(0xffffffffu, cnt_r, av & 31);
+                                            if (lane == (av & 31)) cnt_r += __popc(m[j]);
+                                            if (half) base = S.lim[av] - base - __popc(m[j]);  // from the range's end
+                                        } else {
+                                            base = __shfl_sync(0xffffffffu, base4, j);
+                                        }
+                                        if (pa[j]) {
+                                            const uint32_t at = base + __popc(m[j] & ((1u << lane) - 1u));
+                                            if (!APPROX || at < S.lim[av]) put(j, S.base[av] + at, e_b, true);
+                                            else over = true;
+                                        }
                                     }
-                                    if (pa) {
-                                        const uint32_t before = __popc(m & ((1u << lane) - 1u));
-                                        const unsigned long long at = S.base[av] + base + before;
-                                        if (!APPROX || base + before < S.lim[av])
-                                            put_prop<FAST>(a.bucket, at, dd, e_b | axb, row_b, pidx,
-                                                           outer == q_a ? 0u : 1u);
-                                        else
-                                            over = true;
+                                    if (pb[j]) {
+                                        const uint32_t at = !wl ? pos++ : half ? lim_b - 1u - cnt_r++ : cnt_r++;
+                                        if (!APPROX || at < lim_b) put(j, base_b + at, e_a[j], false);
+                                        else over = true;
                                     }
-                                }
-                                if (ok && lb < kth_b) {
-                                    const uint32_t pos =
-                                        wl ? (half ? lim_b - 1u - cnt_r++ : cnt_r++) : atomicAdd(&S.cnt[slot], 1u);
-                                    const unsigned long long at = base_b + pos;
-                                    if (!APPROX || pos < lim_b)
-                                        put_prop<FAST>(a.bucket, at, dd, e_a | axb, row_b, pidx, outer == q_b ? 0u : 1u);
-                                    else
-                                        over = true;
                                 }
                             }
                         }
                     }
+                    if (PASS == 0 && cnt_w) atomicAdd(&S.cnt[c0 + lane], cnt_w);
                 }
             };
-            if (wl_tile) pairs(std::true_type{});
-            else pairs(std::false_type{});
-            if (PASS == 0) {
-                if (wl_tile ? (cnt_r + cb) != 0 : cb != 0) atomicAdd(&S.cnt[slot], wl_tile ? cnt_r + cb : cb);
+            if constexpr (PASS == 1) {
+                if (wl_tile) pairs(std::true_type{});
+                else pairs(std::false_type{});
+            } else {
+                pairs(std::false_type{});
             }
+            if (PASS == 0 && cb) atomicAdd(&S.cnt[slot], cb);
             if (PASS == 1 && APPROX && wl_tile && cnt_r) atomicAdd(&S.cnt[slot], cnt_r);
             if (PASS == 1 && APPROX && over) atomicOr(a.tc_err, (unsigned)DERR_TC_RANGE);
             asm volatile("tcgen05.fence::before_thread_sync;");
@@ -1229,10 +1313,10 @@ static void launch_tc(const JoinArgs& ja, unsigned tiles, int nsm, size_t bytes,
     const int per_sm_smem = (int)((size_t)smem_sm / (bytes + fa.sharedSizeBytes + (size_t)reserved));
     int regs_sm = 65536;
     cudaDeviceGetAttribute(&regs_sm, cudaDevAttrMaxRegistersPerMultiprocessor, dev);
-    const int per_sm_regs = regs_sm / (((fa.numRegs + 7) & ~7) * tc_threads(PASS));
+    const int per_sm_regs = regs_sm / (((fa.numRegs + 7) & ~7) * tc_threads(PASS, KIND));
     const int per_sm = std::min(std::max(std::min(per_sm_smem, per_sm_regs), 1), TC_TMEM_CTAS);
     const unsigned grid = std::min<unsigned>(tiles, (unsigned)nsm * (unsigned)per_sm);
-    k_join_tc<PASS, KIND, FAST, AUDIT><<<grid, tc_threads(PASS), bytes, st>>>(ja);
+    k_join_tc<PASS, KIND, FAST, AUDIT><<<grid, tc_threads(PASS, KIND), bytes, st>>>(ja);
 }
 
 template <int KIND>
