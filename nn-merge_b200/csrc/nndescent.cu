@@ -1152,10 +1152,60 @@ __device__ __forceinline__ void load_prop(const void* bucket, unsigned long long
     }
 }
 
-// The reference's FP32 distance of rows t and u (the reduced-precision
-// joins' exact value), one non-inlined copy.
-__device__ __noinline__ float merge_exact_l2(const float* x, uint32_t dp, uint32_t t, uint32_t u) {
-    return dist_seq<L2>(x + (size_t)t * dp, x + (size_t)u * dp, (int)dp);
+// The reference's FP32 distances of row t and each wanting lane's row u (the
+// reduced-precision joins' exact values), one non-inlined copy.  A lane
+// reading its own row from global memory touches a line per lane and load
+// instruction: with most lanes wanting, the L1 ran at 98 % of its throughput.
+// Above RC_DIRECT rows they come through shared memory instead, RC_UNITS
+// 16-byte units of each at a time, by copies of consecutive lanes, and each
+// lane sums its own row there, in the reference's order; below it the
+// stages' round trips cost more than they save.  400,000 x 127 FP8 build:
+// 90.8 ms all direct, 84.0 with 16, 84.5 with 8; 1M x 96 BF16: 190.4, 189.2,
+// 190.2.
+constexpr int RC_DIRECT = 16;
+// Targets of at most this many proposals take their exact distances without
+// the bound on the K-th distance (approx_bound: two sorts and 50 shuffles a
+// target): BF16 build 194.0 -> 189.4 ms (190.2 at 8, 189.3 at 24).
+constexpr uint32_t RC_BOUND = 16;
+constexpr int MERGE_AX_BLOCKS = 6;            // per SM (40 registers; eight at 32 spill: 193.3 ms)
+constexpr uint32_t RC_UNITS = 4;              // 64 bytes of every row at a time
+constexpr uint32_t RC_STRIDE = RC_UNITS + 1;  // odd: lanes reading their own rows fall in different banks
+constexpr uint32_t RC_TILE = 33 * RC_STRIDE;  // float4 of a warp: 32 rows and row t
+__device__ __noinline__ float merge_exact_l2(const float* x, uint32_t dp, uint32_t t, uint32_t u, bool want,
+                                             float4* tile) {
+    const uint32_t lane = threadIdx.x & 31, dq = dp >> 2, base = smem_u32(tile);
+    const unsigned todo = __ballot_sync(FULL, want);
+    const float4* x4 = reinterpret_cast<const float4*>(x);
+    const uint32_t c = lane % RC_UNITS;
+    if (__popc(todo) <= RC_DIRECT)
+        return want ? dist_seq<L2>(x + (size_t)t * dp, x + (size_t)u * dp, (int)dp) : 0.f;
+    float acc = 0.f;
+    for (uint32_t c0 = 0; c0 < dq; c0 += RC_UNITS) {
+        if (c0 + c < dq) {
+            if (lane < RC_UNITS) cp_async16(base + (32 * RC_STRIDE + c) * 16, x4 + (size_t)t * dq + c0 + c);
+        }
+#pragma unroll
+        for (uint32_t r0 = 0; r0 < 32; r0 += 32 / RC_UNITS) {
+            const uint32_t r = r0 + lane / RC_UNITS;
+            const uint32_t id = __shfl_sync(FULL, u, r);
+            if (((todo >> r) & 1u) && c0 + c < dq)
+                cp_async16(base + (r * RC_STRIDE + c) * 16, x4 + (size_t)id * dq + c0 + c);
+        }
+        asm volatile("cp.async.wait_all;" ::: "memory");
+        __syncwarp();
+        if (want) {
+            const uint32_t m = min(RC_UNITS, dq - c0);
+            for (uint32_t k = 0; k < m; k++) {
+                const float4 va = tile[32 * RC_STRIDE + k], vb = tile[lane * RC_STRIDE + k];
+                acc = dist_step<L2>(acc, va.x, vb.x);
+                acc = dist_step<L2>(acc, va.y, vb.y);
+                acc = dist_step<L2>(acc, va.z, vb.z);
+                acc = dist_step<L2>(acc, va.w, vb.w);
+            }
+        }
+        __syncwarp();
+    }
+    return acc;
 }
 
 struct MEnt {
@@ -1402,11 +1452,12 @@ __device__ uint32_t approx_bound(const MergeArgs& a, unsigned long long b_first,
 // computes their exact distances at the flush -- so the pool gets what the
 // FP32 join's proposals would give it.
 template <bool APPROX>
-__global__ void __launch_bounds__(MERGE_WARPS * 32, 8) k_merge(MergeArgs a) {
+__global__ void __launch_bounds__(MERGE_WARPS * 32, APPROX ? MERGE_AX_BLOCKS : 8) k_merge(MergeArgs a) {
     __shared__ MEnt sm[MERGE_WARPS][64];
     __shared__ MEnt kept[MERGE_WARPS][32];
     __shared__ MEnt buf[MERGE_WARPS][32];
     __shared__ uint8_t bufax[APPROX ? MERGE_WARPS : 1][32];
+    __shared__ float4 rows[APPROX ? MERGE_WARPS : 1][APPROX ? RC_TILE : 1];
     if (a.ctr->overflow) return;
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const uint32_t t = blockIdx.x * MERGE_WARPS + w;
@@ -1434,7 +1485,8 @@ __global__ void __launch_bounds__(MERGE_WARPS * 32, 8) k_merge(MergeArgs a) {
             uint32_t bound = 0xffffffffu;
             if (APPROX) {
                 nt = __uint_as_float(a.nrm[t]);
-                bound = approx_bound<false>(a, b_first, c, K, cd, ce, nt,
+                if (c <= RC_BOUND) bound = 0x7f800000u;  // infinity
+                else bound = approx_bound<false>(a, b_first, c, K, cd, ce, nt,
                                             reinterpret_cast<unsigned long long*>(&sm[w][0]));
             }
             uint32_t nb = 0;  // entries in buf
@@ -1447,16 +1499,23 @@ __global__ void __launch_bounds__(MERGE_WARPS * 32, 8) k_merge(MergeArgs a) {
                     pd = me.d;
                     pe = me.e;
                     pk = me.k;
-                    if (APPROX && bufax[w][lane]) {
-                        pd = __float_as_uint(merge_exact_l2(a.x, a.dp, t, pe & ID_MASK));
-                        if (pd >= kd0) {
-                            pd = 0xffffffffu;
-                            pe = 0;
-                            pk = ~0ull;
+                }
+                if (APPROX) {
+                    const bool ax = lane < (int)nb && bufax[w][lane];
+                    const unsigned axm = __ballot_sync(FULL, ax);
+                    if (axm) {
+                        const float ex = merge_exact_l2(a.x, a.dp, t, pe & ID_MASK, ax, rows[w]);
+                        if (ax) {
+                            pd = __float_as_uint(ex);
+                            if (pd >= kd0) {
+                                pd = 0xffffffffu;
+                                pe = 0;
+                                pk = ~0ull;
+                            }
                         }
                     }
+                    if (a.count_approx) nrc += __popc(axm);
                 }
-                if (APPROX && a.count_approx) nrc += __popc(__ballot_sync(FULL, lane < (int)nb && bufax[w][lane]));
                 __syncwarp();
                 warp_sort_ment(pd, pk, pe);
                 merge_round(pd, pk, pe, nb, K, cd, ce, ck, sm[w], kept[w]);
@@ -1569,10 +1628,11 @@ __device__ __forceinline__ unsigned long long fm_flush(unsigned long long pool, 
 // One warp per target, as k_merge, on the fast tier's 8-byte proposals;
 // APPROX as there.
 template <bool APPROX>
-__global__ void __launch_bounds__(MERGE_WARPS * 32, 8) k_merge_fast(MergeArgs a) {
+__global__ void __launch_bounds__(MERGE_WARPS * 32, APPROX ? MERGE_AX_BLOCKS : 8) k_merge_fast(MergeArgs a) {
     __shared__ unsigned long long buf[MERGE_WARPS][32];
     __shared__ unsigned long long stage[MERGE_WARPS][32];
     __shared__ uint8_t bufax[APPROX ? MERGE_WARPS : 1][32];
+    __shared__ float4 rows[APPROX ? MERGE_WARPS : 1][APPROX ? RC_TILE : 1];
     if (a.ctr->overflow) return;
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const uint32_t t = blockIdx.x * MERGE_WARPS + w;
@@ -1598,7 +1658,8 @@ __global__ void __launch_bounds__(MERGE_WARPS * 32, 8) k_merge_fast(MergeArgs a)
         uint32_t bound = 0xffffffffu;
         if (APPROX) {
             nt = __uint_as_float(a.nrm[t]);
-            bound = approx_bound<true>(a, b_first, c, K, (uint32_t)(pool >> 32), (uint32_t)(pool >> 2), nt, stage[w]);
+            if (c <= RC_BOUND) bound = 0x7f800000u;  // infinity
+            else bound = approx_bound<true>(a, b_first, c, K, (uint32_t)(pool >> 32), (uint32_t)(pool >> 2), nt, stage[w]);
         }
         uint32_t nb = 0;
         uint32_t nrc = 0, nax = 0;  // rechecks, approximate proposals (count_approx)
@@ -1638,14 +1699,17 @@ __global__ void __launch_bounds__(MERGE_WARPS * 32, 8) k_merge_fast(MergeArgs a)
                 rest = valid && rank >= take;
             }
             unsigned long long bv = FM_EMPTY;
-            if (lane < (int)nb) {
-                bv = buf[w][lane];
-                if (APPROX && bufax[w][lane]) {  // the exact distance replaces d~
-                    const uint32_t ex = __float_as_uint(merge_exact_l2(a.x, a.dp, t, (uint32_t)(bv >> 2) & ID_MASK));
-                    bv = ex < kd0 ? ((unsigned long long)ex << 32) | (uint32_t)bv : FM_EMPTY;
+            if (lane < (int)nb) bv = buf[w][lane];
+            if (APPROX) {
+                const bool axb = lane < (int)nb && bufax[w][lane];
+                const unsigned axm = __ballot_sync(FULL, axb);
+                if (axm) {  // the exact distance replaces d~
+                    const uint32_t ex = __float_as_uint(
+                        merge_exact_l2(a.x, a.dp, t, (uint32_t)(bv >> 2) & ID_MASK, axb, rows[w]));
+                    if (axb) bv = ex < kd0 ? ((unsigned long long)ex << 32) | (uint32_t)bv : FM_EMPTY;
                 }
+                if (a.count_approx) nrc += __popc(axm);
             }
-            if (APPROX && a.count_approx) nrc += __popc(__ballot_sync(FULL, lane < (int)nb && bufax[w][lane]));
             __syncwarp();
             pool = fm_flush(pool, bv, K, stage[w]);
             kth = __shfl_sync(FULL, pool, K - 1);
