@@ -52,19 +52,21 @@
 namespace nnm {
 namespace {
 
-// Consumer threads per CTA: two warps per TMEM lane quarter (warps 0-7) in
-// the emit pass, one (warps 0-3) in the count pass; then the producers, one
-// thread per tile slot, a group for both buffers (u8) or for each
+// Consumer threads per CTA: one warp per TMEM lane quarter (warps 0-3), two
+// (warps 0-7) in the reduced-precision kinds' emit pass; then the producers,
+// one thread per tile slot, a group for both buffers (u8) or for each
 // (reduced-precision kinds).  BF16 and FP8 operand rows leave room for two
 // CTAs on an SM, and their joins waited for the producers, whose reads from
 // tile to tile form one chain (eight consumer warps in the count pass
 // changed nothing): a group per buffer took 6 % off a 1M x 96 BF16 build,
-// 209.1 -> 196.9 ms.  Four u8 CTAs a SM overlap each other.
+// 209.1 -> 196.9 ms (200.8 with four consumer warps in the emit pass).  Four
+// u8 CTAs on an SM overlap each other; three with eight consumer warps in the
+// emit pass took 90.9 ms for a learned 1M x 128 build, four with four 89.2.
 constexpr int TC_PROD = 128;
-__host__ __device__ constexpr int tc_cons(int pass) { return pass == 1 ? 256 : 128; }
+__host__ __device__ constexpr int tc_cons(int pass, uint32_t kind) { return pass == 1 && kind != 0 ? 256 : 128; }
 __host__ __device__ constexpr int tc_prods(uint32_t kind) { return kind != 0 ? 2 : 1; }  // producer groups
 __host__ __device__ constexpr int tc_threads(int pass, uint32_t kind) {
-    return tc_cons(pass) + tc_prods(kind) * TC_PROD;
+    return tc_cons(pass, kind) + tc_prods(kind) * TC_PROD;
 }
 // Columns the epilogue works through together: their reads and tests have no
 // branch between them (1M x 128 u8 build 95.2 -> 92.1 ms; 8: 93.5, 2: 92.0).
@@ -201,14 +203,10 @@ __device__ __forceinline__ uint32_t slot_kth(float kth) {
 //     four with a buffer and tiles of their own): wait until the buffer is
 //     released, write its header and slot metadata, gather the slot vectors
 //     with cp.async, then arrive on its full barrier;
-//   consumers (warps 0-3; in the emit pass warps 0-7, warps w and w + 4
-//     reading TMEM lanes 32 (w % 4) .. + 31 and sharing their columns in
-//     8-column blocks): wait for full[k%2], run the MMA chain (thread 0) and
-//     the epilogue, write the counts, then arrive on empty[k%2].
-// The emit pass takes two warps per lane quarter because its epilogue is
-// latency-bound (under one eligible warp per scheduler with one): 9 % off
-// the pass, at three CTAs per SM instead of four (registers); the count
-// pass, with less to do per pair, measured 6 % slower that way.
+//   consumers (warps 0-3; with eight, warps w and w + 4 reading TMEM lanes
+//     32 (w % 4) .. + 31 and sharing their columns in 8-column blocks): wait
+//     for the buffer's full barrier, run the MMA chain (thread 0) and the
+//     epilogue, write the counts, then arrive on its empty barrier.
 // So the loads of tile k+1 overlap the MMA and epilogue of tile k.  Every
 // mbarrier wait is bounded; a group decides to stop with a barrier-OR over
 // its threads, and the other group then times out on its next wait.
@@ -226,10 +224,10 @@ __device__ __forceinline__ uint32_t slot_kth(float kth) {
 // AUDIT (pass 0 of the reduced-precision kinds): every pair's d~ is also
 // checked against its exact distance.
 template <int PASS, int KIND, bool FAST, bool AUDIT = false>
-__global__ void __launch_bounds__(tc_threads(PASS, KIND), KIND != KIND_U8 ? 2 : PASS == 0 ? 4 : 3) k_join_tc(JoinArgs a) {
+__global__ void __launch_bounds__(tc_threads(PASS, KIND), KIND != KIND_U8 ? 2 : 4) k_join_tc(JoinArgs a) {
     extern __shared__ __align__(1024) unsigned char smem[];
     __shared__ TcShared sh;
-    constexpr uint32_t CONS = tc_cons(PASS), HALVES = CONS / 128, PG = tc_prods(KIND);
+    constexpr uint32_t CONS = tc_cons(PASS, KIND), HALVES = CONS / 128, PG = tc_prods(KIND);
     if (a.ctr->overflow) return;  // a buffer sized ahead was too small: the host reruns
     const uint32_t tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const uint32_t kq = a.kq, nchunk = kq >> 4;
@@ -514,8 +512,8 @@ __global__ void __launch_bounds__(tc_threads(PASS, KIND), KIND != KIND_U8 ? 2 : 
             const int ncol = valid_b ? (int)min(q_b, nn_b) : 0;
             uint32_t cb = 0;
             // Emit pass: rows of at most 32 slots lie inside one lane quarter,
-            // so every proposal to slot s of such a tile comes from the two
-            // warps holding s: each keeps its counter in a register of lane
+            // so every proposal to slot s of such a tile comes from the warp
+            // (or two) holding s: each keeps its counter in a register of lane
             // s % 32 (read by shuffle) instead of shared memory, half 0
             // filling the slot's reserved range from its start, half 1 from
             // its end.
@@ -526,7 +524,7 @@ __global__ void __launch_bounds__(tc_threads(PASS, KIND), KIND != KIND_U8 ? 2 : 
             // one running holds no code of the other (the emit pass is
             // bound by instruction fetch)
             auto pairs = [&](auto wl_kind) {
-                constexpr bool wl = decltype(wl_kind)::value;
+                [[maybe_unused]] constexpr bool wl = decltype(wl_kind)::value;
                 uint32_t blocks = 0;  // 8-column blocks of this lane quarter so far
                 for (uint32_t c0 = c_first; c0 <= quarter * 32; c0 += 32) {
                     // the last column any lane of the warp pairs with
@@ -1295,9 +1293,8 @@ cudaError_t tc_set_attributes(uint32_t kq, uint32_t kind) {
 // One launch of a join variant: a persistent grid of the CTAs that are
 // resident on the SMs at once, or fewer when the host knows the tile count.
 // Residency is at most four CTAs per SM (TMEM: 512 columns, 128 a CTA),
-// three for the u8 emit pass by registers (384 threads of 56), fewer when the
-// tile buffers of wide operand rows fill the shared memory (two for BF16
-// rows of d = 96).  It is counted here from the registers and shared-memory
+// fewer when the tile buffers of wide operand rows fill the shared memory (two
+// for BF16 rows of d = 96).  It is counted here from the registers and shared-memory
 // sizes: the occupancy query knows nothing of TMEM and reported half these
 // counts, and a grid sized larger than the residency leaves a second wave of
 // persistent CTAs whose tiles run last.
