@@ -1294,22 +1294,53 @@ __device__ __forceinline__ void merge_round(uint32_t pd, unsigned long long pk, 
     __syncwarp();
 }
 
-// Bitonic sort of one entry per lane by (dist, key).
+// Ascending bitonic sort of one word per lane.
+__device__ __forceinline__ unsigned long long fm_sort32(unsigned long long v) {
+    const int lane = threadIdx.x & 31;
+#pragma unroll
+    for (int k = 2; k <= 32; k <<= 1)
+#pragma unroll
+        for (int j = k >> 1; j > 0; j >>= 1) {
+            const unsigned long long o = __shfl_xor_sync(FULL, v, j);
+            const bool take_min = ((lane & j) == 0) == ((lane & k) == 0);
+            v = take_min ? min(v, o) : max(v, o);
+        }
+    return v;
+}
+
+// One entry per lane in (dist, key) order (keys are distinct where dist is
+// not that of an empty lane).  The sort moves a word of distance and lane
+// instead of the 16-byte entries; entries of equal distance -- a pair
+// proposed by several rows, mostly two or three of them -- are then put in
+// key order by exchanges between neighbours.
 __device__ __forceinline__ void warp_sort_ment(uint32_t& pd, unsigned long long& pk, uint32_t& pe) {
     const int lane = threadIdx.x & 31;
-    for (int k = 2; k <= 32; k <<= 1)
-        for (int j = k >> 1; j > 0; j >>= 1) {
-            uint32_t od = __shfl_xor_sync(FULL, pd, j);
-            unsigned long long ok = __shfl_xor_sync(FULL, pk, j);
-            uint32_t oe = __shfl_xor_sync(FULL, pe, j);
-            bool take_min = ((lane & j) == 0) == ((lane & k) == 0);
-            bool swap = take_min ? mless(od, ok, pd, pk) : mless(pd, pk, od, ok);
-            if (swap) {
-                pd = od;
+    const unsigned long long v = fm_sort32(((unsigned long long)pd << 32) | (uint32_t)lane);
+    const int src = (int)(v & 31u);
+    pd = (uint32_t)(v >> 32);
+    pk = __shfl_sync(FULL, pk, src);
+    pe = __shfl_sync(FULL, pe, src);
+    const uint32_t dn = __shfl_down_sync(FULL, pd, 1);
+    const unsigned ties = __ballot_sync(FULL, lane < 31 && dn == pd && pd != 0xffffffffu);
+    if (!ties) return;
+    // bit i of ties: lanes i and i + 1 hold equal distances
+    for (;;) {
+        bool moved = false;
+#pragma unroll
+        for (int odd = 0; odd < 2; odd++) {
+            const bool low = ((lane ^ odd) & 1) == 0;  // the lower lane of its pair
+            const int other = low ? lane + 1 : lane - 1;
+            const unsigned long long ok = __shfl_sync(FULL, pk, other & 31);
+            const uint32_t oe = __shfl_sync(FULL, pe, other & 31);
+            const bool eq = other >= 0 && other < 32 && ((ties >> (low ? lane : other)) & 1u);
+            if (eq && (low ? ok < pk : pk < ok)) {
                 pk = ok;
                 pe = oe;
+                moved = true;
             }
         }
+        if (!__any_sync(FULL, moved)) break;
+    }
 }
 
 // Fast-tier merge.  A fast-tier key is a function of the entry (fast_key),
@@ -1331,20 +1362,6 @@ __device__ __forceinline__ unsigned long long fm_word(uint32_t dist_bits, uint32
 __device__ __forceinline__ uint32_t fm_pool_word(unsigned long long v) {
     const uint32_t lo = (uint32_t)v;
     return ((lo >> 2) & ID_MASK) | (((lo & 1u) ^ 1u) << 30) | (((lo >> 1) & 1u) << 31);
-}
-
-// Ascending bitonic sort of one word per lane.
-__device__ __forceinline__ unsigned long long fm_sort32(unsigned long long v) {
-    const int lane = threadIdx.x & 31;
-#pragma unroll
-    for (int k = 2; k <= 32; k <<= 1)
-#pragma unroll
-        for (int j = k >> 1; j > 0; j >>= 1) {
-            const unsigned long long o = __shfl_xor_sync(FULL, v, j);
-            const bool take_min = ((lane & j) == 0) == ((lane & k) == 0);
-            v = take_min ? min(v, o) : max(v, o);
-        }
-    return v;
 }
 
 // Ascending order of a bitonic sequence of one word per lane.
