@@ -215,7 +215,10 @@ __global__ void k_rev_sort_big(RevSortArgs a) {
             for (uint32_t i = threadIdx.x; i < m; i += blockDim.x) seg[cs + i] = sh[i];
             __syncthreads();
         }
-        // phase 2: merge sorted runs pairwise (keys are distinct source rows)
+        // phase 2: merge sorted runs pairwise.  A row that lists this one twice
+        // is here twice (GraphDev::repeats): the odd run's entries go after
+        // equal ones of the even run and the even run's before equal ones of
+        // the odd run, so that copies in different runs take different places.
         uint32_t* src = seg;
         uint32_t* dst = scr;
         for (uint32_t w = BIGSORT_CH; w < len; w <<= 1) {
@@ -227,10 +230,12 @@ __global__ void k_rev_sort_big(RevSortArgs a) {
                 uint32_t oe = min(os + w, len);
                 if (os > len) os = len;
                 uint32_t key = rkey(src[i]);
-                uint32_t lo2 = os, hi2 = oe;  // lower bound of key in the other run
+                // bound of key in the other run: upper for the odd run's entries, lower for the even run's
+                uint32_t lo2 = os, hi2 = oe;
                 while (lo2 < hi2) {
                     uint32_t mid = (lo2 + hi2) >> 1;
-                    if (rkey(src[mid]) < key) lo2 = mid + 1;
+                    const uint32_t o = rkey(src[mid]);
+                    if (o < key || ((run & 1u) && o == key)) lo2 = mid + 1;
                     else hi2 = mid;
                 }
                 dst[pb + (i - rs) + (lo2 - os)] = src[i];

@@ -52,3 +52,36 @@ def test_rows_in_any_order(ctx, tmp_path, n, k):
     pre = n // 2
     g = [np.array([r.choice(size, k, replace=False) for _ in range(size)], np.uint32) for size in (pre, n - pre)]
     check(ctx, tmp_path, x, k, pre, g[0], g[1], 3)
+
+
+def hub_case(n, k, seed):
+    """Rows far from each other and near row 0 (n / 2: row n / 2 of the second
+    half); two rows in three list that hub twice, the others once."""
+    r = np.random.default_rng(seed)
+    x = np.zeros((n, 48), np.float32)
+    for i in range(n):
+        x[i, r.choice(48, 3, replace=False)] = r.integers(60, 90, 3)
+    pre = n // 2
+    for hub in (0, pre):
+        x[hub] = r.integers(0, 9, 48)
+    g = []
+    for size in (pre, n - pre):
+        a = np.zeros((size, k), np.uint32)
+        for i in range(size):
+            a[i] = 1 + r.choice(size - 1, k, replace=False)
+            a[i][a[i] == i] = 0
+            if i:
+                a[i, 0] = 0
+                if i % 3:
+                    a[i, 1] = 0
+        g.append(a)
+    return x, pre, g[0], g[1]
+
+
+@pytest.mark.parametrize("n,k", [(6000, 8), (20000, 6)])
+def test_repeated_rows_across_sorted_runs(ctx, tmp_path, n, k):
+    """Reverse lists of more than 4,096 entries that hold rows twice: the
+    block-wide sort joins runs of 4,096 entries, and both copies of a row have
+    to come through when they lie in different runs."""
+    x, pre, g1, g2 = hub_case(n, k, n)
+    check(ctx, tmp_path, x, k, pre, g1, g2, 7)
