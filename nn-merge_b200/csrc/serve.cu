@@ -217,6 +217,11 @@ __device__ __forceinline__ float warp_dists_short(const float4 (&qr)[QV], const 
     return out;
 }
 
+// NaN distances (of queries or rows with NaN, or infinities that cancel)
+// count as infinite: comparisons of NaN would give the lanes different
+// minima and several new entries the same place in the beam, others none.
+__device__ __forceinline__ float ordered(float d) { return d == d ? d : INFINITY; }
+
 __device__ __forceinline__ bool key_less(float da, uint32_t ia, float db, uint32_t ib) {
     return da < db || (da == db && ia < ib);
 }
@@ -291,7 +296,8 @@ __global__ void __launch_bounds__(FW * 32, DENSE ? 7 : 5) k_serve(ServeArgs a) {
     const float4* x4 = reinterpret_cast<const float4*>(a.x);
     const uint32_t nlast = a.nrows[a.L - 1];
     auto dists = [](const float4(&qr)[QV], const float4* x, uint32_t dp4, uint32_t fid, uint32_t nf, uint32_t lane) {
-        return DENSE ? warp_dists_short<M, QV>(qr, x, dp4, fid, nf, lane) : warp_dists<M, QV>(qr, x, dp4, fid, nf, lane);
+        return ordered(DENSE ? warp_dists_short<M, QV>(qr, x, dp4, fid, nf, lane)
+                             : warp_dists<M, QV>(qr, x, dp4, fid, nf, lane));
     };
     unsigned long long cmps = 0, nexp = 0;
     for (;;) {
@@ -751,7 +757,7 @@ __global__ void __launch_bounds__(TEAM * 32) k_serve_team(ServeArgs a) {
             __syncthreads();
             team_rows<M, QV>(qr, x4, a.dp4, fid, 0, cnt, lane, raw);
             __syncthreads();
-            return raw[lane];
+            return ordered(raw[lane]);
         };
         uint32_t cur = 0, g0;
         float cur_d = 0.f;
