@@ -139,6 +139,14 @@ size_t chunk_for(size_t bytes, int workers) {
     return std::min(std::max(c, (size_t)128 << 10), HostStage::CHUNK);
 }
 
+// A copy's status once its failure is known: copies already under way end
+// first, so that neither the slots (whose event may be the call that failed)
+// nor the caller's memory are still in use.
+cudaError_t settled(Ctx& ctx, cudaError_t e) {
+    if (e != cudaSuccess) cudaStreamSynchronize(ctx.stream);
+    return e;
+}
+
 }  // namespace
 
 void HostStage::release() {
@@ -176,7 +184,7 @@ cudaError_t host_to_dev(Ctx& ctx, void* dst, const void* src, size_t bytes) {
         }
         if (e != cudaSuccess) err = e;
     });
-    return (cudaError_t)err.load();
+    return settled(ctx, (cudaError_t)err.load());
 }
 
 cudaError_t dev_to_host(Ctx& ctx, const HostPiece* pieces, int count) {
@@ -193,7 +201,7 @@ cudaError_t dev_to_host(Ctx& ctx, const HostPiece* pieces, int count) {
             if (pieces[i].host && pieces[i].bytes) {
                 const cudaError_t e = cudaMemcpyAsync(pieces[i].host, pieces[i].dev, pieces[i].bytes,
                                                       cudaMemcpyDeviceToHost, ctx.stream);
-                if (e != cudaSuccess) return e;
+                if (e != cudaSuccess) return settled(ctx, e);
             }
         return cudaStreamSynchronize(ctx.stream);
     }
@@ -238,7 +246,7 @@ cudaError_t dev_to_host(Ctx& ctx, const HostPiece* pieces, int count) {
             if (e == cudaSuccess) len[slot] = n;
         };
         for (int slot = 0; slot < HostStage::SLOTS; slot++) start(slot);
-        for (int slot = 0; len[slot]; slot ^= 1) {
+        for (int slot = 0; e == cudaSuccess && len[slot]; slot ^= 1) {  // ends with the first error
             e = cudaEventSynchronize(s.done[w][slot]);
             if (e != cudaSuccess) break;
             std::memcpy(host[slot], slot_ptr(slot), len[slot]);
@@ -247,7 +255,7 @@ cudaError_t dev_to_host(Ctx& ctx, const HostPiece* pieces, int count) {
         if (e != cudaSuccess) err = e;
     });
     const cudaError_t e = (cudaError_t)err.load();
-    return e != cudaSuccess ? e : cudaStreamSynchronize(ctx.stream);
+    return e != cudaSuccess ? settled(ctx, e) : cudaStreamSynchronize(ctx.stream);
 }
 
 }  // namespace nnm

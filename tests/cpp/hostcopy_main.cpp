@@ -1,0 +1,161 @@
+// hostcopy.cu over a stand-in for the CUDA runtime: copies wait in a queue
+// until an event or the stream is waited for (as a device's DMA may), and a
+// chosen call fails once.  Prints one line per check; exit status 1 on a
+// failed one.
+#include <math.h>
+
+#include <cstdio>
+#include <cstdlib>
+#include <deque>
+#include <map>
+
+// what the headers' device code names (none of it is called here)
+float __fadd_rn(float, float), __fsub_rn(float, float), __fmul_rn(float, float), __fdiv_rn(float, float);
+unsigned __umulhi(unsigned, unsigned);
+int __popc(unsigned), __clz(int);
+
+#include "../../nn-merge_b200/csrc/hostcopy.cu"
+
+namespace {
+struct Copy {
+    void* dst;
+    const void* src;
+    size_t bytes;
+};
+std::mutex mu;
+std::deque<Copy> queue_;
+size_t done_ = 0, issued_ = 0;          // copies carried out, copies issued
+std::map<cudaEvent_t, size_t> marks;    // event -> copies issued before its record
+std::map<const char*, size_t> pinned;   // page-locked ranges
+long calls = 0, fail_at = 0;            // the fail_at-th enqueue or record call fails
+
+void run_to(size_t upto) {
+    while (done_ < upto && !queue_.empty()) {
+        const Copy c = queue_.front();
+        queue_.pop_front();
+        std::memcpy(c.dst, c.src, c.bytes);
+        done_++;
+    }
+}
+bool is_pinned(const void* p) {
+    auto it = pinned.upper_bound(static_cast<const char*>(p));
+    if (it == pinned.begin()) return false;
+    --it;
+    return static_cast<const char*>(p) < it->first + it->second;
+}
+bool fails() { return ++calls == fail_at; }
+}  // namespace
+
+extern "C" {
+cudaError_t cudaMemcpyAsync(void* dst, const void* src, size_t bytes, cudaMemcpyKind kind, cudaStream_t) {
+    std::lock_guard<std::mutex> l(mu);
+    if (fails()) return cudaErrorUnknown;
+    queue_.push_back({dst, src, bytes});
+    issued_++;
+    // pageable host memory is staged (in) or waited for (out) within the call
+    if (!is_pinned(kind == cudaMemcpyHostToDevice ? src : dst)) run_to(issued_);
+    return cudaSuccess;
+}
+cudaError_t cudaEventRecord(cudaEvent_t e, cudaStream_t) {
+    std::lock_guard<std::mutex> l(mu);
+    if (fails()) return cudaErrorUnknown;
+    marks[e] = issued_;
+    return cudaSuccess;
+}
+cudaError_t cudaEventSynchronize(cudaEvent_t e) {
+    std::lock_guard<std::mutex> l(mu);
+    run_to(marks[e]);
+    return cudaSuccess;
+}
+cudaError_t cudaStreamSynchronize(cudaStream_t) {
+    std::lock_guard<std::mutex> l(mu);
+    run_to(issued_);
+    return cudaSuccess;
+}
+cudaError_t cudaEventCreateWithFlags(cudaEvent_t* e, unsigned) {
+    *e = reinterpret_cast<cudaEvent_t>(std::malloc(1));
+    return cudaSuccess;
+}
+cudaError_t cudaEventDestroy(cudaEvent_t e) {
+    std::free(e);
+    return cudaSuccess;
+}
+cudaError_t cudaMallocHost(void** p, size_t bytes) {
+    std::lock_guard<std::mutex> l(mu);
+    *p = std::malloc(bytes);
+    pinned[static_cast<char*>(*p)] = bytes;
+    return cudaSuccess;
+}
+cudaError_t cudaFreeHost(void* p) {
+    std::lock_guard<std::mutex> l(mu);
+    pinned.erase(static_cast<char*>(p));
+    std::free(p);
+    return cudaSuccess;
+}
+cudaError_t cudaPointerGetAttributes(cudaPointerAttributes* a, const void* p) {
+    std::lock_guard<std::mutex> l(mu);
+    a->type = is_pinned(p) ? cudaMemoryTypeHost : cudaMemoryTypeUnregistered;
+    return cudaSuccess;
+}
+cudaError_t cudaGetLastError(void) { return cudaSuccess; }
+cudaError_t cudaSetDevice(int) { return cudaSuccess; }
+cudaError_t cudaMalloc(void** p, size_t bytes) {
+    *p = std::malloc(bytes);
+    return cudaSuccess;
+}
+cudaError_t cudaFree(void* p) {
+    std::free(p);
+    return cudaSuccess;
+}
+}
+
+namespace {
+int bad = 0;
+void check(bool ok, const char* what, size_t bytes, long at) {
+    if (!ok) {
+        bad++;
+        std::printf("FAILED %s, %zu bytes, call %ld\n", what, bytes, at);
+    }
+}
+std::vector<unsigned char> bytes_of(size_t n, unsigned seed) {
+    std::vector<unsigned char> v(n);
+    for (size_t i = 0; i < n; i++) v[i] = (unsigned char)((i * 2654435761u + seed) >> 13);
+    return v;
+}
+
+// A failed call shows in the status, whichever it is, and nothing of the
+// copy is under way when the call returns.
+void errors(size_t n) {
+    long total = 1;
+    for (long at = 0; at < total; at++) {  // 0: none
+        const auto src = bytes_of(n, 1);
+        for (int out = 0; out < 2; out++) {
+            nnm::Ctx ctx;
+            std::vector<unsigned char> dst(n), tail(1000);
+            calls = 0;
+            fail_at = at;
+            cudaError_t e;
+            if (out) {
+                const nnm::HostPiece p[] = {{dst.data(), src.data(), n}, {nullptr, src.data(), n}, {tail.data(), src.data(), 1000}};
+                e = nnm::dev_to_host(ctx, p, 3);
+            } else {
+                e = nnm::host_to_dev(ctx, dst.data(), src.data(), n);
+            }
+            const bool hit = at > 0 && calls >= at;
+            check((e != cudaSuccess) == hit, out ? "status of a copy out" : "status of a copy in", n, at);
+            if (hit) check(queue_.empty(), "nothing under way after an error", n, at);
+            total = std::max(total, calls + 1);
+            cudaStreamSynchronize(nullptr);
+            if (!hit) check(dst == src, "bytes", n, at);
+            if (!hit && out) check(!std::memcmp(tail.data(), src.data(), 1000), "bytes of the last piece", n, at);
+            ctx.stage.release();
+        }
+    }
+    std::printf("errors: %zu bytes, %ld calls\n", n, total - 1);
+}
+}  // namespace
+
+int main() {
+    for (size_t n : {(size_t)1000, (size_t)(2 << 20), (size_t)(9 << 20) + 7}) errors(n);
+    return bad != 0;
+}
