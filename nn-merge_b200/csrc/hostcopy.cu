@@ -163,8 +163,13 @@ void HostStage::release() {
 
 cudaError_t host_to_dev(Ctx& ctx, void* dst, const void* src, size_t bytes) {
     HostStage& s = ctx.stage;
-    if (bytes < PARALLEL_MIN || !pageable(src) || !stage_ready(s))
-        return cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, ctx.stream);
+    const bool paged = pageable(src);
+    if (bytes < PARALLEL_MIN || !paged || !stage_ready(s)) {
+        const cudaError_t e = cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, ctx.stream);
+        // pageable memory is staged within the call; pinned and managed memory
+        // is read while the copy runs
+        return e == cudaSuccess && !paged ? cudaStreamSynchronize(ctx.stream) : e;
+    }
     const int workers = workers_for(bytes);
     const size_t chunk = chunk_for(bytes, workers), chunks = (bytes + chunk - 1) / chunk;
     std::atomic<size_t> next{0};

@@ -31,7 +31,7 @@ struct HostPiece {
 };
 
 // dst[0, bytes) = src, ordered on the context's stream; src may change once
-// the call returns.
+// the call returns (it waits for the copy of pinned or managed memory).
 cudaError_t host_to_dev(Ctx& ctx, void* dst, const void* src, size_t bytes);
 // Every piece's device bytes to its host memory, after the work on the
 // context's stream; complete when the call returns.  Pieces with a null host

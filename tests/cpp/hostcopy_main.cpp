@@ -153,9 +153,32 @@ void errors(size_t n) {
     }
     std::printf("errors: %zu bytes, %ld calls\n", n, total - 1);
 }
+
+// The source changes as soon as the call returns, while copies that still
+// wait run late.
+void sources(size_t n) {
+    const auto src = bytes_of(n, 2);
+    for (int page_locked = 0; page_locked < 2; page_locked++) {
+        nnm::Ctx ctx;
+        std::vector<unsigned char> dst(n);
+        void* p = nullptr;
+        if (page_locked) cudaMallocHost(&p, n);
+        else p = std::malloc(n);
+        std::memcpy(p, src.data(), n);
+        calls = fail_at = 0;
+        check(nnm::host_to_dev(ctx, dst.data(), p, n) == cudaSuccess, "copy in", n, 0);
+        std::memset(p, 0xee, n);
+        cudaStreamSynchronize(nullptr);
+        check(dst == src, page_locked ? "a pinned source that changes" : "a pageable source that changes", n, 0);
+        if (page_locked) cudaFreeHost(p);
+        else std::free(p);
+        ctx.stage.release();
+    }
+}
 }  // namespace
 
 int main() {
     for (size_t n : {(size_t)1000, (size_t)(2 << 20), (size_t)(9 << 20) + 7}) errors(n);
+    for (size_t n : {(size_t)1, (size_t)100000, (size_t)(8 << 20), (size_t)(9 << 20) + 7}) sources(n);
     return bad != 0;
 }
