@@ -77,6 +77,13 @@ int index_upload(Ctx& ctx, IndexDev& ix, const float* x, uint64_t n, uint32_t d,
 // distance and expansion counts) before a run.
 int index_run_exact(Ctx& ctx, IndexDev& ix, const SearchReq& r);
 int index_run_fast(Ctx& ctx, IndexDev& ix, const SearchReq& r);
+// Blocks that an index's per-warp scratch is allocated for when a batch runs
+// `blocks` of them: one an SM, or as soon as a batch has more all that the
+// largest batch runs (full), so that growing batches allocate and clear it
+// twice at most.
+inline uint32_t scratch_blocks(uint32_t blocks, uint32_t full, uint32_t nsm) {
+    return blocks <= nsm ? nsm : blocks < full ? full : blocks;
+}
 // Seeds of nndFlatSrch for every beam width up to beam_max (cached).
 int index_flat_seeds(Ctx& ctx, IndexDev& ix, uint32_t beam_max);
 // Waits for the stream, reads the distance and expansion counts of the last

@@ -625,10 +625,10 @@ int index_run_exact(Ctx& ctx, IndexDev& ix, const SearchReq& r) {
     NNM_CUDA_TRY(cudaFuncSetAttribute(k_search, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     int per_sm = 1;
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_search, SWARPS * 32, smem);
-    const uint32_t blocks = std::min((uint32_t)std::min(std::max(1, per_sm), 4) * (uint32_t)nsm,
-                                     (r.nq + SWARPS - 1) / SWARPS);
+    const uint32_t full = (uint32_t)std::min(std::max(1, per_sm), 4) * (uint32_t)nsm;
+    const uint32_t blocks = std::min(full, (r.nq + SWARPS - 1) / SWARPS);
     const uint32_t words = (uint32_t)((ix.n + 31) / 32);
-    const size_t slots = (size_t)blocks * SWARPS;
+    const size_t slots = (size_t)scratch_blocks(blocks, full, (uint32_t)nsm) * SWARPS;
     if (ix.visited.bytes < slots * words * 4) {
         NNM_CUDA_TRY(ix.visited.ensure(slots * words * 4));
         NNM_CUDA_TRY(cudaMemsetAsync(ix.visited.p, 0, slots * words * 4, st));
