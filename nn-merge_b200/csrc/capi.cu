@@ -576,6 +576,7 @@ int nnm_hmerge_build(nnm_ctx* ctx, const float* x, uint64_t n, uint32_t d, uint3
         rc = nnm::hmerge_build(c, g, [&](Ctx& cc, GraphDev& gg) { return nnm::dpg_layer(cc, dpg, gg, layers); });
     if (!rc) rc = nnm::export_graph(c, g, ids, dists, flags, true);
     float ms = tm.stop();
+    dpg.release(nnm::KEEP_BYTES);
     if (!rc) fill_stats(stats, g, 0, ms);
     else if (layers) nnm_layers_free(layers);
     return rc;
@@ -699,6 +700,7 @@ int nnm_mlp_grad(nnm_ctx* ctx, const nnm_mlp* model, const float* x, uint64_t n,
         if (triplets[i] >= n) return fail(ctx, NNM_ERR_INVALID, "triplet index out of range");
     Ctx& c = ctx->c;
     if (cudaSetDevice(c.device) != cudaSuccess) return fail(ctx, NNM_ERR_NO_DEVICE, "cudaSetDevice failed");
+    nnm::KeepBound kx(c.store.x), ks(c.ws.bucket);
     GraphDev g;
     int rc = upload_plain(c, c.store, g, x, n, d);
     if (!rc) rc = nnm::mlp_grad(c, *model, g.x, (uint32_t)n, g.dp, triplets, ntrip, margin, loss, *grad);
@@ -772,6 +774,7 @@ int nnm_graph_recall(nnm_ctx* ctx, const float* x, uint64_t n, uint32_t d, const
     // the vectors in the context's graph store; the evaluated rows and the
     // first atop ids of their lists, the only ones read, in its workspace
     // (a call used to allocate five buffers, copy all n x k ids and free them)
+    nnm::KeepBound kx(c.store.x), ks(c.ws.bucket), km(c.ws.misc);
     GraphDev g;
     int rc = upload_plain(c, c.store, g, x, n, d);
     std::vector<uint32_t> h((size_t)nrows * (atop + 1));

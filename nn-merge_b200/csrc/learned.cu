@@ -570,18 +570,17 @@ cudaError_t set_fwd_attrs(uint32_t d) {
 
 // Scratch of one training/gradient pass over B triplets, laid out in the
 // context's training workspace (a call allocated and freed 13 buffers, 2-3 ms
-// with the frees' waits).  A workspace above KEEP bytes is given back at the end.
+// with the frees' waits).  A workspace above KEEP_BYTES is given back at the end.
 struct Pass {
     struct Span {
         void* p = nullptr;
         template <class T> T* as() const { return static_cast<T*>(p); }
     };
-    static constexpr size_t KEEP = (size_t)256 << 20;
     DevBuf& arena;
     Span idx, h, t, dz, dh, partial, flat, grad, mom, vel, w1t, w2t, loss, step;
     explicit Pass(Ctx& ctx) : arena(ctx.ws.train) {}
     ~Pass() {
-        if (arena.bytes > KEEP) arena.release();
+        if (arena.bytes > KEEP_BYTES) arena.release();
     }
 };
 

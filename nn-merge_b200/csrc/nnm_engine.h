@@ -36,6 +36,19 @@ struct DevBuf {
     template <class T> T* as() const { return static_cast<T*>(p); }
 };
 
+// Memory that a call other than a build leaves allocated in its context, per
+// buffer that it grew: what takes more is given back when the call returns
+// (allocating and freeing a quarter of a GB is small beside the work on it).
+constexpr size_t KEEP_BYTES = (size_t)256 << 20;
+struct KeepBound {
+    DevBuf& b;
+    size_t had;
+    explicit KeepBound(DevBuf& buf) : b(buf), had(buf.bytes) {}
+    ~KeepBound() {
+        if (b.bytes > KEEP_BYTES && b.bytes > had) b.release();
+    }
+};
+
 // Scratch for one NN-Descent iteration, sized for the largest graph seen.
 struct Workspace {
     DevBuf rcnt, rcur, rtot, roff, rseg, rscr, rofs, rbuf;
@@ -89,7 +102,7 @@ struct DpgState;
 struct Ctx {
     int device = 0;
     DevMlp* init_model = nullptr;  // learned-initialisation model (owned)
-    DpgState* dpg = nullptr;       // H-Merge's DPG lists, reused across calls (grow-only, owned)
+    DpgState* dpg = nullptr;       // H-Merge's DPG lists, reused across calls up to KEEP_BYTES (owned)
     bool prof = false;
     GraphStore store;  // graph arrays, reused across calls (grow-only)
     KStat kjoin, kemit, kmerge;

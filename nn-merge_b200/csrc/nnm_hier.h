@@ -21,10 +21,13 @@ struct DpgState {
     DevBuf ecnt, ecur, eoff, ev, escr, bigseg, counters, tmp;
     uint32_t cap = 0, K = 0, M = 0, rows = 0, n_cap = 0;
     uint32_t last_rounds = 0;
-    void release() {
+    void release(size_t above = 0) {  // if the buffers together hold more than `above` bytes
         DevBuf* all[] = {&gid, &gdist, &glen, &g1id, &g1dist, &g1len, &sid, &sdist, &slen, &tid, &tdist,
                          &tlen, &ecnt, &ecur, &eoff, &ev, &escr, &bigseg, &counters, &tmp};
-        for (auto* b : all) b->release();
+        size_t held = 0;
+        for (auto* b : all) held += b->bytes;
+        if (held > above)
+            for (auto* b : all) b->release();
     }
 };
 
