@@ -38,14 +38,18 @@ namespace nnm {
 namespace {
 constexpr unsigned FULL = 0xffffffffu;
 constexpr int FW = 4;                    // warps per block
-constexpr uint32_t FVCAP = 65536;        // visited ids recorded per warp slot, at most
+// Visited ids recorded per warp slot; a query that visits more clears its
+// whole bitmap (65,536 ids took 0.8 GB an index, 1.1 in the dense form).  A
+// constant: lists as long as the layer or the bitmap, as an argument, cost
+// k_serve 2 to 4 % (L2 and L1, 100,000 x 128, 1,500 to 8,000 queries).
+constexpr uint32_t FVCAP = 16384;
 constexpr uint32_t EXP_BIT = 1u << 31;   // beam entry already expanded
 constexpr uint32_t IDM = 0x7fffffffu;
 constexpr uint32_t FAST_MAX_DP = 512;    // 4 float4 per lane
 constexpr uint32_t WARPS = 20;                          // k_serve: warps per SM
 constexpr uint32_t DENSE_WARPS = 28;                    // .. of its dense form,
 constexpr uint32_t DENSE_QUERIES = 2 * DENSE_WARPS;     // for more queries per SM than these
-constexpr size_t DENSE_SCRATCH = (size_t)256 << 20;     // and at most this much of visited bitmaps and lists
+constexpr size_t DENSE_SCRATCH = (size_t)387 << 20;     // and at most this much of visited bitmaps and lists (259,000 rows)
 constexpr uint32_t GROUP = 4;            // 32-id chunks of a step whose loads and atomics overlap
 constexpr uint32_t WARP_EXTRA = 256 + GROUP * 32 * 4;  // nd, ni and fr after the beam's two arrays
 
@@ -77,7 +81,6 @@ struct ServeArgs {
     const uint32_t* flat_off;    // seeds of beam width b at flat_pool + flat_off[b]
     const uint32_t* flat_pool;
     unsigned* next_q;
-    uint32_t vcap;  // entries of a slot's visited list
     unsigned* overflow;
     unsigned long long* ncmps;
     unsigned long long* nexp;
@@ -294,7 +297,7 @@ __global__ void __launch_bounds__(FW * 32, DENSE ? 7 : 5) k_serve(ServeArgs a) {
     uint32_t* ni = reinterpret_cast<uint32_t*>(nd + 32);
     uint32_t* fr = ni + 32;  // fresh ids of one group of a step
     uint32_t* vis = a.visited + (size_t)slot * a.words;
-    uint32_t* vl = a.vlist + (size_t)slot * a.vcap;
+    uint32_t* vl = a.vlist + (size_t)slot * FVCAP;
     const float4* x4 = reinterpret_cast<const float4*>(a.x);
     const uint32_t nlast = a.nrows[a.L - 1];
     auto dists = [](const float4(&qr)[QV], const float4* x, uint32_t dp4, uint32_t fid, uint32_t nf, uint32_t lane) {
@@ -458,7 +461,7 @@ __global__ void __launch_bounds__(FW * 32, DENSE ? 7 : 5) k_serve(ServeArgs a) {
                 if (lane < cnt) {
                     id = sd[c0 + lane];
                     atomicOr(&vis[id >> 5], 1u << (id & 31));
-                    if (nvis + lane < a.vcap) vl[nvis + lane] = id;
+                    if (nvis + lane < FVCAP) vl[nvis + lane] = id;
                 }
                 nvis += cnt;
                 offer(id, cnt);
@@ -556,7 +559,7 @@ __global__ void __launch_bounds__(FW * 32, DENSE ? 7 : 5) k_serve(ServeArgs a) {
                         if (DENSE)
                             for (uint32_t t = 0; t < a.dp4; t += 8) prefetch_l2(x4 + (size_t)nn[c] * a.dp4 + t);
                         fr[r] = nn[c];
-                        if (nvis + r < a.vcap) vl[nvis + r] = nn[c];
+                        if (nvis + r < FVCAP) vl[nvis + r] = nn[c];
                     }
                     nf += __popc(fb);
                 }
@@ -576,7 +579,7 @@ __global__ void __launch_bounds__(FW * 32, DENSE ? 7 : 5) k_serve(ServeArgs a) {
             if (a.out_d) a.out_d[o] = t < m ? bd[t] : 0.f;
         }
         // clear this query's visited bits
-        if (nvis <= a.vcap) {
+        if (nvis <= FVCAP) {
             for (uint32_t t = lane; t < nvis; t += 32) {
                 const uint32_t id = vl[t];
                 atomicAnd(&vis[id >> 5], ~(1u << (id & 31)));
@@ -1149,13 +1152,8 @@ int index_run_fast(Ctx& ctx, IndexDev& ix, const SearchReq& r) {
         NNM_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&pt, team, TEAM * 32, tsmem));
         use_team = r.nq <= (uint32_t)std::max(pt, 0) * (uint32_t)nsm;
     }
-    // A query that visits more ids than its bitmap has words clears the whole
-    // bitmap, which is no more than clearing them one by one; so a slot's list
-    // needs no more entries (65,536 of them took 0.8 GB an index, 1.1 in the
-    // dense form).
-    const uint32_t vcap = std::min(FVCAP, words);
     // several queries per resident warp: the form with more warps
-    const bool dense_fits = ((size_t)words + vcap) * 4 * DENSE_WARPS * nsm <= DENSE_SCRATCH;
+    const bool dense_fits = ((size_t)words + FVCAP) * 4 * DENSE_WARPS * nsm <= DENSE_SCRATCH;
     const bool dense = !use_team && r.nq > DENSE_QUERIES * (uint32_t)nsm && dense_fits;
     const ServeFn fn = use_team ? team : dense ? pick_warp<true>(ix.metric, qv) : pick_warp<false>(ix.metric, qv);
     const size_t smem = use_team ? tsmem : (size_t)FW * ((size_t)r.beam_max * 8 + WARP_EXTRA);
@@ -1170,7 +1168,7 @@ int index_run_fast(Ctx& ctx, IndexDev& ix, const SearchReq& r) {
             NNM_CUDA_TRY(ix.visited.ensure(slots * words * 4));
             NNM_CUDA_TRY(cudaMemsetAsync(ix.visited.p, 0, slots * words * 4, st));
         }
-        NNM_CUDA_TRY(ix.vlist.ensure(slots * vcap * 4));
+        NNM_CUDA_TRY(ix.vlist.ensure(slots * FVCAP * 4));
     }
     ServeArgs a{};
     a.x = ix.x.as<float>();
@@ -1206,7 +1204,6 @@ int index_run_fast(Ctx& ctx, IndexDev& ix, const SearchReq& r) {
     a.overflow = reinterpret_cast<unsigned*>(c + 4);
     a.ncmps = reinterpret_cast<unsigned long long*>(c + 8);
     a.nexp = reinterpret_cast<unsigned long long*>(c + 16);
-    a.vcap = vcap;
     a.spec_blocks = (uint32_t)nsm;
     fn<<<blocks, (use_team ? TEAM : FW) * 32, smem, st>>>(a); count_launch();
     NNM_CUDA_TRY(cudaGetLastError());

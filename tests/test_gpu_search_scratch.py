@@ -17,8 +17,9 @@ def used():
 
 
 # form: its batches, the first of which has more blocks (of four queries)
-# than SMs; bound on what they keep, queries and results included
-@pytest.mark.parametrize("mode,batches,most", [("fast", [3_100, 3_900, 5_000, 9_000, 20_000], 120),
+# than SMs; bound on what they keep, queries and results included: 4,144 warps
+# of the fast form's bitmaps and lists of 16,384 ids
+@pytest.mark.parametrize("mode,batches,most", [("fast", [3_100, 3_900, 5_000, 9_000, 20_000], 320),
                                                ("exact", [700, 900, 1_500, 2_400, 5_000], 1_000)])
 def test_memory_of_growing_batches(ctx, mode, batches, most):
     x = gaussian_mixture_u8(50_000, d=16, seed=1)
@@ -37,8 +38,8 @@ def test_memory_of_growing_batches(ctx, mode, batches, most):
 
 @pytest.mark.parametrize("n", [33, 2_000, 40_000])
 def test_more_visits_than_list_entries(ctx, n):
-    """A warp per query, dense and not: queries that visit more ids than the
-    bitmap has words (beams near the layer) and few, in turn, give what a
+    """A warp per query, dense and not: queries that visit most of the layer
+    (40,000 rows: more ids than a list holds) and few, in turn, give what a
     block per query gives."""
     r = np.random.default_rng(n)
     x = gaussian_mixture_u8(n, d=8, seed=2)
