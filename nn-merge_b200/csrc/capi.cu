@@ -988,12 +988,9 @@ int index_search_impl(nnm_index* h, const float* q, uint64_t nq, const uint32_t*
     // out, one wait -- five copies from and to pageable memory, each waited
     // for, were 70 us of a 280-us call of one query
     const size_t in_bytes = (size_t)nq * dp * 4 + (beams ? (size_t)nq * 4 : 0), out_bytes = (size_t)nq * out_k * 8;
-    const bool small = !dev && in_bytes + out_bytes + 128 <= nnm::INDEX_IO_BYTES;
-    if (small && !ix.h_io) {
-        void* p = nullptr;
-        if ((rc = cu(cudaMallocHost(&p, nnm::INDEX_IO_BYTES)))) return rc;
-        ix.h_io = static_cast<unsigned char*>(p);
-    }
+    const bool fits = !dev && in_bytes + out_bytes + 128 <= nnm::INDEX_IO_BYTES;
+    if (fits && !ix.h_io) ix.h_io = nnm::pinned_block(nnm::INDEX_IO_BYTES);
+    const bool small = fits && ix.h_io;  // without pinned memory: as a large batch
     // queries with rows of dp floats
     const float* qd = q;
     if (small) {

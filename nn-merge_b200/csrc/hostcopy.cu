@@ -99,13 +99,11 @@ bool pageable(const void* p) {
 bool stage_ready(HostStage& s) {
     if (s.block) return true;
     if (s.failed) return false;
-    void* p = nullptr;
-    bool ok = cudaMallocHost(&p, HostStage::WORKERS * HostStage::SLOTS * HostStage::CHUNK) == cudaSuccess;
-    if (ok) {
-        s.block = static_cast<unsigned char*>(p);
+    s.block = pinned_block(HostStage::WORKERS * HostStage::SLOTS * HostStage::CHUNK);
+    bool ok = s.block != nullptr;
+    if (ok)
         for (auto& w : s.done)
             for (auto& e : w) ok = ok && cudaEventCreateWithFlags(&e, cudaEventDisableTiming) == cudaSuccess;
-    }
     if (!ok) {
         cudaGetLastError();
         s.release();
@@ -148,6 +146,13 @@ cudaError_t settled(Ctx& ctx, cudaError_t e) {
 }
 
 }  // namespace
+
+unsigned char* pinned_block(size_t bytes) {
+    void* p = nullptr;
+    if (cudaMallocHost(&p, bytes) == cudaSuccess) return static_cast<unsigned char*>(p);
+    cudaGetLastError();
+    return nullptr;
+}
 
 void HostStage::release() {
     delete threads;

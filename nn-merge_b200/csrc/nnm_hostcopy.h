@@ -30,6 +30,9 @@ struct HostPiece {
     size_t bytes;
 };
 
+// Pinned memory (freed with cudaFreeHost), or null where there is none: the
+// callers then copy without it.
+unsigned char* pinned_block(size_t bytes);
 // dst[0, bytes) = src, ordered on the context's stream; src may change once
 // the call returns (it waits for the copy of pinned or managed memory).
 cudaError_t host_to_dev(Ctx& ctx, void* dst, const void* src, size_t bytes);

@@ -28,6 +28,8 @@ size_t done_ = 0, issued_ = 0;          // copies carried out, copies issued
 std::map<cudaEvent_t, size_t> marks;    // event -> copies issued before its record
 std::map<const char*, size_t> pinned;   // page-locked ranges
 long calls = 0, fail_at = 0;            // the fail_at-th enqueue or record call fails
+bool no_pinned = false;                 // pinned memory cannot be had
+cudaError_t last_error = cudaSuccess;
 
 void run_to(size_t upto) {
     while (done_ < upto && !queue_.empty()) {
@@ -82,6 +84,7 @@ cudaError_t cudaEventDestroy(cudaEvent_t e) {
 }
 cudaError_t cudaMallocHost(void** p, size_t bytes) {
     std::lock_guard<std::mutex> l(mu);
+    if (no_pinned) return last_error = cudaErrorMemoryAllocation;
     *p = std::malloc(bytes);
     pinned[static_cast<char*>(*p)] = bytes;
     return cudaSuccess;
@@ -97,7 +100,11 @@ cudaError_t cudaPointerGetAttributes(cudaPointerAttributes* a, const void* p) {
     a->type = is_pinned(p) ? cudaMemoryTypeHost : cudaMemoryTypeUnregistered;
     return cudaSuccess;
 }
-cudaError_t cudaGetLastError(void) { return cudaSuccess; }
+cudaError_t cudaGetLastError(void) {
+    const cudaError_t e = last_error;
+    last_error = cudaSuccess;
+    return e;
+}
 cudaError_t cudaSetDevice(int) { return cudaSuccess; }
 cudaError_t cudaMalloc(void** p, size_t bytes) {
     *p = std::malloc(bytes);
@@ -175,10 +182,28 @@ void sources(size_t n) {
         ctx.stage.release();
     }
 }
+
+// Without pinned memory the copies still come through, and no error is left
+// for a later call to report.
+void without_pinned(size_t n) {
+    const auto src = bytes_of(n, 3);
+    nnm::Ctx ctx;
+    std::vector<unsigned char> dst(n), back(n);
+    calls = fail_at = 0;
+    no_pinned = true;
+    check(nnm::pinned_block(n) == nullptr && cudaGetLastError() == cudaSuccess, "no pinned block", n, 0);
+    const nnm::HostPiece p{back.data(), dst.data(), n};
+    check(nnm::host_to_dev(ctx, dst.data(), src.data(), n) == cudaSuccess &&
+              nnm::dev_to_host(ctx, &p, 1) == cudaSuccess && back == src && cudaGetLastError() == cudaSuccess,
+          "copies without pinned memory", n, 0);
+    no_pinned = false;
+    ctx.stage.release();
+}
 }  // namespace
 
 int main() {
     for (size_t n : {(size_t)1000, (size_t)(2 << 20), (size_t)(9 << 20) + 7}) errors(n);
     for (size_t n : {(size_t)1, (size_t)100000, (size_t)(8 << 20), (size_t)(9 << 20) + 7}) sources(n);
+    for (size_t n : {(size_t)1000, (size_t)(9 << 20) + 7}) without_pinned(n);
     return bad != 0;
 }
