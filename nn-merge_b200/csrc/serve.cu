@@ -48,8 +48,7 @@ constexpr uint32_t IDM = 0x7fffffffu;
 constexpr uint32_t FAST_MAX_DP = 512;    // 4 float4 per lane
 constexpr uint32_t WARPS = 20;                          // k_serve: warps per SM
 constexpr uint32_t DENSE_WARPS = 28;                    // .. of its dense form,
-constexpr uint32_t DENSE_QUERIES = 2 * DENSE_WARPS;     // for more queries per SM than these
-constexpr size_t DENSE_SCRATCH = (size_t)387 << 20;     // and at most this much of visited bitmaps and lists (259,000 rows)
+constexpr size_t DENSE_SCRATCH = (size_t)387 << 20;     // with at most this much of visited bitmaps and lists (259,000 rows)
 constexpr uint32_t GROUP = 4;            // 32-id chunks of a step whose loads and atomics overlap
 constexpr uint32_t WARP_EXTRA = 256 + GROUP * 32 * 4;  // nd, ni and fr after the beam's two arrays
 
@@ -278,10 +277,8 @@ __device__ __forceinline__ void prefetch_l2(const void* p) { asm volatile("prefe
 // DENSE, for batches of several queries per resident warp: seven CTAs per SM
 // (72 registers: the rows of a list summed eight at a time, prefetched into L2
 // when their ids are known); otherwise five CTAs (96 registers, 32 rows summed
-// together), whose single query is shorter.  The line: 20,000 queries, 100,000
-// rows, five CTAs against seven: beams 16 872 -> 761 us, 64 2,690 -> 2,442,
-// 32..512 6,492 -> 5,206, d = 160 8,448 -> 5,962; 3,000 queries (one each) 1,726
-// -> 2,062.  At 1M rows the 28 warps' bitmaps (518 MB, allocated and cleared
+// together), whose single query is shorter.  The line between them is
+// dense_queries.  At 1M rows the 28 warps' bitmaps (518 MB, allocated and cleared
 // by an index's first batch) gain 3 to 7 %, not worth it: so at most
 // DENSE_SCRATCH of them and their lists.  A hash table per query instead of a bitmap there took
 // 1.5 times as long.
@@ -1109,6 +1106,27 @@ __global__ void __launch_bounds__(TEAM * 32) k_serve_team(ServeArgs a) {
     }
 }
 
+// The dense form takes batches of more queries per SM than this (0: none).
+// Wider beams visit more rows and so wait more for the bitmaps, which 28 warps
+// an SM push out of the L2 sooner.  Device time, dense / not, at 8,300 to
+// 18,000 queries (56 to 122 an SM; 56 is two for every dense warp):
+//   rows of four float4 a lane, and chi-square: 0.17 to 0.73 from 56 on;
+//   beams 16 and 64: 0.79 to 0.94 and 0.85 to 1.05 from 56 on;
+//   beams 100 to 512, by the bitmaps of the dense form (rows):
+//     16 MB (31,000): 0.94 to 1.08 at 56, 0.89 to 1.01 from 67 on;
+//     64 MB (124,000), to beam 128: 0.98 to 1.12 at 61, 0.92 to 1.04 at 81, 0.87
+//       to 0.96 from 100 on; above: 0.99 to 1.17 at 56 and 61, 0.93 to 1.07 at
+//       81, 0.90 to 0.99 from 100 on;
+//     above, to beam 128: 0.99 to 1.13 at 61, 0.86 to 1.05 at 88, 0.90 to 1.01
+//       from 100 on; wider, one float4 a lane: 1.05 to 1.22 at 61, 0.99 to 1.05
+//       at 108 and 122; two: 1.15 to 1.20 at 61, 0.95 to 0.98 at 108.
+uint32_t dense_queries(int metric, uint32_t qv, uint32_t beam, size_t bitmaps) {
+    if (metric == CHI2 || qv > 2 || beam <= 64) return 56;
+    if (bitmaps <= (size_t)16 << 20) return 64;
+    if (bitmaps <= (size_t)64 << 20) return beam <= 128 ? 72 : 100;
+    return beam <= 128 || qv > 1 ? 100 : 0;
+}
+
 using ServeFn = void (*)(ServeArgs);
 template <int M, bool DENSE>
 ServeFn pick_qv(uint32_t qv) {
@@ -1154,7 +1172,8 @@ int index_run_fast(Ctx& ctx, IndexDev& ix, const SearchReq& r) {
     }
     // several queries per resident warp: the form with more warps
     const bool dense_fits = ((size_t)words + FVCAP) * 4 * DENSE_WARPS * nsm <= DENSE_SCRATCH;
-    const bool dense = !use_team && r.nq > DENSE_QUERIES * (uint32_t)nsm && dense_fits;
+    const uint32_t line = dense_queries((int)ix.metric, qv, r.beam_max, (size_t)words * 4 * DENSE_WARPS * nsm);
+    const bool dense = !use_team && dense_fits && line && r.nq > line * (uint32_t)nsm;
     const ServeFn fn = use_team ? team : dense ? pick_warp<true>(ix.metric, qv) : pick_warp<false>(ix.metric, qv);
     const size_t smem = use_team ? tsmem : (size_t)FW * ((size_t)r.beam_max * 8 + WARP_EXTRA);
     uint32_t blocks = r.nq;
