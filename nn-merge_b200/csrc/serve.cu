@@ -34,6 +34,8 @@
 #include "nnm_hier.h"
 #include "nnm_launch.h"
 
+#pragma nv_diag_suppress 177  // every object of this file (below) uses a part of it
+
 namespace nnm {
 namespace {
 constexpr unsigned FULL = 0xffffffffu;
@@ -615,6 +617,7 @@ __global__ void __launch_bounds__(FW * 32, DENSE ? 7 : 5) k_serve(ServeArgs a) {
 // picks it.  The beam in registers (up to 192 entries) against shared memory:
 // 177 -> 155 us.
 constexpr int TEAM = 4;
+constexpr uint32_t TEAM_MOST = 16;  // blocks an SM: 64 warps
 
 // Distances to rows [first, first + 8) of the cnt <= 32 ids that the lanes
 // hold, into out[0, 8) (shared memory).  NB rows at a time are summed by a
@@ -1106,6 +1109,22 @@ __global__ void __launch_bounds__(TEAM * 32) k_serve_team(ServeArgs a) {
     }
 }
 
+#ifdef NNM_SERVE_FORM
+using ServeFn = void (*)(ServeArgs);
+template <int M>
+ServeFn pick_warp(uint32_t qv, bool dense) {
+    if (dense) return qv == 1 ? k_serve<M, 1, true> : (qv == 2 ? k_serve<M, 2, true> : k_serve<M, 4, true>);
+    return qv == 1 ? k_serve<M, 1, false> : (qv == 2 ? k_serve<M, 2, false> : k_serve<M, 4, false>);
+}
+template <int M, int QV>
+ServeFn pick_team_beam(uint32_t beam) {
+    return beam <= 64 ? k_serve_team<M, QV, 2> : (beam <= 192 ? k_serve_team<M, QV, 6> : k_serve_team<M, QV, 0>);
+}
+template <int M>
+ServeFn pick_team(uint32_t qv, uint32_t beam) {
+    return qv == 1 ? pick_team_beam<M, 1>(beam) : (qv == 2 ? pick_team_beam<M, 2>(beam) : pick_team_beam<M, 4>(beam));
+}
+#else
 // The dense form takes batches of more queries per SM than this (0: none).
 // Wider beams visit more rows and so wait more for the bitmaps, which 28 warps
 // an SM push out of the L2 sooner.  Device time, dense / not, at 8,300 to
@@ -1126,25 +1145,28 @@ uint32_t dense_queries(int metric, uint32_t qv, uint32_t beam, size_t bitmaps) {
     if (bitmaps <= (size_t)64 << 20) return beam <= 128 ? 72 : 100;
     return beam <= 128 || qv > 1 ? 100 : 0;
 }
-
-using ServeFn = void (*)(ServeArgs);
-template <int M, bool DENSE>
-ServeFn pick_qv(uint32_t qv) {
-    return qv == 1 ? k_serve<M, 1, DENSE> : (qv == 2 ? k_serve<M, 2, DENSE> : k_serve<M, 4, DENSE>);
-}
-template <bool DENSE>
-ServeFn pick_warp(int metric, uint32_t qv) {
-    return metric == L2 ? pick_qv<L2, DENSE>(qv) : (metric == L1 ? pick_qv<L1, DENSE>(qv) : pick_qv<CHI2, DENSE>(qv));
-}
-template <int M, int QV>
-ServeFn pick_team_beam(uint32_t beam) {
-    return beam <= 64 ? k_serve_team<M, QV, 2> : (beam <= 192 ? k_serve_team<M, QV, 6> : k_serve_team<M, QV, 0>);
-}
-template <int M>
-ServeFn pick_team(uint32_t qv, uint32_t beam) {
-    return qv == 1 ? pick_team_beam<M, 1>(beam) : (qv == 2 ? pick_team_beam<M, 2>(beam) : pick_team_beam<M, 4>(beam));
-}
+#endif
 }  // namespace
+
+// This file is compiled seven times: for the host side, and for the kernels of
+// each form (NNM_SERVE_FORM: warp, team) and metric.  A form's kernels are a
+// module of their own, so that a program's first search loads the forms it
+// may run and not all 45 (its first one-query call: 28 -> 2 ms), and they
+// compile side by side.
+#define NNM_SERVE_NAME_(form, metric) serve_##form##_##metric
+#define NNM_SERVE_NAME(form, metric) NNM_SERVE_NAME_(form, metric)
+#ifdef NNM_SERVE_FORM
+#define NNM_SERVE_PICK_(form) pick_##form
+#define NNM_SERVE_PICK(form) NNM_SERVE_PICK_(form)
+const void* NNM_SERVE_NAME(NNM_SERVE_FORM, NNM_SERVE_METRIC)(uint32_t qv, uint32_t arg) {
+    return reinterpret_cast<const void*>(NNM_SERVE_PICK(NNM_SERVE_FORM)<NNM_SERVE_METRIC>(qv, arg));
+}
+#else
+// The kernel for qv float4 a lane: arg = the dense form (warp), or the widest
+// beam (team).
+using ServePick = const void* (*)(uint32_t qv, uint32_t arg);
+const void *serve_warp_L2(uint32_t, uint32_t), *serve_warp_L1(uint32_t, uint32_t), *serve_warp_CHI2(uint32_t, uint32_t),
+    *serve_team_L2(uint32_t, uint32_t), *serve_team_L1(uint32_t, uint32_t), *serve_team_CHI2(uint32_t, uint32_t);
 
 int index_run_fast(Ctx& ctx, IndexDev& ix, const SearchReq& r) {
     cudaStream_t st = ctx.stream;
@@ -1160,21 +1182,24 @@ int index_run_fast(Ctx& ctx, IndexDev& ix, const SearchReq& r) {
     const uint32_t words = (ix.n + 31) / 32;
     // a block per query while the blocks resident at once hold them all, and
     // the visited bitmap fits in shared memory
-    const ServeFn team = ix.metric == L2 ? pick_team<L2>(qv, r.beam_max)
-                         : (ix.metric == L1 ? pick_team<L1>(qv, r.beam_max) : pick_team<CHI2>(qv, r.beam_max));
+    const ServePick pick_team = ix.metric == L2 ? serve_team_L2 : (ix.metric == L1 ? serve_team_L1 : serve_team_CHI2);
+    const ServePick pick_warp = ix.metric == L2 ? serve_warp_L2 : (ix.metric == L1 ? serve_warp_L1 : serve_warp_CHI2);
+    const void* fn = nullptr;
     const size_t tsmem = team_smem(words, r.beam_max);
-    bool use_team = tsmem <= (size_t)optin;
+    bool use_team = tsmem <= (size_t)optin && r.nq <= TEAM_MOST * (uint32_t)nsm;
     if (use_team) {
+        const void* team = pick_team(qv, r.beam_max);
         NNM_CUDA_TRY(cudaFuncSetAttribute(team, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tsmem));
         int pt = 0;
         NNM_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&pt, team, TEAM * 32, tsmem));
         use_team = r.nq <= (uint32_t)std::max(pt, 0) * (uint32_t)nsm;
+        if (use_team) fn = team;
     }
     // several queries per resident warp: the form with more warps
     const bool dense_fits = ((size_t)words + FVCAP) * 4 * DENSE_WARPS * nsm <= DENSE_SCRATCH;
     const uint32_t line = dense_queries((int)ix.metric, qv, r.beam_max, (size_t)words * 4 * DENSE_WARPS * nsm);
     const bool dense = !use_team && dense_fits && line && r.nq > line * (uint32_t)nsm;
-    const ServeFn fn = use_team ? team : dense ? pick_warp<true>(ix.metric, qv) : pick_warp<false>(ix.metric, qv);
+    if (!fn) fn = pick_warp(qv, dense);
     const size_t smem = use_team ? tsmem : (size_t)FW * ((size_t)r.beam_max * 8 + WARP_EXTRA);
     uint32_t blocks = r.nq;
     if (!use_team) {
@@ -1224,9 +1249,10 @@ int index_run_fast(Ctx& ctx, IndexDev& ix, const SearchReq& r) {
     a.ncmps = reinterpret_cast<unsigned long long*>(c + 8);
     a.nexp = reinterpret_cast<unsigned long long*>(c + 16);
     a.spec_blocks = (uint32_t)nsm;
-    fn<<<blocks, (use_team ? TEAM : FW) * 32, smem, st>>>(a); count_launch();
-    NNM_CUDA_TRY(cudaGetLastError());
+    void* args[] = {&a};
+    NNM_CUDA_TRY(cudaLaunchKernel(fn, dim3(blocks), dim3((use_team ? TEAM : FW) * 32), args, smem, st)); count_launch();
     return 0;
 }
+#endif
 
 }  // namespace nnm
