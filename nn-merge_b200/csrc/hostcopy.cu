@@ -8,6 +8,8 @@
 // it pass through the slots on the calling thread, with one wait for all
 // pieces.  The threads stay with the context: starting three for each copy
 // cost 0.4 ms.
+#include <unistd.h>
+
 #include <algorithm>
 #include <atomic>
 #include <condition_variable>
@@ -34,6 +36,10 @@ struct CopyThreads {
     int busy = 0;
     bool stop = false;
     std::vector<std::thread> t;
+    // A forked child has this object and not its threads: joining them, or
+    // destroying the condition they wait on, would wait for good.
+    const pid_t owner = getpid();
+    bool here() const { return owner == getpid(); }
 
     // Fewer than asked when the system has no more threads.
     CopyThreads(int device, int n) {
@@ -121,7 +127,7 @@ void run_workers(Ctx& ctx, int workers, const std::function<void(int)>& work) {
         return;
     }
     if (!ctx.stage.threads) ctx.stage.threads = new (std::nothrow) CopyThreads(ctx.device, workers - 1);
-    if (ctx.stage.threads) ctx.stage.threads->run(work);
+    if (ctx.stage.threads && ctx.stage.threads->here()) ctx.stage.threads->run(work);
     else work(0);
 }
 
@@ -155,7 +161,7 @@ unsigned char* pinned_block(size_t bytes) {
 }
 
 void HostStage::release() {
-    delete threads;
+    if (threads && threads->here()) delete threads;
     threads = nullptr;
     for (auto& w : done)
         for (auto& e : w) {

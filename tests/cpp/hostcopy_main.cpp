@@ -3,6 +3,9 @@
 // chosen call fails once.  Prints one line per check; exit status 1 on a
 // failed one.
 #include <math.h>
+#include <signal.h>
+#include <sys/wait.h>
+#include <unistd.h>
 
 #include <cstdio>
 #include <cstdlib>
@@ -199,11 +202,47 @@ void without_pinned(size_t n) {
     no_pinned = false;
     ctx.stage.release();
 }
+
+// A forked child has the context and none of its threads: copies and the end
+// of the context return there (a child of a Python program that holds a
+// context destroys it as it exits), and the parent goes on.
+void forked(size_t n) {
+    const auto src = bytes_of(n, 4);
+    nnm::Ctx ctx;
+    std::vector<unsigned char> dst(n);
+    calls = fail_at = 0;
+    nnm::host_to_dev(ctx, dst.data(), src.data(), n);
+    for (int copy = 0; copy < 2; copy++) {
+        const pid_t pid = fork();
+        if (pid == 0) {
+            if (copy) nnm::host_to_dev(ctx, dst.data(), src.data(), n);
+            ctx.stage.release();
+            _exit(0);
+        }
+        int status = -1;
+        bool ended = false;
+        for (int i = 0; i < 500 && !ended; i++) {
+            ended = waitpid(pid, &status, WNOHANG) == pid;
+            if (!ended) usleep(10000);
+        }
+        if (!ended) {
+            kill(pid, SIGKILL);
+            waitpid(pid, &status, 0);
+        }
+        check(ended && status == 0, copy ? "a copy in a forked child" : "the end of a context in a forked child", n, 0);
+    }
+    std::fill(dst.begin(), dst.end(), 0);
+    nnm::host_to_dev(ctx, dst.data(), src.data(), n);
+    cudaStreamSynchronize(nullptr);
+    check(dst == src, "a copy after a fork", n, 0);
+    ctx.stage.release();
+}
 }  // namespace
 
 int main() {
     for (size_t n : {(size_t)1000, (size_t)(2 << 20), (size_t)(9 << 20) + 7}) errors(n);
     for (size_t n : {(size_t)1, (size_t)100000, (size_t)(8 << 20), (size_t)(9 << 20) + 7}) sources(n);
     for (size_t n : {(size_t)1000, (size_t)(9 << 20) + 7}) without_pinned(n);
+    forked((size_t)(9 << 20) + 7);
     return bad != 0;
 }
