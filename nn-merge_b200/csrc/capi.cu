@@ -2,6 +2,7 @@
 #include <cstdio>
 #include <cstring>
 #include <memory>
+#include <new>
 #include <random>
 #include <string>
 #include <vector>
@@ -777,16 +778,19 @@ int nnm_graph_recall(nnm_ctx* ctx, const float* x, uint64_t n, uint32_t d, const
     nnm::KeepBound kx(c.store.x), ks(c.ws.bucket), km(c.ws.misc);
     GraphDev g;
     int rc = upload_plain(c, c.store, g, x, n, d);
-    std::vector<uint32_t> h((size_t)nrows * (atop + 1));
-    for (uint32_t i = 0; i < nrows; i++) {
-        h[i] = rows[i];
-        for (uint32_t j = 0; j < atop; j++) h[nrows + (size_t)i * atop + j] = ids[(size_t)rows[i] * k + j];
-    }
-    if (!rc && c.ws.bucket.ensure(h.size() * 4 + 4) != cudaSuccess) rc = fail(ctx, NNM_ERR_OOM, "device allocation failed");
+    const size_t words = (size_t)nrows * (atop + 1);
+    std::unique_ptr<uint32_t[]> h(new (std::nothrow) uint32_t[words + 1]);
+    if (!rc && (!h || c.ws.bucket.ensure(words * 4 + 4) != cudaSuccess))
+        rc = fail(ctx, NNM_ERR_OOM, "recall: no memory for the evaluated rows");
     uint32_t* dev = c.ws.bucket.as<uint32_t>();
-    if (!rc && !h.empty() &&
-        cudaMemcpyAsync(dev, h.data(), h.size() * 4, cudaMemcpyHostToDevice, c.stream) != cudaSuccess)
-        rc = fail(ctx, NNM_ERR_CUDA, "recall: copy failed");
+    if (!rc && nrows) {
+        for (uint32_t i = 0; i < nrows; i++) {
+            h[i] = rows[i];
+            for (uint32_t j = 0; j < atop; j++) h[nrows + (size_t)i * atop + j] = ids[(size_t)rows[i] * k + j];
+        }
+        if (cudaMemcpyAsync(dev, h.get(), words * 4, cudaMemcpyHostToDevice, c.stream) != cudaSuccess)
+            rc = fail(ctx, NNM_ERR_CUDA, "recall: copy failed");
+    }
     if (!rc)
         rc = nnm::graph_recall_dev(c, g.x, (uint32_t)n, g.dp, NNM_METRIC_L2, dev + nrows, atop, true, dev, nrows, atop,
                                    recall);
