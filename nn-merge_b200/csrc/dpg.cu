@@ -372,7 +372,7 @@ int dpg_layer(Ctx& ctx, DpgState& s, GraphDev& g, nnm_layers* out) {
         NNM_CUDA_TRY(cudaMemsetAsync(s.ecur.p, 0, (size_t)N * 4, st));
         k_ev_count<<<nblk(N, WPB), WPB * 32, 0, st>>>(s.sid.as<uint32_t>(), s.slen.as<uint32_t>(), N, C,
                                                          s.ecnt.as<uint32_t>()); count_launch();
-        NNM_CUDA_TRY(exclusive_scan(s.ecnt.as<uint32_t>(), s.eoff.as<uint64_t>(), N, s.tmp.as<uint64_t>(), nullptr, st));
+        NNM_CUDA_TRY(exclusive_scan(s.ecnt.as<uint32_t>(), s.eoff.as<uint64_t>(), N, s.tmp.as<uint64_t>(), st));
         k_ev_fill<<<nblk(N, WPB), WPB * 32, 0, st>>>(s.sid.as<uint32_t>(), s.sdist.as<float>(), s.slen.as<uint32_t>(),
                                                         N, C, s.eoff.as<uint64_t>(), s.ecur.as<uint32_t>(),
                                                         s.ev.as<unsigned long long>()); count_launch();
@@ -402,7 +402,7 @@ int dpg_layer(Ctx& ctx, DpgState& s, GraphDev& g, nnm_layers* out) {
     if (out && out->nlayers < 16) {
         // packed on the device, into the offers' buffer (N x C words of its
         // 2 N x C), so that only the lists themselves are copied out
-        NNM_CUDA_TRY(exclusive_scan(s.glen.as<uint32_t>(), s.eoff.as<uint64_t>(), N, s.tmp.as<uint64_t>(), nullptr, st));
+        NNM_CUDA_TRY(exclusive_scan(s.glen.as<uint32_t>(), s.eoff.as<uint64_t>(), N, s.tmp.as<uint64_t>(), st));
         k_dpg_pack<<<nblk(N, WPB), WPB * 32, 0, st>>>(s.gid.as<uint32_t>(), s.glen.as<uint32_t>(), N, C,
                                                       s.eoff.as<uint64_t>(), s.ev.as<uint32_t>()); count_launch();
         const uint32_t L = out->nlayers;

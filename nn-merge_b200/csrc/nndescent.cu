@@ -669,7 +669,7 @@ __host__ __device__ __forceinline__ uint32_t vec_stride(uint32_t units) { return
 // d(a, b) = |a|^2 + |b|^2 - 2 a.b is then an exact integer below 2^24, the
 // value of the reference's sequential float sum of the same terms, so both
 // give the same distances.
-constexpr int VEC_GLOBAL = 0, VEC_U8 = 2;
+constexpr int VEC_GLOBAL = 0, VEC_U8 = 1;
 
 // Tiers 0-3: the row's FP32 vectors staged in shared memory, PS_WARPS[t]
 // warps a row (four rows side by side in a block of tier 0), a TA x TB tile
@@ -1172,7 +1172,10 @@ constexpr int RC_DIRECT = 16;
 // the bound on the K-th distance (approx_bound: two sorts and 50 shuffles a
 // target): BF16 build 194.0 -> 189.4 ms (190.2 at 8, 189.3 at 24).
 constexpr uint32_t RC_BOUND = 16;
-constexpr int MERGE_AX_BLOCKS = 6;            // per SM (40 registers; eight at 32 spill: 193.3 ms)
+// Blocks per SM: 40 registers, with 218 bytes of spills stored and 244 loaded in
+// k_merge<true>, 134 and 180 in k_merge_fast<true>; eight blocks (32 registers)
+// spill more: 189.2 -> 193.3 ms.
+constexpr int MERGE_AX_BLOCKS = 6;
 constexpr uint32_t RC_UNITS = 4;              // 64 bytes of every row at a time
 constexpr uint32_t RC_STRIDE = RC_UNITS + 1;  // odd: lanes reading their own rows fall in different banks
 constexpr uint32_t RC_TILE = 33 * RC_STRIDE;  // float4 of a warp: 32 rows and row t

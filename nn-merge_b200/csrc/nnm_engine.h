@@ -51,7 +51,7 @@ struct KeepBound {
 
 // Scratch for one NN-Descent iteration, sized for the largest graph seen.
 struct Workspace {
-    DevBuf rcnt, rcur, rtot, roff, rseg, rscr, rofs, rbuf;
+    DevBuf rcnt, rcur, roff, rseg, rscr, rofs, rbuf;
     DevBuf cntpos, bcnt, bcur, boff, bucket, bigrev, nflag, scan_tmp;
     DevBuf npairs, poff, pd, tiers, erows;
     DevBuf kth;  // every row's K-th distance, gathered per iteration
@@ -65,7 +65,7 @@ struct Workspace {
     DevBuf train;    // one training or gradient pass of the code network
     DevBuf mlp_err;  // the code network's tensor-core inference: a wait that ran out
     void release_all() {
-        DevBuf* all[] = {&rcnt, &rcur, &rtot, &roff, &rseg, &rscr, &rofs, &rbuf, &cntpos, &bcnt, &bcur,
+        DevBuf* all[] = {&rcnt, &rcur, &roff, &rseg, &rscr, &rofs, &rbuf, &cntpos, &bcnt, &bcur,
                          &boff, &bucket, &bigrev, &nflag, &scan_tmp, &npairs, &poff, &pd, &tiers, &erows, &kth, &rtier,
                          &draws, &mt_ring, &counters, &misc, &train, &mlp_err};
         for (auto* b : all) b->release();

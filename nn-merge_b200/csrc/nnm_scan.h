@@ -25,6 +25,5 @@ cudaError_t exclusive_scans(const ScanJobs& jobs, int count, size_t n, uint64_t*
 // Scratch size (in u64 elements) that the scans need for n inputs.
 size_t scan_temp_elems(size_t n);
 // One plain scan.
-cudaError_t exclusive_scan(const uint32_t* in, uint64_t* out, size_t n, uint64_t* temp, uint64_t* d_total,
-                           cudaStream_t st);
+cudaError_t exclusive_scan(const uint32_t* in, uint64_t* out, size_t n, uint64_t* temp, cudaStream_t st);
 }  // namespace nnm

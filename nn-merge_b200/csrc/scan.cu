@@ -118,10 +118,9 @@ cudaError_t exclusive_scans(const ScanJobs& jobs, int count, size_t n, uint64_t*
     return cudaGetLastError();
 }
 
-cudaError_t exclusive_scan(const uint32_t* in, uint64_t* out, size_t n, uint64_t* temp, uint64_t* d_total,
-                           cudaStream_t st) {
+cudaError_t exclusive_scan(const uint32_t* in, uint64_t* out, size_t n, uint64_t* temp, cudaStream_t st) {
     ScanJobs jobs{};
-    jobs.j[0] = ScanJob{in, nullptr, out, d_total, nullptr, 0, 0};
+    jobs.j[0] = ScanJob{in, nullptr, out, nullptr, nullptr, 0, 0};
     return exclusive_scans(jobs, 1, n, temp, st);
 }
 

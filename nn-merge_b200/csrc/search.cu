@@ -27,8 +27,9 @@
 // shared memory, a coalesced copy each: a lane reading its own row from global
 // memory 16 bytes at a time touched 20 lines per load instruction, and the
 // candidate heap in HBM put an L2 round trip under every level of a pop.
-// Bound: latency of a query's chain (lane 0's heap steps, then list, visited
-// bits and rows), all queries of a batch at once.  2,000 queries, beam 60,
+// Bound: latency of a query's chain (heap steps, then list, visited bits and
+// rows), all queries of a batch at once (72 registers; 86 bytes of spills
+// stored, 112 loaded).  2,000 queries, beam 60,
 // 100,000 x 128 rows: 1,366 -> 1,215 us, the length of the longest query's
 // chain (120 expansions, 2M cycles: offers 1,700 each, 2,300 before; rows
 // 5,000 and a pop 1,350 an expansion, 2,100 before).

@@ -3,7 +3,8 @@
 // laid out for throughput rather than for the reference's float rounding.
 //
 // One warp per query; persistent warps pull queries from a counter, so
-// queries of different beam widths balance.
+// queries of different beam widths balance.  (A batch whose queries all have
+// a resident block takes a block per query: k_serve_team.)
 //   - distances: a whole warp per distance, lane l holding components
 //     [4l, 4l+4) (+128 per further float4) of the query in registers; a
 //     row is one coalesced 512-byte read for d = 128.  Up to 32 distances
@@ -27,7 +28,7 @@
 //     so that the dependent loads (offsets, lists, visited bits, rows) of
 //     several nodes are in flight at once; width 1 is strict best-first.
 //   - visited set: one bitmap per warp slot in HBM, cleared after each query
-//     from the list of ids it set.
+//     from the list of ids it set, or whole where the list was too short.
 #include <algorithm>
 #include <cmath>
 
@@ -279,11 +280,12 @@ __device__ __forceinline__ void prefetch_l2(const void* p) { asm volatile("prefe
 // DENSE, for batches of several queries per resident warp: seven CTAs per SM
 // (72 registers: the rows of a list summed eight at a time, prefetched into L2
 // when their ids are known); otherwise five CTAs (96 registers, 32 rows summed
-// together), whose single query is shorter.  The line between them is
-// dense_queries.  At 1M rows the 28 warps' bitmaps (518 MB, allocated and cleared
-// by an index's first batch) gain 3 to 7 %, not worth it: so at most
-// DENSE_SCRATCH of them and their lists.  A hash table per query instead of a bitmap there took
-// 1.5 times as long.
+// together), whose single query is shorter.  Both spill (bytes stored: 96, 148
+// and 248 by row length for L2 and L1, 168 to 344 for chi-square; dense 48 to
+// 104, 104 to 268); the line between them is dense_queries.  At 1M rows the 28
+// warps' bitmaps (518 MB, allocated and cleared by an index's first batch) gain
+// 3 to 7 %, not worth it: so at most DENSE_SCRATCH of them and their lists.  A
+// hash table per query instead of a bitmap there took 1.5 times as long.
 template <int M, int QV, bool DENSE>
 __global__ void __launch_bounds__(FW * 32, DENSE ? 7 : 5) k_serve(ServeArgs a) {
     extern __shared__ __align__(16) unsigned char smem[];
@@ -614,8 +616,9 @@ __global__ void __launch_bounds__(FW * 32, DENSE ? 7 : 5) k_serve(ServeArgs a) {
 // 100,000 x 128 rows, device time against k_serve's: 1 query 250 -> 155 us,
 // 148 queries 415 -> 239, 592 queries 489 -> 288; faster as long as every
 // query has a resident block (740 here: 472 -> 296), which is the rule that
-// picks it.  The beam in registers (up to 192 entries) against shared memory:
-// 177 -> 155 us.
+// picks it.  At 1, 148 and 700 queries, beams 16 to 256, of k_serve's time:
+// L2 0.52 to 0.82, L1 0.52 to 0.82, chi-square 0.37 to 0.65.  The beam in
+// registers (up to 192 entries) against shared memory: 177 -> 155 us.
 constexpr int TEAM = 4;
 constexpr uint32_t TEAM_MOST = 16;  // blocks an SM: 64 warps
 
