@@ -355,7 +355,8 @@ int nnm_set_init_model(nnm_ctx *ctx, const nnm_mlp *model);
  * computes each distance with a whole warp (coalesced rows, a different
  * float summation order) and keeps the beam as a sorted array in shared
  * memory in place of the two heaps: the same best-first expansion and
- * stopping rule, ties between equal distances broken by id.
+ * stopping rule, ties between equal distances broken by id; a distance that
+ * is NaN counts as infinite.
  *
  * Entry points: NNM_ENTRY_DEFAULT starts every query at rand() % nrows[0]
  * after srand(seed) and descends greedily from layer 0, as the reference.
