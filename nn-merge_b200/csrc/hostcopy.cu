@@ -8,6 +8,7 @@
 // it pass through the slots on the calling thread, with one wait for all
 // pieces.  The threads stay with the context: starting three for each copy
 // cost 0.4 ms.
+#include <sys/mman.h>
 #include <unistd.h>
 
 #include <algorithm>
@@ -36,10 +37,6 @@ struct CopyThreads {
     int busy = 0;
     bool stop = false;
     std::vector<std::thread> t;
-    // A forked child has this object and not its threads: joining them, or
-    // destroying the condition they wait on, would wait for good.
-    const pid_t owner = getpid();
-    bool here() const { return owner == getpid(); }
 
     // Fewer than asked when the system has no more threads.
     CopyThreads(int device, int n) {
@@ -102,11 +99,12 @@ bool pageable(const void* p) {
     return a.type == cudaMemoryTypeUnregistered;
 }
 
+// The slots of the first worker.  A forked child has a stage without its
+// threads and without its memory.
 bool stage_ready(HostStage& s) {
-    if (s.block) return true;
+    if (s.first.p) return s.first.here();
     if (s.failed) return false;
-    s.block = pinned_block(HostStage::WORKERS * HostStage::SLOTS * HostStage::CHUNK);
-    bool ok = s.block != nullptr;
+    bool ok = s.first.make(HostStage::SLOTS * HostStage::CHUNK);
     if (ok)
         for (auto& w : s.done)
             for (auto& e : w) ok = ok && cudaEventCreateWithFlags(&e, cudaEventDisableTiming) == cudaSuccess;
@@ -127,14 +125,16 @@ void run_workers(Ctx& ctx, int workers, const std::function<void(int)>& work) {
         return;
     }
     if (!ctx.stage.threads) ctx.stage.threads = new (std::nothrow) CopyThreads(ctx.device, workers - 1);
-    if (ctx.stage.threads && ctx.stage.threads->here()) ctx.stage.threads->run(work);
+    if (ctx.stage.threads) ctx.stage.threads->run(work);
     else work(0);
 }
 
-int workers_for(size_t bytes) {
+int workers_for(HostStage& s, size_t bytes) {
     const unsigned hw = std::thread::hardware_concurrency();
     const int most = (int)std::min<unsigned>(HostStage::WORKERS, std::max(1u, hw / 2));
-    return bytes < PARALLEL_MIN ? 1 : most;
+    if (bytes < PARALLEL_MIN || most == 1) return 1;
+    if (!s.others.p && !s.others.make((HostStage::WORKERS - 1) * HostStage::SLOTS * HostStage::CHUNK)) return 1;
+    return most;
 }
 
 // Chunks small enough that every worker gets a few.
@@ -153,23 +153,53 @@ cudaError_t settled(Ctx& ctx, cudaError_t e) {
 
 }  // namespace
 
-unsigned char* pinned_block(size_t bytes) {
-    void* p = nullptr;
-    if (cudaMallocHost(&p, bytes) == cudaSuccess) return static_cast<unsigned char*>(p);
-    cudaGetLastError();
-    return nullptr;
+bool PinnedBlock::make(size_t n) {
+    constexpr size_t HUGE = (size_t)2 << 20;
+    n = (n + 4095) & ~(size_t)4095;
+    const size_t align = n >= HUGE ? HUGE : 4096;
+    void* raw = mmap(nullptr, n + align, PROT_READ | PROT_WRITE, MAP_PRIVATE | MAP_ANONYMOUS, -1, 0);
+    if (raw == MAP_FAILED) return false;
+    unsigned char* const r = static_cast<unsigned char*>(raw);
+    unsigned char* const b = r + (align - reinterpret_cast<uintptr_t>(r) % align) % align;
+    if (b > r) munmap(r, b - r);
+    if (b + n < r + n + align) munmap(b + n, r + align - b);
+    if (align == HUGE) madvise(b, n, MADV_HUGEPAGE);
+    // a fork would leave the pages shared, and a write move this process's
+    // away from those that the device knows
+    madvise(b, n, MADV_DONTFORK);
+    if (cudaHostRegister(b, n, cudaHostRegisterDefault) != cudaSuccess) {
+        cudaGetLastError();
+        munmap(b, n);
+        return false;
+    }
+    p = b;
+    bytes = n;
+    owner = getpid();
+    return true;
+}
+
+bool PinnedBlock::here() const { return p && owner == getpid(); }
+
+void PinnedBlock::release() {
+    if (here()) {
+        cudaHostUnregister(p);
+        munmap(p, bytes);
+    }
+    p = nullptr;
 }
 
 void HostStage::release() {
-    if (threads && threads->here()) delete threads;
+    // In a forked child there are no threads to join, and destroying the
+    // condition that they wait on would wait for good.
+    if (threads && first.here()) delete threads;
     threads = nullptr;
     for (auto& w : done)
         for (auto& e : w) {
             if (e) cudaEventDestroy(e);
             e = nullptr;
         }
-    if (block) cudaFreeHost(block);
-    block = nullptr;
+    others.release();
+    first.release();
 }
 
 cudaError_t host_to_dev(Ctx& ctx, void* dst, const void* src, size_t bytes) {
@@ -181,7 +211,7 @@ cudaError_t host_to_dev(Ctx& ctx, void* dst, const void* src, size_t bytes) {
         // is read while the copy runs
         return e == cudaSuccess && !paged ? cudaStreamSynchronize(ctx.stream) : e;
     }
-    const int workers = workers_for(bytes);
+    const int workers = workers_for(s, bytes);
     const size_t chunk = chunk_for(bytes, workers), chunks = (bytes + chunk - 1) / chunk;
     std::atomic<size_t> next{0};
     std::atomic<int> err{cudaSuccess};
@@ -191,7 +221,7 @@ cudaError_t host_to_dev(Ctx& ctx, void* dst, const void* src, size_t bytes) {
             const size_t c = next.fetch_add(1);
             if (c >= chunks) break;
             const size_t o = c * chunk, len = std::min(chunk, bytes - o);
-            unsigned char* p = s.block + ((size_t)w * HostStage::SLOTS + slot) * HostStage::CHUNK;
+            unsigned char* p = s.slot(w, slot);
             e = cudaEventSynchronize(s.done[w][slot]);  // the slot's last copy, of this call or an earlier one
             if (e != cudaSuccess) break;
             std::memcpy(p, static_cast<const unsigned char*>(src) + o, len);
@@ -222,7 +252,7 @@ cudaError_t dev_to_host(Ctx& ctx, const HostPiece* pieces, int count) {
         return cudaStreamSynchronize(ctx.stream);
     }
     if (total == 0) return cudaStreamSynchronize(ctx.stream);
-    const int workers = workers_for(total);
+    const int workers = workers_for(s, total);
     const size_t chunk = chunk_for(total, workers);
     size_t chunks = 0;
     for (int i = 0; i < count; i++)
@@ -247,9 +277,6 @@ cudaError_t dev_to_host(Ctx& ctx, const HostPiece* pieces, int count) {
         cudaError_t e = cudaSuccess;
         unsigned char* host[HostStage::SLOTS] = {};
         size_t len[HostStage::SLOTS] = {};
-        auto slot_ptr = [&](int slot) {
-            return s.block + ((size_t)w * HostStage::SLOTS + slot) * HostStage::CHUNK;
-        };
         auto start = [&](int slot) {  // the next chunk on its way into the slot
             len[slot] = 0;
             const size_t c = next.fetch_add(1);
@@ -257,7 +284,7 @@ cudaError_t dev_to_host(Ctx& ctx, const HostPiece* pieces, int count) {
             const unsigned char* d = nullptr;
             const size_t n = where(c, host[slot], d);
             e = cudaEventSynchronize(s.done[w][slot]);
-            if (e == cudaSuccess) e = cudaMemcpyAsync(slot_ptr(slot), d, n, cudaMemcpyDeviceToHost, ctx.stream);
+            if (e == cudaSuccess) e = cudaMemcpyAsync(s.slot(w, slot), d, n, cudaMemcpyDeviceToHost, ctx.stream);
             if (e == cudaSuccess) e = cudaEventRecord(s.done[w][slot], ctx.stream);
             if (e == cudaSuccess) len[slot] = n;
         };
@@ -265,7 +292,7 @@ cudaError_t dev_to_host(Ctx& ctx, const HostPiece* pieces, int count) {
         for (int slot = 0; e == cudaSuccess && len[slot]; slot ^= 1) {  // ends with the first error
             e = cudaEventSynchronize(s.done[w][slot]);
             if (e != cudaSuccess) break;
-            std::memcpy(host[slot], slot_ptr(slot), len[slot]);
+            std::memcpy(host[slot], s.slot(w, slot), len[slot]);
             start(slot);
         }
         if (e != cudaSuccess) err = e;

@@ -54,7 +54,7 @@ struct IndexDev {
     uint32_t width = 4;  // fast kernel: most unexpanded entries expanded together
     // small batches from host memory: queries, beams, counters and results
     // pass through this pinned block, so that a call waits for the device once
-    unsigned char* h_io = nullptr;
+    PinnedBlock h_io;
     cudaEvent_t ev[3] = {};
     void release();
 };

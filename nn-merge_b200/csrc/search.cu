@@ -743,8 +743,7 @@ void IndexDev::release() {
     DevBuf* all[] = {&x,     &off,   &adj,  &visited, &vlist,  &cand,         &ctr,      &qpad,
                      &beams, &probes, &hid, &scores,  &out,    &flat_off, &flat_pool};
     for (auto* b : all) b->release();
-    if (h_io) cudaFreeHost(h_io);
-    h_io = nullptr;
+    h_io.release();
     for (auto& e : ev) {
         if (e) cudaEventDestroy(e);
         e = nullptr;

@@ -92,6 +92,16 @@ cudaError_t cudaMallocHost(void** p, size_t bytes) {
     pinned[static_cast<char*>(*p)] = bytes;
     return cudaSuccess;
 }
+cudaError_t cudaHostRegister(void* p, size_t bytes, unsigned) {
+    std::lock_guard<std::mutex> l(mu);
+    if (no_pinned) return last_error = cudaErrorMemoryAllocation;
+    pinned[static_cast<char*>(p)] = bytes;
+    return cudaSuccess;
+}
+cudaError_t cudaHostUnregister(void* p) {
+    std::lock_guard<std::mutex> l(mu);
+    return pinned.erase(static_cast<char*>(p)) ? cudaSuccess : cudaErrorUnknown;
+}
 cudaError_t cudaFreeHost(void* p) {
     std::lock_guard<std::mutex> l(mu);
     pinned.erase(static_cast<char*>(p));
@@ -194,7 +204,8 @@ void without_pinned(size_t n) {
     std::vector<unsigned char> dst(n), back(n);
     calls = fail_at = 0;
     no_pinned = true;
-    check(nnm::pinned_block(n) == nullptr && cudaGetLastError() == cudaSuccess, "no pinned block", n, 0);
+    nnm::PinnedBlock b;
+    check(!b.make(n) && !b.p && cudaGetLastError() == cudaSuccess, "no pinned block", n, 0);
     const nnm::HostPiece p{back.data(), dst.data(), n};
     check(nnm::host_to_dev(ctx, dst.data(), src.data(), n) == cudaSuccess &&
               nnm::dev_to_host(ctx, &p, 1) == cudaSuccess && back == src && cudaGetLastError() == cudaSuccess,
@@ -212,6 +223,7 @@ void forked(size_t n) {
     std::vector<unsigned char> dst(n);
     calls = fail_at = 0;
     nnm::host_to_dev(ctx, dst.data(), src.data(), n);
+    cudaStreamSynchronize(nullptr);  // the child's stand-in would carry out what is queued here
     for (int copy = 0; copy < 2; copy++) {
         const pid_t pid = fork();
         if (pid == 0) {
@@ -237,6 +249,31 @@ void forked(size_t n) {
     check(dst == src, "a copy after a fork", n, 0);
     ctx.stage.release();
 }
+
+// Page-locking costs more than a small copy takes (8 MB: 2 to 7 ms), and a
+// program may make a context for one build: a context locks a quarter for
+// copies of one thread, all of it for one that several share.
+void locked() {
+    const auto src = bytes_of((size_t)24 << 20, 5);
+    auto held = [] {
+        size_t n = 0;
+        for (const auto& x : pinned) n += x.second;
+        return n;
+    };
+    nnm::Ctx ctx;
+    std::vector<unsigned char> dst(src.size());
+    calls = fail_at = 0;
+    const nnm::HostPiece small{dst.data(), src.data(), 400000}, large{dst.data(), src.data(), (size_t)10 << 20};
+    nnm::host_to_dev(ctx, dst.data(), src.data(), 1 << 20);
+    check(held() == 0, "nothing locked by a small copy in", held(), 0);
+    nnm::dev_to_host(ctx, &small, 1);
+    check(held() <= (size_t)2 << 20, "memory locked by a small copy out", held(), 0);
+    nnm::dev_to_host(ctx, &large, 1);
+    nnm::host_to_dev(ctx, dst.data(), src.data(), src.size());
+    check(held() <= (size_t)8 << 20, "memory locked by large copies", held(), 0);
+    ctx.stage.release();
+    check(held() == 0, "memory locked after the context", held(), 0);
+}
 }  // namespace
 
 int main() {
@@ -244,5 +281,6 @@ int main() {
     for (size_t n : {(size_t)1, (size_t)100000, (size_t)(8 << 20), (size_t)(9 << 20) + 7}) sources(n);
     for (size_t n : {(size_t)1000, (size_t)(9 << 20) + 7}) without_pinned(n);
     forked((size_t)(9 << 20) + 7);
+    locked();
     return bad != 0;
 }
