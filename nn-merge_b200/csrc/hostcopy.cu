@@ -4,9 +4,9 @@
 // S-Merge of 24 ms); here up to four threads share it, each claiming chunks
 // and passing them through two pinned slots of its own, so that memcpy, page
 // faults and DMA overlap: 51 MB in takes 1.8 ms.  Pinned (or managed) host
-// memory and copies in below PARALLEL_MIN take the plain copy; copies out below
-// it pass through the slots on the calling thread, with one wait for all
-// pieces.  The threads stay with the context: starting three for each copy
+// memory and copies in below SHARED_IN take the plain copy; copies out below
+// SHARED_OUT pass through the slots on the calling thread, with one wait for
+// all pieces.  The threads stay with the context: starting three for each copy
 // cost 0.4 ms.
 #include <sys/mman.h>
 #include <unistd.h>
@@ -86,9 +86,13 @@ struct CopyThreads {
 
 namespace {
 
-// below: waking the threads costs what they save (5 MB in: 0.45 ms plain,
-// 0.65 ms shared; 12 MB: 1.05 and 0.7; 51 MB: 5.0 and 1.8)
-constexpr size_t PARALLEL_MIN = (size_t)8 << 20;
+// below: waking the threads costs what they save.  In, whole calls, plain and
+// shared: 10 MB 0.61 and 0.69 to 1.00 ms, 16 MB 0.94 and 1.06 to 1.11, 20 MB 1.17
+// to 1.31 and 1.22 to 1.24, 28 MB 1.58 and 1.43 to 1.49, 51 MB 2.9 and 2.1 (a host
+// whose driver stages 17 GB/s; at 10 GB/s the copies alone: 5 MB 0.45 and 0.65,
+// 12 MB 1.05 and 0.7, 51 MB 5.0 and 1.8).  Out, where new pages are touched, 10
+// MB: 3.8 and 1.9.
+constexpr size_t SHARED_IN = (size_t)20 << 20, SHARED_OUT = (size_t)8 << 20;
 
 bool pageable(const void* p) {
     cudaPointerAttributes a{};
@@ -129,10 +133,10 @@ void run_workers(Ctx& ctx, int workers, const std::function<void(int)>& work) {
     else work(0);
 }
 
-int workers_for(HostStage& s, size_t bytes) {
+int workers_for(HostStage& s, bool shared) {
     const unsigned hw = std::thread::hardware_concurrency();
     const int most = (int)std::min<unsigned>(HostStage::WORKERS, std::max(1u, hw / 2));
-    if (bytes < PARALLEL_MIN || most == 1) return 1;
+    if (!shared || most == 1) return 1;
     if (!s.others.p && !s.others.make((HostStage::WORKERS - 1) * HostStage::SLOTS * HostStage::CHUNK)) return 1;
     return most;
 }
@@ -205,13 +209,13 @@ void HostStage::release() {
 cudaError_t host_to_dev(Ctx& ctx, void* dst, const void* src, size_t bytes) {
     HostStage& s = ctx.stage;
     const bool paged = pageable(src);
-    if (bytes < PARALLEL_MIN || !paged || !stage_ready(s)) {
+    if (bytes < SHARED_IN || !paged || !stage_ready(s)) {
         const cudaError_t e = cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, ctx.stream);
         // pageable memory is staged within the call; pinned and managed memory
         // is read while the copy runs
         return e == cudaSuccess && !paged ? cudaStreamSynchronize(ctx.stream) : e;
     }
-    const int workers = workers_for(s, bytes);
+    const int workers = workers_for(s, true);
     const size_t chunk = chunk_for(bytes, workers), chunks = (bytes + chunk - 1) / chunk;
     std::atomic<size_t> next{0};
     std::atomic<int> err{cudaSuccess};
@@ -252,7 +256,7 @@ cudaError_t dev_to_host(Ctx& ctx, const HostPiece* pieces, int count) {
         return cudaStreamSynchronize(ctx.stream);
     }
     if (total == 0) return cudaStreamSynchronize(ctx.stream);
-    const int workers = workers_for(s, total);
+    const int workers = workers_for(s, total >= SHARED_OUT);
     const size_t chunk = chunk_for(total, workers);
     size_t chunks = 0;
     for (int i = 0; i < count; i++)

@@ -277,10 +277,10 @@ void locked() {
 }  // namespace
 
 int main() {
-    for (size_t n : {(size_t)1000, (size_t)(2 << 20), (size_t)(9 << 20) + 7}) errors(n);
-    for (size_t n : {(size_t)1, (size_t)100000, (size_t)(8 << 20), (size_t)(9 << 20) + 7}) sources(n);
-    for (size_t n : {(size_t)1000, (size_t)(9 << 20) + 7}) without_pinned(n);
-    forked((size_t)(9 << 20) + 7);
+    for (size_t n : {(size_t)1000, (size_t)(2 << 20), (size_t)(9 << 20) + 7, (size_t)(21 << 20) + 7}) errors(n);
+    for (size_t n : {(size_t)1, (size_t)100000, (size_t)(20 << 20), (size_t)(21 << 20) + 7}) sources(n);
+    for (size_t n : {(size_t)1000, (size_t)(21 << 20) + 7}) without_pinned(n);
+    forked((size_t)(21 << 20) + 7);
     locked();
     return bad != 0;
 }
