@@ -304,19 +304,18 @@ __global__ void k_merge2one(uint32_t* pid, float* pdist, const uint32_t* cpid, c
     // graph may leave unsorted (nnm_merge_init_sgraph): an entry waits for
     // those before it in its own list, so it stands where its list's largest
     // distance so far would.
-    float pm = pd, cm = keepc ? cd : -INFINITY;
+    uint32_t pm = dist_word<true>(__float_as_uint(pd)), cm = keepc ? dist_word<true>(__float_as_uint(cd)) : 0u;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
-        const float p = __shfl_up_sync(FULL, pm, o), c = __shfl_up_sync(FULL, cm, o);
+        const uint32_t p = __shfl_up_sync(FULL, pm, o), c = __shfl_up_sync(FULL, cm, o);
         if (lane >= o) {
-            pm = fmaxf(pm, p);
-            cm = fmaxf(cm, c);
+            pm = max(pm, p);
+            cm = max(cm, c);
         }
     }
     uint32_t pp = lane, cp = __popc(km & ((1u << lane) - 1u));
     for (uint32_t j = 0; j < K; j++) {
-        float od = __shfl_sync(FULL, pm, j);
-        float oc = __shfl_sync(FULL, cm, j);
+        const uint32_t od = __shfl_sync(FULL, pm, j), oc = __shfl_sync(FULL, cm, j);
         if (j < cut && ((km >> j) & 1u) && oc < pm) pp++;  // compensation entries strictly smaller come first
         if (od <= cm) cp++;                                // pool entries with equal distance win
     }

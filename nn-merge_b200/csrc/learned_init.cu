@@ -173,7 +173,7 @@ __device__ void warp_sort64(SortEnt* e, uint32_t cnt) {
 #pragma unroll
     for (int h = 0; h < 2; h++) {
         const uint32_t i = 2 * lane + h;
-        v[h] = i < cnt ? ((unsigned long long)__float_as_uint(e[i].dist) << 32) | e[i].id : ~0ull;
+        v[h] = i < cnt ? ((unsigned long long)dist_word<true>(__float_as_uint(e[i].dist)) << 32) | e[i].id : ~0ull;
     }
     __syncwarp();
 #pragma unroll
@@ -201,7 +201,7 @@ __device__ void warp_sort64(SortEnt* e, uint32_t cnt) {
 #pragma unroll
     for (int h = 0; h < 2; h++) {
         const uint32_t i = 2 * lane + h;
-        if (i < cnt) e[i] = SortEnt{__uint_as_float((uint32_t)(v[h] >> 32)), (uint32_t)v[h]};
+        if (i < cnt) e[i] = SortEnt{__uint_as_float(dist_bits<true>((uint32_t)(v[h] >> 32))), (uint32_t)v[h]};
     }
     __syncwarp();
 }

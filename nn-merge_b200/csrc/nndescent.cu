@@ -1351,11 +1351,16 @@ __device__ __forceinline__ void warp_sort_ment(uint32_t& pd, unsigned long long&
     }
 }
 
+// A start pool in that order, out of line: rare (see k_merge).
+__device__ __noinline__ void sort_pool(uint32_t& cd, unsigned long long& ck, uint32_t& ce) {
+    warp_sort_ment(cd, ck, ce);
+}
+
 // Fast-tier merge.  A fast-tier key is a function of the entry (fast_key),
 // so an entry and its order fit one 64-bit word:
-//   dist bits (63..32) | id (31..2) | new flag (1) | group bit ^ 1 (0)
-// and the words order as (distance, id, ...) (distances are non-negative,
-// so their bits order as the floats).  Copies of an entry -- the same id at
+//   dist_word (63..32) | id (31..2) | new flag (1) | group bit ^ 1 (0)
+// and the words order as (distance, id, ...) (dist_word orders as the
+// floats).  Copies of an entry -- the same id at
 // the same distance -- are adjacent in sorted order, one already in the pool
 // (flag 0) before a proposal, proposals of group 1 before group 0 (as
 // fast_key orders them); the first copy is kept.  The start pool is keyed
@@ -1476,7 +1481,11 @@ __device__ uint32_t approx_bound(const MergeArgs& a, unsigned long long b_first,
 // proposals whose lower bound d~ - err_c (|t|^2 + |u|^2) reaches it and
 // computes their exact distances at the flush -- so the pool gets what the
 // FP32 join's proposals would give it.
-template <bool APPROX>
+// SIGNED (chi-square): distances may be negative, and are compared as
+// dist_word.  A start pool that is not in the order of those words (a caller's
+// graph) is sorted first: the merged positions below are counted in sorted
+// lists, and an unsorted one left some unwritten.
+template <bool APPROX, bool SIGNED>
 __global__ void __launch_bounds__(MERGE_WARPS * 32, APPROX ? MERGE_AX_BLOCKS : 8) k_merge(MergeArgs a) {
     __shared__ MEnt sm[MERGE_WARPS][64];
     __shared__ MEnt kept[MERGE_WARPS][32];
@@ -1495,9 +1504,11 @@ __global__ void __launch_bounds__(MERGE_WARPS * 32, APPROX ? MERGE_AX_BLOCKS : 8
             unsigned long long ck = ~0ull;
             if (lane < (int)K) {
                 ce = a.pid[(size_t)t * K + lane];
-                cd = __float_as_uint(a.pdist[(size_t)t * K + lane]);
+                cd = dist_word<SIGNED>(__float_as_uint(a.pdist[(size_t)t * K + lane]));
                 ck = (unsigned long long)lane;  // start entries precede every proposal of equal distance
             }
+            const uint32_t cprev = __shfl_up_sync(FULL, cd, 1);
+            if (!__all_sync(FULL, lane == 0 || cprev <= cd)) sort_pool(cd, ck, ce);
             uint32_t kd = __shfl_sync(FULL, cd, K - 1);
             unsigned long long kk = __shfl_sync(FULL, ck, K - 1);
             // the K-th distance the join filtered against: an approximate
@@ -1564,7 +1575,7 @@ __global__ void __launch_bounds__(MERGE_WARPS * 32, APPROX ? MERGE_AX_BLOCKS : 8
                     bool valid = false;
                     if (b0 + lane < c) {
                         const Prop p = reinterpret_cast<const Prop*>(a.bucket)[b_first + b0 + lane];
-                        pd = __float_as_uint(p.dist);
+                        pd = dist_word<SIGNED>(__float_as_uint(p.dist));
                         pk = p.key;
                         pe = (p.idg & ID_MASK) | ((p.idg >> 31) << 30) | FLAG_BIT;
                         if (APPROX && (p.idg & APPROX_BIT)) {
@@ -1603,7 +1614,7 @@ __global__ void __launch_bounds__(MERGE_WARPS * 32, APPROX ? MERGE_AX_BLOCKS : 8
             }
             if (lane < (int)K) {
                 a.pid[(size_t)t * K + lane] = ce;
-                a.pdist[(size_t)t * K + lane] = __uint_as_float(cd);
+                a.pdist[(size_t)t * K + lane] = __uint_as_float(dist_bits<SIGNED>(cd));
             }
             if (APPROX && a.count_approx && lane == 0 && nax) {
                 atomicAdd(&a.ctr->approx_props, (unsigned long long)nax);
@@ -1651,8 +1662,8 @@ __device__ __forceinline__ unsigned long long fm_flush(unsigned long long pool, 
 }
 
 // One warp per target, as k_merge, on the fast tier's 8-byte proposals;
-// APPROX as there.
-template <bool APPROX>
+// APPROX and SIGNED as there.
+template <bool APPROX, bool SIGNED>
 __global__ void __launch_bounds__(MERGE_WARPS * 32, APPROX ? MERGE_AX_BLOCKS : 8) k_merge_fast(MergeArgs a) {
     __shared__ unsigned long long buf[MERGE_WARPS][32];
     __shared__ unsigned long long stage[MERGE_WARPS][32];
@@ -1668,7 +1679,8 @@ __global__ void __launch_bounds__(MERGE_WARPS * 32, APPROX ? MERGE_AX_BLOCKS : 8
     if (c) {
         unsigned long long pool = FM_EMPTY;
         if (lane < (int)K)
-            pool = fm_word(__float_as_uint(a.pdist[(size_t)t * K + lane]), a.pid[(size_t)t * K + lane]);
+            pool = fm_word(dist_word<SIGNED>(__float_as_uint(a.pdist[(size_t)t * K + lane])),
+                           a.pid[(size_t)t * K + lane]);
         // the start pool in word order (entries of equal distance by id);
         // a pool the previous merge wrote is in that order already
         const unsigned long long pprev = __shfl_up_sync(FULL, pool, 1);
@@ -1700,7 +1712,7 @@ __global__ void __launch_bounds__(MERGE_WARPS * 32, APPROX ? MERGE_AX_BLOCKS : 8
                 if (b0 + lane < c) {
                     const uint2 p = bp[b0 + lane];
                     // a new entry: flag 1, group bit from the list entry
-                    v = ((unsigned long long)p.x << 32) | ((p.y & ID_MASK) << 2) | 2u | ((p.y >> 31) ^ 1u);
+                    v = ((unsigned long long)dist_word<SIGNED>(p.x) << 32) | ((p.y & ID_MASK) << 2) | 2u | ((p.y >> 31) ^ 1u);
                     if (APPROX && (p.y & APPROX_BIT)) {
                         ax = true;
                         lb = __uint_as_float(p.x) - a.err_c * (nt + __uint_as_float(a.nrm[p.y & ID_MASK]));
@@ -1752,7 +1764,7 @@ __global__ void __launch_bounds__(MERGE_WARPS * 32, APPROX ? MERGE_AX_BLOCKS : 8
         }
         if (lane < (int)K) {
             a.pid[(size_t)t * K + lane] = fm_pool_word(pool);
-            a.pdist[(size_t)t * K + lane] = __uint_as_float((uint32_t)(pool >> 32));
+            a.pdist[(size_t)t * K + lane] = __uint_as_float(dist_bits<SIGNED>((uint32_t)(pool >> 32)));
         }
         if (APPROX && a.count_approx && lane == 0 && nax) {
             atomicAdd(&a.ctr->approx_props, (unsigned long long)nax);
@@ -2155,11 +2167,13 @@ int run_nndescent(Ctx& ctx, GraphDev& g, JoinMode mode, uint32_t split, uint32_t
             rec(3);
             const unsigned mgrid = (n + MERGE_WARPS - 1) / MERGE_WARPS;
             if (g.fast) {
-                if (approx) k_merge_fast<true><<<mgrid, MERGE_WARPS * 32, 0, st>>>(ma);
-                else k_merge_fast<false><<<mgrid, MERGE_WARPS * 32, 0, st>>>(ma);
+                if (approx) k_merge_fast<true, false><<<mgrid, MERGE_WARPS * 32, 0, st>>>(ma);
+                else if (g.metric == CHI2) k_merge_fast<false, true><<<mgrid, MERGE_WARPS * 32, 0, st>>>(ma);
+                else k_merge_fast<false, false><<<mgrid, MERGE_WARPS * 32, 0, st>>>(ma);
             } else {
-                if (approx) k_merge<true><<<mgrid, MERGE_WARPS * 32, 0, st>>>(ma);
-                else k_merge<false><<<mgrid, MERGE_WARPS * 32, 0, st>>>(ma);
+                if (approx) k_merge<true, false><<<mgrid, MERGE_WARPS * 32, 0, st>>>(ma);
+                else if (g.metric == CHI2) k_merge<false, true><<<mgrid, MERGE_WARPS * 32, 0, st>>>(ma);
+                else k_merge<false, false><<<mgrid, MERGE_WARPS * 32, 0, st>>>(ma);
             }
             count_launch();
             k_sum_flags<<<std::min<unsigned>((n + 255) / 256, (unsigned)nsm * 4), 256, 0, st>>>(P<uint8_t>(ws.nflag), n, ctr); count_launch();

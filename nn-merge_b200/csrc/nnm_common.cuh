@@ -58,6 +58,20 @@ __device__ __forceinline__ float dist_seq_rt(int metric, const float* a, const f
     return dist_seq<CHI2>(a, b, dp);
 }
 
+// A distance as an unsigned word of the same order.  L2 and L1 distances are
+// not negative, so their bits are that word; a chi-square distance is where a
+// sum of components is (SIGNED).  ~0 stays above every distance.
+template <bool SIGNED>
+__device__ __forceinline__ uint32_t dist_word(uint32_t bits) {
+    if (!SIGNED) return bits;
+    return min(bits ^ ((uint32_t)((int32_t)bits >> 31) | 0x80000000u), 0xfffffffeu);
+}
+template <bool SIGNED>
+__device__ __forceinline__ uint32_t dist_bits(uint32_t word) {
+    if (!SIGNED) return word;
+    return word ^ (word >> 31 ? 0x80000000u : 0xffffffffu);
+}
+
 // ---------------------------------------------------------------------
 // Device port of libstdc++'s std::sort as the reference calls it on a pool
 // (kgraph.cpp:90, smerge.cpp:150 ...): comparator "a.dist < b.dist",
@@ -70,7 +84,10 @@ struct SortEnt {
     uint32_t id;  // packed pool word
 };
 
-__device__ __forceinline__ bool sless(const SortEnt& a, const SortEnt& b) { return a.dist < b.dist; }
+// NaN after every distance, so that pools are in the order the merges read.
+__device__ __forceinline__ bool sless(const SortEnt& a, const SortEnt& b) {
+    return a.dist < b.dist || (b.dist != b.dist && a.dist == a.dist);
+}
 __device__ __forceinline__ void sswap(SortEnt* a, SortEnt* b) { SortEnt t = *a; *a = *b; *b = t; }
 
 __device__ inline void s_heap_push(SortEnt* f, int hole, int top, SortEnt v) {
