@@ -18,7 +18,10 @@
 //     which the heaps decide -- is the reference's too.  Up to COOP entries
 //     the warp takes a step at once: a push compares every ancestor in its own
 //     lane, a pop picks every node's larger child by ballot and moves the path
-//     from the root together; larger heaps replay the steps on lane 0.  The
+//     from the root together; larger heaps replay the steps on lane 0.  For
+//     wide beams over short rows (serial_heaps) a second form of the kernel
+//     takes every step on lane 0, with the candidate heap all in HBM and the
+//     rows read where they are.  The
 //     neighbours of an expanded node are checked against a per-warp visited
 //     bitmap and their distances computed in parallel first, then offered in
 //     list order.
@@ -28,13 +31,14 @@
 // memory 16 bytes at a time touched 20 lines per load instruction, and the
 // candidate heap in HBM put an L2 round trip under every level of a pop.
 // Bound: latency of a query's chain (heap steps, then list, visited bits and
-// rows), all queries of a batch at once (72 registers; 86 bytes of spills
-// stored, 112 loaded).  2,000 queries, beam 60,
+// rows), all queries of a batch at once (72 registers, 86 bytes of spills
+// stored, 112 loaded; lane 0's form 64, 12 and 12).  2,000 queries, beam 60,
 // 100,000 x 128 rows: 1,366 -> 1,215 us, the length of the longest query's
 // chain (120 expansions, 2M cycles: offers 1,700 each, 2,300 before; rows
 // 5,000 and a pop 1,350 an expansion, 2,100 before).
 #include <algorithm>
 #include <string>
+#include <type_traits>
 #include <vector>
 
 #include "nnm_hier.h"
@@ -256,18 +260,20 @@ enum : unsigned {
 // Shared memory of one warp: the query, the staged rows (an odd number of
 // 16-byte units apart, so that lanes reading their own rows at the same offset
 // fall in different banks), the results heap, the offered distances and ids, the
-// candidate heap's head.
+// candidate heap's head (not in lane 0's form).
 __host__ __device__ constexpr uint32_t row_units(uint32_t dp) { return (dp / 4) | 1u; }
-__host__ __device__ constexpr size_t search_warp_bytes(uint32_t dp, uint32_t beam_cap, uint32_t rb) {
-    return ((size_t)dp * 4 + (size_t)rb * row_units(dp) * 16 + (size_t)(beam_cap + 1) * 8 + 32 * 8 + CAND_SMEM * 8 + 15) &
+__host__ __device__ constexpr size_t search_warp_bytes(bool serial, uint32_t dp, uint32_t beam_cap, uint32_t rb) {
+    return ((size_t)dp * 4 + (size_t)rb * row_units(dp) * 16 + (size_t)(beam_cap + 1) * 8 + 32 * 8 +
+            (serial ? 0 : CAND_SMEM * 8) + 15) &
            ~(size_t)15;
 }
 
 // Exact distances from qv to the rows nn of the lanes with `want` (0 in the
 // others), rb rows at a time through `rows`.
+template <bool STAGED>
 __device__ __forceinline__ float rows_exact(const SearchArgs& a, const float* qv, float4* rows, uint32_t nn, bool want,
                                             int lane) {
-    if (!a.rb) return want ? dist_seq_rt(a.metric, qv, a.x + (size_t)nn * a.dp, a.dp) : 0.f;
+    if (!STAGED || !a.rb) return want ? dist_seq_rt(a.metric, qv, a.x + (size_t)nn * a.dp, a.dp) : 0.f;
     const uint32_t dq = a.dp >> 2, units = row_units(a.dp), base = smem_u32(rows);
     unsigned todo = __ballot_sync(FULL, want);
     float dd = 0.f;
@@ -294,11 +300,12 @@ __device__ __forceinline__ float rows_exact(const SearchArgs& a, const float* qv
     return dd;
 }
 
+template <bool SERIAL>
 __global__ void __launch_bounds__(SWARPS * 32) k_search(SearchArgs a) {
     extern __shared__ __align__(16) unsigned char smem[];
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const uint32_t slot = blockIdx.x * SWARPS + w;
-    unsigned char* base = smem + (size_t)w * search_warp_bytes(a.dp, a.beam_cap, a.rb);
+    unsigned char* base = smem + (size_t)w * search_warp_bytes(SERIAL, a.dp, a.beam_cap, a.rb);
     float* qv = reinterpret_cast<float*>(base);
     float4* rows = reinterpret_cast<float4*>(base + (size_t)a.dp * 4);
     HP* top = reinterpret_cast<HP*>(rows + (size_t)a.rb * row_units(a.dp));
@@ -306,7 +313,10 @@ __global__ void __launch_bounds__(SWARPS * 32) k_search(SearchArgs a) {
     uint32_t* stage_i = reinterpret_cast<uint32_t*>(stage_d + 32);
     uint32_t* vis = a.visited + (size_t)slot * a.words;
     uint32_t* vl = a.vlist + (size_t)slot * VCAP;
-    const CandHeap cand{reinterpret_cast<HP*>(stage_i + 32), a.cand + (size_t)slot * CCAP};
+    using Cand = std::conditional_t<SERIAL, HP*, CandHeap>;
+    Cand cand;
+    if constexpr (SERIAL) cand = a.cand + (size_t)slot * CCAP;
+    else cand = CandHeap{reinterpret_cast<HP*>(stage_i + 32), a.cand + (size_t)slot * CCAP};
     unsigned long long cmps = 0, nexp = 0;
     for (;;) {
         unsigned qi = 0;
@@ -365,7 +375,7 @@ __global__ void __launch_bounds__(SWARPS * 32) k_search(SearchArgs a) {
                 const uint64_t b = off[cur], e = off[cur + 1];  // the list of the node at loop entry
                 for (uint64_t c0 = b; c0 < e; c0 += 32) {
                     const uint32_t nn = c0 + lane < e ? a.adj_all[c0 + lane] : 0u;
-                    const float dd = rows_exact(a, qv, rows, nn, c0 + lane < e, lane);
+                    const float dd = rows_exact<!SERIAL>(a, qv, rows, nn, c0 + lane < e, lane);
                     const uint32_t cnt = (uint32_t)(e - c0 < 32 ? e - c0 : 32);
                     cmps += cnt;
                     for (uint32_t j = 0; j < cnt; j++) {
@@ -393,7 +403,7 @@ __global__ void __launch_bounds__(SWARPS * 32) k_search(SearchArgs a) {
             for (uint32_t c0 = 0; c0 < topk; c0 += 32) {
                 const uint32_t cnt = min(32u, topk - c0);
                 const uint32_t id = lane < cnt ? sd[c0 + lane] : 0u;
-                const float dd = rows_exact(a, qv, rows, id, lane < cnt, lane);
+                const float dd = rows_exact<!SERIAL>(a, qv, rows, id, lane < cnt, lane);
                 if (lane < cnt) {
                     stage_i[lane] = id;
                     stage_d[lane] = dd;
@@ -401,13 +411,27 @@ __global__ void __launch_bounds__(SWARPS * 32) k_search(SearchArgs a) {
                     if (nvis + lane < VCAP) vl[nvis + lane] = id;
                 }
                 __syncwarp();
-                for (uint32_t r = 0; r < cnt; r++) {
-                    if (ncand >= CCAP) {
-                        if (lane == 0) atomicOr(a.overflow, SERR_HEAP);
-                        break;
+                if constexpr (SERIAL) {
+                    if (lane == 0)
+                        for (uint32_t r = 0; r < cnt; r++) {
+                            if (ncand >= CCAP) {
+                                atomicOr(a.overflow, SERR_HEAP);
+                                break;
+                            }
+                            heap_push(cand, ncand, HP{-stage_d[r], stage_i[r]});
+                            heap_push(top, ntop, HP{stage_d[r], stage_i[r]});
+                        }
+                    ncand = __shfl_sync(FULL, ncand, 0);
+                    ntop = __shfl_sync(FULL, ntop, 0);
+                } else {
+                    for (uint32_t r = 0; r < cnt; r++) {
+                        if (ncand >= CCAP) {
+                            if (lane == 0) atomicOr(a.overflow, SERR_HEAP);
+                            break;
+                        }
+                        warp_push(cand, ncand, HP{-stage_d[r], stage_i[r]}, lane);
+                        warp_push(top, ntop, HP{stage_d[r], stage_i[r]}, lane);
                     }
-                    warp_push(cand, ncand, HP{-stage_d[r], stage_i[r]}, lane);
-                    warp_push(top, ntop, HP{stage_d[r], stage_i[r]}, lane);
                 }
                 __syncwarp();
                 nvis += cnt;
@@ -417,9 +441,10 @@ __global__ void __launch_bounds__(SWARPS * 32) k_search(SearchArgs a) {
         } else {
             start_ok = cur < a.nrows[a.L - 1];  // false only after a failed greedy check
             if (start_ok) {
-                warp_push(cand, ncand, HP{-cur_d, cur}, lane);
-                warp_push(top, ntop, HP{cur_d, cur}, lane);
+                ncand = ntop = 1;
                 if (lane == 0) {
+                    cand[0] = HP{-cur_d, cur};
+                    top[0] = HP{cur_d, cur};
                     atomicOr(&vis[cur >> 5], 1u << (cur & 31));
                     vl[0] = cur;
                 }
@@ -427,14 +452,15 @@ __global__ void __launch_bounds__(SWARPS * 32) k_search(SearchArgs a) {
         }
         __syncwarp();
         if (!start_ok) nvis = 0;
-        float lwbnd = start_ok ? top[0].f : 0.f;
+        float lwbnd = start_ok ? __shfl_sync(FULL, top[0].f, 0) : 0.f;
         const uint32_t nlast = a.nrows[a.L - 1];
         uint32_t expansions = 0;
         while (ncand > 0) {
             // Every heap update ends with a warp barrier; a value read from a
             // heap is broadcast, so that lanes cannot disagree on it whatever
             // the compiler does with the read.
-            HP c = cand.s[0];
+            HP c{0.f, 0u};
+            if (lane == 0) c = cand[0];
             c.f = __shfl_sync(FULL, c.f, 0);
             c.id = __shfl_sync(FULL, c.id, 0);
             __syncwarp();
@@ -443,7 +469,12 @@ __global__ void __launch_bounds__(SWARPS * 32) k_search(SearchArgs a) {
                 if (lane == 0) atomicOr(a.overflow, c.id >= nlast ? SERR_BAD_ID : SERR_BEAM_CAP);
                 break;
             }
-            warp_pop(cand, ncand, lane);
+            if constexpr (SERIAL) {
+                if (lane == 0) heap_pop(cand, ncand);
+                ncand = __shfl_sync(FULL, ncand, 0);
+            } else {
+                warp_pop(cand, ncand, lane);
+            }
             nexp++;
             const uint64_t b = off[c.id], e = off[c.id + 1];
             for (uint64_t c0 = b; c0 < e; c0 += 32) {
@@ -459,7 +490,7 @@ __global__ void __launch_bounds__(SWARPS * 32) k_search(SearchArgs a) {
                     }
                 }
                 const unsigned fb = __ballot_sync(FULL, fresh);
-                const float dd = rows_exact(a, qv, rows, nn, fresh, lane);
+                const float dd = rows_exact<!SERIAL>(a, qv, rows, nn, fresh, lane);
                 if (fresh) {
                     const uint32_t r = __popc(fb & ((1u << lane) - 1u));
                     if (nvis + r < VCAP) vl[nvis + r] = nn;
@@ -471,19 +502,38 @@ __global__ void __launch_bounds__(SWARPS * 32) k_search(SearchArgs a) {
                 if (nvis > VCAP) vis_overflow = true;
                 cmps += nf;
                 __syncwarp();
-                for (uint32_t r = 0; r < nf; r++) {  // offers in list order (lysearch.cpp:284-295)
-                    const float dj = __shfl_sync(FULL, stage_d[r], 0);
-                    const uint32_t ij = __shfl_sync(FULL, stage_i[r], 0);
-                    const float worst = __shfl_sync(FULL, top[0].f, 0);
-                    __syncwarp();
-                    if (worst > dj || ntop < topk) {
-                        if (ncand >= CCAP) {
-                            if (lane == 0) atomicOr(a.overflow, SERR_HEAP);
-                            continue;
+                // offers in list order (lysearch.cpp:284-295)
+                if constexpr (SERIAL) {
+                    if (lane == 0)
+                        for (uint32_t r = 0; r < nf; r++) {
+                            const float dj = stage_d[r];
+                            if (top[0].f > dj || ntop < topk) {
+                                if (ncand >= CCAP) {
+                                    atomicOr(a.overflow, SERR_HEAP);
+                                    continue;
+                                }
+                                heap_push(cand, ncand, HP{-dj, stage_i[r]});
+                                heap_push(top, ntop, HP{dj, stage_i[r]});
+                                if (ntop > topk) heap_pop(top, ntop);
+                            }
                         }
-                        warp_push(cand, ncand, HP{-dj, ij}, lane);
-                        warp_push(top, ntop, HP{dj, ij}, lane);
-                        if (ntop > topk) warp_pop(top, ntop, lane);
+                    ncand = __shfl_sync(FULL, ncand, 0);
+                    ntop = __shfl_sync(FULL, ntop, 0);
+                } else {
+                    for (uint32_t r = 0; r < nf; r++) {
+                        const float dj = __shfl_sync(FULL, stage_d[r], 0);
+                        const uint32_t ij = __shfl_sync(FULL, stage_i[r], 0);
+                        const float worst = __shfl_sync(FULL, top[0].f, 0);
+                        __syncwarp();
+                        if (worst > dj || ntop < topk) {
+                            if (ncand >= CCAP) {
+                                if (lane == 0) atomicOr(a.overflow, SERR_HEAP);
+                                continue;
+                            }
+                            warp_push(cand, ncand, HP{-dj, ij}, lane);
+                            warp_push(top, ntop, HP{dj, ij}, lane);
+                            if (ntop > topk) warp_pop(top, ntop, lane);
+                        }
                     }
                 }
                 __syncwarp();
@@ -498,14 +548,27 @@ __global__ void __launch_bounds__(SWARPS * 32) k_search(SearchArgs a) {
             if (a.out_d) a.out_d[o + t] = 0.f;
         }
         __syncwarp();
-        while (ntop > 0) {
-            const uint32_t loc = ntop - 1;
-            if (loc < a.out_k && lane == 0) {
-                a.out_ids[o + loc] = top[0].id;
-                if (a.out_d) a.out_d[o + loc] = top[0].f;
-            }
+        if constexpr (SERIAL) {
+            if (lane == 0)
+                while (ntop > 0) {
+                    const uint32_t loc = ntop - 1;
+                    if (loc < a.out_k) {
+                        a.out_ids[o + loc] = top[0].id;
+                        if (a.out_d) a.out_d[o + loc] = top[0].f;
+                    }
+                    heap_pop(top, ntop);
+                }
             __syncwarp();
-            warp_pop(top, ntop, lane);
+        } else {
+            while (ntop > 0) {
+                const uint32_t loc = ntop - 1;
+                if (loc < a.out_k && lane == 0) {
+                    a.out_ids[o + loc] = top[0].id;
+                    if (a.out_d) a.out_d[o + loc] = top[0].f;
+                }
+                __syncwarp();
+                warp_pop(top, ntop, lane);
+            }
         }
         // clear the visited bits of this query
         if (!vis_overflow) {
@@ -607,6 +670,21 @@ int index_upload(Ctx& ctx, IndexDev& ix, const float* x, uint64_t n, uint32_t d,
     return 0;
 }
 
+// Which form of k_search a batch takes.  The warp's heap steps save time while
+// the heaps stay within COOP entries; past that they are lane 0's either way,
+// and what the form costs besides (barriers, broadcasts, a heap in two parts)
+// shows the more the shorter a row is.  Flat seeds fill both heaps at once, so
+// its line lies lower.  Whole warp against lane 0, geometric means over 1, 17,
+// 300 and 2,000 queries, us: descent, d = 64: beam 100 756 / 759, 128 911 / 877,
+// 300 1,791 / 1,654; d = 24: beam 64 581 / 588, 100 896 / 852; d = 96: beam 128
+// 910 / 928, 200 1,377 / 1,306; d = 128: beam 64 542 / 636, 300 2,405 / 2,410,
+// 900 6,331 / 6,737; d = 512: beam 900 8,989 / 8,909.  Flat, d = 64: beam 64
+// 588 / 600, 100 970 / 878, 300 2,002 / 1,603; d = 128: beam 100 1,160 / 1,200,
+// 200 1,949 / 1,796; d = 512: beam 200 2,084 / 2,188, 300 3,512 / 3,074.
+static bool serial_heaps(uint32_t dp, uint32_t beam, bool flat) {
+    return flat ? beam > std::min(48 + dp / 2, COOP) : dp < 128 && beam > 48 + dp;
+}
+
 int index_run_exact(Ctx& ctx, IndexDev& ix, const SearchReq& r) {
     cudaStream_t st = ctx.stream;
     const uint32_t dp = ix.dp;
@@ -614,18 +692,20 @@ int index_run_exact(Ctx& ctx, IndexDev& ix, const SearchReq& r) {
     cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, ctx.device);
     // rows staged at a time: 16 while four blocks fit on an SM, fewer for long
     // rows and wide beams, none where two rows no longer fit beside the heaps
-    auto bytes_of = [&](uint32_t rb) { return (size_t)SWARPS * search_warp_bytes(dp, r.beam_max, rb) + 64; };
-    uint32_t rb = 16;
+    const bool serial = serial_heaps(dp, r.beam_max, r.flat != 0);
+    auto bytes_of = [&](uint32_t rb) { return (size_t)SWARPS * search_warp_bytes(serial, dp, r.beam_max, rb) + 64; };
+    uint32_t rb = serial ? 0 : 16;
     while (rb > 2 && bytes_of(rb) > 56 * 1024) rb /= 2;
     if (bytes_of(rb) > 112 * 1024) rb = 0;
     const size_t smem = bytes_of(rb);
-    if (smem > 200 * 1024 + (size_t)SWARPS * CAND_SMEM * 8) {
+    if (smem > 200 * 1024 + (serial ? 0 : (size_t)SWARPS * CAND_SMEM * 8)) {
         ctx.last_error = "beam too wide for shared memory at this dimension";
         return 1;
     }
-    NNM_CUDA_TRY(cudaFuncSetAttribute(k_search, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    const auto kern = serial ? k_search<true> : k_search<false>;
+    NNM_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     int per_sm = 1;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_search, SWARPS * 32, smem);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, SWARPS * 32, smem);
     const uint32_t full = (uint32_t)std::min(std::max(1, per_sm), 4) * (uint32_t)nsm;
     const uint32_t blocks = std::min(full, (r.nq + SWARPS - 1) / SWARPS);
     const uint32_t words = (uint32_t)((ix.n + 31) / 32);
@@ -673,7 +753,7 @@ int index_run_exact(Ctx& ctx, IndexDev& ix, const SearchReq& r) {
     a.overflow = reinterpret_cast<unsigned*>(c + 4);
     a.ncmps = reinterpret_cast<unsigned long long*>(c + 8);
     a.nexp = reinterpret_cast<unsigned long long*>(c + 16);
-    k_search<<<blocks, SWARPS * 32, smem, st>>>(a); count_launch();
+    kern<<<blocks, SWARPS * 32, smem, st>>>(a); count_launch();
     NNM_CUDA_TRY(cudaGetLastError());
     return 0;
 }
