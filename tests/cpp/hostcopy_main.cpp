@@ -14,7 +14,7 @@
 
 // what the headers' device code names (none of it is called here)
 float __fadd_rn(float, float), __fsub_rn(float, float), __fmul_rn(float, float), __fdiv_rn(float, float);
-unsigned __umulhi(unsigned, unsigned);
+unsigned __umulhi(unsigned, unsigned), min(unsigned, unsigned);
 int __popc(unsigned), __clz(int);
 
 #include "../../nn-merge_b200/csrc/hostcopy.cu"
