@@ -993,12 +993,16 @@ int index_search_impl(nnm_index* h, const float* q, uint64_t nq, const uint32_t*
     // for, were 70 us of a 280-us call of one query
     const size_t in_bytes = (size_t)nq * dp * 4 + (beams ? (size_t)nq * 4 : 0), out_bytes = (size_t)nq * out_k * 8;
     const bool fits = !dev && in_bytes + out_bytes + 128 <= nnm::INDEX_IO_BYTES;
-    const bool small = fits && (ix.h_io.p || ix.h_io.make(nnm::INDEX_IO_BYTES));  // without pinned memory: as a large batch
+    if (fits && !ix.h_io && cudaMallocHost(reinterpret_cast<void**>(&ix.h_io), nnm::INDEX_IO_BYTES) != cudaSuccess) {
+        cudaGetLastError();
+        ix.h_io = nullptr;
+    }
+    const bool small = fits && ix.h_io;  // without pinned memory: as a large batch
     // queries with rows of dp floats
     const float* qd = q;
     if (small) {
         if ((rc = cu(ix.qpad.ensure(in_bytes)))) return rc;
-        float* hq = reinterpret_cast<float*>(ix.h_io.p);
+        float* hq = reinterpret_cast<float*>(ix.h_io);
         if (dp == d) std::memcpy(hq, q, (size_t)nq * d * 4);
         else
             for (uint64_t i = 0; i < nq; i++) {
@@ -1067,7 +1071,7 @@ int index_search_impl(nnm_index* h, const float* q, uint64_t nq, const uint32_t*
     cudaEventRecord(ev[2], st);
     uint64_t ncmps = 0, nexp = 0;
     if (small) {
-        unsigned char* hc = ix.h_io.p + ((in_bytes + 63) & ~(size_t)63);  // counters, then the results
+        unsigned char* hc = ix.h_io + ((in_bytes + 63) & ~(size_t)63);  // counters, then the results
         if (!rc) rc = cu(cudaMemcpyAsync(hc, ix.ctr.p, 24, cudaMemcpyDeviceToHost, st));
         if (!rc) rc = cu(cudaMemcpyAsync(hc + 32, oi, out_d ? out_bytes : out_bytes / 2, cudaMemcpyDeviceToHost, st));
         if (!rc) rc = cu(cudaStreamSynchronize(st));

@@ -54,7 +54,9 @@ struct IndexDev {
     uint32_t width = 4;  // fast kernel: most unexpanded entries expanded together
     // small batches from host memory: queries, beams, counters and results
     // pass through this pinned block, so that a call waits for the device once
-    PinnedBlock h_io;
+    // (cudaMallocHost: a part of what the context's counters lie in, where
+    // registering pages cost the index's first search 110 to 300 us)
+    unsigned char* h_io = nullptr;
     cudaEvent_t ev[3] = {};
     void release();
 };

@@ -823,7 +823,8 @@ void IndexDev::release() {
     DevBuf* all[] = {&x,     &off,   &adj,  &visited, &vlist,  &cand,         &ctr,      &qpad,
                      &beams, &probes, &hid, &scores,  &out,    &flat_off, &flat_pool};
     for (auto* b : all) b->release();
-    h_io.release();
+    if (h_io) cudaFreeHost(h_io);
+    h_io = nullptr;
     for (auto& e : ev) {
         if (e) cudaEventDestroy(e);
         e = nullptr;
